@@ -11,15 +11,16 @@
 //                           u = beta (v - g a),   o = g c + kq u,   S <- g S + k u^T
 //                       (the same sums as the four steps above, regrouped so that a token needs one reduction over row groups).
 //                       The CTAs of a sequence also advance its convolution state, a share of the channels each.
-//   delta_chunk_kernel  the same recurrence 32 tokens at a time for prompt portions (see there).
+//   delta_mma_kernel    the same recurrence 32 tokens at a time on the tensor pipe for prompt portions: a decay per head, up to 128 channels
+//   delta_chunk_kernel  the same 16 tokens at a time on the FMA pipe, for the other prompt portions (decays per channel, up to 256 channels)
 // With a decay per head and key CHANNEL (g a vector, S <- diag(g) S) the token kernel scales every row of S first and then follows the
 // four steps, and the chunk kernel works with the running sums L_t of each channel: the token-by-token products take
 // exp(L_t - L_j) inside their sums, the keys and queries that meet the state carry exp(L_t), those that enter it exp(L_n - L_j).
 // Both states live in fp32 in pools of state slots; a sequence whose first new token sits at position 0 starts from zeros.
-// Everything here is plain fp32 FMA code.
+// All arithmetic is fp32: FMA code, or products of three bf16 parts per number (scan_mma.cuh).
 #include <type_traits>
 
-#include "scan_common.cuh"
+#include "scan_mma.cuh"
 
 namespace {
 
@@ -165,13 +166,12 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
 // The convolution state of a sequence after a portion: the last taps - 1 inputs of (what it held, this portion).  Slot i reads slot
 // i + len or the portion, never a slot below itself, so one thread per channel shifts in place.  The channels are spread over the
 // CTAs (head, value slice) of the sequence; nothing else in a scan kernel reads this state.
-__device__ __forceinline__ void advance_conv_state(const nvc_delta_prep& p, int r0, int r1, bool fresh, int slot) {
+__device__ __forceinline__ void advance_conv_state(const nvc_delta_prep& p, int r0, int r1, bool fresh, int slot, int part, int parts, int thread, int threads) {
   const int C = 2 * p.kv_heads * p.dim + p.heads * p.vdim, len = r1 - r0, keep = p.taps - 1;
   if (keep == 0) return;
   float* cs = p.conv_state + (int64_t)slot * keep * C;
-  const int part = blockIdx.y * gridDim.z + blockIdx.z, parts = gridDim.y * gridDim.z;
   const int qk = p.kv_heads * p.dim;
-  for (int c = part * blockDim.x + threadIdx.x; c < C; c += parts * blockDim.x) {
+  for (int c = part * threads + thread; c < C; c += parts * threads) {
     const int col = c < qk ? p.q_off + c : (c < 2 * qk ? p.k_off + c - qk : p.v_off + c - 2 * qk);
     for (int i = 0; i < keep; ++i) {
       const int src = len - keep + i;                 // portion index
@@ -203,7 +203,7 @@ __global__ void delta_scan_kernel(const DeltaArgs a) {
   const int r1 = p.cu_seqlens ? p.cu_seqlens[b + 1] : b + 1;
   const bool fresh = p.positions[r0] == 0;
   const int slot = p.state_slots[b];
-  advance_conv_state(p, r0, r1, fresh, slot);
+  advance_conv_state(p, r0, r1, fresh, slot, blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z, threadIdx.x, blockDim.x);
   const int d0 = rg * DPT;
   float S[DPT];
   float* sp = a.state + (((int64_t)slot * p.heads + h) * p.dim) * p.vdim;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 3) delta_chunk_kernel(c
   const int r1 = p.cu_seqlens ? p.cu_seqlens[b + 1] : b + 1;
   const bool fresh = p.positions[r0] == 0;
   const int slot = p.state_slots[b];
-  advance_conv_state(p, r0, r1, fresh, slot);
+  advance_conv_state(p, r0, r1, fresh, slot, blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z, threadIdx.x, blockDim.x);
   float* sp = a.state + (((int64_t)slot * p.heads + h) * dim) * p.vdim;
   for (int i = threadIdx.x; i < dz * COLS; i += THREADS) {
     const int d = i / COLS, c = i % COLS;
@@ -575,6 +575,243 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 3) delta_chunk_kernel(c
   }
 }
 
+// ---- one decay per head and keys of up to 128 numbers: chunks of 32 tokens with every product on the tensor pipe (scan_mma.cuh says how the warps
+// share the work).  In the notation above and with (.)^T for a state warp's 16 value columns,
+//   B^T = beta (v^T - exp(L) S^T K^T);      U_0 = X_0 B_0,   U_1 = X_1 (B_1 - A_10 U_0)      for the chunk's two halves of 16 tokens,
+//   O^T = exp(L) S^T Q^T + U^T P^T;         S^T <- exp(L_n) S^T + (exp(L_n - L) U)^T K
+// where A (strictly lower, with beta and decays) and P are the token-by-token products and X_i the inverse of I + A_ii, found column by
+// column with forward substitution in fp32 by the preparing warp that computed the block.  B, U and O never leave a state warp's registers.
+constexpr int kHT = 16;                  // tokens of a half
+constexpr int kHP = kHT + 8;             // row stride of a half's planes
+__host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 5 * kMT * 4; }
+
+template <int KS>
+__global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, const int vecv) {
+  constexpr int DZ = 16 * KS, DP = DZ + 8;
+  constexpr float kLog2e = 1.4426950408889634f;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ int which;
+  __shared__ __align__(16) float nts[2][kHT * kDA];       // A of a half, transposed, for its inversion
+  pdl_trigger();
+  const nvc_delta_prep& p = a.p;
+  const int slices = (p.vdim + kMC - 1) / kMC, h = blockIdx.x / slices, v0 = (blockIdx.x % slices) * kMC;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
+  const int hk = h / (p.heads / p.kv_heads);
+  const int dim = p.dim, cols = min(kMC, p.vdim - v0);
+  pdl_wait();
+  const int b = sequence_of_rank(p.cu_seqlens, p.B, blockIdx.y, &which);
+  const int r0 = p.cu_seqlens[b], r1 = p.cu_seqlens[b + 1], chunks = (r1 - r0 + kMT - 1) / kMT;
+  if (chunks == 0) return;
+  const bool fresh = p.positions[r0] == 0;
+  const int slot = p.state_slots[b];
+  struct Buffer { Planes Q, K, P, X0, X1, A10; float *V, *beta, *Lh, *Ll, *from, *to; };
+  auto buffer = [&](int i) {
+    uint8_t* q = smem + (i & 1) * delta_buf(DZ);
+    uint8_t* x = q + 2 * kMT * DP * 6 + kMT * kMP * 6;
+    float* v = reinterpret_cast<float*>(x + 3 * kHT * kHP * 6);
+    float* l = v + kMT * kMV;               // beta; running sums in two parts; decay from the chunk's start to a token, from a token to its end
+    return Buffer{planes(q, kMT, DP), planes(q + kMT * DP * 6, kMT, DP), planes(q + 2 * kMT * DP * 6, kMT, kMP), planes(x, kHT, kHP),
+                  planes(x + kHT * kHP * 6, kHT, kHP), planes(x + 2 * kHT * kHP * 6, kHT, kHP), v, l, l + kMT, l + 2 * kMT, l + 3 * kMT, l + 4 * kMT};
+  };
+  if (w >= 4) {
+    // ------------------------------------------------ preparing warps
+    const int pw = w - 4;
+    RowTile<DZ> q, k;
+    RowTile<kMC> v;
+    float2 gb = make_float2(0.f, 0.f);        // (log2 decay, beta) of a token; none behind the end
+    auto fetch = [&](int i) {
+      const int64_t row = r0 + i * kMT;
+      const int n = r1 - (int)row;
+      q.load(p.q_out + row * p.ldq + hk * dim, p.ldq, dim, n, a.vec, pw, lane);
+      k.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, n, a.vec, pw, lane);
+      v.load(p.v_out + row * p.ldv + h * p.vdim + v0, p.ldv, cols, n, vecv, pw, lane);
+      if (pw == 3) {
+        const float* x = p.gb_out + ((row + lane) * p.heads + h) * 2;
+        gb = lane < n ? make_float2(x[0] * kLog2e, x[1]) : make_float2(0.f, 0.f);
+      }
+    };
+    fetch(0);
+    for (int i = 0; i < chunks; ++i) {
+      const Buffer bf = buffer(i);
+      if (i >= 2) bar_sync(kEmpty + (i & 1), 256);
+      q.split_to(bf.Q, pw, lane);
+      k.split_to(bf.K, pw, lane);
+      v.store_to(bf.V, kMV, pw, lane);
+      if (pw == 3) {
+        // running sums in 64 bits: over 32 tokens they reach 40 and more, and what is exponentiated are their differences
+        double l = (double)gb.x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double up = __shfl_up_sync(0xffffffffu, l, o);
+          if (lane >= o) l += up;
+        }
+        const float hi = (float)l;
+        bf.Lh[lane] = hi;
+        bf.Ll[lane] = (float)(l - (double)hi);
+        bf.from[lane] = ex2(hi);
+        bf.to[lane] = ex2((float)(__shfl_sync(0xffffffffu, l, 31) - l));
+        bf.beta[lane] = gb.y;
+      }
+      if (i + 1 < chunks) fetch(i + 1);
+      bar_sync(kPrepare, 128);
+      auto decay = [&](int t, int j) { return ex2((bf.Lh[t] - bf.Lh[j]) + (bf.Ll[t] - bf.Ll[j])); };
+      // warps 0 and 1: the diagonal blocks of A and their inverses; 2: P (16, 0) and A_10; 3: P (0, 0) and P (16, 16)
+      float x[2][4];
+      if (pw < 2) {
+        const int t0 = kHT * pw;
+        token_products<KS>(x, bf.K, t0, bf.K, t0, lane);
+        float* nt = nts[pw];
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = g + 4 * (e & 2), j = 8 * y + 2 * tq + (e & 1);
+            nt[j * kDA + t] = j < t ? bf.beta[t0 + t] * (decay(t0 + t, t0 + j) * x[y][e]) : 0.f;
+          }
+        __syncwarp();
+        const int col = lane & 15;            // a column of the inverse per lane (both halves of the warp do the same)
+        float z[kHT];
+#pragma unroll
+        for (int t = 0; t < kHT; ++t) z[t] = t == col ? 1.f : 0.f;
+#pragma unroll
+        for (int j = 0; j + 1 < kHT; ++j)
+#pragma unroll
+          for (int t4 = (j + 1) / 4 * 4; t4 < kHT; t4 += 4) {
+            const float4 m = *reinterpret_cast<const float4*>(nt + j * kDA + t4);
+            if (t4 > j) z[t4] = fmaf(-m.x, z[j], z[t4]);
+            if (t4 + 1 > j) z[t4 + 1] = fmaf(-m.y, z[j], z[t4 + 1]);
+            if (t4 + 2 > j) z[t4 + 2] = fmaf(-m.z, z[j], z[t4 + 2]);
+            z[t4 + 3] = fmaf(-m.w, z[j], z[t4 + 3]);
+          }
+        const Planes X = pw ? bf.X1 : bf.X0;
+#pragma unroll
+        for (int t = 0; t < kHT / 2; ++t) {                 // rows 0 .. 7 by the left lanes, 8 .. 15 by the right ones
+          const float mine = lane < kHT ? z[t] : z[t + kHT / 2], right = __shfl_down_sync(0xffffffffu, mine, 1);
+          if (!(lane & 1)) store_pair(X, t + (lane & kHT) / 2, col, mine, right);
+        }
+      } else {
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          const bool isa = pw == 2 && half;
+          const int t0 = pw == 2 ? kHT : kHT * half, j0 = pw == 2 ? 0 : kHT * half;
+          token_products<KS>(x, isa ? bf.K : bf.Q, t0, bf.K, j0, lane);
+          const Planes M = isa ? bf.A10 : bf.P;
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const int t = t0 + g + 4 * e, j = j0 + 8 * y + 2 * tq;
+              const float f = isa ? bf.beta[t] : 1.f;
+              store_pair(M, isa ? t - kHT : t, j, j <= t ? f * (decay(t, j) * x[y][e]) : 0.f,
+                         j + 1 <= t ? f * (decay(t, j + 1) * x[y][e + 1]) : 0.f);
+            }
+        }
+      }
+      if (i == 0) advance_conv_state(p, r0, r1, fresh, slot, blockIdx.x, gridDim.x, threadIdx.x - 128, 128);      // nothing here reads that state
+      bar_arrive(kFull + (i & 1), 256);
+    }
+    return;
+  }
+  // -------------------------------------------------- state warps
+  const int c = w * 16 + g;
+  float* sp = a.state + (((int64_t)slot * p.heads + h) * dim) * p.vdim + v0;
+  float S[2 * KS][4];
+  load_state<KS>(S, sp, p.vdim, dim, c, cols, fresh, lane);
+  using Two = float(*)[2][4];
+  for (int i = 0; i < chunks; ++i) {
+    const Buffer bf = buffer(i);
+    const int64_t row = r0 + i * kMT;
+    const int n = min(kMT, r1 - (int)row);
+    bar_sync(kFull + (i & 1), 256);
+    float u[4][4], o[4][4];                   // right sides, then U; outputs
+    {
+      float kr[4][4] = {}, qr[4][4] = {}, kx[4][4] = {}, qx[4][4] = {};
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[t][e] = o[t][e] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        FragA s;
+        FragB x[4];
+        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1]);
+        load_b(x, bf.K, 0, 16 * ks, lane);
+        if (ks < KS / 2) mma_high(kx, s, x);
+        else mma_high(u, s, x);
+        mma_small(kr, s, x);
+        load_b(x, bf.Q, 0, 16 * ks, lane);
+        if (ks < KS / 2) mma_high(qx, s, x);
+        else mma_high(o, s, x);
+        mma_small(qr, s, x);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int tt = 8 * t + 2 * tq + (e & 1);
+          const float f = bf.from[tt];
+          u[t][e] = bf.beta[tt] * (bf.V[tt * kMV + c + 4 * (e & 2)] - f * ((u[t][e] + kx[t][e]) + kr[t][e]));
+          o[t][e] = f * ((o[t][e] + qx[t][e]) + qr[t][e]);
+        }
+    }
+    FragA f;
+    auto solve = [&](float (&x)[2][4], const Planes& X) {     // x <- x X^T;  f: its parts
+      frag_of_tiles(f, x[0], x[1]);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[t][e] = 0.f;
+      add_tokens(x, f, X, 0, 0, lane);
+      frag_of_tiles(f, x[0], x[1]);
+    };
+    solve(*reinterpret_cast<Two>(u), bf.X0);
+    {
+      float m[2][4] = {};
+      add_tokens(m, f, bf.A10, 0, 0, lane);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[2 + t][e] -= m[t][e];
+    }
+    add_tokens(o, f, bf.P, 0, 0, lane);
+    solve(*reinterpret_cast<Two>(u + 2), bf.X1);
+    add_tokens(*reinterpret_cast<Two>(o + 2), f, bf.P, 16, 16, lane);
+    // ---- the state behind the chunk
+    FragA us[2];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) u[t][e] *= bf.to[8 * t + 2 * tq + (e & 1)];
+    frag_of_tiles(us[0], u[0], u[1]);
+    frag_of_tiles(us[1], u[2], u[3]);
+    state_update<KS>(S, bf.from[kMT - 1], us, bf.K, lane);
+    if (i + 2 < chunks) bar_arrive(kEmpty + (i & 1), 256);
+    float* op = a.o + row * a.ldo + h * p.vdim + v0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int tt = 8 * t + 2 * tq + (e & 1), cc = c + 4 * (e & 2);
+        if (tt < n && cc < cols) op[(int64_t)tt * a.ldo + cc] = o[t][e];
+      }
+  }
+  store_state<KS>(S, sp, p.vdim, dim, c, cols, lane);
+}
+
+template <int KS>
+cudaError_t launch_delta_mma(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) {
+  const nvc_delta_prep& p = a.p;
+  constexpr int smem = 2 * delta_buf(16 * KS);
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(delta_mma_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  const int vecv = (p.vdim & 3) == 0 && (p.ldv & 3) == 0 && (reinterpret_cast<uintptr_t>(p.v_out) & 15) == 0;
+  return nvc_launch(ctx, delta_mma_kernel<KS>, dim3(p.heads * ((p.vdim + kMC - 1) / kMC), p.B), dim3(256), smem, st, a, vecv);
+}
+
 template <int C, int NW, bool CH>
 cudaError_t launch_delta_chunk(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) {
   constexpr int COLS = 32 * C * (NW / 4);
@@ -636,10 +873,12 @@ extern "C" int nvc_delta_rule_scan(nvc_ctx* ctx, const nvc_delta_prep* p, float*
   DeltaArgs a{*p, 0, 0, o, ldo, state};
   const int dim = p->dim;
   if (p->cu_seqlens && max_qlen >= 8 && dim <= 256) {
-    // prompt portions: 16 tokens at a time (keys of more than 256 numbers stay token by token)
+    // prompt portions (keys of more than 256 numbers stay token by token).  The tensor pipe keeps 16 columns x all channels of the state in
+    // a warp's registers, which is what ends it at 128 channels; decays per channel are no factors of a product of rows
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     a.vec = dim % 4 == 0 && p->ldq % 4 == 0 && p->ldk % 4 == 0 && al16(p->q_out) && al16(p->k_out) && al16(p->channel_g);
-    const cudaError_t ce = p->channel_a ? launch_delta_chunk_sized<true>(ctx, a, nvc_stream(stream)) : launch_delta_chunk_sized<false>(ctx, a, nvc_stream(stream));
+    const cudaError_t ce = !p->channel_a && dim <= 128 ? (dim <= 64 ? launch_delta_mma<4>(ctx, a, nvc_stream(stream)) : launch_delta_mma<8>(ctx, a, nvc_stream(stream)))
+                           : p->channel_a ? launch_delta_chunk_sized<true>(ctx, a, nvc_stream(stream)) : launch_delta_chunk_sized<false>(ctx, a, nvc_stream(stream));
     NVC_CUDA_CHECK(ctx, ce);
     ctx->launches++;
     return NVC_OK;

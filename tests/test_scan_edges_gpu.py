@@ -1,0 +1,91 @@
+"""The chunked recurrences on the tensor pipe at their edges - chunk and half-chunk lengths, channel and column counts around the tiles, more
+sequences than are ordered by length - against the recurrences written out in 64 bits.  Bound: an fp32 number keeps 24 bits through the three
+bf16 parts, so what is left is the rounding of fp32 sums of up to 128 + 32 terms per chunk, carried by a state whose decays sum to below 20
+tokens: 2e-6 of the largest value is four times the 5e-7 of that."""
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+F64 = torch.float64
+LENS = {"edges": [1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97], "one": [70], "many": [5 + i % 3 for i in range(300)]}
+
+
+@pytest.fixture(scope="module")
+def ops():
+    return importlib.import_module("nano-vllm-candle_b200.ops")
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def rows(lens, g, *shape):
+    return torch.randn(sum(lens), *shape, generator=g).to(DEV)
+
+
+def close(got, want):
+    return float((got.to(F64) - want).abs().max()) <= 2e-6 * max(1.0, float(want.abs().max()))
+
+
+def shapes(vdims):
+    return [(d, vd, "edges") for d in (1, 20, 64, 65, 127, 128) for vd in vdims[:1]] + [(128, vd, "edges") for vd in vdims[1:]] + [(32, 16, "many"), (128, 64, "one")]
+
+
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("dim,vdim,which", shapes([33, 1, 63, 64, 65, 130]))
+def test_decayed_scan_edges(ctx, ops, dim, vdim, which, fixed):
+    lens, H, G = LENS[which], 2, 1
+    g = torch.Generator().manual_seed(dim * 131 + vdim)
+    B = len(lens)
+    q, k, v, skip = rows(lens, g, G, dim) * dim ** -0.5, rows(lens, g, G, dim) * dim ** -0.5, rows(lens, g, H, vdim), rows(lens, g, H, vdim)
+    ld = -rows(lens, g, H).abs()
+    decay, sw = torch.tensor([0.0, 0.95], device=DEV), torch.tensor([0.5, -1.0], device=DEV)
+    slots = torch.randperm(B, generator=g).to(torch.int32).to(DEV)
+    state = torch.randn(B, H, dim, vdim, generator=g).to(DEV)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    first = [b % 2 * 3 for b in range(B)]                    # every other sequence goes on from its state
+    S0, pos = state.to(F64), i32([first[b] + t for b, n in enumerate(lens) for t in range(n)])
+    o = ops.decay_scan(ctx, q.view(-1, G * dim), k.view(-1, G * dim), v.view(-1, H * vdim), state, slots, i32(cu.tolist()), pos, H, G, dim, vdim,
+                       decay=decay if fixed else None, log_decay=None if fixed else ld, skip=None if fixed else skip.view(-1, H * vdim),
+                       skip_w=None if fixed else sw, max_qlen=max(lens))
+    keep = decay.to(F64).expand(sum(lens), H) if fixed else ld.to(F64).exp()
+    for b, n in enumerate(lens):
+        S = S0[slots[b]] * (first[b] > 0)
+        for t in range(int(cu[b]), int(cu[b + 1])):
+            S = S * keep[t][:, None, None] + k[t].to(F64).expand(H, dim)[:, :, None] * v[t].to(F64)[:, None]
+            want = torch.einsum("hdv,hd->hv", S, q[t].to(F64).expand(H, dim))
+            if not fixed:
+                want = want + sw.to(F64)[:, None] * skip[t].to(F64)
+            if n > 90 or t in (int(cu[b]), int(cu[b + 1]) - 1):
+                assert close(o[t].view(H, vdim), want), (b, t)
+        assert close(state[slots[b]], S), b
+
+
+@pytest.mark.parametrize("dim,vdim,which", shapes([33, 1, 63, 64, 65, 130]))
+def test_delta_rule_edges(ctx, ops, dim, vdim, which):
+    lens, H, G, taps = LENS[which], 2, 1, 2
+    g = torch.Generator().manual_seed(dim * 137 + vdim)
+    B, C = len(lens), 2 * G * dim + H * vdim
+    x = rows(lens, g, C + 2 * H)
+    slots = torch.randperm(B, generator=g).to(torch.int32).to(DEV)
+    state, cs = torch.randn(B, H, dim, vdim, generator=g).to(DEV) * 0.5, torch.randn(B, taps - 1, C, generator=g).to(DEV)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    first = [b % 2 * 3 for b in range(B)]
+    S0, pos = state.to(F64), i32([first[b] + t for b, n in enumerate(lens) for t in range(n)])
+    o, q, k, v, gb = ops.delta_rule(ctx, x, (0, G * dim, 2 * G * dim, C, C + H), H, G, dim, vdim, taps, torch.randn(taps, C, generator=g).to(DEV), cs, state, slots,
+                                    i32(cu.tolist()), pos, torch.zeros(H, device=DEV), torch.full((H,), -1.0, device=DEV), max_qlen=max(max(lens), 8))
+    q, k, v = q.to(F64).view(-1, G, dim).expand(-1, H, dim), k.to(F64).view(-1, G, dim).expand(-1, H, dim), v.to(F64).view(-1, H, vdim)
+    gb = gb.to(F64).view(-1, H, 2)
+    for b, n in enumerate(lens):
+        S = S0[slots[b]] * (first[b] > 0)
+        for t in range(int(cu[b]), int(cu[b + 1])):
+            S = S * gb[t, :, 0].exp()[:, None, None]
+            u = gb[t, :, 1][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None]
+            if n > 90 or t in (int(cu[b]), int(cu[b + 1]) - 1):
+                assert close(o[t].view(H, vdim), torch.einsum("hdv,hd->hv", S, q[t])), (b, t)
+        assert close(state[slots[b]], S), b
+        assert torch.equal(cs[slots[b]][0], x[int(cu[b + 1]) - 1, :C]), b
