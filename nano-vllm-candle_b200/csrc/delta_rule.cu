@@ -585,6 +585,19 @@ constexpr int kHT = 16;                  // tokens of a half
 constexpr int kHP = kHT + 8;             // row stride of a half's planes
 __host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 5 * kMT * 4; }
 
+// decays between the tokens of a thread's numbers in a 16 x 16 block, from running sums in two parts
+struct Decays {
+  float th[2], tl[2], jh[4], jl[4];
+  __device__ __forceinline__ void load(const float* Lh, const float* Ll, int t0, int j0, int lane) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { th[i] = Lh[t0 + (lane >> 2) + 8 * i]; tl[i] = Ll[t0 + (lane >> 2) + 8 * i]; }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { jh[i] = Lh[j0 + 2 * (lane & 3) + (i & 1) + 4 * (i & 2)]; jl[i] = Ll[j0 + 2 * (lane & 3) + (i & 1) + 4 * (i & 2)]; }
+  }
+  // number e of tile y
+  __device__ __forceinline__ float operator()(int y, int e) const { return ex2((th[e >> 1] - jh[2 * y + (e & 1)]) + (tl[e >> 1] - jl[2 * y + (e & 1)])); }
+};
+
 template <int KS>
 __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, const int vecv) {
   constexpr int DZ = 16 * KS, DP = DZ + 8;
@@ -654,11 +667,12 @@ __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, co
       }
       if (i + 1 < chunks) fetch(i + 1);
       bar_sync(kPrepare, 128);
-      auto decay = [&](int t, int j) { return ex2((bf.Lh[t] - bf.Lh[j]) + (bf.Ll[t] - bf.Ll[j])); };
       // warps 0 and 1: the diagonal blocks of A and their inverses; 2: P (16, 0) and A_10; 3: P (0, 0) and P (16, 16)
       float x[2][4];
       if (pw < 2) {
         const int t0 = kHT * pw;
+        Decays f;
+        f.load(bf.Lh, bf.Ll, t0, t0, lane);
         token_products<KS>(x, bf.K, t0, bf.K, t0, lane);
         float* nt = nts[pw];
 #pragma unroll
@@ -666,7 +680,7 @@ __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, co
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int t = g + 4 * (e & 2), j = 8 * y + 2 * tq + (e & 1);
-            nt[j * kDA + t] = j < t ? bf.beta[t0 + t] * (decay(t0 + t, t0 + j) * x[y][e]) : 0.f;
+            nt[j * kDA + t] = j < t ? bf.beta[t0 + t] * (f(y, e) * x[y][e]) : 0.f;
           }
         __syncwarp();
         const int col = lane & 15;            // a column of the inverse per lane (both halves of the warp do the same)
@@ -694,6 +708,9 @@ __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, co
         for (int half = 0; half < 2; ++half) {
           const bool isa = pw == 2 && half;
           const int t0 = pw == 2 ? kHT : kHT * half, j0 = pw == 2 ? 0 : kHT * half;
+          Decays f;
+          f.load(bf.Lh, bf.Ll, t0, j0, lane);
+          const float b0 = isa ? bf.beta[t0 + g] : 1.f, b1 = isa ? bf.beta[t0 + g + 8] : 1.f;
           token_products<KS>(x, isa ? bf.K : bf.Q, t0, bf.K, j0, lane);
           const Planes M = isa ? bf.A10 : bf.P;
 #pragma unroll
@@ -701,9 +718,8 @@ __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, co
 #pragma unroll
             for (int e = 0; e < 4; e += 2) {
               const int t = t0 + g + 4 * e, j = j0 + 8 * y + 2 * tq;
-              const float f = isa ? bf.beta[t] : 1.f;
-              store_pair(M, isa ? t - kHT : t, j, j <= t ? f * (decay(t, j) * x[y][e]) : 0.f,
-                         j + 1 <= t ? f * (decay(t, j + 1) * x[y][e + 1]) : 0.f);
+              const float be = e ? b1 : b0;
+              store_pair(M, isa ? t - kHT : t, j, j <= t ? be * (f(y, e) * x[y][e]) : 0.f, j + 1 <= t ? be * (f(y, e + 1) * x[y][e + 1]) : 0.f);
             }
         }
       }

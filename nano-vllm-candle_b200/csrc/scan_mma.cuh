@@ -55,12 +55,13 @@ __device__ __forceinline__ void mma_high(float (&acc)[NT][4], const FragA& a, co
 }
 
 __device__ __forceinline__ void ldsm4(uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr) : "memory");
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm4_t(uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr) : "memory");
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr));
 }
 
+// (Planes are written and read by volatile asm alone, which keeps its order, barriers included: no memory clobbers.)
 // Matrices in shared memory are kept as three planes of bf16 parts, `rows` rows of `ld` numbers each (ld = a multiple of 16 plus 8, so that the
 // eight rows of an 8 x 8 block fall into different banks).
 struct Planes {
@@ -105,7 +106,7 @@ __device__ __forceinline__ void store_pair(const Planes& m, int r, int c, float 
   uint32_t v[3];
   split_pair(x, y, v[0], v[1], v[2]);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(m.at(r, c) + i * m.plane), "r"(v[i]) : "memory");
+  for (int i = 0; i < 3; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(m.at(r, c) + i * m.plane), "r"(v[i]));
 }
 // four neighbouring numbers (c a multiple of 4)
 __device__ __forceinline__ void store_quad(const Planes& m, int r, int c, const float4& x) {
@@ -113,7 +114,7 @@ __device__ __forceinline__ void store_quad(const Planes& m, int r, int c, const 
   split_pair(x.x, x.y, u[0], u[1], u[2]);
   split_pair(x.z, x.w, v[0], v[1], v[2]);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(m.at(r, c) + i * m.plane), "r"(u[i]), "r"(v[i]) : "memory");
+  for (int i = 0; i < 3; ++i) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(m.at(r, c) + i * m.plane), "r"(u[i]), "r"(v[i]));
 }
 constexpr int kMT = 32;                 // tokens per chunk
 constexpr int kMC = 64;                 // value columns per CTA: 16 for each of its four state warps
