@@ -4,13 +4,15 @@
 // or per head) and a constant factor on the output.  Rows of sequence b are the LAST q_len positions of its context; row at position i
 // sees keys max(0, i - window + 1) .. i (window), the keys of its own chunk i - i % chunk .. i (chunk), or 0 .. i (neither).
 //
-// Three kernels:
+// Four kernels:
+//   prefill_attn_v2_kernel (prefill_attn_v2.cuh)  bf16 prompt portions of 128-number heads, no chunk, cap or per-head gate: tcgen05
 //   attn_shared_decode_kernel (attn_shared_decode.cuh)  bf16, one row per sequence, values = leading numbers of 64- or 128-number key rows
 //   attn_wide_mma_kernel (attn_wide_mma.cuh)  bf16 storage, dim and vdim multiples of 16 up to 128: tensor pipe
 //   attn_wide_simt_kernel                      any sizes, both storage formats, plain fp32 FMA: the exact mode
 // The last takes the keys of a row in tiles that start at the row's own first visible key, so the order of every sum depends on
 // the row's position alone - not on how the prompt was cut, on the batch or on the pages.
 #include "typed.cuh"
+#include "internal.h"
 #include "attn_wide_mma.cuh"
 
 namespace {
@@ -153,7 +155,11 @@ extern "C" int nvc_attn_paged_wide(nvc_ctx* ctx, const void* q, int ldq, const v
               "bad strides");
   WideArgs a{q, k_cache, v_cache, out, ldq, ldk, ldv, ldo, block_tables, context_lens, cu_seqlens, bt_stride, B, block_size, s};
   if (dtype == NVC_DT_BF16 && attn_wide_mma_takes(s, ldq, ldk, ldv, ldo, block_size)) {
-    int rc = attn_wide_mma_launch(ctx, a.q, a.k_cache, a.v_cache, a.out, ldq, ldk, ldv, ldo, block_tables, context_lens, cu_seqlens, bt_stride,
+    int rc = nvc_prefill_attn_gated(ctx, reinterpret_cast<const nvc_bf16*>(q), ldq, reinterpret_cast<const nvc_bf16*>(k_cache), ldk,
+                                          reinterpret_cast<const nvc_bf16*>(v_cache), ldv, block_tables, bt_stride, context_lens, cu_seqlens, B, rows, max_qlen,
+                                          block_size, s, reinterpret_cast<nvc_bf16*>(out), ldo, stream);
+    if (rc != NVC_ENOTIMPL) return rc;
+    rc = attn_wide_mma_launch(ctx, a.q, a.k_cache, a.v_cache, a.out, ldq, ldk, ldv, ldo, block_tables, context_lens, cu_seqlens, bt_stride,
                                   B, rows, max_qlen, block_size, s, nvc_stream(stream));
     if (rc != NVC_ENOTIMPL) return rc;
   }

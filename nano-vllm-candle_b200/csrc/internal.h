@@ -34,3 +34,7 @@ int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
 int nvc_prefill_attn_init(nvc_ctx* ctx);
 int nvc_paged_decode_init(nvc_ctx* ctx);
 }
+// prompt portions of nvc_attn_paged_wide on the tcgen05 kernel, or NVC_ENOTIMPL (nothing launched)
+int nvc_prefill_attn_gated(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* k_cache, int ldk, const nvc_bf16* v_cache, int ldv,
+                           const int32_t* block_tables, int bt_stride, const int32_t* context_lens, const int32_t* cu_seqlens_q, int B, int rows, int max_qlen,
+                           int block_size, const nvc_attn_spec& s, nvc_bf16* out, int ldo, void* stream);

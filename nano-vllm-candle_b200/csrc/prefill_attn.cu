@@ -20,6 +20,8 @@
 #include "ptx.cuh"
 #include "internal.h"
 
+#include <algorithm>
+
 int g_nvc_debug[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 extern "C" int nvc_debug_set(int key, int value) {
   if (key < 0 || key >= 8) return NVC_EINVAL;
@@ -52,8 +54,9 @@ struct PagedKV {                              // kPaged only
   // shared key / value rows only
   const float* bias;                          // sigmoid weights: [nh], added to the scores
   const float* key_scale;                     // sigmoid weights: [slots], a factor on the scores of a cached key
-  const float* gate;                          // sigmoid weights: fp32 [rows, ldg], a sigmoid gate on every output number
+  const float* gate;                          // sigmoid weights and kGated: fp32 [rows, ldg], a sigmoid gate on every output number
   int ldg;
+  float out_scale;                            // kGated: a constant factor on the output
 };
 
 int make_tma_heads(nvc_ctx* ctx, CUtensorMap* map, const void* base, int heads, int64_t tokens, int ld, int box_rows = 128) {
@@ -90,7 +93,7 @@ cudaError_t launch_v2(nvc_ctx* ctx, int QT, int nh, int kv, int B, cudaStream_t 
 
 extern "C" int nvc_prefill_attn_init(nvc_ctx* ctx) {
   for (auto k : {v2::prefill_attn_v2_kernel<false, v2::kPlain>, v2::prefill_attn_v2_kernel<true, v2::kPlain>,
-                 v2::prefill_attn_v2_kernel<true, v2::kWindow>, v2::prefill_attn_v2_kernel<true, v2::kShared>, v2::prefill_attn_v2_kernel<true, v2::kSigmoid>})
+                 v2::prefill_attn_v2_kernel<true, v2::kWindow>, v2::prefill_attn_v2_kernel<true, v2::kGated>, v2::prefill_attn_v2_kernel<true, v2::kShared>, v2::prefill_attn_v2_kernel<true, v2::kSigmoid>})
     NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v2::kSmemBytes));
   return NVC_OK;
 }
@@ -220,13 +223,44 @@ extern "C" int nvc_prefill_attn_shared(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
   if (rc) return rc;
   rc = make_tma_heads(ctx, &tk, cache, kv, (int64_t)num_blocks * block_size, kv * 128, box_rows);
   if (rc) return rc;
-  PagedKV pk{block_tables, context_lens, bt_stride, block_size, box_rows, s.sink, s.window, s.bias, s.key_scale, s.gate, s.ldg};
+  PagedKV pk{block_tables, context_lens, bt_stride, block_size, box_rows, s.sink, s.window, s.bias, s.key_scale, s.gate, s.ldg, 1.f};
   const int QT = (max_seqlen_q + 127) / 128;
   const float scale_log2e = s.scale * 1.4426950408889634f;
   if (sig)
     NVC_CUDA_CHECK(ctx, (launch_v2<true, v2::kSigmoid>(ctx, QT, nh, kv, B, nvc_stream(stream), tq, tk, tk, cu_seqlens_q, scale_log2e, out, ldo, pk)));
   else
     NVC_CUDA_CHECK(ctx, (launch_v2<true, v2::kShared>(ctx, QT, nh, kv, B, nvc_stream(stream), tq, tk, tk, cu_seqlens_q, scale_log2e, out, ldo, pk)));
+  NVC_CUDA_CHECK(ctx, cudaGetLastError());
+  ctx->launches++;
+  return NVC_OK;
+}
+
+// Prompt portions of nvc_attn_paged_wide on the tcgen05 kernel: softmax over separate keys and values of 128 numbers per head with an optional
+// window, sink, gate and factor.  NVC_ENOTIMPL (nothing launched): a shape or a variant that the other kernels take.
+// The kernel works on tiles of 128 rows of one sequence and head, the mma.sync one on 64 rows of a key head's query heads: with rows of few
+// tokens per sequence most of a tile is empty.  MEASURED
+int nvc_prefill_attn_gated(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* k_cache, int ldk, const nvc_bf16* v_cache, int ldv,
+                           const int32_t* block_tables, int bt_stride, const int32_t* context_lens, const int32_t* cu_seqlens_q, int B, int rows, int max_qlen,
+                           int block_size, const nvc_attn_spec& s, nvc_bf16* out, int ldo, void* stream) {
+  auto al16 = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
+  if (!cu_seqlens_q || max_qlen < 64 || rows < 32 * B || s.dim != 128 || s.vdim != 128 || s.weights != NVC_ATTN_SOFTMAX || s.chunk || s.softcap != 0.f || s.gate_per_head ||
+      s.key_scale || k_cache == v_cache || !(block_size >= 16 && (block_size >= 128 ? block_size % 128 == 0 : 128 % block_size == 0)) ||
+      ((ldq | ldk | ldv | ldo) & 7) || (s.gate && ((s.ldg & 3) || !al16(s.gate))) || !al16(q) || !al16(k_cache) || !al16(v_cache) || !al16(out) || !ctx->encode_tiled)
+    return NVC_ENOTIMPL;
+  const int nh = s.heads, kv = s.kv_heads, box_rows = block_size < v2::kKT ? block_size : v2::kKT;
+  const int QT = (std::min(max_qlen, rows) + 127) / 128;
+  if ((long long)QT * nh * B > 0x7fffffffLL) return NVC_ENOTIMPL;
+  // the pool's number of rows is not known here: boxes lie inside the pages that the block tables name, so any bound above them will do
+  constexpr int64_t kRows = (int64_t)1 << 31;
+  CUtensorMap tq, tk, tv;
+  int rc = make_tma_heads(ctx, &tq, q, nh, rows, ldq);
+  if (!rc) rc = make_tma_heads(ctx, &tk, k_cache, kv, kRows, ldk, box_rows);
+  if (!rc) rc = make_tma_heads(ctx, &tv, v_cache, kv, kRows, ldv, box_rows);
+  if (rc) return rc;
+  PagedKV pk{};
+  pk.block_tables = block_tables; pk.context_lens = context_lens; pk.bt_stride = bt_stride; pk.block_size = block_size; pk.box_rows = box_rows;
+  pk.sink = s.sink; pk.window = s.window; pk.gate = s.gate; pk.ldg = s.ldg; pk.out_scale = s.out_scale;
+  NVC_CUDA_CHECK(ctx, (launch_v2<true, v2::kGated>(ctx, QT, nh, kv, B, nvc_stream(stream), tq, tk, tv, cu_seqlens_q, s.scale * 1.4426950408889634f, out, ldo, pk)));
   NVC_CUDA_CHECK(ctx, cudaGetLastError());
   ctx->launches++;
   return NVC_OK;

@@ -50,7 +50,7 @@ constexpr int kNumBars = 2 + 2 * kKStages + 2 * kVStages + 2 + 4;
 constexpr int kSmemBytes = 115712;
 static_assert(kOffBar + kNumBars * 8 + 16 + 768 <= kSmemBytes, "shared memory budget for two CTAs per SM");
 constexpr int kTmemCols = 256;                 // S / P (double-buffered): columns [0, 64) and [64, 128); O: [128, 256)
-enum { kPlain = 0, kShared = 1, kSigmoid = 2, kWindow = 3 };
+enum { kPlain = 0, kShared = 1, kSigmoid = 2, kWindow = 3, kGated = 4 };     // kGated: kWindow (or no window) with an output gate and a factor
 // shared tiles: stages of the one ring; the key factors of a stage take the place of a fourth tile
 template <int kMode> struct SharedRing { static constexpr int kStages = kMode == kSigmoid ? 3 : 4; };
 constexpr int kOffScale = kOffK + 3 * kKBytes;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(192, 2)
 prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                        const __grid_constant__ CUtensorMap tma_v, const int32_t* __restrict__ cu_seqlens, const Sched sc,
                        float scale_log2e, nvc_bf16* __restrict__ out, int ldo, const PagedKV pk) {
-  constexpr bool kSep = kMode == kPlain || kMode == kWindow;       // keys and values are separate tensors
+  constexpr bool kSep = kMode == kPlain || kMode == kWindow || kMode == kGated;       // keys and values are separate tensors
   pdl_trigger();
   const int num_items = sc.num_items, nh = sc.nh.d;
   extern __shared__ __align__(1024) uint8_t smem_v2[];
@@ -340,14 +340,14 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
       const int n = ge.n_tiles;
       const float bias = kMode == kSigmoid && pk.bias ? __ldg(pk.bias + x.h) * 1.4426950408889634f : 0.f;
       // rows past the sequence are not stored; their gate row is clamped to the last real one
-      const float* grow = kMode == kSigmoid && pk.gate
+      const float* grow = (kMode == kSigmoid || kMode == kGated) && pk.gate
                               ? pk.gate + (int64_t)(ge.seq_start + min(x.qt * 128 + r, ge.seq_len - 1)) * pk.ldg + x.h * 128 : nullptr;
-      if (kMode == kSigmoid && grow) {               // the row's gate is needed behind the last tile: on its way to L2 until then
+      if ((kMode == kSigmoid || kMode == kGated) && grow) {               // the row's gate is needed behind the last tile: on its way to L2 until then
 #pragma unroll
         for (int c = 0; c < 4; ++c) asm volatile("prefetch.global.L2 [%0];" ::"l"(grow + c * 32));
       }
       // with a window a row's first tiles may hold none of its keys: a finite floor keeps every difference of maxima defined
-      float m = kMode == kShared || kMode == kWindow ? -1e30f : -INFINITY, l = 0.f;                 // m: the maximum the exponentials are taken against (may lag the true one)
+      float m = kMode == kShared || kMode == kWindow || kMode == kGated ? -1e30f : -INFINITY, l = 0.f;                 // m: the maximum the exponentials are taken against (may lag the true one)
       for (int j = 0; j < n; ++j) {
         const uint32_t gi = g + j;
         const uint32_t s_addr = tmem_s + (gi & 1) * kKT + lane_addr;
@@ -410,7 +410,7 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
             for (int i = 0; i < kKT; ++i)
               if (i > lim) sv[i] = 0xff800000u;
           }
-          if ((kMode == kShared || kMode == kWindow) && pk.window > 0 && t0 <= ge.q0 + 127 - pk.window) {
+          if ((kMode == kShared || kMode == kWindow || kMode == kGated) && pk.window > 0 && t0 <= ge.q0 + 127 - pk.window) {
             const int first = ge.q0 + r - pk.window + 1 - t0;      // first visible column of this row
 #pragma unroll
             for (int i = 0; i < kKT; ++i)
@@ -499,7 +499,7 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
       ptx::mbar_wait(o_full, kMode == kSigmoid ? (n_done & 1) : ((g + n - 1) & 1));
       ptx::tcgen05_fence_after();
       if (kPaged && kMode != kSigmoid && pk.sink) l += exp2f(__ldg(pk.sink + x.h) * 1.4426950408889634f - m);   // the sink: in the denominator, without a value
-      const float inv = kMode == kSigmoid ? 1.0f : 1.0f / l;
+      const float inv = kMode == kSigmoid ? 1.0f : (kMode == kGated ? pk.out_scale / l : 1.0f / l);
       // this warp's 32 rows x 128 head dims leave through its staging buffer: 8 lanes per row, 128 contiguous bytes each
       RowStage st = make_row_stage(gen + kOffStage + quad * 4096, out, 0, NVC_EPI_NONE, (int64_t)ldo,
                                    ge.seq_start + x.qt * 128 + quad * 32, ge.seq_start + ge.seq_len, x.h * 128, 128, nh * 128);
@@ -511,7 +511,7 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
         float f[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) * inv;
-        if (kMode == kSigmoid && grow) {
+        if ((kMode == kSigmoid || kMode == kGated) && grow) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             const float4 z = *reinterpret_cast<const float4*>(grow + c * 32 + i);

@@ -9,7 +9,8 @@
 //   value blending                           v <- (1 - lambda) v + lambda v_first, or v_first <- v in the layer that provides it
 //   v *= v_scale                             (a constant weight of the mixer, so that every attention kernel can leave it out)
 //   stores                                   q to its buffer; k and v to rows of a paged cache (slot mapping) or to plain rows
-// One warp per (token, head) of q, k or v; a head is staged in shared memory so that any pairing reads its partner.  The purely
+// Heads of up to 128 numbers whose rows allow 16-byte accesses: four heads (or pairs of small heads) of a token per warp, in registers
+// (prep_heads_kernel).  Other shapes: one warp per (token, head), staged in shared memory so that any pairing reads its partner.  The purely
 // element-wise case (bias and silu only, plain fp32 rows out) runs a flat kernel with 16-byte accesses instead.  With a short causal
 // convolution behind the bias, or norms that span the whole query / key projection, one CTA takes a whole token (prep_token_kernel).
 #include "typed.cuh"
@@ -94,6 +95,113 @@ __global__ void qkv_prep_kernel(const PrepArgs a) {
 }
 
 
+// four neighbouring numbers in the storage format with one store
+__device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
+  uint2 u;
+  u.x = pack_bf16(v.x, v.y);
+  u.y = pack_bf16(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = u;
+}
+
+// Heads of up to 4 L numbers: L lanes with four numbers each, 32 / L heads side by side, four of those per warp and all of one token, so that
+// four 16-byte loads per lane are in flight and the token's angles and the norm weights are read once for all of them.  A head never
+// leaves its lanes' registers: neighbouring pairs turn inside a lane, (i, i + rot_dims / 2) by exchange.  Bound by memory: MEASURED
+template <typename TQ, typename TKV, int L>
+__global__ void __launch_bounds__(128) prep_heads_kernel(const PrepArgs a) {
+  constexpr int U = 4, HP = 32 / L;
+  pdl_trigger();
+  const nvc_qkv_prep& p = a.p;
+  const int lane = threadIdx.x & 31, j = 4 * (lane & (L - 1));
+  const int units = p.q_heads + 2 * p.kv_heads, groups = (units + U * HP - 1) / (U * HP);
+  const int64_t wu = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (wu >= (int64_t)a.N * groups) return;
+  const int n = (int)(wu / groups), u0 = (int)(wu % groups) * U * HP + lane / L;
+  // what no kernel of the step writes: before the wait
+  const int64_t krow = p.slot_mapping ? p.slot_mapping[n] : n;
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+  float4 wq = one, wk = one, c0 = one, c1 = one;
+  if (p.q_norm && j < p.dim) {
+    wq = __ldg(reinterpret_cast<const float4*>(p.q_norm + j));
+    wk = __ldg(reinterpret_cast<const float4*>(p.k_norm + j));
+  }
+  const int half = p.rot_dims >> 1;
+  if (j < p.rot_dims) {       // (cos, sin) of the angles of this lane's numbers: two pairs, or four
+    const float* tab = p.rot_table + (int64_t)p.positions[n] * p.rot_dims;
+    const float4* cs = reinterpret_cast<const float4*>(tab + (p.rot_half ? 2 * (j < half ? j : j - half) : j));
+    c0 = __ldg(cs);
+    if (p.rot_half) c1 = __ldg(cs + 1);
+  }
+  pdl_wait();
+  const float* in = p.in + (int64_t)n * p.ldi;
+  float4 x[U];
+  int kind[U], h[U];          // 0: query, 1: key, 2: value, 3: none
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    const int u = u0 + i * HP;
+    kind[i] = u < p.q_heads ? 0 : (u < p.q_heads + p.kv_heads ? 1 : (u < units ? 2 : 3));
+    h[i] = kind[i] == 0 ? u : (kind[i] == 1 ? u - p.q_heads : u - p.q_heads - p.kv_heads);
+    const int w = kind[i] == 2 ? p.vdim : p.dim;
+    if (j >= w) kind[i] = 3;
+    x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kind[i] != 3) {
+      const int col = (kind[i] == 0 ? p.q_off : (kind[i] == 1 ? p.k_off : p.v_off)) + h[i] * w + j;
+      x[i] = *reinterpret_cast<const float4*>(in + col);
+      if (p.bias) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + col));
+        x[i].x += b.x; x[i].y += b.y; x[i].z += b.z; x[i].w += b.w;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    float4 v = x[i];
+    if (p.act == NVC_PREP_ACT_SILU) { v.x *= sigmoid_f32(v.x); v.y *= sigmoid_f32(v.y); v.z *= sigmoid_f32(v.z); v.w *= sigmoid_f32(v.w); }
+    float r = 1.f;
+    if (p.q_norm || p.unit_norm) {
+      float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      r = 1.0f / sqrtf(ss / (float)p.dim + p.eps);
+    }
+    if (kind[i] < 2) {
+      const float4 w = kind[i] == 0 ? wq : wk;
+      v.x = v.x * r * w.x; v.y = v.y * r * w.y; v.z = v.z * r * w.z; v.w = v.w * r * w.w;
+    }
+    if (p.rot_dims) {
+      if (p.rot_half) {
+        const int from = (lane & ~(L - 1)) | (((j < half ? j + half : j - half) >> 2) & (L - 1));
+        const float s = j < half ? -1.f : 1.f;
+        const float4 z = make_float4(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from), __shfl_sync(0xffffffffu, v.z, from),
+                                     __shfl_sync(0xffffffffu, v.w, from));
+        if (kind[i] < 2 && j < p.rot_dims)
+          v = make_float4(v.x * c0.x + s * z.x * c0.y, v.y * c0.z + s * z.y * c0.w, v.z * c1.x + s * z.z * c1.y, v.w * c1.z + s * z.w * c1.w);
+      } else if (kind[i] < 2 && j < p.rot_dims) {
+        v = make_float4(v.x * c0.x - v.y * c0.y, v.y * c0.x + v.x * c0.y, v.z * c0.z - v.w * c0.w, v.w * c0.z + v.z * c0.w);
+      }
+    }
+    if (kind[i] == 0) {
+      store4(reinterpret_cast<TQ*>(p.q_out) + (int64_t)n * p.ldq + h[i] * p.dim + j, v);
+    } else if (kind[i] == 1) {
+      const float s = p.k_scale;
+      if (krow >= 0) store4(reinterpret_cast<TKV*>(p.k_out) + krow * p.ldk + h[i] * p.dim + j, make_float4(v.x * s, v.y * s, v.z * s, v.w * s));
+    } else if (kind[i] == 2) {
+      if (p.blend != NVC_BLEND_NONE) {
+        float4* first = reinterpret_cast<float4*>(p.v_first + (int64_t)n * p.ldvf + h[i] * p.vdim + j);
+        if (p.blend == NVC_BLEND_PROVIDE) {
+          *first = v;
+        } else {
+          const float lam = __ldg(p.lambda), m = 1.0f - lam;
+          const float4 f = *first;
+          v = make_float4(m * v.x + lam * f.x, m * v.y + lam * f.y, m * v.z + lam * f.z, m * v.w + lam * f.w);
+        }
+      }
+      const float s = p.v_scale;
+      if (krow >= 0) store4(reinterpret_cast<TKV*>(p.v_out) + krow * p.ldv + h[i] * p.vdim + j, make_float4(v.x * s, v.y * s, v.z * s, v.w * s));
+    }
+  }
+}
+
 // The element-wise case (no norm, no rotation, no blending, no scale, plain fp32 rows out): q, k, v = act(in + bias), four numbers per
 // thread.  CTA = (token, block of 256 x 4 columns of [q | k | v]).
 __global__ void __launch_bounds__(256) prep_flat_kernel(const PrepArgs a) {
@@ -116,15 +224,6 @@ __global__ void __launch_bounds__(256) prep_flat_kernel(const PrepArgs a) {
   }
   if (p.act == NVC_PREP_ACT_SILU) { v.x *= sigmoid_f32(v.x); v.y *= sigmoid_f32(v.y); v.z *= sigmoid_f32(v.z); v.w *= sigmoid_f32(v.w); }
   *reinterpret_cast<float4*>(out) = v;
-}
-
-// four neighbouring numbers in the storage format with one store
-__device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
-  uint2 u;
-  u.x = pack_bf16(v.x, v.y);
-  u.y = pack_bf16(v.z, v.w);
-  *reinterpret_cast<uint2*>(p) = u;
 }
 
 __device__ __forceinline__ int prep_find_seq(const int32_t* cu, int B, int row) {
@@ -433,6 +532,20 @@ int launch_prep(nvc_ctx* ctx, const nvc_qkv_prep* p, int N, void* stream) {
   PrepArgs a{*p, N};
   const int64_t units = (int64_t)N * (p->q_heads + 2 * p->kv_heads);
   const int wmax = p->dim > p->vdim ? p->dim : p->vdim;
+  // every quad of a head on a 16-byte boundary, and no pair split over quads
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const bool vec = wmax <= 128 && ((p->dim | p->vdim | p->q_off | p->k_off | p->v_off | p->ldi | p->ldq | p->ldk | p->ldv | p->rot_dims) & 3) == 0 &&
+                   (!p->rot_half || (p->rot_dims & 7) == 0) && (p->blend == NVC_BLEND_NONE || ((p->ldvf & 3) == 0 && al16(p->v_first))) && al16(p->in) &&
+                   al16(p->bias) && al16(p->q_norm) && al16(p->k_norm) && al16(p->rot_table) && al16(p->q_out) && al16(p->k_out) && al16(p->v_out);
+  if (vec) {
+    const int lanes = wmax <= 64 ? 16 : 32, per = 4 * (32 / lanes);
+    const int64_t warps = (int64_t)N * ((p->q_heads + 2 * p->kv_heads + per - 1) / per);
+    NVC_REQUIRE(ctx, (warps + 3) / 4 <= 0x7fffffffLL, NVC_ESHAPE, "too many rows");
+    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, lanes == 16 ? prep_heads_kernel<TQ, TKV, 16> : prep_heads_kernel<TQ, TKV, 32>, dim3((unsigned)((warps + 3) / 4)),
+                                   dim3(128), 0, nvc_stream(stream), a));
+    ctx->launches++;
+    return NVC_OK;
+  }
   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, qkv_prep_kernel<TQ, TKV>, dim3((unsigned)((units + 3) / 4)), dim3(128), (size_t)4 * wmax * sizeof(float),
                                  nvc_stream(stream), a));
   ctx->launches++;
