@@ -108,33 +108,37 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
 // four 16-byte loads per lane are in flight and the token's angles and the norm weights are read once for all of them.  A head never
 // leaves its lanes' registers: neighbouring pairs turn inside a lane, (i, i + rot_dims / 2) by exchange.  Bound by memory: MEASURED
 template <typename TQ, typename TKV, int L>
-__global__ void __launch_bounds__(128) prep_heads_kernel(const PrepArgs a) {
+__global__ void __launch_bounds__(256) prep_heads_kernel(const PrepArgs a) {
   constexpr int U = 4, HP = 32 / L;
   pdl_trigger();
   const nvc_qkv_prep& p = a.p;
   const int lane = threadIdx.x & 31, j = 4 * (lane & (L - 1));
-  const int units = p.q_heads + 2 * p.kv_heads, groups = (units + U * HP - 1) / (U * HP);
-  const int64_t wu = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (wu >= (int64_t)a.N * groups) return;
-  const int n = (int)(wu / groups), u0 = (int)(wu % groups) * U * HP + lane / L;
-  // what no kernel of the step writes: before the wait
+  const int units = p.q_heads + 2 * p.kv_heads, n = blockIdx.x;
+  const int u0 = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * U * HP + lane / L;
+  // the slot, the position and what hangs on them are written by no kernel of the step.  Few CTAs (a decode step): before the wait.  Else behind
+  // the row's loads: position -> angles in front of them would put two more latencies into every warp
+  const bool early = gridDim.x <= 1024;
   const int64_t krow = p.slot_mapping ? p.slot_mapping[n] : n;
+  const int pos = p.rot_dims ? p.positions[n] : 0;
   const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
   float4 wq = one, wk = one, c0 = one, c1 = one;
-  if (p.q_norm && j < p.dim) {
-    wq = __ldg(reinterpret_cast<const float4*>(p.q_norm + j));
-    wk = __ldg(reinterpret_cast<const float4*>(p.k_norm + j));
-  }
   const int half = p.rot_dims >> 1;
-  if (j < p.rot_dims) {       // (cos, sin) of the angles of this lane's numbers: two pairs, or four
-    const float* tab = p.rot_table + (int64_t)p.positions[n] * p.rot_dims;
-    const float4* cs = reinterpret_cast<const float4*>(tab + (p.rot_half ? 2 * (j < half ? j : j - half) : j));
-    c0 = __ldg(cs);
-    if (p.rot_half) c1 = __ldg(cs + 1);
-  }
+  auto statics = [&] {
+    if (p.q_norm && j < p.dim) {
+      wq = __ldg(reinterpret_cast<const float4*>(p.q_norm + j));
+      wk = __ldg(reinterpret_cast<const float4*>(p.k_norm + j));
+    }
+    if (j < p.rot_dims) {       // (cos, sin) of the angles of this lane's numbers: two pairs, or four
+      const float* tab = p.rot_table + (int64_t)pos * p.rot_dims;
+      const float4* cs = reinterpret_cast<const float4*>(tab + (p.rot_half ? 2 * (j < half ? j : j - half) : j));
+      c0 = __ldg(cs);
+      if (p.rot_half) c1 = __ldg(cs + 1);
+    }
+  };
+  if (early) statics();
   pdl_wait();
   const float* in = p.in + (int64_t)n * p.ldi;
-  float4 x[U];
+  float4 x[U], b[U];
   int kind[U], h[U];          // 0: query, 1: key, 2: value, 3: none
 #pragma unroll
   for (int i = 0; i < U; ++i) {
@@ -143,30 +147,42 @@ __global__ void __launch_bounds__(128) prep_heads_kernel(const PrepArgs a) {
     h[i] = kind[i] == 0 ? u : (kind[i] == 1 ? u - p.q_heads : u - p.q_heads - p.kv_heads);
     const int w = kind[i] == 2 ? p.vdim : p.dim;
     if (j >= w) kind[i] = 3;
-    x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    x[i] = b[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (kind[i] != 3) {
       const int col = (kind[i] == 0 ? p.q_off : (kind[i] == 1 ? p.k_off : p.v_off)) + h[i] * w + j;
       x[i] = *reinterpret_cast<const float4*>(in + col);
-      if (p.bias) {
-        const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + col));
-        x[i].x += b.x; x[i].y += b.y; x[i].z += b.z; x[i].w += b.w;
-      }
+      if (p.bias) b[i] = __ldg(reinterpret_cast<const float4*>(p.bias + col));
     }
+  }
+  if (!early) statics();
+  float r[U];
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    float4& v = x[i];
+    v = make_float4(v.x + b[i].x, v.y + b[i].y, v.z + b[i].z, v.w + b[i].w);
+    if (p.act == NVC_PREP_ACT_SILU) { v.x *= sigmoid_f32(v.x); v.y *= sigmoid_f32(v.y); v.z *= sigmoid_f32(v.z); v.w *= sigmoid_f32(v.w); }
+    r[i] = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  }
+  if (p.q_norm || p.unit_norm) {
+    // the four sums by exchange: a lane ends with one of them (which: two bits of its number), so that a root and a division serve four heads
+    const bool hi = lane & (L / 2), lo = lane & (L / 4);
+    float s0 = (hi ? r[2] : r[0]) + __shfl_xor_sync(0xffffffffu, hi ? r[0] : r[2], L / 2), s1 = (hi ? r[3] : r[1]) + __shfl_xor_sync(0xffffffffu, hi ? r[1] : r[3], L / 2);
+    float ss = (lo ? s1 : s0) + __shfl_xor_sync(0xffffffffu, lo ? s0 : s1, L / 4);
+#pragma unroll
+    for (int o = L / 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    ss = 1.0f / sqrtf(ss / (float)p.dim + p.eps);
+#pragma unroll
+    for (int i = 0; i < U; ++i) r[i] = __shfl_sync(0xffffffffu, ss, (lane & ~(L - 1)) | (i & 2 ? L / 2 : 0) | (i & 1 ? L / 4 : 0));
+  } else {
+#pragma unroll
+    for (int i = 0; i < U; ++i) r[i] = 1.f;
   }
 #pragma unroll
   for (int i = 0; i < U; ++i) {
     float4 v = x[i];
-    if (p.act == NVC_PREP_ACT_SILU) { v.x *= sigmoid_f32(v.x); v.y *= sigmoid_f32(v.y); v.z *= sigmoid_f32(v.z); v.w *= sigmoid_f32(v.w); }
-    float r = 1.f;
-    if (p.q_norm || p.unit_norm) {
-      float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-#pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      r = 1.0f / sqrtf(ss / (float)p.dim + p.eps);
-    }
     if (kind[i] < 2) {
       const float4 w = kind[i] == 0 ? wq : wk;
-      v.x = v.x * r * w.x; v.y = v.y * r * w.y; v.z = v.z * r * w.z; v.w = v.w * r * w.w;
+      v.x = v.x * r[i] * w.x; v.y = v.y * r[i] * w.y; v.z = v.z * r[i] * w.z; v.w = v.w * r[i] * w.w;
     }
     if (p.rot_dims) {
       if (p.rot_half) {
@@ -538,11 +554,10 @@ int launch_prep(nvc_ctx* ctx, const nvc_qkv_prep* p, int N, void* stream) {
                    (!p->rot_half || (p->rot_dims & 7) == 0) && (p->blend == NVC_BLEND_NONE || ((p->ldvf & 3) == 0 && al16(p->v_first))) && al16(p->in) &&
                    al16(p->bias) && al16(p->q_norm) && al16(p->k_norm) && al16(p->rot_table) && al16(p->q_out) && al16(p->k_out) && al16(p->v_out);
   if (vec) {
-    const int lanes = wmax <= 64 ? 16 : 32, per = 4 * (32 / lanes);
-    const int64_t warps = (int64_t)N * ((p->q_heads + 2 * p->kv_heads + per - 1) / per);
-    NVC_REQUIRE(ctx, (warps + 3) / 4 <= 0x7fffffffLL, NVC_ESHAPE, "too many rows");
-    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, lanes == 16 ? prep_heads_kernel<TQ, TKV, 16> : prep_heads_kernel<TQ, TKV, 32>, dim3((unsigned)((warps + 3) / 4)),
-                                   dim3(128), 0, nvc_stream(stream), a));
+    // a CTA per token, or several when a token has more than 8 warps of heads
+    const int lanes = wmax <= 64 ? 16 : 32, per = 4 * (32 / lanes), groups = (p->q_heads + 2 * p->kv_heads + per - 1) / per, warps = std::min(groups, 8);
+    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, lanes == 16 ? prep_heads_kernel<TQ, TKV, 16> : prep_heads_kernel<TQ, TKV, 32>,
+                                   dim3((unsigned)N, (unsigned)((groups + warps - 1) / warps)), dim3(32 * warps), 0, nvc_stream(stream), a));
     ctx->launches++;
     return NVC_OK;
   }
