@@ -576,7 +576,7 @@ typedef struct nvc_delta_prep {
    * the recurrence then multiplies row d of a head's state by that channel's decay.  NULL: one decay per head */
   const float* channel_a; int ldca; float* channel_g;
 } nvc_delta_prep;
-int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int max_qlen, void* stream);   /* max_qlen: the longest portion (a bound will do) */
+int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int max_qlen, void* stream);   /* max_qlen: the longest portion, or any number */
 /* The recurrence, per (sequence, head) with state S [dim, vdim] fp32 in state [slots, heads, dim, vdim]:
  *   S <- g S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q        (head h reads q / k head h / (heads / kv_heads))
  * token by token over rows cu_seqlens[b] .. cu_seqlens[b + 1] (row b when cu_seqlens == NULL); a sequence starts from zeros when

@@ -20,6 +20,7 @@
 // All arithmetic is fp32: FMA code, or products of three bf16 parts per number (scan_mma.cuh).
 #include <type_traits>
 
+#include "conv_tile.cuh"
 #include "scan_mma.cuh"
 
 namespace {
@@ -35,8 +36,7 @@ struct DeltaArgs {
 
 __device__ __forceinline__ float softplus_f32(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
-// grid (token tiles of the longest portion, units, sequences): the sequence comes from the block index, so a warp's first loads are
-// its sequence's bounds and nothing has to be searched; CTAs behind a sequence's last token leave at once
+// grid (row tiles, units): a warp per (row, unit), the row's sequence by a search.  Decode steps, and shapes that delta_prep_tile_kernel does not take
 // TAPS: the convolution's taps when they are 2 .. 4 (all inputs of a channel are in flight at once), 0: any number of them
 template <int TAPS>
 __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
@@ -45,11 +45,14 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
   const nvc_delta_prep& p = a.p;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int units = 2 * p.kv_heads + p.heads + 1;
-  const int b = blockIdx.z, uu = blockIdx.y;
-  const int r0 = p.cu_seqlens ? p.cu_seqlens[b] : b;
-  const int r1 = p.cu_seqlens ? p.cu_seqlens[b + 1] : b + 1;
-  const int n = r0 + blockIdx.x * (blockDim.x >> 5) + wid;
-  if (n >= r1) return;
+  const int n = blockIdx.x * (blockDim.x >> 5) + wid, uu = blockIdx.y;
+  if (n >= a.N || (p.cu_seqlens && n >= p.cu_seqlens[p.B])) return;
+  int b = n, r0 = n;
+  if (p.cu_seqlens) {
+    b = 0;
+    for (int i = 1; i < p.B; i += 32) b += __popc(__ballot_sync(0xffffffffu, i + lane < p.B && p.cu_seqlens[i + lane] <= n));
+    r0 = p.cu_seqlens[b];
+  }
   const float* in = p.in + (int64_t)n * p.ldi;
   if (uu >= units) {
     // ---- log decays of one head's key channels
@@ -162,6 +165,92 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
   for (int j = lane; j < width; j += 32) out[j] *= r;
 }
 
+
+// Prompt portions with 16-byte rows, heads of up to 128 numbers and 1 .. 4 taps: a warp takes 8 neighbouring rows of 128 channels (conv_tile.cuh).
+// Tasks of a tile of rows: the q and k heads (a head in L lanes, its length by exchange: one root and division per row), the v channels, the
+// heads' decays and betas, and the decays per channel.  Bound by memory and the exponentials: 4 480 rows of 16 heads of 128 over 8 take 43 us
+// (150 MB: 3.5 TB/s), one warp per (row, head) that read every row once per tap 84 us.
+template <int TAPS, int L>
+__global__ void __launch_bounds__(128) delta_prep_tile_kernel(const DeltaArgs a) {
+  constexpr int TT = 8, HP = 32 / L;
+  pdl_trigger();
+  const nvc_delta_prep& p = a.p;
+  const int lane = threadIdx.x & 31, n0 = blockIdx.x * TT;
+  int task = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int qk = p.kv_heads * p.dim, vw = p.heads * p.vdim, C = 2 * qk + vw;
+  const int t_qk = (2 * p.kv_heads + HP - 1) / HP, t_v = (vw + 127) / 128;
+  pdl_wait();
+  const int cnt = min(TT, min(a.N, p.cu_seqlens[p.B]) - n0);          // rows behind the last sequence are left alone
+  if (cnt <= 0) return;
+  if (task < t_qk + t_v) {
+    const bool head = task < t_qk;
+    const int hu = task * HP + lane / L, j = 4 * (lane % L), cv = 128 * (task - t_qk) + 4 * lane;
+    const bool on = head ? hu < 2 * p.kv_heads && j < p.dim : cv < vw;
+    const bool is_q = hu < p.kv_heads;
+    const int c = head ? hu * p.dim + j : 2 * qk + cv;                 // channel
+    const int col = head ? (is_q ? p.q_off + c : p.k_off + c - qk) : p.v_off + cv;
+    float4 y[TT];
+    conv_tile<TAPS, TT>(y, p.in + col, p.ldi, p.conv_state + c, C, p.conv_w + c, make_float4(0.f, 0.f, 0.f, 0.f), p.cu_seqlens, p.state_slots, p.positions, p.B,
+                        n0, cnt, on, lane);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) y[i] = silu4(y[i]);
+    if (!head) {
+#pragma unroll
+      for (int i = 0; i < TT; ++i)
+        if (on && i < cnt) *reinterpret_cast<float4*>(p.v_out + (int64_t)(n0 + i) * p.ldv + cv) = y[i];
+      return;
+    }
+    float ss[TT];
+#pragma unroll
+    for (int i = 0; i < TT; ++i) ss[i] = y[i].x * y[i].x + y[i].y * y[i].y + y[i].z * y[i].z + y[i].w * y[i].w;
+    int which;
+    bool writer;
+    const float sum = group_sum8(ss, L, lane & (L - 1), &which, &writer);
+    const float r = (is_q ? p.q_scale : 1.f) / sqrtf(sum + p.unit_eps);
+    float* out = is_q ? p.q_out + c : p.k_out + c - qk;
+    const int ld = is_q ? p.ldq : p.ldk;
+#pragma unroll
+    for (int i = 0; i < TT; ++i) {
+      const float f = __shfl_sync(0xffffffffu, r, (lane & ~(L - 1)) | (i & 4 ? L / 2 : 0) | (i & 2 ? L / 4 : 0) | (i & 1 ? L / 8 : 0));
+      if (on && i < cnt) *reinterpret_cast<float4*>(out + (int64_t)(n0 + i) * ld) = make_float4(y[i].x * f, y[i].y * f, y[i].z * f, y[i].w * f);
+    }
+    return;
+  }
+  task -= t_qk + t_v;
+  if (task == 0) {
+    // ---- decay and beta of every head
+    for (int e = lane; e < cnt * p.heads; e += 32) {
+      const int n = n0 + e / p.heads, h = e % p.heads;
+      const float* in = p.in + (int64_t)n * p.ldi;
+      float* gb = p.gb_out + ((int64_t)n * p.heads + h) * 2;
+      if (!p.channel_a) gb[0] = -expf(__ldg(p.A_log + h)) * softplus_f32(in[p.a_off + h] + __ldg(p.dt_bias + h));       // log of the decay
+      gb[1] = sigmoid_f32(in[p.b_off + h]);
+    }
+    return;
+  }
+  // ---- log decays of the heads' key channels
+  const int c = 128 * (task - 1) + 4 * lane;
+  if (!p.channel_a || c >= p.heads * p.dim) return;
+  const float na = -expf(__ldg(p.A_log + c / p.dim));
+  const float4 u = __ldg(reinterpret_cast<const float4*>(p.dt_bias + c));
+  float4 x[TT];
+#pragma unroll
+  for (int i = 0; i < TT; ++i) x[i] = i < cnt ? *reinterpret_cast<const float4*>(p.channel_a + (int64_t)(n0 + i) * p.ldca + c) : u;
+#pragma unroll
+  for (int i = 0; i < TT; ++i)
+    if (i < cnt)
+      *reinterpret_cast<float4*>(p.channel_g + (int64_t)(n0 + i) * p.heads * p.dim + c) =
+          make_float4(na * softplus_f32(x[i].x + u.x), na * softplus_f32(x[i].y + u.y), na * softplus_f32(x[i].z + u.z), na * softplus_f32(x[i].w + u.w));
+}
+
+template <int TAPS>
+cudaError_t launch_prep_tile(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) {
+  const nvc_delta_prep& p = a.p;
+  const int hp = p.dim <= 64 ? 2 : 1;
+  const int tasks = (2 * p.kv_heads + hp - 1) / hp + (p.heads * p.vdim + 127) / 128 + 1 + (p.channel_a ? (p.heads * p.dim + 127) / 128 : 0);
+  return nvc_launch(ctx, hp == 2 ? delta_prep_tile_kernel<TAPS, 16> : delta_prep_tile_kernel<TAPS, 32>, dim3((unsigned)((a.N + 7) / 8), (unsigned)((tasks + 3) / 4)),
+                    dim3(128), 0, st, a);
+}
 
 // The convolution state of a sequence after a portion: the last taps - 1 inputs of (what it held, this portion).  Slot i reads slot
 // i + len or the portion, never a slot below itself, so one thread per channel shifts in place.  The channels are spread over the
@@ -861,7 +950,7 @@ int check_prep(nvc_ctx* ctx, const nvc_delta_prep* p) {
 
 }  // namespace
 
-extern "C" int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int max_qlen, void* stream) {
+extern "C" int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int /*max_qlen*/, void* stream) {
   int rc = check_prep(ctx, p);
   if (rc) return rc;
   NVC_REQUIRE(ctx, p->cu_seqlens || N == p->B, NVC_EINVAL, "rows without cu_seqlens: one per sequence");
@@ -872,10 +961,17 @@ extern "C" int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, 
                   (!p->channel_a || (al16(p->channel_a) && al16(p->channel_g) && al16(p->dt_bias)));
   DeltaArgs a{*p, N, vec, nullptr, 0, nullptr};
   const int units = 2 * p->kv_heads + p->heads + 1 + (p->channel_a ? p->heads : 0);
-  const int longest = p->cu_seqlens ? std::min(N, std::max(max_qlen, 1)) : 1;
   NVC_REQUIRE(ctx, units <= 65535 && p->B <= 65535, NVC_ESHAPE, "more than 65 535 heads or sequences");
-  const int warps = longest >= 4 ? 4 : 1;
-  const dim3 grid((unsigned)((longest + warps - 1) / warps), units, p->B);
+  // portions of 4 tokens and more on average: shorter ones start a new history with nearly every row
+  if (p->cu_seqlens && vec && (!p->channel_a || p->ldca % 4 == 0) && p->dim <= 128 && p->taps <= 4 && N >= 4 * p->B) {
+    cudaStream_t st = nvc_stream(stream);
+    NVC_CUDA_CHECK(ctx, p->taps == 1 ? launch_prep_tile<1>(ctx, a, st) : (p->taps == 2 ? launch_prep_tile<2>(ctx, a, st)
+                                                                                       : (p->taps == 3 ? launch_prep_tile<3>(ctx, a, st) : launch_prep_tile<4>(ctx, a, st))));
+    ctx->launches++;
+    return NVC_OK;
+  }
+  const int warps = p->cu_seqlens ? 4 : 1;
+  const dim3 grid((unsigned)((N + warps - 1) / warps), units);
   auto* kernel = p->taps == 2 ? delta_prep_kernel<2> : (p->taps == 3 ? delta_prep_kernel<3> : (p->taps == 4 ? delta_prep_kernel<4> : delta_prep_kernel<0>));
   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, kernel, grid, dim3(32 * warps), 0, nvc_stream(stream), a));
   ctx->launches++;

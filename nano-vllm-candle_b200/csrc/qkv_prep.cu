@@ -106,7 +106,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
 
 // Heads of up to 4 L numbers: L lanes with four numbers each, 32 / L heads side by side, four of those per warp and all of one token, so that
 // four 16-byte loads per lane are in flight and the token's angles and the norm weights are read once for all of them.  A head never
-// leaves its lanes' registers: neighbouring pairs turn inside a lane, (i, i + rot_dims / 2) by exchange.  Bound by memory: MEASURED
+// leaves its lanes' registers: neighbouring pairs turn inside a lane, (i, i + rot_dims / 2) by exchange.  Bound by issue slots: 4 480 rows of 16 + 8 + 8 heads of 128 take 39 us (110 MB: 2.8 TB/s), one warp per
+// head with 4-byte accesses 81 us.
 template <typename TQ, typename TKV, int L>
 __global__ void __launch_bounds__(256) prep_heads_kernel(const PrepArgs a) {
   constexpr int U = 4, HP = 32 / L;

@@ -706,8 +706,7 @@ def delta_rule(ctx, x, offs, heads: int, kv_heads: int, dim: int, vdim: int, tap
                    _a(state_slots), _a(cu_seqlens), _a(positions), _a(A_log), _a(dt_bias), unit_eps, dim ** -0.5 if q_scale is None else q_scale,
                    _a(q), _a(k), _a(v), q.stride(0), k.stride(0), v.stride(0), _a(gb), state_slots.numel(), _a(channel_a),
                    channel_a.stride(0) if channel_a is not None else 0, _a(channel_g))
-    longest = int((cu_seqlens[1:] - cu_seqlens[:-1]).max().item()) if cu_seqlens is not None else 1
-    check(ctx.l.nvc_delta_prep_run(ctx.h, C.byref(p), N, longest, _stream()), "nvc_delta_prep_run", ctx.h)
+    check(ctx.l.nvc_delta_prep_run(ctx.h, C.byref(p), N, max(N, 1), _stream()), "nvc_delta_prep_run", ctx.h)
     check(ctx.l.nvc_delta_rule_scan(ctx.h, C.byref(p), _ptr(o), o.stride(0), _ptr(state), max_qlen, _stream()), "nvc_delta_rule_scan", ctx.h)
     return o, q, k, v, gb
 
