@@ -688,8 +688,14 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
                                 int K, const nvc_bf16* qw, const nvc_bf16* kw, float eps, const float* cos_sin,
                                 const int32_t* positions, const int32_t* slot_mapping, nvc_bf16* k_cache, nvc_bf16* v_cache,
                                 int nh, int kv, void* stream) {
-  // below ~8k rows the last wave's longer epilogue is exposed and the fusion loses (4 096 x 4 096 x 1 024: 48.3 vs 46.7 us)
-  if (M < 8192 || N != (nh + 2 * kv) * 128 || K % BK != 0) return NVC_ENOTIMPL;
+  if (N != (nh + 2 * kv) * 128 || K % BK != 0) return NVC_ENOTIMPL;
+  // The fusion saves a pass over the rows and lengthens the epilogue, of which all but the last wave's runs under the next tile's main loop.
+  // K >= 2 048: it wins from about 1 500 rows on (one call against two kernels: 1 500 x 6 144 x 4 096 57 / 63 us, 3 000 x 4 096 x 2 048 51 / 62,
+  // 4 096 x 6 144 x 4 096 167 / 191, 6 555 x 4 096 x 2 048 115 / 151; 1 000 rows 54 / 52).  Shorter k-loops hide less of it: below 8 192 rows it wins
+  // where the last wave is at least 2/5 full (6 555 x 4 096 x 1 024, 5.6 waves: 90 / 104; 5 500, 4.8: 65 / 70) and loses else (6 000, 5.2: 97 / 89;
+  // 3 500, 3.03: 62 / 58; 4 096, 3.5: even)
+  const int pairs = ctx->num_sms / 2, rem = ((M + 255) / 256) * ((N + 255) / 256) % pairs;
+  if (K >= 2048 ? M < 1500 : M < 8192 && (M < 4097 || 5 * rem < 2 * pairs)) return NVC_ENOTIMPL;
   int nt = 256, S = 1;
   choose_schedule(ctx, M, N, K / BK, &nt, &S);
   if (nt != 256 || S != 1) return NVC_ENOTIMPL;
