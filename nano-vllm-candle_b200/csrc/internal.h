@@ -21,6 +21,7 @@ int nvc_gemm_bf16_trace(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16
 // set max-dynamic-smem attributes of every kernel instantiation (called once per context)
 int nvc_gemm_init(nvc_ctx* ctx);
 int nvc_gemm_pair_init(nvc_ctx* ctx);
+int nvc_gemm_grouped_init(nvc_ctx* ctx);
 // CTA-pair (cta_group::2) GEMM for M > 128; force_splits 0 = choose the in-cluster split-K factor
 int nvc_gemm_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
                   int N, int K, int force_splits, int epi, void* stream, long long* trace);
