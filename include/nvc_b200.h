@@ -191,6 +191,9 @@ int nvc_gemm_bf16_act(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* 
  * their rows of C are written and mean nothing.  act: NVC_ACT_NONE or NVC_ACT_RELU2. */
 int nvc_gemm_bf16_grouped(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_dtype,
                           int M_cap, int Nout, int K, const int32_t* tile_group, int groups, int act, void* stream);
+/* The same; the rows of the tiles that are skipped become zeros. */
+int nvc_gemm_bf16_grouped_zero(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_dtype,
+                               int M_cap, int Nout, int K, const int32_t* tile_group, int groups, int act, void* stream);
 
 /* The same fused kernel with the tanh form of gelu on the gate (gated feed-forward of the Karuzen family):
  *   act[M, I] = gelu_tanh(A Wgate^T) * (A Wup^T),  gelu_tanh(z) = 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))),
@@ -379,6 +382,9 @@ int nvc_moe_sort_padded(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, i
  * where src_rows[r] < 0.  bf16 rows, width and strides multiples of 8. */
 int nvc_gather_rows_bf16(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out,
                          int ld_out, int rows_cap, int width, void* stream);
+/* The same; the rows from *num_rows to rows_cap are filled with `value`. */
+int nvc_gather_rows_bf16_fill(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out,
+                              int ld_out, int rows_cap, int width, nvc_bf16 value, void* stream);
 /* out[n, :H] = sum_t topk_w[n, t] * y[pos[n * top + t], :H] + gate[n] * shared[n, :H]   (fp32; shared / gate optional). */
 int nvc_moe_combine(nvc_ctx* ctx, const void* y, int y_dtype, int ldy, const int32_t* pos, const float* topk_w, int top,
                     const void* shared, int shared_dtype, int lds, const float* gate, float* out, int ldo, int N, int H,
@@ -547,6 +553,9 @@ int nvc_moe_route_logits_ex(nvc_ctx* ctx, const float* z, int ldz, const float* 
  * tile_group -1. */
 int nvc_moe_sort_padded_ex(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets,
                            int32_t* src_rows, int32_t* pos, int32_t* tile_group, int tiles_cap, void* stream);
+/* The same (align > 1, with a tile_group); src_rows is `tail` behind the last group, up to tiles_cap * align. */
+int nvc_moe_sort_padded_fill(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets,
+                             int32_t* src_rows, int32_t* pos, int32_t* tile_group, int tiles_cap, int tail, void* stream);
 /* nvc_moe_combine where the experts from E_real on are identity experts: a pair (n, t) with topk_idx[n, t] >= E_real contributes
  * topk_w[n, t] * x[n, :H] instead of a row of y. */
 int nvc_moe_combine_identity(nvc_ctx* ctx, const void* y, int y_dtype, int ldy, const int32_t* pos, const float* topk_w,

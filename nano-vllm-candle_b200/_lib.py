@@ -109,8 +109,10 @@ def _declare(l: C.CDLL) -> None:
         "nvc_moe_sort": [_vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp],
         "nvc_moe_sort_padded": [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp],
         "nvc_gather_rows_bf16": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _vp],
+        "nvc_gather_rows_bf16_fill": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, C.c_uint16, _vp],
         "nvc_gemm_bf16_act": [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
         "nvc_gemm_bf16_grouped": [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i, _i, _vp],
+        "nvc_gemm_bf16_grouped_zero": [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i, _i, _vp],
         "nvc_moe_combine": [_vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _i, _i, _i, _vp],
         "nvc_latent_attn_paged": [_vp, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _i, _i, _vp, _sz, _vp],
         "nvc_embed_gather_scaled_f32": [_vp, _vp, _vp, _i, _i, _f, _vp, _i, _i, _i, _vp],
@@ -133,6 +135,7 @@ def _declare(l: C.CDLL) -> None:
         "nvc_act_mul_p": [_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _vp],
         "nvc_moe_route_logits_ex": [_vp, _vp, _i, _vp, _i, _i, _f, _i, _i, _i, _vp, _vp, _vp, _i, _vp],
         "nvc_moe_sort_padded_ex": [_vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp],
+        "nvc_moe_sort_padded_fill": [_vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _vp],
         "nvc_moe_combine_identity": [_vp, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _vp],
         "nvc_delta_prep_run": [_vp, _vp, _i, _i, _vp],
         "nvc_delta_rule_scan": [_vp, _vp, _vp, _i, _vp, _i, _vp],

@@ -158,7 +158,7 @@ __global__ void moe_route_kernel(const T* __restrict__ h, int ldh, const float* 
 // 32).  Within an expert the pairs keep token order, so the layout - and every sum downstream - is deterministic.
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int32_t* __restrict__ idx, int P, int top, int E, int E_real, int align, int32_t* __restrict__ offsets,
-                int32_t* __restrict__ src_rows, int32_t* __restrict__ pos, int32_t* __restrict__ tile_group, int tiles_cap) {
+                int32_t* __restrict__ src_rows, int32_t* __restrict__ pos, int32_t* __restrict__ tile_group, int tiles_cap, int tail_cap, int tail) {
   extern __shared__ int32_t sm[];   // [32][E] counts -> starts, then [E + 1] offsets, then [E] sizes
   int32_t* cnt = sm;
   int32_t* off = sm + 32 * E;
@@ -192,6 +192,7 @@ moe_sort_kernel(const int32_t* __restrict__ idx, int P, int top, int E, int E_re
     }
     if (tile_group)
       for (int t = off[E] / align + threadIdx.x; t < tiles_cap; t += blockDim.x) tile_group[t] = -1;
+    for (int r = off[E] + threadIdx.x; r < tail_cap; r += blockDim.x) src_rows[r] = tail;       // behind the last group
   }
   for (int e = threadIdx.x; e < E; e += blockDim.x) {    // counts -> first position of (warp, expert)
     int a = off[e];
@@ -219,16 +220,21 @@ moe_sort_kernel(const int32_t* __restrict__ idx, int P, int top, int E, int E_re
   }
 }
 
-// out[r] = in[src_rows[r]] for r < *num_rows (a device count), zeros where src_rows[r] < 0; 16 bytes per thread
+// out[r] = in[src_rows[r]] for r < *num_rows (a device count), zeros where src_rows[r] < 0, `two` (a pair of bf16) behind them when fill is set;
+// 16 bytes per thread
 __global__ void gather_rows_kernel(const uint4* __restrict__ in, int ld_in, const int32_t* __restrict__ src_rows,
                                    const int32_t* __restrict__ num_rows, uint4* __restrict__ out, int ld_out, int rows_cap, int per_row,
-                                   int rows_per_cta) {
+                                   int rows_per_cta, int fill, uint32_t two) {
   pdl_trigger();
   pdl_wait();
   const int n = min(rows_cap, *num_rows);
   for (int i = threadIdx.x; i < rows_per_cta * per_row; i += blockDim.x) {
     const int r = blockIdx.x * rows_per_cta + i / per_row, c = i % per_row;
-    if (r >= n) break;
+    if (r >= n) {
+      if (!fill || r >= rows_cap) break;
+      out[(int64_t)r * ld_out + c] = make_uint4(two, two, two, two);
+      continue;
+    }
     const int src = src_rows[r];
     out[(int64_t)r * ld_out + c] = src >= 0 ? in[(int64_t)src * ld_in + c] : make_uint4(0u, 0u, 0u, 0u);
   }
@@ -354,21 +360,32 @@ int nvc_moe_sort_padded(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, i
   return nvc_moe_sort_padded_ex(ctx, topk_idx, N, top, E, E, align, offsets, src_rows, pos, tile_group, tiles_cap, stream);
 }
 
-int nvc_moe_sort_padded_ex(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets,
-                           int32_t* src_rows, int32_t* pos, int32_t* tile_group, int tiles_cap, void* stream) {
+static int sort_padded(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets, int32_t* src_rows, int32_t* pos,
+                       int32_t* tile_group, int tiles_cap, int tail_cap, int tail, void* stream) {
   NVC_REQUIRE(ctx, ctx && topk_idx && offsets && src_rows && pos, NVC_EINVAL, "null pointer");
   NVC_REQUIRE(ctx, E_real >= 0 && E_real <= E, NVC_EINVAL, "E_real must be in [0, E]");
   NVC_REQUIRE(ctx, N >= 0 && top > 0 && E > 0 && E <= 320 && align >= 1, NVC_EINVAL, "bad sizes");
   NVC_REQUIRE(ctx, !tile_group || (align > 1 && (int64_t)tiles_cap * align >= (int64_t)N * top + (int64_t)E * (align - 1)), NVC_EINVAL,
               "tile_group needs align > 1 and room for every group's padding");
   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, moe_sort_kernel, dim3(1), dim3(1024), (size_t)(34 * E + 1) * sizeof(int32_t), nvc_stream(stream),
-                                 topk_idx, N * top, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap));
+                                 topk_idx, N * top, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, tail_cap, tail));
   ctx->launches++;
   return NVC_OK;
 }
 
-int nvc_gather_rows_bf16(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out,
-                         int ld_out, int rows_cap, int width, void* stream) {
+int nvc_moe_sort_padded_ex(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets,
+                           int32_t* src_rows, int32_t* pos, int32_t* tile_group, int tiles_cap, void* stream) {
+  return sort_padded(ctx, topk_idx, N, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, 0, 0, stream);
+}
+
+int nvc_moe_sort_padded_fill(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, int E, int E_real, int align, int32_t* offsets,
+                             int32_t* src_rows, int32_t* pos, int32_t* tile_group, int tiles_cap, int tail, void* stream) {
+  NVC_REQUIRE(ctx, align > 1 && tile_group, NVC_EINVAL, "groups of rows and their table are wanted");
+  return sort_padded(ctx, topk_idx, N, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, tiles_cap * align, tail, stream);
+}
+
+static int gather(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out, int ld_out, int rows_cap, int width,
+                  int fill, nvc_bf16 value, void* stream) {
   NVC_REQUIRE(ctx, ctx && in && src_rows && num_rows && out, NVC_EINVAL, "null pointer");
   NVC_REQUIRE(ctx, rows_cap >= 0 && width > 0 && width % 8 == 0 && ld_in % 8 == 0 && ld_out % 8 == 0 && ld_in >= width && ld_out >= width,
               NVC_ESHAPE, "width and row strides must be multiples of 8");
@@ -378,9 +395,19 @@ int nvc_gather_rows_bf16(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int3
   const int rows_per_cta = std::max(1, 256 / per_row);
   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, gather_rows_kernel, dim3((rows_cap + rows_per_cta - 1) / rows_per_cta), dim3(256), 0, nvc_stream(stream),
                                  reinterpret_cast<const uint4*>(in), ld_in / 8, src_rows, num_rows, reinterpret_cast<uint4*>(out), ld_out / 8,
-                                 rows_cap, per_row, rows_per_cta));
+                                 rows_cap, per_row, rows_per_cta, fill, (uint32_t)value * 0x10001u));
   ctx->launches++;
   return NVC_OK;
+}
+
+int nvc_gather_rows_bf16(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out,
+                         int ld_out, int rows_cap, int width, void* stream) {
+  return gather(ctx, in, ld_in, src_rows, num_rows, out, ld_out, rows_cap, width, 0, 0, stream);
+}
+
+int nvc_gather_rows_bf16_fill(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* src_rows, const int32_t* num_rows, nvc_bf16* out,
+                              int ld_out, int rows_cap, int width, nvc_bf16 value, void* stream) {
+  return gather(ctx, in, ld_in, src_rows, num_rows, out, ld_out, rows_cap, width, 1, value, stream);
 }
 
 int nvc_moe_combine(nvc_ctx* ctx, const void* y, int y_dtype, int ldy, const int32_t* pos, const float* topk_w, int top,
