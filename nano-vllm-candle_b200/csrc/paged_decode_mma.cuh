@@ -16,6 +16,17 @@
 // kWarps = 4: 96 KB of rings, 2 CTAs per SM (296 resident).  kWarps = 2: 48 KB, 4 CTAs per SM (592
 // resident): the same bytes in flight per SM, but a grid of 297..592 CTAs (Qwen3-0.6B at batch 64:
 // 512) is resident at once instead of running 1.7 waves with a synchronised bubble between them.
+//
+// kTeams, for grids beyond the 4-warp residency without splits: what a unit (sequence, kv head, head chunk) costs follows its context length, which
+// only the device knows, so the kernel decides there.  A warp's ring covers about 15 GB/s whatever else the SM does, so among contexts of different
+// lengths the longest ones set the time.  When the longest exceeds 7/4 of the average, units are taken longest first, by teams of four warps where
+// two CTAs per SM hold a good part of them (kWarps = 4, fewer than 6 units per SM), by teams of two in larger grids (kWarps = 2), where the order alone
+// evens the ends out.  Otherwise teams of two, all resident at once, as without kTeams; one level lower (5/4) the ordered form loses at 64 contexts of
+// 300 - 600 (22.4 -> 27.1 us against 22.4 -> 22.9).  Up to 4 units per SM the grid is the 2 * SMs resident CTAs, and a CTA takes a second unit from the short
+// end: a grid of one CTA per unit, half of them without work, ends 1 us later.  8 kv heads, cold cache, a kernel between the calls, before -> after:
+//   64 contexts of 200 - 1 500: 49.2 -> 35.4 us (4.76 TB/s)     40 of 50 - 4 000: 111 -> 51.4        63 of 200 and one of 8 000: 176 -> 93
+//   128 of 200 - 1 500: 79.5 -> 65.6     256 of 100 - 3 000: 171 -> 140 (6.37 TB/s)      300 of 100 - 3 000: 192 -> 162      100 of 20 - 900: 33.8 -> 30.1
+//   64 of 513: 28.4 -> 28.1      64 of 1 000 - 1 400: 59.2 -> 58.7      256 of 1 024: 166.2 -> 167.7       64 of 30 - 350: 16.1 -> 16.8 (reading the lengths)
 #pragma once
 #include "common.cuh"
 
@@ -55,34 +66,117 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 }
 // group_total: query heads per kv head; gchunk: heads of the group handled by one CTA (<= 16).
 // num_splits > 1: every split parks its (m, l, o) partial in part_o / part_ml for paged_decode_combine_kernel.
-template <int kWarps>
+// kTeams: a one-dimensional grid, with a CTA per unit or two units per CTA; no splits.
+template <int kWarps, bool kTeams = false>
 __global__ void __launch_bounds__(kWarps * 32, kWarps == 4 ? 2 : 4)
 paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* __restrict__ k_cache,
                         const nvc_bf16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_blocks,
                         const int32_t* __restrict__ context_lens, int nh, int kv, int group_total, int gchunk,
                         int block_size, float scale_log2e, nvc_bf16* __restrict__ out, float* __restrict__ part_o,
-                        float* __restrict__ part_ml, int num_splits) {
-  constexpr int kThreads = kWarps * 32;
-  constexpr int kCtaTok = kWarps * kTileTok;          // tokens per CTA iteration
+                        float* __restrict__ part_ml, int num_splits, int B) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   // The dependency wait comes AFTER the first K / V tiles are in flight (see below): context_lens and
   // block_tables are step inputs (copied before the step's first kernel), and the only cache rows a
   // kernel of this step writes are the newest token's (position ctx_len - 1: K2 of this layer).
   const int chunks = (group_total + gchunk - 1) / gchunk;
-  const int kvh = blockIdx.x / chunks;
-  const int chunk = blockIdx.x - kvh * chunks;
+  const int lane = threadIdx.x & 31;
+  const int quad = lane >> 2, tq = lane & 3;          // accumulator row (quad, quad + 8), column pair tq
+  int team_warps = kWarps, team = 0, b = blockIdx.y, unit_c = blockIdx.x;
+  int blk_first, ctx_len, most = 0;
+  bool uneven = false;
+  const int KC = kv * chunks, units = KC * B;
+  const bool one_wave = kWarps > 2 && (int)gridDim.x < units;       // kTeams: two units per CTA at most
+  int u = blockIdx.x;
+  if constexpr (kTeams) {
+    int sum = 0;
+    // the first loads of the teams of two go out with the lengths: no second latency where these are equal
+    // (one wave: the second teams start where the first ones end, so that every SM gets its share)
+    team = threadIdx.x >> 6;
+    if (kWarps > 2) u = one_wave ? blockIdx.x + team * gridDim.x : 2 * blockIdx.x + team;
+    const int b2 = min(u / KC, B - 1);
+    blk_first = __ldg(block_tables + (int64_t)b2 * max_blocks);
+    ctx_len = __ldg(context_lens + b2);
+#pragma unroll 2
+    for (int i = lane; i < B; i += 32) {
+      const int x = max(__ldg(context_lens + i), 0);
+      sum += x;
+      most = max(most, x);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    most = __reduce_max_sync(0xffffffffu, most);
+    uneven = 4ll * B * most > 7ll * sum && most >= 128;       // below it all is start-up
+    team_warps = uneven ? kWarps : 2;
+    if (team_warps != 2) {
+      team = 0;
+      u = blockIdx.x;
+    }
+    if (u >= units) return;
+  }
+#pragma unroll 1
+  for (;;) {                                          // a unit; kTeams: the second one of the CTA, if it has one
+  if constexpr (kTeams) {
+    b = u / KC;
+    unit_c = u - b * KC;
+    if (uneven) {
+      // the sequence that `b` longer ones precede: counts of 128 levels of length (in the warp's own part of the ring, free so far; lane 0 has the
+      // four highest), their running sum, then the place among those of the level
+      int* const count = reinterpret_cast<int*>(smem + (threadIdx.x >> 5) * (kStages * kStageBytes));
+      const float f = 127.9f / (float)most;
+      auto place = [&](int i) { return i < B ? 127 - (int)((float)max(__ldg(context_lens + i), 0) * f) : -1; };
+      reinterpret_cast<int4*>(count)[lane] = make_int4(0, 0, 0, 0);
+      __syncwarp();
+#pragma unroll 1
+      for (int i = lane; i < B; i += 32) atomicAdd(count + place(i), 1);
+      __syncwarp();
+      const int4 c = reinterpret_cast<int4*>(count)[lane];
+      const int mine = c.x + c.y + c.z + c.w;
+      int before = mine;
+#pragma unroll
+      for (int w = 1; w < 32; w <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, before, w);
+        if (lane >= w) before += t;
+      }
+      before -= mine;
+      const int holder = __ffs(__ballot_sync(0xffffffffu, b >= before && b < before + mine)) - 1;
+      int level = 4 * lane, k = b - before;
+      if (k >= c.x) { k -= c.x; ++level;
+        if (k >= c.y) { k -= c.y; ++level;
+          if (k >= c.z) { k -= c.z; ++level; } } }
+      level = __shfl_sync(0xffffffffu, level, holder);
+      k = __shfl_sync(0xffffffffu, k, holder);
+#pragma unroll 1
+      for (int i = lane; i - lane < B; i += 32) {
+        const unsigned at = __ballot_sync(0xffffffffu, place(i) == level);
+        const int n = __popc(at);
+        if (k < n) {
+          b = i - lane + __fns(at, 0, k + 1);
+          break;
+        }
+        k -= n;
+      }
+    }
+  }
+  const int kThreads = 32 * team_warps, kCtaTok = team_warps * kTileTok;      // of the team; tokens per iteration
+  const int warp = (threadIdx.x >> 5) - (kTeams ? team * team_warps : 0), tid = threadIdx.x - (kTeams ? team * kThreads : 0);
+  uint8_t* const team_smem = smem + (kTeams ? team * team_warps * kStages * kStageBytes : 0);
+  auto team_sync = [&] {
+    if constexpr (kTeams) asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(kThreads) : "memory");
+    else __syncthreads();
+  };
+  const int kvh = unit_c / chunks;
+  const int chunk = unit_c - kvh * chunks;
   const int head0 = kvh * group_total + chunk * gchunk;
   const int G = min(gchunk, group_total - chunk * gchunk);
-  const int b = blockIdx.y, split = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int quad = lane >> 2, tq = lane & 3;          // accumulator row (quad, quad + 8), column pair tq
+  const int split = kTeams ? 0 : blockIdx.z;
 
   // independent first loads, issued together: the context length and the first block id (the block of this warp's
   // first tile whenever the CTA starts at tile 0) - one load latency instead of two before the first cp.async
   const int32_t* bt = block_tables + (int64_t)b * max_blocks;
-  const int blk_first = __ldg(bt);
-  const int ctx_len = __ldg(context_lens + b);
+  if (!kTeams || uneven) {
+    blk_first = __ldg(bt);
+    ctx_len = __ldg(context_lens + b);
+  }
   const int n_tiles = (ctx_len + kCtaTok - 1) / kCtaTok;
   const int tiles_per_split = (n_tiles + num_splits - 1) / num_splits;
   const int t_begin = split * tiles_per_split;
@@ -93,7 +187,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
   for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
-  const uint32_t ring = smem_u32(smem) + warp * (kStages * kStageBytes);
+  const uint32_t ring = smem_u32(team_smem) + warp * (kStages * kStageBytes);
   const int my_tiles = t_end - t_begin;                // CTA tiles; this warp's tile i covers tokens (t_begin+i)*kCtaTok + 16w
 
   // issue the loads of warp tile i into ring stage i % kStages (empty group if i is out of range); rows past the
@@ -244,10 +338,10 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
 
 
   // ---- merge the warps through shared memory (the rings are dead now)
-  __syncthreads();
-  float* sm_m = reinterpret_cast<float*>(smem);                    // [kWarps][16]
-  float* sm_l = sm_m + kWarps * 16;                                // [kWarps][16]
-  float* sm_o = sm_l + kWarps * 16;                                // [kWarps][16][128]
+  team_sync();
+  float* sm_m = reinterpret_cast<float*>(team_smem);                    // [warps][16]
+  float* sm_l = sm_m + team_warps * 16;                // [warps][16]
+  float* sm_o = sm_l + team_warps * 16;                // [warps][16][128]
   if (tq == 0) {
     sm_m[warp * 16 + quad] = m0;
     sm_m[warp * 16 + quad + 8] = m1;
@@ -262,16 +356,18 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
     r0[0] = o[nt][0]; r0[1] = o[nt][1];
     r1[0] = o[nt][2]; r1[1] = o[nt][3];
   }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < G * 128; idx += kThreads) {
+  team_sync();
+  for (int idx = tid; idx < G * 128; idx += kThreads) {
     const int g = idx >> 7, d = idx & 127;
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm_m[w * 16 + g]);
+    for (int w = 0; w < kWarps; ++w)
+      if (!kTeams || w < team_warps) M = fmaxf(M, sm_m[w * 16 + g]);
     float L = 0.f, O = 0.f;
     if (M != -INFINITY) {
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
+        if (kTeams && w >= team_warps) break;
         const float wt = fast_exp2(sm_m[w * 16 + g] - M);
         L += sm_l[w * 16 + g] * wt;
         O += sm_o[(w * 16 + g) * 128 + d] * wt;
@@ -286,6 +382,11 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
       __stcg(part_o + p * 128 + d, O);
       if (d == 0) { __stcg(part_ml + p * 2, M); __stcg(part_ml + p * 2 + 1, L); }
     }
+  }
+  if (!kTeams || !one_wave || team_warps == 2) break;
+  u = 2 * (int)gridDim.x - 1 - u;                     // the longest ones' CTAs take the shortest ones of the rest, or none
+  if (u >= units || u < (int)gridDim.x) break;
+  team_sync();                                        // the sums have been read
   }
 }
 
