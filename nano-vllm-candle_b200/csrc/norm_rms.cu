@@ -7,7 +7,7 @@
 //   nvc_head_gate                 per-head output stage of a mixer: optional division by the head's root mean square, times a
 //                                 sigmoid or silu gate, times a constant
 // Every kernel exists for bf16 and fp32 storage; arithmetic is fp32.
-#include "typed.cuh"
+#include "gate_rows.cuh"
 
 namespace {
 
@@ -367,6 +367,13 @@ int nvc_head_gate_w(nvc_ctx* ctx, const float* o, int ldo, const float* gate, in
   const int64_t units = (int64_t)N * heads;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const int vec = vdim % 4 == 0 && ldo % 4 == 0 && ldout % 4 == 0 && (!gate || ldg % 4 == 0) && al16(o) && al16(gate) && al16(weight) && al16(out);
+  if (vec && vdim <= 1024 && units < (1 << 30)) {
+    NVC_DISPATCH_DT(out_dtype, T,
+                    NVC_CUDA_CHECK(ctx, launch_gate_rows(ctx, nvc_stream(stream), o, ldo, gate, ldg, weight, 0, reinterpret_cast<T*>(out), ldout, heads, vdim, norm,
+                                                         0, eps, act, out_scale, N)));
+    ctx->launches++;
+    return NVC_OK;
+  }
   NVC_DISPATCH_DT(out_dtype, T,
                   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, head_gate_kernel<T>, dim3((unsigned)((units + 3) / 4)), dim3(128), 0,
                                                  nvc_stream(stream), o, ldo, gate, ldg, weight, reinterpret_cast<T*>(out), ldout, heads, vdim, norm,

@@ -1,0 +1,37 @@
+"""Output stage of a mixer in groups of columns: widths around the lanes' shares, grids under and over the point where a warp takes several units, and
+rows whose last units end inside a warp, against 64-bit arithmetic.  Bounds: a mean of up to 1 028 squares, a root, an exponential and three products
+in 32 bits stay below 3e-6 relative; bf16 results add their rounding, 2^-8."""
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+ops = importlib.import_module("nano-vllm-candle_b200.ops")
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,groups,size", [
+    (3, 3, 4), (3167, 3, 4), (5, 3, 60), (3161, 3, 64), (1, 1, 68), (3163, 3, 128), (9473, 1, 124), (7, 3, 132), (4741, 2, 256), (3, 5, 260),
+    (343, 3, 512), (341, 3, 512), (411, 10, 516), (1367, 3, 1024), (5, 3, 1024), (2, 2, 1028)])
+def test_gate_rows(ctx, rows, groups, size, dt):
+    g = torch.Generator(device=DEV).manual_seed(rows + size)
+    W = groups * size
+    o, z = (torch.randn(rows, W + 4, generator=g, device=DEV) for _ in range(2))
+    o, z = o[:, 4:] * 3, z[:, :W]
+    w = 1 + 0.2 * torch.randn(W, generator=g, device=DEV)
+    o64, z64, w64 = o.double().view(rows, groups, size), z.double().view(rows, groups, size), w.double().view(groups, size)
+    norm = lambda x: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6)  # noqa: E731
+    silu, sig = z64 * torch.sigmoid(z64), torch.sigmoid(z64)
+    head = lambda gate, n, act, s: ops.head_gate_w(ctx, o, gate, w[:size].contiguous(), groups, size, n, 1e-6, act, s, out_dtype=dt)  # noqa: E731
+    for got, want in [
+        (head(z, True, "silu", 0.6), norm(o64) * w64[0] * silu * 0.6),
+        (head(z, False, "sigmoid", 1.0), o64 * w64[0] * sig),
+        (head(None, True, "silu", 1.0), norm(o64) * w64[0]),
+        (ops.group_norm_gate(ctx, o, z, w, groups, size, True, 1e-6, "silu", out_dtype=dt), norm(o64 * silu) * w64),
+        (ops.group_norm_gate(ctx, o, z, w, groups, size, False, 1e-6, "sigmoid", out_dtype=dt), norm(o64) * w64 * sig),
+        (ops.group_norm_gate(ctx, o, None, None, groups, size, False, 1e-6, "silu", out_dtype=dt), norm(o64)),
+    ]:
+        err = ((got.double().view(want.shape) - want).abs() / (want.abs() + 1e-6)).max()
+        assert float(err) <= 3e-6 + (2 ** -8 if dt == torch.bfloat16 else 0), float(err)
