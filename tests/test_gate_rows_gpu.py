@@ -1,4 +1,4 @@
-"""Output stage of a mixer in groups of columns: widths around the lanes' shares, grids under and over the point where a warp takes several units, and
+"""Output stage of a mixer in groups of columns, and the units of a feed-forward layer: widths around the lanes' shares, grids under and over the point where a warp takes several units, and
 rows whose last units end inside a warp, against 64-bit arithmetic.  Bounds: a mean of up to 1 028 squares, a root, an exponential and three products
 in 32 bits stay below 3e-6 relative; bf16 results add their rounding, 2^-8."""
 import importlib
@@ -35,3 +35,26 @@ def test_gate_rows(ctx, rows, groups, size, dt):
     ]:
         err = ((got.double().view(want.shape) - want).abs() / (want.abs() + 1e-6)).max()
         assert float(err) <= 3e-6 + (2 ** -8 if dt == torch.bfloat16 else 0), float(err)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,F", [(4736, 8), (4737, 24), (4739, 264), (4738, 1536), (4741, 2056), (9001, 768)])
+@pytest.mark.parametrize("kind", [1, 2, 3, 4, 5])
+def test_units_of_many_rows(ctx, rows, F, kind, dt):
+    """Four rows per CTA: the numbers of one row per CTA, the last rows included, and a neighbour's buffer untouched."""
+    g = torch.Generator(device=DEV).manual_seed(rows + F)
+    x = (torch.randn(rows, 2 * F, generator=g, device=DEV) * 2).to(dt)
+    act = lambda t: ops.act_mul_p(ctx, t, F, F, kind, 3.0, 1.7)  # noqa: E731
+    got = act(x)
+    for lo, n in ((0, 9), (rows // 2, 5), (rows - 7, 7)):
+        assert torch.equal(got[lo:lo + n], act(x[lo:lo + n]))
+    a, b = x[:, :F].double(), x[:, F:].double()
+    if kind == 5:
+        want = a * torch.sigmoid(a) * b
+        assert float(((got.double() - want).abs() / (want.abs() + 1e-6)).max()) <= 3e-6 + (2 ** -8 if dt == torch.bfloat16 else 0)
+    if kind == 1:
+        want = torch.relu(a).square()
+        assert float(((got.double() - want).abs() / (want + 1e-6)).max()) <= 1e-6 + (2 ** -8 if dt == torch.bfloat16 else 0)
+        ops.check(ctx.l.nvc_act_mul(ctx.h, x.data_ptr(), 2 * F, x.data_ptr(), 2 * F, 0 if dt == torch.bfloat16 else 1, rows, F, F, kind,
+                                    torch.cuda.current_stream().cuda_stream), "nvc_act_mul", ctx.h)
+        assert torch.equal(x[:, :F], got) and torch.equal(x[:, F:].double(), b)
