@@ -245,7 +245,7 @@ int nvc_store_kvcache(nvc_ctx* ctx, const nvc_bf16* k, const nvc_bf16* v, int ld
  * fused qkv buffer); cu_seqlens: i32 [B+1] (device); sequence b owns rows
  * cu_seqlens[b]..cu_seqlens[b+1], positions 0..len (no cached prefix).
  * out: bf16 [N, nh*hd], head-major like the reference (:276-277).  GQA: q head h reads
- * kv head h / (nh/kv) (:236-256).  hd must be 128. */
+ * kv head h / (nh/kv) (:236-256).  hd must be 128, scale positive. */
 int nvc_prefill_attn_varlen(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* k, int ldk,
                             const nvc_bf16* v, int ldv, const int32_t* cu_seqlens, int B,
                             int total_tokens, int max_seqlen, int nh, int kv, int hd, float scale,
@@ -257,7 +257,8 @@ int nvc_prefill_attn_varlen(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_
  * context_lens[b] tokens whose K / V are read from the paged cache through block_tables
  * [B, bt_stride] (this step's k / v must already be stored there).  Causal: q row i sees keys
  * 0 .. context_lens[b] - q_len_b + i.  Cache rows past the context may hold anything (NaN included).
- * block_size in {16, 32, 64} or a multiple of 128. */
+ * block_size in {16, 32, 64} or a multiple of 128.  Here and in the forms below a scale that is not positive takes the
+ * kernels of nvc_attn_paged_wide. */
 int nvc_prefill_attn_paged(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* k_cache,
                            const nvc_bf16* v_cache, const int32_t* block_tables, int bt_stride,
                            const int32_t* context_lens, const int32_t* cu_seqlens_q, int B,

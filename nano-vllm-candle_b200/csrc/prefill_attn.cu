@@ -112,6 +112,7 @@ extern "C" int nvc_prefill_attn_varlen(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
               "pointers must be 16-byte aligned");
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
   if (B == 0 || total_tokens == 0 || max_seqlen == 0) return NVC_OK;
+  NVC_REQUIRE(ctx, scale > 0.f, NVC_EINVAL, "the scale must be positive");      // the kernel masks and takes maxima before it scales
   CUtensorMap tq, tk, tv;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_tokens, ldq);
   if (rc) return rc;
@@ -176,6 +177,11 @@ extern "C" int nvc_prefill_attn_paged_window(nvc_ctx* ctx, const nvc_bf16* q, in
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
   if (B == 0 || total_q_tokens == 0 || max_seqlen_q == 0) return NVC_OK;
   const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
+  if (!(scale > 0.f)) {                      // the kernel masks and takes maxima before it scales; the other one scales first
+    const nvc_attn_spec s{nh, kv, hd, hd, scale, window, sink, nullptr, 0, 1.f, 0.f, 0, 0, NVC_ATTN_SOFTMAX, nullptr, nullptr};
+    return nvc_attn_paged_wide(ctx, q, ldq, k_cache, kv * hd, v_cache, kv * hd, block_tables, bt_stride, context_lens, cu_seqlens_q, B, total_q_tokens, max_seqlen_q,
+                               block_size, &s, out, ldo, NVC_DT_BF16, stream);
+  }
   CUtensorMap tq, tk, tv;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_q_tokens, ldq);
   if (rc) return rc;
@@ -218,6 +224,9 @@ extern "C" int nvc_prefill_attn_shared(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
   if (B == 0 || total_q_tokens == 0 || max_seqlen_q == 0) return NVC_OK;
   const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
+  if (!sig && !(s.scale > 0.f))              // as above; sigmoid weights are made key by key and take any scale
+    return nvc_attn_paged_wide(ctx, q, ldq, cache, kv * 128, cache, kv * 128, block_tables, bt_stride, context_lens, cu_seqlens_q, B, total_q_tokens, max_seqlen_q,
+                               block_size, spec, out, ldo, NVC_DT_BF16, stream);
   CUtensorMap tq, tk;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_q_tokens, ldq);
   if (rc) return rc;
@@ -236,7 +245,8 @@ extern "C" int nvc_prefill_attn_shared(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
 }
 
 // Prompt portions of nvc_attn_paged_wide on the tcgen05 kernel: softmax over separate keys and values of 128 numbers per head with an optional
-// window, sink, gate and factor.  NVC_ENOTIMPL (nothing launched): a shape or a variant that the other kernels take.
+// window, sink, gate and factor.  NVC_ENOTIMPL (nothing launched): a shape or a variant that the other kernels take, and a scale that is not
+// positive: this kernel masks with -inf and takes the maximum of the plain scores, and multiplies afterwards.
 // The kernel works on tiles of 128 rows of one sequence and head, the mma.sync one on 64 rows of a key head's query heads: with portions
 // of few tokens most of a tile is empty, so portions of 64 tokens and batches of 32 rows per sequence are where it starts.  16 heads over 8, with
 // gate and sink, against the mma.sync kernel: 1 x 64 rows 20 / 20 us, behind 3 000 tokens 58 / 250; 64 x 64 rows 37 / 86, behind 3 000 270 / 1 069;
@@ -245,7 +255,7 @@ int nvc_prefill_attn_gated(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_b
                            const int32_t* block_tables, int bt_stride, const int32_t* context_lens, const int32_t* cu_seqlens_q, int B, int rows, int max_qlen,
                            int block_size, const nvc_attn_spec& s, nvc_bf16* out, int ldo, void* stream) {
   auto al16 = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
-  if (!cu_seqlens_q || max_qlen < 64 || rows < 32 * B || s.dim != 128 || s.vdim != 128 || s.weights != NVC_ATTN_SOFTMAX || s.chunk || s.softcap != 0.f || s.gate_per_head ||
+  if (!cu_seqlens_q || !(s.scale > 0.f) || max_qlen < 64 || rows < 32 * B || s.dim != 128 || s.vdim != 128 || s.weights != NVC_ATTN_SOFTMAX || s.chunk || s.softcap != 0.f || s.gate_per_head ||
       s.key_scale || k_cache == v_cache || !(block_size >= 16 && (block_size >= 128 ? block_size % 128 == 0 : 128 % block_size == 0)) ||
       ((ldq | ldk | ldv | ldo) & 7) || (s.gate && ((s.ldg & 3) || !al16(s.gate))) || !al16(q) || !al16(k_cache) || !al16(v_cache) || !al16(out) || !ctx->encode_tiled)
     return NVC_ENOTIMPL;

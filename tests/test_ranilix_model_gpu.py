@@ -281,6 +281,19 @@ def test_long_portions_of_the_causal_half_beside_decoded_tokens(monkeypatch, fla
         r.close()
 
 
+def test_long_portions_with_a_negative_scale():
+    """A causal half whose keys of 128 numbers are met with a negative scale: the tcgen05 attention cannot take it."""
+    cfg = cfg_d()
+    for layer in cfg["layers"]:
+        mix = layer["mixer"].get("left", layer["mixer"])
+        mix["scale"] = -mix["scale"]
+    r = Rig(cfg, "bfloat16", blocks=32, seed=12)
+    try:
+        r.check({"w": toks(200, r.cfg["vocab"], 64)}, [[("w", 9)], [("w", 130)], [("w", 61)]])
+    finally:
+        r.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("gap", [11, 12, 13])
 def test_one_token_before_and_after_the_window_edge(dtype, gap):

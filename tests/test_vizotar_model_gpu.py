@@ -275,6 +275,19 @@ def test_sizes_of_the_tensor_pipe_routes(monkeypatch, dtype, tc):
         r.close()
 
 
+def test_long_portions_with_a_negative_scale():
+    """Attention whose keys of 128 numbers are met with a negative scale: the tcgen05 attention cannot take it."""
+    cfg = cfg_c(all_experts=True)
+    for layer in cfg["layers"]:
+        if "left" in layer["mixer"]:
+            layer["mixer"]["left"]["scale"] *= -1.0
+    r = Rig(cfg, "bfloat16", blocks=32, seed=12)
+    try:
+        r.check({"w": toks(200, r.cfg["vocab"], 64)}, [[("w", 9)], [("w", 130)], [("w", 61)]])
+    finally:
+        r.close()
+
+
 def sharp_window_model(window, seed=30, special=50, dim=16, vdim=32):
     """One parallel layer whose attention head 0 scores the token `special` far above every other key, and whose memory half is switched
     off (its closing norm weight is zero), so that the token reaches later positions through attention ONLY: the embedding gives that
