@@ -50,6 +50,9 @@ struct Cfg {
   static_assert(kStages >= 2, "need at least a double buffer");
 };
 
+// the tiles the choice may take have the extended variant; those of 16 and 96 columns are reached by force_bn only
+constexpr bool has_ext(int bn) { return bn != 16 && bn != 96; }
+
 __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
   int old;
   asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
@@ -57,7 +60,7 @@ __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
 }
 
 // kExt: the variant with the element-wise and the clamped epilogues; the plain variant compiles them out
-template <int BN, int KPS, int CL, bool kExt = false>
+template <int BN, int KPS, bool kExt = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                          void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total,
@@ -88,10 +91,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   const int kb_end = min(k_blocks_total, kb_begin + k_blocks_per_split);
   const int num_kb = kb_end - kb_begin;
   const int num_it = (num_kb + KPS - 1) / KPS;       // pipeline iterations (stages consumed)
-  // CL > 1: the CL CTAs of a cluster work on CL adjacent n-tiles of the same m-tile / k-range and share
-  // the activation tile: each loads 1/CL of its rows and multicasts them to all (a_box_rows = rows per CTA)
-  const uint32_t cta_rank = CL > 1 ? ptx::cluster_ctarank() : 0u;
-  constexpr uint16_t kMask = (uint16_t)((1u << CL) - 1u);
 
   if (warp == 0 && lane == 0) {
     ptx::tma_prefetch_desc(&tma_a);
@@ -101,7 +100,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     if (lane == 0) {
       for (int s = 0; s < cfg::kStages; ++s) {
         ptx::mbar_init(full_bar(s), 2);   // two producers: warp 0 (A sub-tiles) and warp 2 (W sub-tiles)
-        ptx::mbar_init(empty_bar(s), CL);   // released by the MMA warps of all CTAs that received the multicast
+        ptx::mbar_init(empty_bar(s), 1);
       }
       ptx::mbar_init(tmem_full_bar, 1);
       ptx::fence_barrier_init();
@@ -114,7 +113,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
-  if (CL > 1) ptx::cluster_sync_all();   // peers' barriers are initialised before anyone multicasts into them
   // Weights are never written by a kernel, so their first kPrefetchKb k-blocks are pulled into L2
   // BEFORE the dependency wait (overlapping the predecessor), and the producer keeps prefetching
   // that far ahead of its shared-memory ring: a CTA's ring (~190 KB) covers only ~60 B/clk at HBM
@@ -144,12 +142,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   if (warp == 0 || warp == 2) {
     // ------------------------------------------------------------ TMA producers
     const bool is_a = warp == 0;
-    // bytes ONE box delivers into this CTA per k-block (A: all CL slices land here)
-    const uint32_t sub_bytes = is_a ? (uint32_t)a_box_rows * CL * (BK * 2) : (uint32_t)cfg::kBytesB;
+    // bytes ONE box delivers per k-block
+    const uint32_t sub_bytes = is_a ? (uint32_t)a_box_rows * (BK * 2) : (uint32_t)cfg::kBytesB;
     const uint32_t sub_stride = is_a ? (uint32_t)cfg::kBytesA : (uint32_t)cfg::kBytesB;
     const CUtensorMap* map = is_a ? &tma_a : &tma_b;
-    const int row0 = is_a ? m_tile * BM + (int)cta_rank * a_box_rows : n_tile * BN;
-    const uint32_t off = is_a ? cta_rank * (uint32_t)a_box_rows * (BK * 2) : (uint32_t)(KPS * cfg::kBytesA);
+    const int row0 = is_a ? m_tile * BM : n_tile * BN;
+    const uint32_t off = is_a ? 0u : (uint32_t)(KPS * cfg::kBytesA);
     for (int it = is_a ? 0 : w_pre; it < num_it; ++it) {
       const int s = it % cfg::kStages;
       if (it >= cfg::kStages) ptx::mbar_wait(empty_bar(s), ((it / cfg::kStages) & 1) ^ 1u);   // first lap: slots are free
@@ -159,12 +157,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         const uint32_t dst = smem_base + s * cfg::kStageBytes + off;
         const int k0 = (kb_begin + it * KPS) * BK;
 #pragma unroll
-        for (int j = 0; j < KPS; ++j) {
-          if (j < nsub) {
-            if (CL > 1 && is_a) ptx::tma_load_2d_mcast(dst + j * sub_stride, map, full_bar(s), k0 + j * BK, row0, kMask);
-            else ptx::tma_load_2d(dst + j * sub_stride, map, full_bar(s), k0 + j * BK, row0);
-          }
-        }
+        for (int j = 0; j < KPS; ++j)
+          if (j < nsub) ptx::tma_load_2d(dst + j * sub_stride, map, full_bar(s), k0 + j * BK, row0);
         if (!is_a && prefetch_w) {       // stay kPrefetchKb k-blocks ahead in L2
 #pragma unroll
           for (int j = 0; j < KPS; ++j) {
@@ -203,8 +197,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
             }
           }
         }
-        if (CL > 1) ptx::umma_commit_mcast(empty_bar(s), kMask);   // every CTA of the cluster wrote into this stage
-        else ptx::umma_commit(empty_bar(s));       // stage reusable once these MMAs have read it
+        ptx::umma_commit(empty_bar(s));            // stage reusable once these MMAs have read it
         if (it == num_it - 1) {
           ptx::umma_commit(tmem_full_bar);    // accumulator complete
           if (tr) trace[80] = clock64();
@@ -377,7 +370,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     }
   }
   __syncthreads();
-  if (CL > 1 || ks_cluster) ptx::cluster_sync_all();   // nobody exits while a peer may still arrive on its barriers / read its smem
+  if (ks_cluster) ptx::cluster_sync_all();   // nobody exits while a peer may still read its smem
   if (warp == 1) {
     ptx::tcgen05_fence_after();
     ptx::tmem_dealloc(tmem_base, cfg::kTmemCols);
@@ -401,15 +394,14 @@ int make_tma_2d(nvc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t inner
   return NVC_OK;
 }
 
-template <int BN, int KPS, int CL>
+template <int BN, int KPS>
 int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
            int N, int K, int splits, int ks_cluster, int epi, cudaStream_t stream, long long* trace) {
   using cfg = Cfg<BN, KPS>;
   CUtensorMap ta, tb;
-  // a single partial m-tile only needs the rows that exist (rounded to the 8-row swizzle atom per
-  // cluster CTA); each CTA of a cluster loads a_rows / CL of them
-  const int a_rows = M >= BM ? BM : ((M + 8 * CL - 1) / (8 * CL)) * (8 * CL);
-  int rc = make_tma_2d(ctx, &ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, a_rows / CL);
+  // a single partial m-tile only needs the rows that exist (rounded to the 8-row swizzle atom)
+  const int a_rows = M >= BM ? BM : (M + 7) / 8 * 8;
+  int rc = make_tma_2d(ctx, &ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, a_rows);
   if (rc) return rc;
   rc = make_tma_2d(ctx, &tb, W, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN);
   if (rc) return rc;
@@ -417,20 +409,17 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   const int kb_per = (kb_total + splits - 1) / splits;
   const int eff_splits = (kb_total + kb_per - 1) / kb_per;   // no empty splits
   const int n_tiles = (N + BN - 1) / BN;
-  NVC_REQUIRE(ctx, n_tiles % CL == 0, NVC_ESHAPE, "n-tiles must divide by the cluster size");
   dim3 grid(n_tiles, (M + BM - 1) / BM, eff_splits);
   // ks_cluster: the eff_splits CTAs of one output tile form a cluster (1,1,S) and reduce over DSMEM
-  const int ks = (ks_cluster && CL == 1 && eff_splits > 1 && eff_splits <= 8) ? 1 : 0;
+  const int ks = (ks_cluster && eff_splits > 1 && eff_splits <= 8) ? 1 : 0;
   NVC_REQUIRE(ctx, !ks || (size_t)BN * BM * 4 <= (size_t)cfg::kStages * cfg::kStageBytes, NVC_EINVAL, "ring too small for the partial tile");
-  // the extended variant exists for CL = 1 (the element-wise and the clamped epilogues never use clusters)
-  constexpr bool kHasExt = CL == 1;
   const bool ext = nvc_epi_unary(epi) || nvc_epi_glu_clamp(epi);
-  NVC_REQUIRE(ctx, !ext || kHasExt, NVC_EINVAL, "products with an element-wise epilogue need a cluster size of 1");
-  auto kernel = gemm_bf16_tcgen05_kernel<BN, KPS, CL, false>;
-  if constexpr (kHasExt) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, CL, true>; }
+  NVC_REQUIRE(ctx, !ext || has_ext(BN), NVC_EINVAL, "no element-wise epilogue on this tile");
+  auto kernel = gemm_bf16_tcgen05_kernel<BN, KPS, false>;
+  if constexpr (has_ext(BN)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true>; }
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
-                                          stream, dim3(CL, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
-                                          kb_per, a_rows / CL,
+                                          stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
+                                          kb_per, a_rows,
                                           // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring:
                                           // helps the short, latency-bound k-loops of decode (K <= 3072: 5.1 vs 5.7 us), costs
                                           // 2 - 8 % on the long ones (K 12288 at M 64: 23.2 -> 21.6 us without it) and at M >= 256
@@ -442,11 +431,8 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 }
 
 // (BN, KPS) instantiations.  KPS > 1 (several k-blocks per mbarrier round trip) is for short,
-// latency-bound CTAs (decode); KPS = 1 keeps the deepest ring for long compute-bound k-loops.
-// CL > 1: cluster of CL CTAs along N sharing the activation tile through TMA multicast (decode).
-#define NVC_GEMM_CONFIGS(X)                                                                          \
-  X(256, 1, 1) X(128, 1, 1) X(128, 2, 1) X(64, 2, 1) X(64, 4, 1) X(32, 4, 1)                       \
-  X(16, 4, 8) X(16, 4, 4) X(32, 4, 4) X(32, 4, 8) X(64, 4, 4) X(64, 2, 4) X(96, 2, 4) X(128, 2, 4) X(128, 1, 4) X(256, 1, 2)
+// latency-bound CTAs (decode); KPS = 1 keeps the deepest ring for long compute-bound k-loops.  The last two are reached by force_bn only.
+#define NVC_GEMM_CONFIGS(X) X(256, 1) X(128, 1) X(128, 2) X(64, 2) X(64, 4) X(32, 4) X(16, 4) X(96, 2)
 
 // Tile choice, fitted to tools/gemm_microbench.py (CUDA-graph timing + CTA phase traces) on B200:
 //  * a CTA ingests ~60 B/clk through TMA when the operands stream from HBM, so a k-block costs
@@ -456,9 +442,8 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 //    k-blocks per pipeline stage; split-K through the L2 workspace costs >= 6 us (ticket atomic +
 //    reduction round trips) and never won in the sweep, so it is only used when forced.
 void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, int* bn_out, int* kps_out, int* splits_out,
-                   int* cl_out, int* ks_out) {
+                   int* ks_out) {
   *splits_out = 1;
-  *cl_out = 1;
   *ks_out = 0;
   if (M <= BM) {
     // Decode (one m-tile).  Cycle model fitted to CTA phase traces (tools/gemm_microbench.py --trace-decode):
@@ -519,11 +504,11 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
 }  // namespace
 
 extern "C" int nvc_gemm_init(nvc_ctx* ctx) {
-#define X(BN, KPS, CL)                                                                                                   \
-  NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, CL, false>,                                 \
+#define X(BN, KPS)                                                                                                       \
+  NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, false>,                                     \
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS>::kSmemBytes));      \
-  if (CL == 1)                                                                                                           \
-    NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, 1, true>,                                 \
+  if constexpr (has_ext(BN))                                                                                             \
+    NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, true>,                                    \
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS>::kSmemBytes));
   NVC_GEMM_CONFIGS(X)
 #undef X
@@ -576,27 +561,24 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   }
   if (force_bn == 512 || vocab_pair || (force_bn == 0 && M > BM && g_nvc_gemm_pair))
     return nvc_gemm_pair(ctx, A, lda, W, C, ldc, out_dtype == NVC_DT_F32, M, Nout, K, force_splits, epi, stream, trace);
-  int bn, kps, splits, cl = 1, ks = 0;
-  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, &bn, &kps, &splits, &cl, &ks);
-  if (force_bn) {          // force_bn = BN + 1000 * KPS + 10000 * CL (KPS 0: the first instantiation of that BN)
+  int bn, kps, splits, ks = 0;
+  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, &bn, &kps, &splits, &ks);
+  if (force_bn) {          // force_bn = BN + 1000 * KPS (KPS 0: the first instantiation of that BN); a digit in front of KPS has no meaning
     bn = force_bn % 1000;
     kps = (force_bn / 1000) % 10;
-    cl = force_bn / 10000;
-    if (cl == 0) cl = 1;
     if (kps == 0) kps = bn >= 128 ? 1 : (bn == 64 ? 2 : 4);
     ks = 0;
     splits = 1;
   }
   // force_splits: 1..99 = split-K through the global workspace; 100 + S = split-K inside a cluster (1,1,S), S <= 8
-  if (force_splits >= 100) { splits = force_splits - 100; ks = 1; cl = 1; }
+  if (force_splits >= 100) { splits = force_splits - 100; ks = 1; }
   else if (force_splits) { splits = force_splits; ks = 0; }
   NVC_REQUIRE(ctx, !ks || splits <= 8, NVC_EINVAL, "cluster split-K supports at most 8 splits");
   if (epi != NVC_EPI_NONE) {       // the fused epilogue lives in the direct-store path: no split-K, tiles of >= 32 columns
     NVC_REQUIRE(ctx, force_splits == 0 || force_splits == 1, NVC_EINVAL, "fused epilogue cannot be combined with split-K");
     splits = 1;
     ks = 0;
-    if (bn < 32) { bn = 32; kps = 4; cl = 1; }
-    if (nvc_epi_unary(epi) || nvc_epi_glu_clamp(epi)) cl = 1;          // (every (bn, kps) the choice returns has a CL = 1 instantiation)
+    if (bn < 32) { bn = 32; kps = 4; }
   }
   if (splits > K / BK) splits = K / BK;
   const int tiles = ((M + BM - 1) / BM) * ((Nout + bn - 1) / bn);
@@ -606,8 +588,8 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   }
   cudaStream_t st = nvc_stream(stream);
   const int f32 = out_dtype == NVC_DT_F32;
-#define X(BN, KPS, CL) \
-  if (bn == BN && kps == KPS && cl == CL) return launch<BN, KPS, CL>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
+#define X(BN, KPS) \
+  if (bn == BN && kps == KPS) return launch<BN, KPS>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
   NVC_GEMM_CONFIGS(X)
 #undef X
   NVC_REQUIRE(ctx, false, NVC_EINVAL, "unsupported tile configuration");
