@@ -141,6 +141,13 @@ extern "C" int nvc_attn_paged_wide(nvc_ctx* ctx, const void* q, int ldq, const v
                                    const int32_t* block_tables, int bt_stride, const int32_t* context_lens, const int32_t* cu_seqlens,
                                    int B, int rows, int max_qlen, int block_size, const nvc_attn_spec* spec, void* out, int ldo, int dtype,
                                    void* stream) {
+  return nvc_attn_paged_wide_on(ctx, q, ldq, k_cache, ldk, v_cache, ldv, block_tables, bt_stride, context_lens, cu_seqlens, B, rows, max_qlen, block_size, spec, out,
+                                ldo, dtype, stream, true);
+}
+
+int nvc_attn_paged_wide_on(nvc_ctx* ctx, const void* q, int ldq, const void* k_cache, int ldk, const void* v_cache, int ldv, const int32_t* block_tables, int bt_stride,
+                           const int32_t* context_lens, const int32_t* cu_seqlens, int B, int rows, int max_qlen, int block_size, const nvc_attn_spec* spec, void* out,
+                           int ldo, int dtype, void* stream, bool tcgen05) {
   NVC_REQUIRE(ctx, ctx && q && k_cache && v_cache && block_tables && context_lens && spec && out, NVC_EINVAL, "null pointer");
   const nvc_attn_spec& s = *spec;
   NVC_REQUIRE(ctx, B > 0 && rows >= B && block_size > 0 && bt_stride > 0 && max_qlen >= 1, NVC_EINVAL, "bad sizes");
@@ -155,9 +162,10 @@ extern "C" int nvc_attn_paged_wide(nvc_ctx* ctx, const void* q, int ldq, const v
               "bad strides");
   WideArgs a{q, k_cache, v_cache, out, ldq, ldk, ldv, ldo, block_tables, context_lens, cu_seqlens, bt_stride, B, block_size, s};
   if (dtype == NVC_DT_BF16 && attn_wide_mma_takes(s, ldq, ldk, ldv, ldo, block_size)) {
-    int rc = nvc_prefill_attn_gated(ctx, reinterpret_cast<const nvc_bf16*>(q), ldq, reinterpret_cast<const nvc_bf16*>(k_cache), ldk,
-                                          reinterpret_cast<const nvc_bf16*>(v_cache), ldv, block_tables, bt_stride, context_lens, cu_seqlens, B, rows, max_qlen,
-                                          block_size, s, reinterpret_cast<nvc_bf16*>(out), ldo, stream);
+    int rc = !tcgen05 ? NVC_ENOTIMPL
+                      : nvc_prefill_attn_gated(ctx, reinterpret_cast<const nvc_bf16*>(q), ldq, reinterpret_cast<const nvc_bf16*>(k_cache), ldk,
+                                               reinterpret_cast<const nvc_bf16*>(v_cache), ldv, block_tables, bt_stride, context_lens, cu_seqlens, B, rows, max_qlen,
+                                               block_size, s, reinterpret_cast<nvc_bf16*>(out), ldo, stream);
     if (rc != NVC_ENOTIMPL) return rc;
     rc = attn_wide_mma_launch(ctx, a.q, a.k_cache, a.v_cache, a.out, ldq, ldk, ldv, ldo, block_tables, context_lens, cu_seqlens, bt_stride,
                                   B, rows, max_qlen, block_size, s, nvc_stream(stream));

@@ -35,6 +35,10 @@ int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
 int nvc_prefill_attn_init(nvc_ctx* ctx);
 int nvc_paged_decode_init(nvc_ctx* ctx);
 }
+// nvc_attn_paged_wide with its tcgen05 route for prompt portions on or off (the switch of a model's body)
+int nvc_attn_paged_wide_on(nvc_ctx* ctx, const void* q, int ldq, const void* k_cache, int ldk, const void* v_cache, int ldv, const int32_t* block_tables, int bt_stride,
+                           const int32_t* context_lens, const int32_t* cu_seqlens, int B, int rows, int max_qlen, int block_size, const nvc_attn_spec* spec, void* out,
+                           int ldo, int dtype, void* stream, bool tcgen05);
 // prompt portions of nvc_attn_paged_wide on the tcgen05 kernel, or NVC_ENOTIMPL (nothing launched)
 int nvc_prefill_attn_gated(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* k_cache, int ldk, const nvc_bf16* v_cache, int ldv,
                            const int32_t* block_tables, int bt_stride, const int32_t* context_lens, const int32_t* cu_seqlens_q, int B, int rows, int max_qlen,

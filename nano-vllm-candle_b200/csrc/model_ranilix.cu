@@ -327,8 +327,8 @@ struct RanilixBody : nvc_body_base {
                                      nd ? r->d_cu2 : r->d_cu, s.B - nd, s.N - nd, s.max_chunk, a.heads, a.kv_heads, a.dim, bs,
                                      r->opt.num_kvcache_blocks, a.scale, ob + (size_t)nd * w.ow, w.ow, r->stream);
     } else {
-      rc = nvc_attn_paged_wide(ctx, q, p.ldq, w.k_cache, p.ldk, w.v_cache, p.ldv, r->d_bt, cap, r->d_ctx, s.decode ? nullptr : r->d_cu, s.B,
-                               s.N, s.decode ? 1 : s.max_seqlen, bs, &sp, ao, w.ow, dt, r->stream);
+      rc = nvc_attn_paged_wide_on(ctx, q, p.ldq, w.k_cache, p.ldk, w.v_cache, p.ldv, r->d_bt, cap, r->d_ctx, s.decode ? nullptr : r->d_cu, s.B,
+                                  s.N, s.decode ? 1 : s.max_seqlen, bs, &sp, ao, w.ow, dt, r->stream, use_flash);
     }
     mark(r, "attention");
     return rc;

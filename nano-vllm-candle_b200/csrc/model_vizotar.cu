@@ -457,8 +457,8 @@ struct VizotarBody : nvc_body_base {
                                          nd ? r->d_cu2 : r->d_cu, s.B - nd, s.N - nd, s.max_chunk, a.heads, a.kv_heads, 128, bs,
                                          r->opt.num_kvcache_blocks, a.scale, a.window, w.sink, reinterpret_cast<nvc_bf16*>(ao) + (size_t)nd * w.owp, w.owp, st);
     } else {
-      rc = nvc_attn_paged_wide(ctx, q, p.ldq, rs.k_cache, p.ldk, rs.v_cache, p.ldv, r->d_bt, cap, r->d_ctx, s.decode ? nullptr : r->d_cu, s.B, s.N,
-                               s.decode ? 1 : s.max_seqlen, bs, &sp, ao, w.owp, dt, st);
+      rc = nvc_attn_paged_wide_on(ctx, q, p.ldq, rs.k_cache, p.ldk, rs.v_cache, p.ldv, r->d_bt, cap, r->d_ctx, s.decode ? nullptr : r->d_cu, s.B, s.N,
+                                  s.decode ? 1 : s.max_seqlen, bs, &sp, ao, w.owp, dt, st, use_flash);
     }
     mark(r, "attention");
     return rc;

@@ -281,6 +281,22 @@ def test_long_portions_of_the_causal_half_beside_decoded_tokens(monkeypatch, fla
         r.close()
 
 
+def test_the_switch_keeps_portions_off_tcgen05(monkeypatch):
+    """Portions behind a window, keys and values of 128 numbers: the two settings of the switch are two kernels with sums in another order,
+    so some of 140 x 180 logits differ in their last bits."""
+    cfg = R.make_config(vocab=180, width=192, layers=[R.with_mlp(R.attention_cfg(2, 1, 128, 128, window=70, rot_dims=64, scale=0.1), 128)])
+    got = []
+    for flash in ("1", "0"):
+        monkeypatch.setenv("NVC_RANILIX_FLASH", flash)
+        r = Rig(cfg, "bfloat16", blocks=24, seed=12)
+        try:
+            r.check({"w": toks(140, 180, 64)}, [[("w", 140)]])
+            got.append(r.replay({"w": toks(140, 180, 64)}, [[("w", 140)]])["w"])
+        finally:
+            r.close()
+    assert not np.array_equal(*got)
+
+
 def test_long_portions_with_a_negative_scale():
     """A causal half whose keys of 128 numbers are met with a negative scale: the tcgen05 attention cannot take it."""
     cfg = cfg_d()
