@@ -654,7 +654,7 @@ int run_scan(nvc_ctx* ctx, const RetArgs& a, int B, int max_qlen, void* stream) 
     // the tensor pipe keeps 16 columns x all channels of the state in a warp's registers, which is what ends it at 128 channels; at 128 x 64
     // over eight prompts of 245 to 1 050 tokens, 32 heads: 168 us, the FMA form 640
     if constexpr (MODE != kMemory) {
-      if (dim <= 128) {
+      if (dim <= 128 && B <= 65535) {            // sequences lie along the grid's second dimension there
         ce = dim <= 64 ? launch_decay_mma<4, MODE>(ctx, a, B, nvc_stream(stream)) : launch_decay_mma<8, MODE>(ctx, a, B, nvc_stream(stream));
         NVC_CUDA_CHECK(ctx, ce);
         ctx->launches++;

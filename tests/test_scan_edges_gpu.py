@@ -89,3 +89,20 @@ def test_delta_rule_edges(ctx, ops, dim, vdim, which):
                 assert close(o[t].view(H, vdim), torch.einsum("hdv,hd->hv", S, q[t])), (b, t)
         assert close(state[slots[b]], S), b
         assert torch.equal(cs[slots[b]][0], x[int(cu[b + 1]) - 1, :C]), b
+
+
+def test_decayed_scan_over_more_sequences_than_a_grid_dimension(ctx, ops):
+    """65 600 portions of five tokens in one call against the same in two calls (which run on the tensor pipe)."""
+    B, n, d, vd = 65600, 5, 16, 16
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q, k, v = (torch.randn(B * n, w, generator=g, device=DEV) * 0.25 for w in (d, d, vd))
+    ld = -torch.rand(B * n, 1, generator=g, device=DEV)
+    pos = torch.arange(n, device=DEV, dtype=torch.int32).repeat(B)
+
+    def run(b0, b1):
+        cu = torch.arange(0, (b1 - b0) * n + 1, n, device=DEV, dtype=torch.int32)
+        state, at = torch.zeros(b1 - b0, 1, d, vd, device=DEV), slice(b0 * n, b1 * n)
+        o = ops.decay_scan(ctx, q[at], k[at], v[at], state, torch.arange(b1 - b0, device=DEV, dtype=torch.int32), cu, pos[at], 1, 1, d, vd, log_decay=ld[at], max_qlen=n)
+        return o, state
+    for a, x, y in zip(run(0, B), run(0, B // 2), run(B // 2, B)):
+        assert close(a, torch.cat([x, y]).to(F64))
