@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int units = 2 * p.kv_heads + p.heads + 1;
   const int n = blockIdx.x * (blockDim.x >> 5) + wid, uu = blockIdx.y;
-  if (n >= a.N || (p.cu_seqlens && n >= p.cu_seqlens[p.B])) return;
+  if (n >= a.N || (p.cu_seqlens && (n < p.cu_seqlens[0] || n >= p.cu_seqlens[p.B]))) return;
   int b = n, r0 = n;
   if (p.cu_seqlens) {
     b = 0;
@@ -175,12 +175,13 @@ __global__ void __launch_bounds__(128) delta_prep_tile_kernel(const DeltaArgs a)
   constexpr int TT = 8, HP = 32 / L;
   pdl_trigger();
   const nvc_delta_prep& p = a.p;
-  const int lane = threadIdx.x & 31, n0 = blockIdx.x * TT;
+  const int lane = threadIdx.x & 31;
   int task = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int qk = p.kv_heads * p.dim, vw = p.heads * p.vdim, C = 2 * qk + vw;
   const int t_qk = (2 * p.kv_heads + HP - 1) / HP, t_v = (vw + 127) / 128;
   pdl_wait();
-  const int cnt = min(TT, min(a.N, p.cu_seqlens[p.B]) - n0);          // rows behind the last sequence are left alone
+  // rows in front of the first sequence and behind the last are left alone
+  const int n0 = max((int)blockIdx.x * TT, p.cu_seqlens[0]), cnt = min((int)(blockIdx.x + 1) * TT, min(a.N, p.cu_seqlens[p.B])) - n0;
   if (cnt <= 0) return;
   if (task < t_qk + t_v) {
     const bool head = task < t_qk;

@@ -106,3 +106,27 @@ def test_decayed_scan_over_more_sequences_than_a_grid_dimension(ctx, ops):
         return o, state
     for a, x, y in zip(run(0, B), run(0, B // 2), run(B // 2, B)):
         assert close(a, torch.cat([x, y]).to(F64))
+
+
+@pytest.mark.parametrize("front,behind,lens", [(5, 0, [13, 20]), (8, 3, [40]), (3, 9, [1, 1, 30]), (6, 2, [2, 1])])
+def test_delta_rule_leaves_rows_outside_the_sequences_alone(ctx, ops, front, behind, lens):
+    """Rows in front of the first sequence and behind the last one are in the call's rows: the sequences between them come out as without them."""
+    H, G, dim, vdim, taps, B = 2, 1, 64, 64, 4, len(lens)
+    g = torch.Generator().manual_seed(front)
+    C = 2 * G * dim + H * vdim
+    x = torch.randn(front + sum(lens) + behind, C + 2 * H, generator=g).to(DEV)
+    w = torch.randn(taps, C, generator=g).to(DEV)
+    S, cs = torch.randn(B, H, dim, vdim, generator=g).to(DEV) * 0.5, torch.randn(B, taps - 1, C, generator=g).to(DEV)
+    cu = torch.tensor([0] + lens).cumsum(0)
+
+    def run(x, cu, pos):
+        s, c = S.clone(), cs.clone()
+        out = ops.delta_rule(ctx, x, (0, G * dim, 2 * G * dim, C, C + H), H, G, dim, vdim, taps, w, c, s, i32(list(range(B))), i32(cu.tolist()), i32(pos),
+                             torch.zeros(H, device=DEV), torch.full((H,), -1.0, device=DEV), max_qlen=max(lens))
+        return out, s, c
+    pos = [b % 2 * 7 + t for b, n in enumerate(lens, 1) for t in range(n)]          # the first sequence goes on from its state
+    want, s0, c0 = run(x[front:front + sum(lens)].contiguous(), cu, pos)
+    got, s1, c1 = run(x, cu + front, [0] * front + pos + [0] * behind)
+    for a, b in zip(got, want):
+        assert torch.equal(a[front:front + sum(lens)], b)
+    assert torch.equal(s0, s1) and torch.equal(c0, c1)
