@@ -347,7 +347,7 @@ int nvc_latent_norm_store(nvc_ctx* ctx, const float* in, int ldi, int n0, int of
                           float eps, void* out0, int ld0, void* cache, int ldc, const int32_t* slot_mapping, int dtype, int N,
                           void* stream);
 /* kind NVC_ACT_GELU_TANH_MUL: out[n, j] = gelu_tanh(in[n, j]) * in[n, Fp + j];  NVC_ACT_RELU2: out[n, j] = max(in[n, j], 0)^2;
- * j < F.  in and out may alias for NVC_ACT_RELU2. */
+ * j < F.  out may be in itself: with ldo == ldi and, for two halves, Fp >= F (else NVC_EINVAL). */
 int nvc_act_mul(nvc_ctx* ctx, const void* in, int ldi, void* out, int ldo, int dtype, int N, int F, int Fp, int kind, void* stream);
 /* C[b] = act(A[b] . W[b]^T), any sizes (fp32 operands: FMA pipe, plain IEEE; bf16 operands with 16-byte-aligned rows - lda,
  * ldw, sa, sw, K multiples of 8 - tensor pipe with fp32 accumulators, other bf16 shapes: FMA pipe): A [M, K] (+ b * sa), W [N, K] (+ b * sw), C [M, N] (+ b * sc),

@@ -119,7 +119,8 @@ __global__ void act_mul_kernel(const T* __restrict__ in, int ldi, T* __restrict_
 // rows fill the chip so (32 per SM; one pass per row: rows of two passes lost 4 % with R = 4), else 1.  Against a CTA of 64 to 256 threads per row that tests the
 // kind per number, cold cache, gated units, bf16 rows x columns: 64 x 1 536: 2.0 -> 1.4 us; 512 x 3 072: 4.8 -> 3.8; 4 000 x 1 536: 9.5 -> 8.5; 10 048 x 1 536: 20.0 -> 17.2 gelu
 // (5.4 TB/s), 20.7 -> 19.6 clamped; 8 192 x 64: 15.3 -> 4.7; 16 000 x 256: 11.6 -> 6.5; fp32 10 048 x 1 536: 32.8 -> 27.0; squared relu 10 048 x 1 536: 12.2 -> 8.8 (7.0 TB/s)
-// `in` and `out` may be the same buffer: a CTA has read its rows' columns before it writes them.
+// `in` and `out` may be the same rows (one stride, the second halves behind the first ones): a number is written by the thread that has read it, and
+// nobody else reads it.
 template <typename T, int kKind, int R>
 __global__ void __launch_bounds__(512) act_mul_rows_kernel(const T* in, int ldi, T* out, int ldo, int N, int F, int Fp, float p0, float p1) {
   pdl_trigger();
@@ -231,6 +232,8 @@ int nvc_act_mul_p(nvc_ctx* ctx, const void* in, int ldi, void* out, int ldo, int
   const bool two = kind == NVC_ACT_GELU_TANH_MUL || kind == NVC_ACT_GLU_CLAMP || kind == NVC_ACT_SILU_MUL;
   NVC_REQUIRE(ctx, N >= 0 && F > 0 && (two || kind == NVC_ACT_RELU2 || kind == NVC_ACT_GELU_TANH), NVC_EINVAL, "bad arguments");
   NVC_REQUIRE(ctx, ldo >= F && ldi >= (two ? Fp + F : F), NVC_EINVAL, "bad strides");
+  // with other strides, or halves that overlap, a CTA would write what another one (a thread, what another one) still has to read
+  NVC_REQUIRE(ctx, in != out || ((ldi == ldo || N <= 1) && (!two || Fp >= F)), NVC_EINVAL, "in place: one row stride, and the second half behind the first");
   if (N == 0) return NVC_OK;
   const int per = dtype == NVC_DT_F32 ? 4 : 8;
   const bool vec = F % per == 0 && Fp % per == 0 && ldi % per == 0 && ldo % per == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 &&

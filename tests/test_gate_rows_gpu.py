@@ -58,3 +58,18 @@ def test_units_of_many_rows(ctx, rows, F, kind, dt):
         ops.check(ctx.l.nvc_act_mul(ctx.h, x.data_ptr(), 2 * F, x.data_ptr(), 2 * F, 0 if dt == torch.bfloat16 else 1, rows, F, F, kind,
                                     torch.cuda.current_stream().cuda_stream), "nvc_act_mul", ctx.h)
         assert torch.equal(x[:, :F], got) and torch.equal(x[:, F:].double(), b)
+
+
+@pytest.mark.parametrize("kind,F,Fp", [(2, 256, 256), (2, 250, 264), (1, 256, 256), (2, 256, 128)])
+@pytest.mark.parametrize("ldo", [0, 8])
+def test_units_in_place(ctx, kind, F, Fp, ldo):
+    """out inside in: the same numbers as out of place where every number is written by the thread that read it, an error elsewhere."""
+    N, two = 200, kind == 2
+    x = torch.randn(N, (Fp + F if two else F) + 8, generator=torch.Generator().manual_seed(F)).bfloat16().to(DEV)
+    want = torch.empty(N, F, dtype=torch.bfloat16, device=DEV)
+    call = lambda out, ld: ctx.l.nvc_act_mul(ctx.h, x.data_ptr(), x.stride(0), out.data_ptr(), ld, 0, N, F, Fp, kind, torch.cuda.current_stream().cuda_stream)  # noqa: E731
+    assert call(want, F) == 0
+    ok = ldo == 0 and (not two or Fp >= F)
+    assert (call(x, x.stride(0) - ldo) == 0) == ok
+    if ok:
+        assert torch.equal(x[:, :F], want)
