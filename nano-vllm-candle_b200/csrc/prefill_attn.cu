@@ -111,8 +111,8 @@ extern "C" int nvc_prefill_attn_varlen(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
   NVC_REQUIRE(ctx, ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0, NVC_EINVAL,
               "pointers must be 16-byte aligned");
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
-  if (B == 0 || total_tokens == 0 || max_seqlen == 0) return NVC_OK;
   NVC_REQUIRE(ctx, scale > 0.f, NVC_EINVAL, "the scale must be positive");      // the kernel masks and takes maxima before it scales
+  if (B == 0 || total_tokens == 0 || max_seqlen == 0) return NVC_OK;
   CUtensorMap tq, tk, tv;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_tokens, ldq);
   if (rc) return rc;
@@ -176,12 +176,12 @@ extern "C" int nvc_prefill_attn_paged_window(nvc_ctx* ctx, const nvc_bf16* q, in
               NVC_EINVAL, "pointers must be 16-byte aligned");
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
   if (B == 0 || total_q_tokens == 0 || max_seqlen_q == 0) return NVC_OK;
-  const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
   if (!(scale > 0.f)) {                      // the kernel masks and takes maxima before it scales; the other one scales first
     const nvc_attn_spec s{nh, kv, hd, hd, scale, window, sink, nullptr, 0, 1.f, 0.f, 0, 0, NVC_ATTN_SOFTMAX, nullptr, nullptr};
     return nvc_attn_paged_wide(ctx, q, ldq, k_cache, kv * hd, v_cache, kv * hd, block_tables, bt_stride, context_lens, cu_seqlens_q, B, total_q_tokens, max_seqlen_q,
                                block_size, &s, out, ldo, NVC_DT_BF16, stream);
   }
+  const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
   CUtensorMap tq, tk, tv;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_q_tokens, ldq);
   if (rc) return rc;
@@ -223,10 +223,10 @@ extern "C" int nvc_prefill_attn_shared(nvc_ctx* ctx, const nvc_bf16* q, int ldq,
   NVC_REQUIRE(ctx, al16(q) && al16(cache) && al16(out) && al16(s.gate) && al16(s.key_scale), NVC_EINVAL, "pointers must be 16-byte aligned");
   NVC_REQUIRE(ctx, ctx->encode_tiled != nullptr, NVC_EDEVICE, "cuTensorMapEncodeTiled unavailable");
   if (B == 0 || total_q_tokens == 0 || max_seqlen_q == 0) return NVC_OK;
-  const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
   if (!sig && !(s.scale > 0.f))              // as above; sigmoid weights are made key by key and take any scale
     return nvc_attn_paged_wide(ctx, q, ldq, cache, kv * 128, cache, kv * 128, block_tables, bt_stride, context_lens, cu_seqlens_q, B, total_q_tokens, max_seqlen_q,
                                block_size, spec, out, ldo, NVC_DT_BF16, stream);
+  const int box_rows = block_size < v2::kKT ? block_size : v2::kKT;
   CUtensorMap tq, tk;
   int rc = make_tma_heads(ctx, &tq, q, nh, total_q_tokens, ldq);
   if (rc) return rc;
