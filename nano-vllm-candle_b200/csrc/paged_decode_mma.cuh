@@ -164,7 +164,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
     if constexpr (kTeams) asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(kThreads) : "memory");
     else __syncthreads();
   };
-  const int kvh = unit_c / chunks;
+  const int kvh = (kTeams ? (unsigned)unit_c : blockIdx.x) / chunks;      // unsigned: a shorter division in front of the first load
   const int chunk = unit_c - kvh * chunks;
   const int head0 = kvh * group_total + chunk * gchunk;
   const int G = min(gchunk, group_total - chunk * gchunk);
