@@ -89,7 +89,9 @@ int paged_decode_impl(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* 
   // residency runs as 2-warp CTAs: Qwen3-0.6B at batch 64 (512 CTAs on 148 SMs) is ONE resident wave instead of
   // 1.7 waves of 4-warp CTAs (28.5 -> 26.6 us), 384 CTAs 26.5 -> 21.1 us, 1024 CTAs 54.7 -> 49.8 us, 2048 CTAs equal;
   // below it the 4-warp CTAs (with KV splits) win (profiles/r02_pd_warps_split_sweep.txt).  NVC_PD_WARPS / nvc_debug_set(5, w) force it (microbench, tests).
-  // Without splits such a grid decides between teams of two and four from the context lengths (paged_decode_mma.cuh) unless the warps are forced.
+  // Up to twice that residency and 128 sequences, and where contexts may exceed 512 tokens, such a grid decides between teams of two and four from the
+  // context lengths (paged_decode_mma.cuh) unless the warps are forced.  Below it start-up is what counts, and the decision's share shows: 64 contexts of 200
+  // 13.6 / 14.1 us, of 64 8.2 / 8.7, of 30 - 350 16.0 / 16.7; 64 of 513 27.8 / 27.9.
   int warps = base > 2 * ctx->num_sms ? 2 : 4;
   bool forced = g_nvc_debug[5] == 2 || g_nvc_debug[5] == 4;
   if (const char* e = getenv("NVC_PD_WARPS")) {
@@ -122,12 +124,9 @@ int paged_decode_impl(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf16* 
     part_o = reinterpret_cast<float*>(workspace);
     part_ml = part_o + (size_t)B * nh * splits * hd;
   }
-  if (splits == 1 && warps == 2 && !forced) {
-    const bool many = base >= 6 * ctx->num_sms;
-    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, many ? pdmma::paged_decode_mma_kernel<2, true> : pdmma::paged_decode_mma_kernel<4, true>,
-                                   dim3(base <= 4 * ctx->num_sms ? 2 * ctx->num_sms : base), dim3(many ? 64 : 128),
-                                   (size_t)(many ? pdmma::smem_bytes<2>() : pdmma::smem_bytes<4>()), st, q, ldq, k_cache, v_cache, block_tables, max_blocks,
-                                   context_lens, nh, kv, group, G, block_size, scale_log2e, out, part_o, part_ml, 1, B));
+  if (splits == 1 && warps == 2 && !forced && base <= 4 * ctx->num_sms && B <= 128 && (int64_t)max_blocks_hint * block_size > 512) {
+    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, pdmma::paged_decode_mma_kernel<4, true>, dim3(2 * ctx->num_sms), dim3(128), (size_t)pdmma::smem_bytes<4>(), st, q, ldq,
+                                   k_cache, v_cache, block_tables, max_blocks, context_lens, nh, kv, group, G, block_size, scale_log2e, out, part_o, part_ml, 1, B));
     NVC_CUDA_CHECK(ctx, cudaGetLastError());
     ctx->launches++;
     return NVC_OK;
@@ -157,8 +156,6 @@ extern "C" int nvc_paged_decode_init(nvc_ctx* ctx) {
                                            pdmma::smem_bytes<4>()));
   NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(pdmma::paged_decode_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            pdmma::smem_bytes<2>()));
-  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(pdmma::paged_decode_mma_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            pdmma::smem_bytes<2>())));
   NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(pdmma::paged_decode_mma_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             pdmma::smem_bytes<4>())));
   // device address of the static scratch (ctx creation runs with ctx->device current)

@@ -17,16 +17,15 @@
 // resident): the same bytes in flight per SM, but a grid of 297..592 CTAs (Qwen3-0.6B at batch 64:
 // 512) is resident at once instead of running 1.7 waves with a synchronised bubble between them.
 //
-// kTeams, for grids beyond the 4-warp residency without splits: what a unit (sequence, kv head, head chunk) costs follows its context length, which
-// only the device knows, so the kernel decides there.  A warp's ring covers about 15 GB/s whatever else the SM does, so among contexts of different
-// lengths the longest ones set the time.  When the longest exceeds 7/4 of the average, units are taken longest first, by teams of four warps where
-// two CTAs per SM hold a good part of them (kWarps = 4, fewer than 6 units per SM), by teams of two in larger grids (kWarps = 2), where the order alone
-// evens the ends out.  Otherwise teams of two, all resident at once, as without kTeams; one level lower (5/4) the ordered form loses at 64 contexts of
-// 300 - 600 (22.4 -> 27.1 us against 22.4 -> 22.9).  Up to 4 units per SM the grid is the 2 * SMs resident CTAs, and a CTA takes a second unit from the short
-// end: a grid of one CTA per unit, half of them without work, ends 1 us later.  8 kv heads, cold cache, a kernel between the calls, before -> after:
-//   64 contexts of 200 - 1 500: 49.2 -> 35.4 us (4.76 TB/s)     40 of 50 - 4 000: 111 -> 51.4        63 of 200 and one of 8 000: 176 -> 93
-//   128 of 200 - 1 500: 79.5 -> 65.6     256 of 100 - 3 000: 171 -> 140 (6.37 TB/s)      300 of 100 - 3 000: 192 -> 162      100 of 20 - 900: 33.8 -> 30.1
-//   64 of 513: 28.4 -> 28.1      64 of 1 000 - 1 400: 59.2 -> 58.7      256 of 1 024: 166.2 -> 167.7       64 of 30 - 350: 16.1 -> 16.8 (reading the lengths)
+// kTeams, for grids beyond the 4-warp residency without splits, up to twice that: what a unit (sequence, kv head, head chunk) costs follows its
+// context length, which only the device knows, so the kernel decides there.  A warp's ring covers about 15 GB/s whatever else the SM does, so among
+// contexts of different lengths the longest ones set the time.  When the longest exceeds 7/4 of the average, units are taken longest first, by teams of
+// four warps; a CTA takes a second unit from the short end.  Otherwise teams of two, all resident at once, as without kTeams; one level lower (5/4) the
+// ordered form loses at 64 contexts of 300 - 600.  The first tile of the teams of two is on its way before the lengths are looked at: it costs the ordered form
+// little, and where the lengths are equal nothing waits for them.  Larger grids, and batches of more than 128, run without kTeams: CTAs are many, each would
+// read all the lengths, and 1 024 contexts of 30 - 300 took 174 us where the plain form takes 105.
+// The number of warps that share a sequence, and with it the order of its sums, follows the OTHER lengths of the batch in this range: the same batch repeats
+// itself bit by bit, the same sequence in another batch need not.
 #pragma once
 #include "common.cuh"
 
@@ -66,7 +65,7 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 }
 // group_total: query heads per kv head; gchunk: heads of the group handled by one CTA (<= 16).
 // num_splits > 1: every split parks its (m, l, o) partial in part_o / part_ml for paged_decode_combine_kernel.
-// kTeams: a one-dimensional grid, with a CTA per unit or two units per CTA; no splits.
+// kTeams: four warps, a one-dimensional grid of at least half as many CTAs as units; no splits, up to 128 sequences.
 template <int kWarps, bool kTeams = false>
 __global__ void __launch_bounds__(kWarps * 32, kWarps == 4 ? 2 : 4)
 paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* __restrict__ k_cache,
@@ -74,6 +73,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
                         const int32_t* __restrict__ context_lens, int nh, int kv, int group_total, int gchunk,
                         int block_size, float scale_log2e, nvc_bf16* __restrict__ out, float* __restrict__ part_o,
                         float* __restrict__ part_ml, int num_splits, int B) {
+  static_assert(!kTeams || kWarps == 4, "teams of two or all four");
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   // The dependency wait comes AFTER the first K / V tiles are in flight (see below): context_lens and
@@ -83,45 +83,32 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
   const int lane = threadIdx.x & 31;
   const int quad = lane >> 2, tq = lane & 3;          // accumulator row (quad, quad + 8), column pair tq
   int team_warps = kWarps, team = 0, b = blockIdx.y, unit_c = blockIdx.x;
-  int blk_first, ctx_len, most = 0;
-  bool uneven = false;
+  int blk_first, ctx_len, most = 0, stage0 = 0;
+  int lens[4];                                        // kTeams: this lane's share of the lengths
+  bool uneven = false, decided = !kTeams;
   const int KC = kv * chunks, units = KC * B;
-  const bool one_wave = kWarps > 2 && (int)gridDim.x < units;       // kTeams: two units per CTA at most
   int u = blockIdx.x;
   if constexpr (kTeams) {
-    int sum = 0;
-    // the first loads of the teams of two go out with the lengths: no second latency where these are equal
-    // (one wave: the second teams start where the first ones end, so that every SM gets its share)
+    // teams of two, until the lengths are known: the second teams start where the first ones end, so that every SM gets its share
     team = threadIdx.x >> 6;
-    if (kWarps > 2) u = one_wave ? blockIdx.x + team * gridDim.x : 2 * blockIdx.x + team;
+    team_warps = 2;
+    u = blockIdx.x + team * gridDim.x;
     const int b2 = min(u / KC, B - 1);
     blk_first = __ldg(block_tables + (int64_t)b2 * max_blocks);
     ctx_len = __ldg(context_lens + b2);
-#pragma unroll 2
-    for (int i = lane; i < B; i += 32) {
-      const int x = max(__ldg(context_lens + i), 0);
-      sum += x;
-      most = max(most, x);
-    }
-    sum = __reduce_add_sync(0xffffffffu, sum);
-    most = __reduce_max_sync(0xffffffffu, most);
-    uneven = 4ll * B * most > 7ll * sum && most >= 128;       // below it all is start-up
-    team_warps = uneven ? kWarps : 2;
-    if (team_warps != 2) {
-      team = 0;
-      u = blockIdx.x;
-    }
-    if (u >= units) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lens[i] = lane + 32 * i < B ? max(__ldg(context_lens + lane + 32 * i), 0) : 0;
   }
 #pragma unroll 1
-  for (;;) {                                          // a unit; kTeams: the second one of the CTA, if it has one
+  for (;;) {                                          // a unit; kTeams: once more when the lengths turn out uneven, and the CTA's second unit
   if constexpr (kTeams) {
     b = u / KC;
     unit_c = u - b * KC;
     if (uneven) {
-      // the sequence that `b` longer ones precede: counts of 128 levels of length (in the warp's own part of the ring, free so far; lane 0 has the
-      // four highest), their running sum, then the place among those of the level
-      int* const count = reinterpret_cast<int*>(smem + (threadIdx.x >> 5) * (kStages * kStageBytes));
+      // the sequence that `b` longer ones precede: counts of 128 levels of length (lane 0 has the four highest), their running sum, then the place
+      // among those of the level
+      __shared__ __align__(16) int counts[kWarps][128];
+      int* const count = counts[threadIdx.x >> 5];
       const float f = 127.9f / (float)most;
       auto place = [&](int i) { return i < B ? 127 - (int)((float)max(__ldg(context_lens + i), 0) * f) : -1; };
       reinterpret_cast<int4*>(count)[lane] = make_int4(0, 0, 0, 0);
@@ -199,7 +186,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
         const int bi = tok0 / block_size;
         const int blk = bi == 0 ? blk_first : __ldg(bt + bi);
         const int64_t slot0 = (int64_t)blk * block_size + (tok0 % block_size);
-        const uint32_t st = ring + (i % kStages) * kStageBytes;
+        const uint32_t st = ring + ((i + stage0) % kStages) * kStageBytes;
         const int c = lane & 15;                       // 16-byte chunk of the 256-byte row
 #pragma unroll
         for (int rr = 0; rr < 8; ++rr) {
@@ -223,13 +210,29 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
     return i >= my_tiles || tok0 >= ctx_len || tok0 + kTileTok <= ctx_len - 1;
   };
   int pre = 0;
-  if (safe(0)) {
+  if ((decided || u < units) && safe(0)) {
     issue(0);
     pre = 1;
-    if (safe(1)) {
-      issue(1);
-      pre = 2;
+  }
+  if constexpr (kTeams) {
+    if (!decided) {
+      decided = true;
+      const int sum = __reduce_add_sync(0xffffffffu, lens[0] + lens[1] + lens[2] + lens[3]);
+      most = __reduce_max_sync(0xffffffffu, max(max(lens[0], lens[1]), max(lens[2], lens[3])));
+      uneven = 4ll * B * most > 7ll * sum && most >= 128;       // below it all is start-up
+      if (uneven) {
+        team_warps = kWarps;
+        team = 0;
+        u = blockIdx.x;
+        stage0 = pre;                                 // the tile that is on its way keeps its stage until tile 2 needs it
+        continue;
+      }
+      if (u >= units) return;
     }
+  }
+  if (pre == 1 && safe(1)) {
+    issue(1);
+    pre = 2;
   }
   pdl_wait();
   // ---- Q as A fragments: 8 k-steps of 16 dims; rows >= G are zero
@@ -249,13 +252,14 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
   }
   if (pre < 1) issue(0);
   if (pre < 2) issue(1);
+  if (kTeams && stage0) cp_async_wait<2>();
   for (int i = 0; i < my_tiles; ++i) {
     issue(i + 2);
     cp_async_wait<2>();                               // tile i has landed (two younger groups may be in flight)
     __syncwarp();
     const int tok0 = (t_begin + i) * kCtaTok + warp * kTileTok;
     if (tok0 < ctx_len) {                             // warp-uniform
-      const uint32_t st = ring + (i % kStages) * kStageBytes;
+      const uint32_t st = ring + ((i + stage0) % kStages) * kStageBytes;
       // ---- S = Q K^T: two n-tiles of 8 tokens, fp32
       float s[2][4];
 #pragma unroll
@@ -383,7 +387,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
       if (d == 0) { __stcg(part_ml + p * 2, M); __stcg(part_ml + p * 2 + 1, L); }
     }
   }
-  if (!kTeams || !one_wave || team_warps == 2) break;
+  if (!kTeams || team_warps == 2) break;
   u = 2 * (int)gridDim.x - 1 - u;                     // the longest ones' CTAs take the shortest ones of the rest, or none
   if (u >= units || u < (int)gridDim.x) break;
   team_sync();                                        // the sums have been read
