@@ -46,12 +46,19 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int units = 2 * p.kv_heads + p.heads + 1;
   const int n = blockIdx.x * (blockDim.x >> 5) + wid, uu = blockIdx.y;
-  if (n >= a.N || (p.cu_seqlens && (n < p.cu_seqlens[0] || n >= p.cu_seqlens[p.B]))) return;
+  if (n >= a.N) return;
   int b = n, r0 = n;
   if (p.cu_seqlens) {
-    b = 0;
-    for (int i = 1; i < p.B; i += 32) b += __popc(__ballot_sync(0xffffffffu, i + lane < p.B && p.cu_seqlens[i + lane] <= n));
-    r0 = p.cu_seqlens[b];
+    // the last sequence that starts at or in front of the row; its start comes with the search, no second load
+    const int end = p.cu_seqlens[p.B];
+    b = -1;
+    for (int i = 0; i < p.B; i += 32) {
+      const int c = i + lane < p.B ? p.cu_seqlens[i + lane] : 0x7fffffff, k = __popc(__ballot_sync(0xffffffffu, c <= n));
+      if (k == 0) break;
+      b = i + k - 1;
+      r0 = __shfl_sync(0xffffffffu, c, k - 1);
+    }
+    if (b < 0 || n >= end) return;             // in front of the first sequence, or behind the last
   }
   const float* in = p.in + (int64_t)n * p.ldi;
   if (uu >= units) {
@@ -963,8 +970,9 @@ extern "C" int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, 
   DeltaArgs a{*p, N, vec, nullptr, 0, nullptr};
   const int units = 2 * p->kv_heads + p->heads + 1 + (p->channel_a ? p->heads : 0);
   NVC_REQUIRE(ctx, units <= 65535 && p->B <= 65535, NVC_ESHAPE, "more than 65 535 heads or sequences");
-  // portions of 4 tokens and more on average: shorter ones start a new history with nearly every row
-  if (p->cu_seqlens && vec && (!p->channel_a || p->ldca % 4 == 0) && p->dim <= 128 && p->taps <= 4 && N >= 4 * p->B) {
+  // From 512 rows on - fewer do not fill the chip with tiles of rows (16 heads of 128 over 8, rows / this: 10 rows 2.8 / 5.9 us, 256 5.5 / 6.8, 640 11.3 / 8.9) - and
+  // from 4 tokens per portion on average: shorter ones start a new history with nearly every row
+  if (p->cu_seqlens && vec && (!p->channel_a || p->ldca % 4 == 0) && p->dim <= 128 && p->taps <= 4 && N >= 512 && N >= 4 * p->B) {
     cudaStream_t st = nvc_stream(stream);
     NVC_CUDA_CHECK(ctx, p->taps == 1 ? launch_prep_tile<1>(ctx, a, st) : (p->taps == 2 ? launch_prep_tile<2>(ctx, a, st)
                                                                                        : (p->taps == 3 ? launch_prep_tile<3>(ctx, a, st) : launch_prep_tile<4>(ctx, a, st))));

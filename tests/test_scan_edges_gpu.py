@@ -108,7 +108,7 @@ def test_decayed_scan_over_more_sequences_than_a_grid_dimension(ctx, ops):
         assert close(a, torch.cat([x, y]).to(F64))
 
 
-@pytest.mark.parametrize("front,behind,lens", [(5, 0, [13, 20]), (8, 3, [40]), (3, 9, [1, 1, 30]), (6, 2, [2, 1])])
+@pytest.mark.parametrize("front,behind,lens", [(5, 0, [13, 20]), (8, 3, [40]), (3, 9, [1, 1, 30]), (6, 2, [2, 1]), (5, 3, [13, 520]), (12, 0, [600]), (3, 6, [1, 1, 511])])
 def test_delta_rule_leaves_rows_outside_the_sequences_alone(ctx, ops, front, behind, lens):
     """Rows in front of the first sequence and behind the last one are in the call's rows: the sequences between them come out as without them."""
     H, G, dim, vdim, taps, B = 2, 1, 64, 64, 4, len(lens)
@@ -130,3 +130,37 @@ def test_delta_rule_leaves_rows_outside_the_sequences_alone(ctx, ops, front, beh
     for a, b in zip(got, want):
         assert torch.equal(a[front:front + sum(lens)], b)
     assert torch.equal(s0, s1) and torch.equal(c0, c1)
+
+
+PORTIONS = {"few": [1, 2, 3, 7, 8, 9, 500], "one": [523], "many": [4 + i % 9 for i in range(140)]}
+
+
+@pytest.mark.parametrize("H,G,dim,vdim,taps", [(2, 1, 64, 64, 4), (3, 1, 20, 132, 2), (2, 2, 128, 8, 1), (5, 5, 4, 4, 3), (4, 2, 68, 64, 4)])
+@pytest.mark.parametrize("which", list(PORTIONS))
+@pytest.mark.parametrize("channels", [False, True])
+def test_delta_preparation_in_tiles_of_rows(ctx, ops, H, G, dim, vdim, taps, which, channels):
+    """512 rows and more in one call (tiles of rows) against the portions one by one (a warp per row and head).  Both are fp32 with at most 4 taps
+    and 128 squares in another order: 2e-6 of the largest value."""
+    lens = PORTIONS[which] if which != "one" else [511, 523]
+    B, g = len(lens), torch.Generator().manual_seed(dim + taps)
+    C = 2 * G * dim + H * vdim
+    ld = (C + 2 * H + 3) // 4 * 4
+    x = torch.randn(sum(lens), ld, generator=g).to(DEV)
+    w, cs = torch.randn(taps, C, generator=g).to(DEV), torch.randn(B, max(taps - 1, 1), C, generator=g).to(DEV)
+    ca = torch.randn(sum(lens), H * dim, generator=g).to(DEV) if channels else None
+    A, dt = torch.randn(H, generator=g).to(DEV), torch.randn(H * dim if channels else H, generator=g).to(DEV)
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    pos = [b % 2 * 5 + t for b, n in enumerate(lens) for t in range(n)]
+
+    def run(a, b):
+        r = slice(cu[a], cu[b])
+        out = ops.delta_rule(ctx, x[r], (0, G * dim, 2 * G * dim, C, C + H), H, G, dim, vdim, taps, w, cs.clone(), torch.zeros(B, H, dim, vdim, device=DEV),
+                             i32(list(range(a, b))), i32([c - cu[a] for c in cu[a:b + 1]]), i32(pos[r]), A, dt, max_qlen=max(lens), channel_a=ca[r].contiguous() if channels else None)
+        return out[1:]                                   # q, k, v and (log decay, beta)
+    parts = [run(b, b + 1) for b in range(B)] if which != "one" else [run(0, 1)]
+    whole = run(0, B)
+    for i, got in enumerate(whole):
+        want = torch.cat([p[i] for p in parts]).to(F64)
+        if i == 3 and channels:                          # the decay per head is not written then
+            got, want = got[:, 1::2], want[:, 1::2]
+        assert close(got[:want.shape[0]], want), i
