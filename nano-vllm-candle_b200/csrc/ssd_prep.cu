@@ -180,8 +180,10 @@ extern "C" int nvc_ssd_prep_run(nvc_ctx* ctx, const nvc_ssd_prep* p, int N, void
   const int gn = p->groups * p->state;
   const bool vec = ((p->vdim | gn | p->ldi | p->xbc_off | p->ldx | p->ldbc) & 3) == 0 && al16(p->in) && al16(p->conv_w) && al16(p->conv_b) &&
                    al16(p->conv_state) && al16(p->x_out) && al16(p->v_out) && al16(p->b_out) && al16(p->c_out);
-  // portions of 4 tokens and more on average: shorter ones start a new history with nearly every row
-  if (vec && p->cu_seqlens && p->taps <= 4 && N >= 4 * p->B) {
+  // Tiles of rows from 2 048 rows on, and from 1 024 where portions are long: a tile takes the ends of portions one after another, about 1 us each, and fewer
+  // tiles do not fill the chip.  2 560 channels, a CTA per row / this: 10 rows 6.2 / 8.9 us, 256 7.5 / 9.6, 512 beside 63 single tokens 11.6 / 17.4,
+  // one portion of 1 050 14.0 / 10.9, 256 portions of 10 42.4 / 34.7, 512 of 20 146 / 95
+  if (vec && p->cu_seqlens && p->taps <= 4 && N >= 4 * p->B && (N >= 2048 || (N >= 1024 && N >= 256 * (int64_t)p->B))) {
     auto* kernel = p->taps == 1 ? ssd_prep_tile_kernel<1> : (p->taps == 2 ? ssd_prep_tile_kernel<2> : (p->taps == 3 ? ssd_prep_tile_kernel<3> : ssd_prep_tile_kernel<4>));
     NVC_CUDA_CHECK(ctx, nvc_launch(ctx, kernel, dim3((unsigned)((N + 7) / 8), (unsigned)((C + 511) / 512)), dim3(128), 0, nvc_stream(stream), a));
   } else if (vec) {

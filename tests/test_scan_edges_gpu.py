@@ -164,3 +164,27 @@ def test_delta_preparation_in_tiles_of_rows(ctx, ops, H, G, dim, vdim, taps, whi
         if i == 3 and channels:                          # the decay per head is not written then
             got, want = got[:, 1::2], want[:, 1::2]
         assert close(got[:want.shape[0]], want), i
+
+
+@pytest.mark.parametrize("H,vdim,Gs,state,taps", [(3, 64, 1, 64, 4), (2, 4, 1, 12, 2), (5, 132, 1, 20, 3), (34, 16, 2, 8, 1)])
+@pytest.mark.parametrize("lens", [[700, 330], [9 + i % 2 for i in range(230)], [1, 1023, 1100]])
+def test_state_space_preparation_in_tiles_of_rows(ctx, ops, H, vdim, Gs, state, taps, lens):
+    """Rows enough for tiles against the same in calls that are not, each portion cut from its neighbours: fp32 sums of 4 taps, 2e-6."""
+    g = torch.Generator().manual_seed(H + vdim)
+    B, C = len(lens), H * vdim + 2 * Gs * state
+    x = torch.randn(sum(lens), (C + H + 3) // 4 * 4, generator=g).to(DEV)
+    w, bias = torch.randn(taps, C, generator=g).to(DEV), torch.randn(C, generator=g).to(DEV)
+    cs = torch.randn(B, max(taps - 1, 1), C, generator=g).to(DEV)
+    A, dt = torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    pos = [b % 2 * 5 + t for b, n in enumerate(lens) for t in range(n)]
+
+    def run(a, b, step):
+        st, out = cs.clone(), []
+        for r0 in range(cu[a], cu[b], step):
+            r1 = min(r0 + step, cu[b])
+            sel = [k for k in range(a, b) if cu[k] < r1 and cu[k + 1] > r0]
+            out.append(ops.ssd_prep(ctx, x[r0:r1], 0, C, H, vdim, Gs, state, taps, w, bias, st, i32(sel), i32([max(cu[k], r0) - r0 for k in sel] + [r1 - r0]), i32(pos[r0:r1]), A, dt))
+        return [torch.cat(t) for t in zip(*out)] + [st]
+    for got, want in zip(run(0, B, 1 << 20), run(0, B, 400)):
+        assert close(got, want.to(F64))
