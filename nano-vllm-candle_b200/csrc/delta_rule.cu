@@ -998,7 +998,10 @@ extern "C" int nvc_delta_rule_scan(nvc_ctx* ctx, const nvc_delta_prep* p, float*
     // a warp's registers, which is what ends it at 128 channels; decays per channel are no factors of a product of rows
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     a.vec = dim % 4 == 0 && p->ldq % 4 == 0 && p->ldk % 4 == 0 && al16(p->q_out) && al16(p->k_out) && al16(p->channel_g);
-    const cudaError_t ce = !p->channel_a && dim <= 128 && p->B <= 65535 ? (dim <= 64 ? launch_delta_mma<4>(ctx, a, nvc_stream(stream)) : launch_delta_mma<8>(ctx, a, nvc_stream(stream)))
+    // Portions of up to 16 tokens fill half of a 32-token chunk, and a CTA there has its SM for itself: it wins while the CTAs are few (one portion of
+    // 10 tokens, 16 heads of 128 x 128: 15.0 -> 11.6 us; 8 portions, 256 CTAs: 23.2 -> 22.8) and loses among many (64 portions of 10: 127 -> 173)
+    const bool brief = max_qlen <= 16 && (int64_t)p->B * p->heads * ((p->vdim + kMC - 1) / kMC) > 2 * ctx->num_sms;
+    const cudaError_t ce = !p->channel_a && dim <= 128 && p->B <= 65535 && !brief ? (dim <= 64 ? launch_delta_mma<4>(ctx, a, nvc_stream(stream)) : launch_delta_mma<8>(ctx, a, nvc_stream(stream)))
                            : p->channel_a ? launch_delta_chunk_sized<true>(ctx, a, nvc_stream(stream)) : launch_delta_chunk_sized<false>(ctx, a, nvc_stream(stream));
     NVC_CUDA_CHECK(ctx, ce);
     ctx->launches++;

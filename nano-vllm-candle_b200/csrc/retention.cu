@@ -654,7 +654,10 @@ int run_scan(nvc_ctx* ctx, const RetArgs& a, int B, int max_qlen, void* stream) 
     // the tensor pipe keeps 16 columns x all channels of the state in a warp's registers, which is what ends it at 128 channels; at 128 x 64
     // over eight prompts of 245 to 1 050 tokens, 32 heads: 168 us, the FMA form 640
     if constexpr (MODE != kMemory) {
-      if (dim <= 128 && B <= 65535) {            // sequences lie along the grid's second dimension there
+      // portions of up to 16 tokens over states that do not fit in L2: the FMA kernel's slices of 128 columns read them better (256 portions of 10 tokens, 16 heads of
+      // 128 x 128, 1 GB of states: 581 us, here 642; 64 portions: 161, here 121; heads of 64 x 64: 282, here 258)
+      const bool brief = max_qlen <= 16 && vdim > 64 && (int64_t)B * heads >= 16 * ctx->num_sms;
+      if (dim <= 128 && B <= 65535 && !brief) {  // sequences lie along the grid's second dimension there
         ce = dim <= 64 ? launch_decay_mma<4, MODE>(ctx, a, B, nvc_stream(stream)) : launch_decay_mma<8, MODE>(ctx, a, B, nvc_stream(stream));
         NVC_CUDA_CHECK(ctx, ce);
         ctx->launches++;

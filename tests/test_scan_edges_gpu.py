@@ -10,7 +10,7 @@ import torch
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 F64 = torch.float64
-LENS = {"edges": [1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97], "one": [70], "many": [5 + i % 3 for i in range(300)]}
+LENS = {"edges": [1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97], "one": [70], "many": [5 + i % 3 for i in range(300)], "crowd": [17 + i % 3 for i in range(260)]}
 
 
 @pytest.fixture(scope="module")
@@ -31,7 +31,7 @@ def close(got, want):
 
 
 def shapes(vdims):
-    return [(d, vd, "edges") for d in (1, 20, 64, 65, 127, 128) for vd in vdims[:1]] + [(128, vd, "edges") for vd in vdims[1:]] + [(32, 16, "many"), (128, 64, "one")]
+    return [(d, vd, "edges") for d in (1, 20, 64, 65, 127, 128) for vd in vdims[:1]] + [(128, vd, "edges") for vd in vdims[1:]] + [(32, 16, "many"), (32, 16, "crowd"), (128, 64, "one")]
 
 
 @pytest.mark.parametrize("fixed", [False, True])
@@ -91,18 +91,18 @@ def test_delta_rule_edges(ctx, ops, dim, vdim, which):
         assert torch.equal(cs[slots[b]][0], x[int(cu[b + 1]) - 1, :C]), b
 
 
-def test_decayed_scan_over_more_sequences_than_a_grid_dimension(ctx, ops):
-    """65 600 portions of five tokens in one call against the same in two calls (which run on the tensor pipe)."""
-    B, n, d, vd = 65600, 5, 16, 16
+@pytest.mark.parametrize("B,n,H,d,vd", [(65600, 5, 1, 16, 16), (1300, 9, 2, 64, 80)])
+def test_decayed_scan_over_more_sequences_than_the_tensor_pipe_takes(ctx, ops, B, n, H, d, vd):
+    """More sequences than a grid dimension holds, and many brief portions: one call (FMA) against the same in two (tensor pipe)."""
     g = torch.Generator(device=DEV).manual_seed(3)
-    q, k, v = (torch.randn(B * n, w, generator=g, device=DEV) * 0.25 for w in (d, d, vd))
-    ld = -torch.rand(B * n, 1, generator=g, device=DEV)
+    q, k, v = (torch.randn(B * n, H * w, generator=g, device=DEV) * 0.25 for w in (d, d, vd))
+    ld = -torch.rand(B * n, H, generator=g, device=DEV)
     pos = torch.arange(n, device=DEV, dtype=torch.int32).repeat(B)
 
     def run(b0, b1):
         cu = torch.arange(0, (b1 - b0) * n + 1, n, device=DEV, dtype=torch.int32)
-        state, at = torch.zeros(b1 - b0, 1, d, vd, device=DEV), slice(b0 * n, b1 * n)
-        o = ops.decay_scan(ctx, q[at], k[at], v[at], state, torch.arange(b1 - b0, device=DEV, dtype=torch.int32), cu, pos[at], 1, 1, d, vd, log_decay=ld[at], max_qlen=n)
+        state, at = torch.zeros(b1 - b0, H, d, vd, device=DEV), slice(b0 * n, b1 * n)
+        o = ops.decay_scan(ctx, q[at], k[at], v[at], state, torch.arange(b1 - b0, device=DEV, dtype=torch.int32), cu, pos[at], H, H, d, vd, log_decay=ld[at], max_qlen=n)
         return o, state
     for a, x, y in zip(run(0, B), run(0, B // 2), run(B // 2, B)):
         assert close(a, torch.cat([x, y]).to(F64))
