@@ -551,8 +551,8 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
     return nvc_gemm_pair_swapped(ctx, A, lda, W, reinterpret_cast<float*>(C), ldc, M, Nout, K, stream, trace);
   // Narrow products over many rows (a router: 64 columns) fill few CTA pairs and are one k-loop long: the narrowest 1-CTA tiles that stay in one wave
   // (us, pair / this: 1 000 x 64 x 1 024 8.1 / 4.7, 4 000 x 64 x 2 048 10.8 / 7.0, 4 000 x 256 x 1 024 10.6 / 6.1, 16 000 x 128 x 1 024 11.6 / 8.4; two waves lose:
-  // 16 000 x 256 x 2 048 17.5 / 23.5, and so does a long k-loop over few rows: 200 x 64 x 4 096 8.2 / 10.8)
-  if (force_bn == 0 && force_splits == 0 && epi == NVC_EPI_NONE && M > BM && Nout <= 256 && K <= 2048) {
+  // 16 000 x 256 x 2 048 17.5 / 23.5, and so does a long k-loop over few rows: 200 x 64 x 4 096 8.2 / 10.8, 160 x 16 x 2 048 6.4 / 6.7, 384 x 16 x 2 048 9.0 / 6.7)
+  if (force_bn == 0 && force_splits == 0 && epi == NVC_EPI_NONE && M > BM && Nout <= 256 && K <= (M <= 2 * BM ? 1536 : 2048)) {
     for (int bn : {32, 64, 128})
       if ((int64_t)((M + BM - 1) / BM) * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
         force_bn = bn + (bn == 128 ? 2000 : 4000);
