@@ -688,7 +688,8 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
                                 int K, const nvc_bf16* qw, const nvc_bf16* kw, float eps, const float* cos_sin,
                                 const int32_t* positions, const int32_t* slot_mapping, nvc_bf16* k_cache, nvc_bf16* v_cache,
                                 int nh, int kv, void* stream) {
-  if (N != (nh + 2 * kv) * 128 || K % BK != 0) return NVC_ENOTIMPL;
+  auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  if (N != (nh + 2 * kv) * 128 || K % BK != 0 || lda < K || (lda | ldc) % 8 || !al16(A) || !al16(W) || !al16(C)) return NVC_ENOTIMPL;
   // The fusion saves a pass over the rows and lengthens the epilogue, of which all but the last wave's runs under the next tile's main loop.
   // K >= 2 048: it wins from about 1 500 rows on (one call against two kernels: 1 500 x 6 144 x 4 096 57 / 63 us, 3 000 x 4 096 x 2 048 51 / 62,
   // 4 096 x 6 144 x 4 096 167 / 191, 6 555 x 4 096 x 2 048 115 / 151; 1 000 rows 54 / 52).  Shorter k-loops hide less of it: below 8 192 rows it wins

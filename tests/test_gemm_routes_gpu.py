@@ -10,6 +10,18 @@ pytestmark = pytest.mark.gpu
 BF16 = torch.bfloat16
 
 
+def test_projection_refuses_rows_that_overlap(ctx):
+    """A row stride below the row's length is an error in the fused range too."""
+    M, nh, kv, K = 1600, 4, 2, 2048
+    N = (nh + 2 * kv) * 128
+    a, w, qkv = (torch.zeros(n, m, dtype=BF16, device="cuda") for n, m in ((M, K), (N, K), (M, N)))
+    one, tab, pos = torch.ones(128, dtype=BF16, device="cuda"), ctx.rope_table(1e6, 128, M), torch.arange(M, dtype=torch.int32, device="cuda")
+    call = lambda lda: ctx.l.nvc_qkv_proj_norm_rope(ctx.h, a.data_ptr(), lda, w.data_ptr(), qkv.data_ptr(), M, K, one.data_ptr(), one.data_ptr(), 1e-6,  # noqa: E731
+                                                    tab.data_ptr(), pos.data_ptr(), None, None, None, nh, kv, 128, torch.cuda.current_stream().cuda_stream)
+    assert call(K) == 0 and call(K - 8) != 0 and call(K // 2) != 0
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("M", [129, 200, 1000, 2368, 2369, 18944, 18945])
 @pytest.mark.parametrize("N", [16, 48, 64, 240, 256])
 @pytest.mark.parametrize("K", [64, 192, 2048])
