@@ -694,9 +694,9 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
   // K >= 2 048: it wins from about 1 500 rows on (one call against two kernels: 1 500 x 6 144 x 4 096 57 / 63 us, 3 000 x 4 096 x 2 048 51 / 62,
   // 4 096 x 6 144 x 4 096 167 / 191, 6 555 x 4 096 x 2 048 115 / 151; 1 000 rows 54 / 52).  Shorter k-loops hide less of it: below 8 192 rows it wins
   // where the last wave is at least 2/5 full (6 555 x 4 096 x 1 024, 5.6 waves: 90 / 104; 5 500, 4.8: 65 / 70) and loses else (6 000, 5.2: 97 / 89;
-  // 3 500, 3.03: 62 / 58; 4 096, 3.5: even)
-  const int pairs = ctx->num_sms / 2, rem = ((M + 255) / 256) * ((N + 255) / 256) % pairs;
-  if (K >= 2048 ? M < 1500 : M < 8192 && (M < 4097 || 5 * rem < 2 * pairs)) return NVC_ENOTIMPL;
+  // 3 500, 3.03: 62 / 58; 4 096, 3.5: even; 4 100 - 4 608, 3.7 - 3.9: 46 / 47 - 50)
+  const int pairs = ctx->num_sms / 2, rem = ((M + 255) / 256) * ((N + 255) / 256) % pairs, last = rem ? rem : pairs;
+  if (K >= 2048 ? M < 1500 : M < 8192 && (M <= 4096 || 5 * last < 2 * pairs)) return NVC_ENOTIMPL;
   int nt = 256, S = 1;
   choose_schedule(ctx, M, N, K / BK, &nt, &S);
   if (nt != 256 || S != 1) return NVC_ENOTIMPL;

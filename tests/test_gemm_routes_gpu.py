@@ -10,6 +10,30 @@ pytestmark = pytest.mark.gpu
 BF16 = torch.bfloat16
 
 
+@pytest.mark.parametrize("M,nh,kv,K", [(1500, 4, 2, 2048), (1501, 32, 8, 4096), (3001, 16, 8, 2048), (5500, 16, 8, 1024), (6000, 16, 8, 1024), (6555, 16, 8, 1024),
+                                       (8191, 8, 4, 512), (2400, 5, 1, 2048),
+                                       (5120, 66, 4, 512)])      # 740 tiles: ten full waves on 74 pairs of SMs
+def test_fused_projection_between_its_thresholds(ctx, nvc, M, nh, kv, K):
+    g = torch.Generator().manual_seed(M + K)
+    N, slots = (nh + 2 * kv) * 128, M + 64
+    a, w = torch.randn(M, K, generator=g).to(BF16).cuda(), (torch.randn(N, K, generator=g) / math.sqrt(K)).to(BF16).cuda()
+    qw, kw = ((1 + 0.2 * torch.randn(128, generator=g)).to(BF16).cuda() for _ in range(2))
+    pos = torch.randint(0, 2000, (M,), generator=g, dtype=torch.int32).cuda()
+    slot = torch.randperm(slots, generator=g)[:M].to(torch.int32)
+    slot[2] = -1
+    slot, tab, got = slot.cuda(), ctx.rope_table(1e6, 128, 2000), []
+    for off in (0, 1):
+        nvc.lib().nvc_debug_set(7, off)
+        try:
+            kc = torch.zeros(slots, kv, 128, dtype=BF16, device="cuda")
+            vc = torch.zeros_like(kc)
+            got.append((ctx.qkv_proj_norm_rope(a, w, qw, kw, 1e-6, tab, pos, nh, kv, 128, slot_mapping=slot, k_cache=kc, v_cache=vc), kc, vc))
+        finally:
+            nvc.lib().nvc_debug_set(7, 0)
+    for x, y in zip(*got):
+        assert torch.equal(x.view(torch.int16), y.view(torch.int16))
+
+
 def test_projection_refuses_rows_that_overlap(ctx):
     """A row stride below the row's length is an error in the fused range too."""
     M, nh, kv, K = 1600, 4, 2, 2048
