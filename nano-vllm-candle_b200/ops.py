@@ -442,8 +442,9 @@ def moe_sort_padded(ctx, idx: torch.Tensor, E: int, align: int = 128):
 def gather_rows(ctx, x: torch.Tensor, src: torch.Tensor, num_rows: torch.Tensor) -> torch.Tensor:
     """out[r] = x[src[r]] for r < num_rows[0] (zeros where src[r] < 0); rows behind num_rows keep the fill value."""
     out = torch.empty(src.numel(), x.shape[1], dtype=x.dtype, device=x.device)
+    three = 0x4040 if x.dtype == torch.bfloat16 else int(torch.full((1,), 3, dtype=x.dtype).view(torch.int16)[0])     # 3.0 in the rows' 16-bit type
     check(ctx.l.nvc_gather_rows_bf16_fill(ctx.h, _ptr(x), x.stride(0), _ptr(src), _ptr(num_rows), _ptr(out), out.stride(0), src.numel(),
-                                          x.shape[1], 0x4040, _stream()), "nvc_gather_rows_bf16_fill", ctx.h)       # 0x4040: 3.0
+                                          x.shape[1], three, _stream()), "nvc_gather_rows_bf16_fill", ctx.h)
     return out
 
 

@@ -39,3 +39,12 @@ def test_grouped_product(ctx, ops, tokens, E, E_real, top, N, K, dt, act):
         want = want.clamp(min=0) ** 2 if act else want
         tol = (1e-5 if dt == torch.float32 else 2.0 ** -8) * float(want.abs().max() if len(rows) else 0)
         assert ((y[rows].double() - want).abs() <= tol).all(), k
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_gathered_rows_of_any_16_bit_type(ctx, ops, dt):
+    """Rows are copied as they are; those behind the last group hold 3 in their own type."""
+    x = torch.randn(9, 64, generator=torch.Generator().manual_seed(1)).to(dt).to(DEV)
+    src, n = torch.tensor([4, -1, 0, 7, 7], dtype=torch.int32, device=DEV), torch.tensor([3], dtype=torch.int32, device=DEV)
+    got = ops.gather_rows(ctx, x, src, n)
+    assert torch.equal(got[0], x[4]) and (got[1] == 0).all() and torch.equal(got[2], x[0]) and (got[3:] == 3).all()
