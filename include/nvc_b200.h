@@ -505,7 +505,7 @@ int nvc_attn_paged_wide(nvc_ctx* ctx, const void* q, int ldq, const void* k_cach
  * cu_seqlens[b] .. cu_seqlens[b + 1], or row b when cu_seqlens == NULL).  state: fp32 [slots, heads, dim, vdim]; sequence b
  * uses slot state_slots[b], starts from zeros when positions[first row] == 0 and leaves its last state in the slot.
  * q, k, v, o: fp32 rows.  max_qlen: the longest portion; above 4 tokens the recurrence runs 32 tokens at a time (the same
- * sums regrouped, fp32 FMA), else token by token. */
+ * sums regrouped; up to 128 key channels on the tensor pipe, every number as three bf16 parts, else fp32 FMA), else token by token. */
 int nvc_retention_scan(nvc_ctx* ctx, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, float* o, int ldo,
                        float* state, const int32_t* state_slots, const int32_t* cu_seqlens, const int32_t* positions,
                        const float* decay, int B, int max_qlen, int heads, int dim, int vdim, void* stream);
@@ -586,11 +586,12 @@ typedef struct nvc_delta_prep {
    * the recurrence then multiplies row d of a head's state by that channel's decay.  NULL: one decay per head */
   const float* channel_a; int ldca; float* channel_g;
 } nvc_delta_prep;
-int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int max_qlen, void* stream);   /* max_qlen: the longest portion, or any number */
+int nvc_delta_prep_run(nvc_ctx* ctx, const nvc_delta_prep* p, int N, int max_qlen, void* stream);   /* max_qlen: not used */
 /* The recurrence, per (sequence, head) with state S [dim, vdim] fp32 in state [slots, heads, dim, vdim]:
  *   S <- g S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q        (head h reads q / k head h / (heads / kv_heads))
  * token by token over rows cu_seqlens[b] .. cu_seqlens[b + 1] (row b when cu_seqlens == NULL); a sequence starts from zeros when
- * positions[first row] == 0; portions of 8 tokens and more (max_qlen) run 32 tokens at a time (the same sums regrouped, fp32 FMA).
+ * positions[first row] == 0.  Portions of 8 tokens and more (max_qlen) run several tokens at a time, the same sums regrouped: 32 on the tensor pipe
+ * with every number as three bf16 parts (one decay per head, dim up to 128), 16 in fp32 FMA (decays per channel, dim up to 256).
  * Also advances the convolution state of nvc_delta_prep_run (p->in still holds the step's rows). */
 int nvc_delta_rule_scan(nvc_ctx* ctx, const nvc_delta_prep* p, float* o, int ldo, float* state, int max_qlen, void* stream);
 
