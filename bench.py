@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""Benchmark of the Qwen3 forward hot path (BASELINE.json metric: decode tok/s).
+"""Benchmark of the Qwen3 forward hot path (metric: decode tok/s).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 \
         --master-port P bench.py --gpus N --steps K --warmup W
 
-Headline workload: BASELINE.json configs[1] - Qwen3-0.6B bf16, batch 64, 512-token prompts, decode
+Headline workload: Qwen3-0.6B bf16, batch 64, 512-token prompts, decode
 with ignore_eos, paged KV cache block size 256, random-init (synthetic seeded) weights.  A "step" is
 ONE decode step of the whole batch.  N > 1 runs the same batch tensor-parallel (TP = N, one process
 per GPU, all-reduce after each row-parallel linear): strong scaling.
@@ -20,13 +20,13 @@ One JSON line on stdout (rank 0):
             fp32 oracle (one full-recompute forward each; every generated token must be within 4e-2
             of the oracle's best logit at its step), and - under TP - whether all ranks produced the
             same tokens.  A failed check makes the process exit non-zero.
-  north_star  sub-record: BASELINE.json configs[2]'s decode phase - Qwen3-8B, batch 256, context
+  north_star  sub-record: the decode phase of Qwen3-8B, batch 256, context
             ~1024, device-generated weights - with its own value / clocks and TWO rooflines (paged
             decode vs HBM, layer GEMMs vs the bf16 tensor peak, burst and sustained)
   cpu_baseline  the oracle's restatement of the reference algorithm on the host cores (bounded sample)
 
 --impl reference times that CPU restatement alone (the reference crate is Rust + candle and cannot
-be built on this image; see DESIGN.md).
+be built on this image).
 """
 from __future__ import annotations
 
@@ -51,7 +51,7 @@ CPU_SAMPLE_SEQS = 1          # sequences of the batch the CPU legs process per s
 PARITY_SEQS = 2              # sequences of the benchmarked batch checked against the fp32 oracle
 PARITY_TOL = 4e-2            # worst allowed logit deficit of a generated token (same as tests/test_e2e_gpu.py)
 
-NS_MODEL = "qwen3-8b"        # north-star sub-record (decode phase)
+NS_MODEL = "qwen3-8b"        # second record: decode phase of the 8B model
 NS_BATCH = 256
 NS_PROMPT_LEN = 1000         # + warm-up + timed steps = context ~1024 at timing
 
@@ -78,7 +78,7 @@ def _peaks() -> dict:
         return {"hbm_gbs": float(d["hbm_gbs"]), "bf16_burst": float(d["bf16_tflops"]),
                 "bf16_sustained": float(d.get("bf16_tflops_sustained", d["bf16_tflops"])),
                 "source": "measured (MEASURED_PEAKS.json)"}
-    return {"hbm_gbs": 6650.0, "bf16_burst": 1590.0, "bf16_sustained": 1400.0, "source": "fallback (B200_PROFILING.md)"}
+    return {"hbm_gbs": 6650.0, "bf16_burst": 1590.0, "bf16_sustained": 1400.0, "source": "fallback"}
 
 
 def _host_threads() -> int:
@@ -176,7 +176,7 @@ def cpu_kv_cached_decode(steps: int, model=None):
     """The same fp32 arithmetic on the same host cores WITH a KV cache and last-token logits
     (oracle.Qwen3OracleKVCached - not the reference's algorithm): one sequence, 512-token prompt prefilled once
     (untimed), `steps` timed single-token decode steps.  Separates the algorithmic speed-up (what a KV cache buys
-    the reference on its own hardware) from the hardware speed-up (SURVEY.md section 8d).  Returns tok/s."""
+    the reference on its own hardware) from the hardware speed-up.  Returns tok/s."""
     import torch
     from oracle import qwen3_oracle as O
     synth = importlib.import_module("nano-vllm-candle_b200.synth")

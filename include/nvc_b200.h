@@ -3,7 +3,7 @@
  * behind nano-vllm-candle's layer / runner API.
  *
  * The reference crate has no FFI of its own: its boundary is a set of Rust traits and
- * inherent methods that call candle tensor ops (SURVEY.md section 8b).  Each entry point
+ * inherent methods that call candle tensor ops.  Each entry point
  * below names the reference interface (file:line, relative to the reference crate root)
  * whose body it replaces; INTEGRATION.md shows the Rust `extern "C"` block and the
  * candle CustomOp wrapper a maintainer would add.
@@ -251,7 +251,7 @@ int nvc_prefill_attn_varlen(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_
                             int total_tokens, int max_seqlen, int nh, int kv, int hd, float scale,
                             nvc_bf16* out, void* stream);
 
-/* K4 (paged). The same kernel for sequences with a cached prefix (prefix caching, SURVEY.md 8f.1;
+/* K4 (paged). The same kernel for sequences with a cached prefix (prefix caching;
  * upstream nano-vllm passes block_table to flash_attn_varlen_func for this): q rows of sequence b
  * are the LAST q_len_b = cu_seqlens_q[b+1] - cu_seqlens_q[b] positions of a context of
  * context_lens[b] tokens whose K / V are read from the paged cache through block_tables
@@ -300,7 +300,7 @@ int nvc_paged_decode_attn(nvc_ctx* ctx, const nvc_bf16* q, int ldq, const nvc_bf
                           float scale, nvc_bf16* out, void* workspace, size_t workspace_bytes,
                           void* stream);
 
-/* K5, allocation-free variant.  No counterpart in the reference: added at the request of the run's operators for
+/* K5, allocation-free variant.  No counterpart in the reference: for
  * callers that cannot call cudaMalloc (CUDA graph capture, tight serving loops, harnesses that forbid it).  Same
  * kernels and results as nvc_paged_decode_attn; the KV-split partials go to a static device array inside the
  * library (nvc_paged_decode_static_scratch_bytes() = 4 MiB per GPU, held until exit) instead of a caller workspace.

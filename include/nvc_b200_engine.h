@@ -154,14 +154,14 @@ int nvc_safetensors_read_bf16(const nvc_safetensors* st, const char* name, nvc_b
  * src/engine/llm_engine.rs:135-142). */
 int nvc_runner_prefill(nvc_runner* r, const int32_t* ids, const int32_t* positions, const int32_t* cu_seqlens,
                        const int32_t* slot_mapping, int B, int N, int max_seqlen, int32_t* out_tokens);
-/* Prefill step whose sequences may have a cached prefix (prefix caching, SURVEY 8f.1): the N new
+/* Prefill step whose sequences may have a cached prefix (prefix caching): the N new
  * tokens of sequence b are positions context_lens[b] - q_len_b .. context_lens[b] - 1 and attend
  * to ALL context_lens[b] tokens, read from the paged cache through block_tables [B, max_blocks]
  * (the new tokens' K/V are scattered to slot_mapping first, as in every step). */
 int nvc_runner_prefill_paged(nvc_runner* r, const int32_t* ids, const int32_t* positions, const int32_t* cu_seqlens,
                              const int32_t* slot_mapping, const int32_t* block_tables, int max_blocks,
                              const int32_t* context_lens, int B, int N, int max_seqlen, int32_t* out_tokens);
-/* Mixed step (chunked prefill, SURVEY 8f.2): the first num_decode sequences have exactly one query
+/* Mixed step (chunked prefill): the first num_decode sequences have exactly one query
  * token (cu_seqlens[b] == b) and attend through the paged DECODE kernel (K5); the other B -
  * num_decode sequences are prompt chunks of any length through the paged PREFILL kernel (K4
  * paged); everything else (embedding, norms, GEMMs, KV store, head) runs once over all N tokens.
@@ -212,7 +212,7 @@ typedef struct nvc_scheduler_config {
   int32_t eos;
   int32_t num_kvcache_blocks;
   int32_t kvcache_block_size;
-  /* Beyond the reference (SURVEY.md section 8f); 0 = the reference's behaviour. */
+  /* Beyond the reference; 0 = the reference's behaviour. */
   int32_t enable_prefix_caching;   /* 8f.1: hash-chained dedup of full KV blocks (upstream nano-vllm's
                                       BlockManager, which block_manager.rs:24-29 says it will mirror)     */
   int32_t enable_chunked_prefill;  /* 8f.2: one step = the decode tokens of the running sequences + as many prompt

@@ -1,5 +1,5 @@
 // K9: tensor-parallel collectives.  The reference has none (src/tp.rs:1-70 is config only,
-// src/layers/linear.rs:184-198 does no all-reduce); north_star (4) adds an all-reduce after
+// src/layers/linear.rs:184-198 does no all-reduce); tensor parallelism needs one after
 // each row-parallel linear.  NCCL is resolved at run time with dlopen so that the library
 // loads (and TP=1 runs) without it; with torch in the process this binds to the same
 // libnccl.so.2 torch already loaded.

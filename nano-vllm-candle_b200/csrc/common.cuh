@@ -80,7 +80,7 @@ static inline cudaStream_t nvc_stream(void* s) { return reinterpret_cast<cudaStr
 // kernel of the step produces; operands no kernel of the step writes (weights, norm vectors, rope
 // table, positions / slot_mapping / block_tables / context_lens, older cache rows) may be fetched
 // ahead of the wait - the early-launch chain can be several kernels deep, so "written two kernels
-// ago" is NOT safe before the wait (DESIGN.md 4.3).
+// ago" is NOT safe before the wait.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t nvc_launch_cluster3(const nvc_ctx* ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                               size_t smem, cudaStream_t stream, dim3 cluster, Args&&... args) {

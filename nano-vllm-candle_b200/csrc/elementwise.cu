@@ -511,7 +511,7 @@ extern "C" int nvc_argmax_last(nvc_ctx* ctx, const float* logits, int ld, int32_
 }
 
 // ------------------------------------------------------------------------------------
-// K8s temperature sampling on device (SURVEY 8f.3).  Replaces Qwen3ModelRunner::sample_token
+// K8s temperature sampling on device.  Replaces Qwen3ModelRunner::sample_token
 // (llm_engine.rs:97-133: softmax((l - max) / max(T, 1e-6)) then WeightedIndex with an UNSEEDED
 // rand::rng(), i.e. not reproducible) by the Gumbel-max form of the same categorical draw:
 //   token = argmax_i ( l_i / T + g_i ),  g_i = -log(-log(u_i)),  u_i uniform in (0, 1)

@@ -9,7 +9,7 @@
 //                 can_append, may_append grows the table when len % block_size == 1)
 //   Scheduler     src/engine/scheduler.rs:58-250     (same control flow, statement by statement)
 //   LLMEngine     src/engine/llm_engine.rs:209-326
-// plus the integer contract the north_star adds (N1 slot_mapping, N2 block_tables), written
+// plus the integer contract of the paged cache (N1 slot_mapping, N2 block_tables), written
 // only in terms of the Sequence helpers the reference exposes (sequence.rs:73-91).
 #include <algorithm>
 #include <cstdint>
@@ -36,7 +36,7 @@ struct Sequence {
   size_t num_tokens = 0;
   size_t num_prompt_tokens = 0;
   size_t num_cached_tokens = 0;
-  size_t num_computed_tokens = 0;   // chunked prefill (SURVEY 8f.2): tokens whose K / V are in the cache
+  size_t num_computed_tokens = 0;   // chunked prefill: tokens whose K / V are in the cache
   double temperature = 1.0;
   size_t max_tokens = 64;
   bool ignore_eos = false;
@@ -109,7 +109,7 @@ struct FreeList {
 
 // BlockManager (block_manager.rs:31-99).  The reference's is an admitted stub (:24-29); this one
 // keeps its method set and follows upstream nano-vllm's allocator, which the reference says its
-// API mirrors: FIFO free list, ref-counted blocks and - when `prefix_caching` is on (SURVEY 8f.1) -
+// API mirrors: FIFO free list, ref-counted blocks and - when `prefix_caching` is on -
 // hash-chained dedup of FULL blocks.  One rule is added to upstream's: a block is taken from the
 // cache only if at least one token of the sequence is left to compute ((i+1)*block_size < len),
 // otherwise a fully cached prompt would schedule a prefill step with no query tokens.
@@ -345,7 +345,7 @@ struct Scheduler {
     waiting.push_front(seq);
   }
 
-  // Chunked prefill (SURVEY 8f.2; no counterpart in the reference, whose schedule() is either a
+  // Chunked prefill (no counterpart in the reference, whose schedule() is either a
   // whole-prompt prefill step or a decode step, scheduler.rs:106-111).  One step =
   //   1. every running sequence, in queue order as schedule_decode visits them: a sequence with one
   //      pending token (decode, or the last token of its prompt) appends exactly as in
@@ -451,14 +451,14 @@ struct nvc_engine {
   std::vector<SeqPtr> batch;
   bool batch_is_prefill = false;
   bool batch_valid = false;
-  bool chunked = false;                        // chunked prefill / mixed steps (SURVEY 8f.2)
+  bool chunked = false;                        // chunked prefill / mixed steps
   int num_decode = 0;                          // leading one-token sequences of the batch
   std::vector<int32_t> q_lens, emit;           // per sequence of the batch
   std::vector<int32_t> ids, positions, cu_seqlens, slot_mapping, block_tables, context_lens, out_tokens;
   std::vector<int64_t> seq_ids;
   std::vector<int32_t> state_slots;            // per sequence of the batch (-1 when the model keeps no recurrent state)
   int max_blocks = 0, max_seqlen = 0;
-  bool sampling = false;                       // on-device temperature sampling (SURVEY 8f.3)
+  bool sampling = false;                       // on-device temperature sampling
   uint64_t sampling_seed = 0;
   std::vector<float> temps;
   std::vector<uint64_t> streams;

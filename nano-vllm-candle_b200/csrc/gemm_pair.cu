@@ -43,7 +43,7 @@ constexpr int kRingBudget = 200 * 1024;
 // schedule overlaps the epilogue).  NT in [128, 256): one narrower MMA per k-step, two accumulator stages - more,
 // smaller tiles when 256-wide ones quantise badly onto the 74 pairs (96 tiles = two waves of which the second is 30 %
 // full; 128 tiles of 192 = two full waves of 3/4 the work each).  (Wide tiles, NT in (256, 512] as two MMAs per k-step
-// into one accumulator stage, measured no gain - 8B gate_up at batch 256: 53.1 vs 53.6 us - and were deleted in round 2.)
+// into one accumulator stage, measured no gain - 8B gate_up at batch 256: 53.1 vs 53.6 us - and are gone.)
 template <int NT>
 struct PairCfg {
   static_assert(NT == 64 || (NT >= 128 && NT <= 256 && NT % 32 == 0), "tile width");

@@ -1,4 +1,4 @@
-// Native HF checkpoint loading behind the C ABI (SURVEY 8f.3): config.json, safetensors files
+// Native HF checkpoint loading behind the C ABI: config.json, safetensors files
 // (single or sharded through model.safetensors.index.json), bf16 / f16 / f32 tensors, tied
 // embeddings.  Replaces Qwen3Config::from_hf_dir (src/models/qwen3.rs:77-101) and
 // Qwen3ForCausalLM::from_hf_dir (:515-536), which goes through candle's VarBuilder over ONE

@@ -1,6 +1,6 @@
 // K9 on NVLS: all-reduce through the NVSwitch multicast object of the TP group, fused with the residual
 // add and RMSNorm that always follow a row-parallel linear (o_proj: src/layers/linear.rs:184-198; down_proj:
-// src/models/qwen3.rs:326 - the reference has no collective there, north_star (4) adds one).
+// src/models/qwen3.rs:326 - the reference has no collective there, tensor parallelism needs one).
 //
 // Every rank owns one physical buffer (cuMemCreate) that is bound into ONE multicast object
 // (cuMulticastCreate / AddDevice / BindMem) and mapped twice: at a unicast address (this rank's copy) and

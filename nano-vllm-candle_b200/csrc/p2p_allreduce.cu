@@ -209,7 +209,7 @@ extern "C" int nvc_p2p_allreduce_rmsnorm(nvc_ctx* ctx, int slot, const float* re
   const int threads = ((H / 8 + 31) / 32) * 32;
   cudaStream_t st = nvc_stream(stream);
   // (a two-shot variant - reduce-scatter by peer loads, all-gather by peer stores, second flag barrier - measured slower at
-  // every size on 8 x B200, 44 vs 39 us for 2 MB, and was deleted in round 2; large messages go through the switch, nvls_allreduce.cu)
+  // every size on 8 x B200, 44 vs 39 us for 2 MB, and is gone; large messages go through the switch, nvls_allreduce.cu)
 #define NVC_AR(TPV)                                                                                              \
   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, p2p_allreduce_rmsnorm_kernel<TPV>, dim3(N), dim3(threads), 0, st,          \
                                  (uint8_t* const*)ctx->p2p_peer_d, ctx->p2p_state, ctx->tp_rank, off,            \

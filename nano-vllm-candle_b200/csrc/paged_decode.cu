@@ -192,7 +192,7 @@ extern "C" int nvc_paged_decode_attn(nvc_ctx* ctx, const nvc_bf16* q, int ldq, c
                                   nh, kv, hd, block_size, scale, out, workspace, workspace_bytes, stream);
 }
 
-// K5 without any allocation (no counterpart in the reference; added at the request of the run's operators): the same
+// K5 without any allocation (no counterpart in the reference): the same
 // kernels as nvc_paged_decode_attn, the KV-split partials in the library's static device array (4 MiB) instead of a caller
 // workspace.  Calls no cudaMalloc / cudaFree; every call on a device shares the one array, so calls that overlap on the GPU
 // (two streams) race - serialise them.  Nothing has to start at zero: every (sequence, head, split) partial the combine

@@ -7,10 +7,10 @@
 // The kernel is prefill_attn_v2.cuh (persistent grid, 128-row q tiles x 64-token kv tiles, TMA over 3-D tensor maps
 // {head_dim, head, token} so q / k / v are read in place from the fused qkv rows, S / P / O in tensor memory); this file
 // holds the tensor maps, the launchers and the C ABI.  The first-generation kernel (one CTA per SM, 128-token kv tiles,
-// output accumulator in registers: 215-396 TFLOP/s, profiles/r01_s14_prefill_attn_v2.md) was deleted in round 2.
+// output accumulator in registers: 215-396 TFLOP/s, profiles/r01_s14_prefill_attn_v2.md) is gone.
 // FLOPs per (sequence, head): 4 * 128 * T^2 / 2 (causal).
 //
-// kPaged = true (prefix caching, SURVEY 8f.1): the q rows of sequence b are its LAST q_len
+// kPaged = true (prefix caching): the q rows of sequence b are its LAST q_len
 // positions of a context of context_lens[b] tokens; K / V tiles are read from the paged cache
 // through block_tables (one TMA box per block, or per 64 tokens when block_size >= 64), after
 // qk_norm_rope_store has scattered this step's k / v there.  Cache rows past the context may

@@ -53,9 +53,9 @@ class SchedulerConfig:
     eos: int = 0
     num_kvcache_blocks: int = 0
     kvcache_block_size: int = 256
-    enable_prefix_caching: bool = False      # beyond the reference (SURVEY 8f.1); off = reference behaviour
+    enable_prefix_caching: bool = False      # beyond the reference; off = reference behaviour
 
-    enable_chunked_prefill: bool = False     # beyond the reference (SURVEY 8f.2): mixed prefill / decode steps
+    enable_chunked_prefill: bool = False     # beyond the reference: mixed prefill / decode steps
     max_model_len: int = 0                   # 0 = the runner's: a sequence that reaches it finishes, a longer prompt is refused
 
     def with_chunked_prefill(self, on: bool = True):
@@ -139,7 +139,7 @@ def _cfg(H, L, nh, kv, I, V=151936, maxpos=40960, bos=151643, eos=151645) -> Qwe
                        bos_token_id=bos, eos_token_id=eos)
 
 
-# Published Qwen3 dense shapes (SURVEY.md section 8) + a toy shape for fast tests.
+# Published Qwen3 dense shapes + a toy shape for fast tests.
 MODEL_CONFIGS: Dict[str, Qwen3Config] = {
     "qwen3-0.6b": _cfg(1024, 28, 16, 8, 3072),
     "qwen3-8b": _cfg(4096, 36, 32, 8, 12288),
@@ -185,7 +185,7 @@ class Qwen3ModelRunner:
     Greedy by default: a step returns argmax with the reference's tie rule (last maximum).  The
     reference's temperature path draws from an unseeded RNG (llm_engine.rs:128) and cannot be
     reproduced; `set_sampling` / `LLMEngine.set_sampling` arm the seeded on-device sampler instead
-    (Gumbel-max on Philox noise, SURVEY 8f.3).  Steps: `prefill` (whole prompts), `decode` (one token
+    (Gumbel-max on Philox noise).  Steps: `prefill` (whole prompts), `decode` (one token
     per sequence, CUDA graph), `step_mixed` (chunked prefill: decode rows + prompt chunks)."""
 
     def __init__(self, ctx, cfg: Qwen3Config, num_kvcache_blocks: int, kvcache_block_size: int = 256,

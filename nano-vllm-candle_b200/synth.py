@@ -1,8 +1,8 @@
 """Seeded synthetic Qwen3 checkpoints and prompts (data generation only: numpy on the host,
 no model math; shared by bench.py, the tests and the oracle's golden-vector generator).
 
-No Qwen3 weights exist on this box or the GPU box, and the reference's own random-init
-constructors are broken (SURVEY.md section 3.5), so "random-init" means: an HF-format
+No Qwen3 weights are at hand, and the reference's own random-init
+constructors are broken, so "random-init" means: an HF-format
 checkpoint with seeded tensors, loaded through the from_hf_dir path
 (src/models/qwen3.rs:515-536 tensor names and shapes).
 
@@ -97,7 +97,7 @@ def write_hf_dir(path: str, cfg, weights: Dict[str, torch.Tensor]) -> None:
 
 
 def make_prompts(num: int, length, vocab: int, seed: int) -> List[List[int]]:
-    """Uniform random token ids in [0, vocab) (BASELINE.md section 4).  `length` is an int
+    """Uniform random token ids in [0, vocab).  `length` is an int
     or an inclusive (lo, hi) range."""
     rng = np.random.Generator(np.random.PCG64(seed))
     out = []

@@ -6,7 +6,7 @@ anything from this directory.  Only ``tests/``, ``__graft_entry__.smoke()``
 and ``bench.py``'s ``cpu_baseline`` / ``--impl reference`` legs use it, and
 only as the checker / the timed CPU baseline.
 
-Parity status (see DESIGN.md section "Oracle"):
+Parity status:
   * Linear, RMSNorm, SiluAndMul, TP shard arithmetic, GQA interleave:
     pinned by the reference's own unit-test vectors (tests/test_oracle_goldens.py).
   * RoPE: pinned by the reference's norm-preservation properties only.

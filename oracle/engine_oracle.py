@@ -8,10 +8,10 @@ Reference files followed:
 
 The reference BlockManager is an admitted stub (block_manager.rs:24-29: identity
 block_table, always-true capacity).  `BlockManagerStub` restates it as written;
-`BlockManager` is the real allocator the north_star contract needs (free list,
+`BlockManager` is the real allocator the paged cache needs (free list,
 disjoint ids), following upstream nano-vllm's rule which the reference says its API
 mirrors (block_manager.rs:26-29); `BlockManagerPrefix` adds upstream's hash-chained
-prefix cache (SURVEY section 8f item 1).
+prefix cache.
 The slot_mapping rule (N1) is expressed only with the Sequence helpers the reference
 exposes (sequence.rs:73-91).
 """
@@ -441,7 +441,7 @@ class Scheduler:
 
 
 class SchedulerChunked(Scheduler):
-    """Chunked prefill with mixed prefill / decode steps (SURVEY section 8f item 2).  The reference
+    """Chunked prefill with mixed prefill / decode steps.  The reference
     has no such mode (scheduler.rs:106-111 is prefill-step-or-decode-step); this restates the
     rule the C++ engine implements, written independently from the same specification:
 

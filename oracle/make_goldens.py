@@ -2,12 +2,12 @@
 
     python -m oracle.make_goldens [--model qwen3-0.6b] [--prompt-seeds 1 2 3 ...]
 
-Qwen3-0.6B shapes, synthetic checkpoint seed 0, ONE sequence, 32-token
+The golden workload: Qwen3-0.6B shapes, synthetic checkpoint seed 0, ONE sequence, 32-token
 prompt (uniform ids, seed = prompt seed), 64 greedy tokens, ignore_eos, run with the
 reference's algorithm (full recompute every step, all-position logits, host argmax with the
 last-maximum tie rule).  For every step the top-2 logit gap is recorded: greedy identity
 between a bf16 path and the fp32 reference is only meaningful on prompts whose minimum gap is
-well above the bf16 path's logit error (hard part 1).  The first prompt
+well above the bf16 path's logit error.  The first prompt
 seed whose minimum gap is >= --min-gap becomes the asserted fixture; the others are recorded
 with their gaps.
 """

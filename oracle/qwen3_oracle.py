@@ -71,7 +71,7 @@ class Qwen3Config:
         return d
 
 
-# Published Qwen3 dense configs (SURVEY.md section 8 table).
+# Published Qwen3 dense configs.
 MODEL_CONFIGS: Dict[str, Qwen3Config] = {
     "qwen3-0.6b": Qwen3Config(),
     "qwen3-8b": Qwen3Config(hidden_size=4096, num_hidden_layers=36, num_attention_heads=32,
@@ -293,7 +293,7 @@ class Qwen3OracleKVCached:
     positions are kept per layer, a step computes only the new positions and logits only for the
     last one.  Not the reference's algorithm (it recomputes everything each step,
     src/engine/llm_engine.rs:146-189) - it exists so that bench.py can separate the ALGORITHMIC
-    speed-up (KV cache, last-token logits) from the hardware speed-up (SURVEY.md section 8d), and
+    speed-up (KV cache, last-token logits) from the hardware speed-up, and
     tests/test_oracle_goldens.py checks it against the full-recompute oracle."""
 
     def __init__(self, model: Qwen3Oracle, max_len: int):

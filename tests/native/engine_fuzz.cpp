@@ -2,7 +2,7 @@
 //
 // Links csrc/engine.cpp and csrc/hf_loader.cpp against a STUB model runner defined here, so that the
 // engine -> runner call path (which the Python CPU tests cannot reach: a real runner needs a device) is exercised:
-// the stub checks every step's inputs against the integer contract of SURVEY 8 N1-N3 (slot_mapping, block_tables,
+// the stub checks every step's inputs against the integer contract (slot_mapping, block_tables,
 // context_lens, cu_seqlens) exactly as csrc/runner.cu validates them, and answers next = last token + 1 like
 // DummyModelRunner (llm_engine.rs:20-33).  It also keeps a model of the paged KV cache (g_kv below).  Random valid and
 // invalid call sequences; any contract violation, sanitizer report or wrong output aborts.  test_native_asan.py also
@@ -450,7 +450,7 @@ int main(int argc, char** argv) {
     for (int guard = 0; guard < 20000 && !nvc_engine_is_finished(e); ++guard) {
       nvc_step_output out;
       g_trace += " drain";
-      if (nvc_engine_step(e, &out) != 0) break;                      // e.g. the reference-mode stall (DESIGN.md section 5)
+      if (nvc_engine_step(e, &out) != 0) break;                      // e.g. the reference-mode stall
     }
     if (nvc_engine_is_finished(e)) {
       REQUIRE(nvc_engine_num_free_blocks(e) == cfg.num_kvcache_blocks);

@@ -1,7 +1,7 @@
 """End-to-end GPU parity: the whole hot path (runner + engine through the C ABI) against the
 oracle's full-recompute fp32 forward on the same synthetic checkpoints.
 
-Tolerances (BASELINE.json north_star): logits max-abs <= 2e-2 and cosine >= 0.999 against the
+Tolerances: logits max-abs <= 2e-2 and cosine >= 0.999 against the
 fp32 reference; greedy tokens identical.  Token identity between a bf16 path and an fp32
 reference is only decidable where the reference's top-2 logit gap exceeds the bf16 path's
 logit error, so a mismatch is accepted ONLY at a step whose recorded fp32 gap is below
@@ -130,7 +130,7 @@ def test_greedy_generation_with_preemption_tiny(tiny):
 
 
 def test_prefix_caching_generation_matches_oracle_tiny(tiny):
-    """with prefix caching on, sequences that share full KV blocks skip them in
+    """With prefix caching on, sequences that share full KV blocks skip them in
     prefill (paged K4 reads the prefix through block_tables); every token must still be the
     oracle's full-recompute greedy choice up to numerical ties, and the cache must have hit."""
     cfg, runner, fp32, _ = tiny
@@ -155,7 +155,7 @@ def test_prefix_caching_generation_matches_oracle_tiny(tiny):
 def test_prefix_cached_prefill_logits_match_uncached(tiny):
     """The same prompt prefilled twice, the second time with its first blocks served from the
     cache: last-token logits agree with the uncached run to bf16 rounding and with the oracle
-    within the north_star tolerance."""
+    within the logit tolerance."""
     cfg, runner, fp32, _ = tiny
     bs = 16
     prompt = synth.make_prompts(1, 4 * bs + 7, cfg.vocab_size, 950)[0]
@@ -185,7 +185,7 @@ def test_prefix_cached_prefill_logits_match_uncached(tiny):
 
 
 def test_chunked_prefill_generation_matches_oracle_tiny(tiny):
-    """mixed steps (decode tokens through paged decode attention next to prompt chunks
+    """Mixed steps (decode tokens through paged decode attention next to prompt chunks
     through paged prefill attention, one pass of everything else over all tokens).  Prompts longer
     than the 24-token budget are split over steps while earlier sequences keep decoding; every
     token must be the fp32 oracle's full-recompute greedy choice up to numerical ties."""
@@ -212,7 +212,7 @@ def test_chunked_prefill_generation_matches_oracle_tiny(tiny):
 def test_mixed_step_logits_match_whole_prompt_prefill(tiny):
     """One prompt prefilled whole (K4 varlen) and again in three chunks riding along with two
     decoding sequences (nvc_runner_step_mixed): last-token logits agree to bf16 rounding and with
-    the fp32 oracle within the north_star tolerance; the decode rows of the mixed step equal a
+    the fp32 oracle within the logit tolerance; the decode rows of the mixed step equal a
     plain decode step's logits for the same state within the same tolerance."""
     cfg, runner, fp32, _ = tiny
     bs = 16
@@ -285,7 +285,7 @@ def test_mixed_step_rejects_inconsistent_inputs(tiny):
 
 
 def test_on_device_sampling_is_reproducible_and_follows_the_oracle(tiny):
-    """SURVEY 8f.3: temperature sampling on device (seeded Gumbel-max).  Same seed -> same tokens;
+    """Temperature sampling on device (seeded Gumbel-max).  Same seed -> same tokens;
     every sampled token, teacher-forced through the fp32 oracle with the same Philox stream
     (seq_id, step), must be within tolerance of the oracle's best perturbed score."""
     from oracle import sampling_oracle as S
@@ -310,7 +310,7 @@ def test_on_device_sampling_is_reproducible_and_follows_the_oracle(tiny):
         for i, t in enumerate(toks):
             row = logits[len(p) - 1 + i].numpy()
             sc = S.gumbel_scores(row, T, seed, S.stream_id(sid, i))
-            # logits within 2e-2 of the oracle (north_star) -> scores within 2e-2 / T, both sides
+            # logits within 2e-2 of the oracle -> scores within 2e-2 / T, both sides
             assert sc.max() - sc[t] <= 2 * 2e-2 / T + 1e-4, f"seq {sid} step {i}: token {t} is {sc.max() - sc[t]:.4f} below the best draw"
             exact += int(S.sample(row, T, seed, S.stream_id(sid, i)) == t)
             total += 1
@@ -334,7 +334,7 @@ def test_causality_property(tiny):
 
 @pytest.mark.parametrize("name", ["qwen3-0.6b_cfg0.json"])
 def test_config0_golden_tokens(ctx, name):
-    """BASELINE config 0 (Qwen3-0.6B shapes, 1 seq, 32-token prompt, 64 greedy tokens): tokens and
+    """The golden workload (Qwen3-0.6B shapes, 1 seq, 32-token prompt, 64 greedy tokens): tokens and
     top logits committed by oracle/make_goldens.py from the fp32 full-recompute oracle."""
     path = os.path.join(GOLD, name)
     if not os.path.exists(path):
@@ -366,7 +366,7 @@ def test_config0_golden_tokens(ctx, name):
             n16 = next((i for i, (a, b) in enumerate(zip(toks, case["tokens_bf16_mode"])) if a != b), len(toks))
             diag(f"[golden {g['model']} prompt seed {case['prompt_seed']}] top-8 logit max-abs err {err:.4e}; tokens equal to "
                  f"fp32 oracle for {n32}/{len(toks)}, to bf16-mode oracle for {n16}/{len(toks)}; min fp32 gap {case['min_gap_fp32']:.4f}")
-            assert err <= 2e-2, "step-0 logits outside the north_star tolerance"
+            assert err <= 2e-2, "step-0 logits outside the logit tolerance"
             _teacher_forced_check(fp32, case["prompt"], toks, 4e-2, f"golden {g['model']} seed {case['prompt_seed']}")
             if n32 < len(toks):
                 gap = case["gaps_fp32"][n32]

@@ -139,7 +139,7 @@ def test_kv_pool_exhaustion_is_an_error_not_an_abort():
         cpp.step()                   # the reference asserts here (scheduler.rs:175-178)
 
 
-# ----------------------------------------------------------------------------- prefix caching (SURVEY 8f.1)
+# ----------------------------------------------------------------------------- prefix caching
 def _shared_prefix_prompts(rng, bs, n, n_prefixes=3):
     """Prompts that share block-aligned and unaligned prefixes, plus exact duplicates."""
     prefixes = [rng.integers(10, 1000, size=int(rng.integers(1, 5)) * bs + int(rng.integers(0, bs))).tolist()
@@ -223,7 +223,7 @@ def test_prefix_caching_off_is_the_default_and_never_caches():
     assert si.cu_seqlens.tolist() == [0, 40] and cpp.prefix_cache_stats() == (0, 0)
 
 
-# ----------------------------------------------------------------------------- chunked prefill (SURVEY 8f.2)
+# ----------------------------------------------------------------------------- chunked prefill
 def _mk_chunked(max_num_seqs, budget, nblocks, bs, eos=0, prefix=False):
     cfg = eng.SchedulerConfig().with_max_num_seqs(max_num_seqs).with_max_num_batched_tokens(budget) \
         .with_eos(eos).with_kvcache(nblocks, bs).with_prefix_caching(prefix).with_chunked_prefill(True)
@@ -346,7 +346,7 @@ def test_chunked_prefill_decode_tokens_ride_along_with_a_new_prompt():
 
 
 def test_chunked_prefill_bounds_all_running_sequences():
-    """SURVEY 8f.2: max_num_seqs bounds the running set, not one scheduling round (scheduler.rs:118)."""
+    """max_num_seqs bounds the running set, not one scheduling round (scheduler.rs:118)."""
     cpp, _ = _mk_chunked(2, 64, 32, 16)
     sp = eng.SamplingParams(1.0, 4, True)
     for i in range(5):
@@ -490,7 +490,7 @@ def test_preempted_sequence_that_outgrew_the_budget_stalls_the_reference_but_not
     """Found by the fuzz test: with max_num_batched_tokens = 14, a 14-token prompt that is preempted after 19
     generated tokens can never be prefilled again (33 > 14: scheduler.rs:125-130 refuses, then the decode stage has
     nothing to schedule and the reference asserts, :175-178).  The C++ engine reports it as a status; the chunked
-    scheduler (SURVEY 8f.2) re-prefills the sequence in chunks and finishes."""
+    scheduler re-prefills the sequence in chunks and finishes."""
     bs, nblocks, max_tokens = 16, 8, 20
     prompts = [[100], [100], [100], [100] * 14]
     cpp, orc = _mk(4, 14, nblocks, bs, eos=7)
@@ -615,7 +615,7 @@ def test_engine_c_abi_survives_random_call_sequences():
 
 
 def test_revived_cached_block_stays_ready_for_later_hits():
-    """chunked prefill + prefix caching.  A finishes (its blocks go to the free list, hashes kept); B takes
+    """Chunked prefill + prefix caching.  A finishes (its blocks go to the free list, hashes kept); B takes
     them back from the cache; C, admitted while B is still running, must hit the same blocks - a revived block keeps
     its `ready` flag (its K / V are still there).  The oracle mirrors the rule; both must count the same hits."""
     bs = 4
@@ -639,7 +639,7 @@ def test_revived_cached_block_stays_ready_for_later_hits():
 
 
 def test_max_model_len_finishes_sequences_and_refuses_long_prompts():
-    """the engine knows the longest sequence the runner holds.  A sequence that grows to it finishes like
+    """The engine knows the longest sequence the runner holds.  A sequence that grows to it finishes like
     one that reached max_tokens (instead of failing a later step with 'position out of range'); a prompt that is
     longer is refused at add_request."""
     cfg = eng.SchedulerConfig(4, 256, -1, 32, 16)

@@ -216,7 +216,7 @@ def test_argmax_last_index(ctx, B, V):
     assert torch.equal(val.cpu(), logits.max(dim=1).values)
 
 
-# ----------------------------------------------------------------------------- K8s sampling (SURVEY 8f.3)
+# ----------------------------------------------------------------------------- K8s sampling
 @pytest.mark.parametrize("B,V,offset", [(5, 2048, 0), (3, 151936, 0), (4, 18992, 37984), (100, 32768, 0), (64, 151936, 0)])
 def test_sample_gumbel_matches_oracle(ctx, B, V, offset):
     """Device Gumbel-max draw against oracle/sampling_oracle.py (same Philox counters).  The noise

@@ -1,6 +1,6 @@
 """Host side under AddressSanitizer + UBSan: tests/native/engine_fuzz.cpp links csrc/engine.cpp and
 csrc/hf_loader.cpp against a stub model runner that checks every step's inputs against the integer
-contract (slot_mapping / block_tables / context_lens / cu_seqlens, SURVEY 8 N1-N3) the way csrc/runner.cu
+contract (slot_mapping / block_tables / context_lens / cu_seqlens) the way csrc/runner.cu
 validates them, and drives random call sequences + mutated checkpoint files.  CPU only; no oracle involved."""
 import os
 import shutil

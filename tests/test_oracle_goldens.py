@@ -1,5 +1,5 @@
 """Pins the CPU oracle against every golden vector / known-answer test the reference's own test
-suite holds for this path that can run without real Qwen3 weights (SURVEY.md section 8c)."""
+suite holds for this path that can run without real Qwen3 weights."""
 import json
 import os
 
@@ -184,7 +184,7 @@ def test_hf_transformers_crosscheck():
 
 
 def test_kv_cached_cpu_variant_equals_full_recompute():
-    """the KV-cached CPU variant that bench.py times next to the reference algorithm is the
+    """The KV-cached CPU variant that bench.py times next to the reference algorithm is the
     same arithmetic - prefill in two chunks + decode steps reproduce the full-recompute logits."""
     import torch
     from oracle import synth

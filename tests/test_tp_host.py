@@ -89,7 +89,7 @@ def _free_port():
 
 
 def _rank_main_chunked(rank, world, port, q):
-    """Chunked prefill (SURVEY 8f.2) under TP: the scheduler is replicated, so every rank must build
+    """Chunked prefill under TP: the scheduler is replicated, so every rank must build
     the same mixed batches (ids / positions / cu_seqlens / slots / block tables / emit mask) with
     requests arriving while others are mid-prompt."""
     os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), RANK=str(rank), WORLD_SIZE=str(world))

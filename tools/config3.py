@@ -1,10 +1,10 @@
-"""BASELINE config 3: Qwen3-8B bf16 on 1 x B200, batch 256 mixed prefill / decode, paged KV cache
-block size 256 (SURVEY.md section 8d: half of the sequences arrive at step 0, half staggered so
+"""Qwen3-8B bf16 on 1 x B200, batch 256 mixed prefill / decode, paged KV cache
+block size 256 (half of the sequences arrive at step 0, half staggered so
 that prefill and decode work interleave; prompt lengths uniform [256, 1024] seed 3; 256 decode
 tokens, ignore-eos).  Runs the whole job through LLMEngine.step() twice:
 
   reference scheduling   a step is a whole-prompt prefill step OR a decode step (scheduler.rs:106-111)
-  chunked prefill        mixed steps under a token budget (SURVEY 8f.2)
+  chunked prefill        mixed steps under a token budget
 
 and reports wall-clock job throughput plus the time between consecutive tokens of a sequence
 (the stall a running sequence sees while prompts are prefilled).
@@ -114,7 +114,7 @@ def main():
     rows = [run(eng, runner, cfg, prompts, arrivals, a.decode_tokens, nblocks, ref_budget, False)]
     for b in a.budget:
         rows.append(run(eng, runner, cfg, prompts, arrivals, a.decode_tokens, nblocks, max(b, B), True))
-    out = dict(config="BASELINE configs[2]: %s bf16, 1 x B200, batch %d mixed prefill/decode, block size 256" % (a.model, B),
+    out = dict(config="%s bf16, 1 x B200, batch %d mixed prefill/decode, block size 256" % (a.model, B),
                prompt_lens="uniform[%d, %d] seed 3 (sum %d)" % (a.min_prompt, a.max_prompt, int(lens.sum())),
                arrivals="half at step 0, then one sequence every second step", decode_tokens_per_seq=a.decode_tokens,
                timing="wall clock around the whole job through LLMEngine schedule / runner step / post_process", runs=rows)

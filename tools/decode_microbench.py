@@ -1,4 +1,4 @@
-"""GPU microbenchmark of the paged decode attention kernel: achieved HBM GB/s for the BASELINE
+"""GPU microbenchmark of the paged decode attention kernel: achieved HBM GB/s for the Qwen3
 shapes, timed with CUDA graphs over several distinct KV pools (working set >> L2)."""
 import importlib
 import json

@@ -1,13 +1,13 @@
 """Parity + latency of the NVLS (NVSwitch multicast) all-reduce kernels, one process per GPU:
 
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 \
-        --master-port 29513 tools/nvls_check.py --out gpurun_out/nvls_N.jsonl
+        --master-port 29513 tools/nvls_check.py --out nvls_N.jsonl
 
 For every (rows, hidden, mode): each rank holds its own partial sums; the kernel's output (sum over ranks
 + residual, RMSNorm) is compared with a torch fp32 evaluation of the same expression on the all-gathered
 partials (test driver: torch is the checker here, not the product), and the outputs of all ranks must be
 bit-identical.  Then the same call is timed back to back from a CUDA graph (28 calls per replay, max over
-ranks), next to the peer-load kernel of round 1 and NCCL all-reduce + the norm kernel."""
+ranks), next to the peer-load kernel and NCCL all-reduce + the norm kernel."""
 import argparse
 import ctypes as C
 import importlib

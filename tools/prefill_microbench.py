@@ -1,5 +1,5 @@
 """GPU microbenchmark of the prefill attention kernel (K4): TFLOP/s (causal flops 4 * nh * 128 * T^2 / 2 per
-sequence) for the BASELINE shapes, both kernel generations, CUDA events around back-to-back launches over
+sequence) for the Qwen3 shapes, both kernel generations, CUDA events around back-to-back launches over
 distinct qkv buffers (working set >> L2 where the shape allows)."""
 import importlib
 import json

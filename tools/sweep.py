@@ -1,4 +1,4 @@
-"""Throughput sweep for the BASELINE.md table: prefill tok/s and decode tok/s at several batch
+"""Throughput sweep table: prefill tok/s and decode tok/s at several batch
 sizes for one model (synthetic device-generated weights), with the HBM / tensor roofline
 fractions.  One process per GPU (TP = WORLD_SIZE) when launched with torch.distributed.run.
 
