@@ -21,9 +21,12 @@
 // context length, which only the device knows, so the kernel decides there.  A warp's ring covers about 15 GB/s whatever else the SM does, so among
 // contexts of different lengths the longest ones set the time.  When the longest exceeds 7/4 of the average, units are taken longest first, by teams of
 // four warps; a CTA takes a second unit from the short end.  Otherwise teams of two, all resident at once, as without kTeams; one level lower (5/4) the
-// ordered form loses at 64 contexts of 300 - 600.  The first tile of the teams of two is on its way before the lengths are looked at: it costs the ordered form
-// little, and where the lengths are equal nothing waits for them.  Larger grids, and batches of more than 128, run without kTeams: CTAs are many, each would
-// read all the lengths, and 1 024 contexts of 30 - 300 took 174 us where the plain form takes 105.
+// ordered form loses at 64 contexts of 300 - 600.  The first tile of the teams of two is on its way before the lengths are looked at, so that where they are
+// equal nothing waits for them.  Cold cache, a kernel between the calls, without teams -> with them:
+//   64 contexts of 200 - 1 500: 49.0 -> 34.9 us (4.8 TB/s)     40 of 50 - 4 000: 111 -> 51.3     63 of 200 and one of 8 000: 176 -> 94     128 of 200 - 1 500: 46.8 -> 36.1
+//   64 of 513: 28.3 -> 27.8     64 of 1 024: 47.2 -> 47.2     64 of 1 000 - 1 400: 59.0 -> 57.8     64 of 300 - 600: 25.8 -> 26.2     72 of 600: 34.2 -> 34.9     40 of 800: 29.4 -> 30.2
+// Larger grids, and batches of more than 128, run without kTeams: CTAs are many, each would read all the lengths, and 1 024 contexts of 30 - 300 took
+// 174 us where the plain form takes 105.
 // The number of warps that share a sequence, and with it the order of its sums, follows the OTHER lengths of the batch in this range: the same batch repeats
 // itself bit by bit, the same sequence in another batch need not.
 #pragma once
@@ -83,7 +86,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
   const int lane = threadIdx.x & 31;
   const int quad = lane >> 2, tq = lane & 3;          // accumulator row (quad, quad + 8), column pair tq
   int team_warps = kWarps, team = 0, b = blockIdx.y, unit_c = blockIdx.x;
-  int blk_first, ctx_len, most = 0, stage0 = 0;
+  int blk_first, ctx_len, most = 0;
   int lens[4];                                        // kTeams: this lane's share of the lengths
   bool uneven = false, decided = !kTeams;
   const int KC = kv * chunks, units = KC * B;
@@ -186,7 +189,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
         const int bi = tok0 / block_size;
         const int blk = bi == 0 ? blk_first : __ldg(bt + bi);
         const int64_t slot0 = (int64_t)blk * block_size + (tok0 % block_size);
-        const uint32_t st = ring + ((i + stage0) % kStages) * kStageBytes;
+        const uint32_t st = ring + (i % kStages) * kStageBytes;
         const int c = lane & 15;                       // 16-byte chunk of the 256-byte row
 #pragma unroll
         for (int rr = 0; rr < 8; ++rr) {
@@ -209,6 +212,7 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
     const int tok0 = (t_begin + i) * kCtaTok + warp * kTileTok;
     return i >= my_tiles || tok0 >= ctx_len || tok0 + kTileTok <= ctx_len - 1;
   };
+  if (kTeams && uneven) cp_async_wait<0>();           // the tile that went out before the decision has landed: its stage is free
   int pre = 0;
   if ((decided || u < units) && safe(0)) {
     issue(0);
@@ -224,7 +228,6 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
         team_warps = kWarps;
         team = 0;
         u = blockIdx.x;
-        stage0 = pre;                                 // the tile that is on its way keeps its stage until tile 2 needs it
         continue;
       }
       if (u >= units) return;
@@ -252,14 +255,13 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
   }
   if (pre < 1) issue(0);
   if (pre < 2) issue(1);
-  if (kTeams && stage0) cp_async_wait<2>();
   for (int i = 0; i < my_tiles; ++i) {
     issue(i + 2);
     cp_async_wait<2>();                               // tile i has landed (two younger groups may be in flight)
     __syncwarp();
     const int tok0 = (t_begin + i) * kCtaTok + warp * kTileTok;
     if (tok0 < ctx_len) {                             // warp-uniform
-      const uint32_t st = ring + ((i + stage0) % kStages) * kStageBytes;
+      const uint32_t st = ring + (i % kStages) * kStageBytes;
       // ---- S = Q K^T: two n-tiles of 8 tokens, fp32
       float s[2][4];
 #pragma unroll
