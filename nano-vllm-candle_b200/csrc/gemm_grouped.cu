@@ -4,7 +4,8 @@
 //
 // A persistent grid, one CTA per SM, walks the 128 x BN tiles, the column tiles of a row tile first (they share its rows, and neighbouring row
 // tiles of a group its weights, through L2):
-//   warp 0     TMA producer: 128 x 64 boxes of A and BN x 64 boxes of W, a ring of four (BN 256) or six (BN 128) stages that runs on into the next tile
+//   warp 0     TMA producer: 128 x 64 boxes of A and BN x 64 boxes of W, a ring of four (BN 256), six (128) or four (64, two k-blocks
+//              each) stages that runs on into the next tile
 //   warp 1     tcgen05.mma M 128, N BN, K 16; two accumulators in tensor memory, so that a tile's epilogue runs under the next one's main loop
 //   warps 2-5  epilogue: tcgen05.ld, activation, rows through a staging buffer (RowStage)
 // What bounds it: a k-block brings (128 + BN) x 128 bytes into shared memory for 2 BN cycles of the tensor pipe, 96 and 128 bytes per cycle where an
@@ -16,6 +17,9 @@
 #include "internal.h"
 #include "gemm_epilogue.cuh"
 
+#include <algorithm>
+#include <cmath>
+
 namespace {
 
 constexpr int BM = 128;
@@ -25,8 +29,9 @@ constexpr int kThreads = 192;
 template <int BN>
 struct GroupedCfg {
   static constexpr int kBytesA = BM * BK * 2, kBytesB = BN * BK * 2;
-  static constexpr int kStageBytes = kBytesA + kBytesB;
-  static constexpr int kStages = BN == 256 ? 4 : 6;                          // 192 KB
+  static constexpr int KPS = BN == 64 ? 2 : 1;                               // k-blocks per stage: a round trip over the barriers is long beside a narrow one
+  static constexpr int kStageBytes = KPS * (kBytesA + kBytesB);
+  static constexpr int kStages = BN == 128 ? 6 : 4;                          // 192 KB
   static constexpr int kOffStaging = kStages * kStageBytes;                  // 4 KB per epilogue warp
   static constexpr int kOffBar = kOffStaging + 4 * 4096;
   static constexpr int kNumBars = 2 * kStages + 4;                           // full, empty, accumulator full x 2, accumulator empty x 2
@@ -83,14 +88,20 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       const int grp = next, m = tile / n_tiles, n = tile - m * n_tiles;
       next = group_of(tile + gridDim.x);
       if (grp < 0) continue;
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+      for (int kb = 0; kb < num_kb; kb += cfg::KPS, ++it) {
         const int s = it % cfg::kStages;
         ptx::mbar_wait(empty_bar(s), ((it / cfg::kStages) & 1) ^ 1u);      // first lap: falls through
         if (ptx::elect_one()) {
-          ptx::mbar_arrive_expect_tx(full_bar(s), cfg::kStageBytes);
-          const uint32_t dst = base + s * cfg::kStageBytes;
-          ptx::tma_load_2d(dst + cfg::kBytesA, &tma_b, full_bar(s), kb * BK, grp * N + n * BN);
-          ptx::tma_load_2d(dst, &tma_a, full_bar(s), kb * BK, m * BM);
+          const int nsub = min(cfg::KPS, num_kb - kb);
+          ptx::mbar_arrive_expect_tx(full_bar(s), (uint32_t)(nsub * (cfg::kBytesA + cfg::kBytesB)));
+#pragma unroll
+          for (int j = 0; j < cfg::KPS; ++j) {
+            if (j < nsub) {
+              const uint32_t dst = base + s * cfg::kStageBytes + j * (cfg::kBytesA + cfg::kBytesB);
+              ptx::tma_load_2d(dst + cfg::kBytesA, &tma_b, full_bar(s), (kb + j) * BK, grp * N + n * BN);
+              ptx::tma_load_2d(dst, &tma_a, full_bar(s), (kb + j) * BK, m * BM);
+            }
+          }
         }
         __syncwarp();
       }
@@ -106,17 +117,23 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       const int acc = ti & 1;
       ptx::mbar_wait(acc_empty(acc), ((ti >> 1) & 1) ^ 1u);                // its last tile has been read out
       ptx::tcgen05_fence_after();
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+      for (int kb = 0; kb < num_kb; kb += cfg::KPS, ++it) {
         const int s = it % cfg::kStages;
         ptx::mbar_wait(full_bar(s), (it / cfg::kStages) & 1);
         ptx::tcgen05_fence_after();
         if (ptx::elect_one()) {
-          const uint32_t a_lo = a_lo0 + s * (cfg::kStageBytes >> 4), b_lo = a_lo + (cfg::kBytesA >> 4);
+          const int nsub = min(cfg::KPS, num_kb - kb);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            ptx::umma_bf16_ss(tmem + acc * BN, ptx::umma_desc(a_lo + 2 * k, desc_hi), ptx::umma_desc(b_lo + 2 * k, desc_hi), idesc, (kb | k) != 0 ? 1u : 0u);
+          for (int j = 0; j < cfg::KPS; ++j) {
+            if (j < nsub) {
+              const uint32_t a_lo = a_lo0 + ((s * cfg::kStageBytes + j * (cfg::kBytesA + cfg::kBytesB)) >> 4), b_lo = a_lo + (cfg::kBytesA >> 4);
+#pragma unroll
+              for (int k = 0; k < BK / 16; ++k)
+                ptx::umma_bf16_ss(tmem + acc * BN, ptx::umma_desc(a_lo + 2 * k, desc_hi), ptx::umma_desc(b_lo + 2 * k, desc_hi), idesc, (kb | j | k) != 0 ? 1u : 0u);
+            }
+          }
           ptx::umma_commit(empty_bar(s));
-          if (kb == num_kb - 1) ptx::umma_commit(acc_full(acc));
+          if (kb + cfg::KPS >= num_kb) ptx::umma_commit(acc_full(acc));
         }
         __syncwarp();
       }
@@ -199,6 +216,7 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 extern "C" int nvc_gemm_grouped_init(nvc_ctx* ctx) {
   NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_grouped_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, GroupedCfg<256>::kSmemBytes));
   NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_grouped_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, GroupedCfg<128>::kSmemBytes));
+  NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_grouped_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, GroupedCfg<64>::kSmemBytes));
   return NVC_OK;
 }
 
@@ -217,9 +235,18 @@ static int grouped(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, 
   if (M_cap == 0) return NVC_OK;
   const int epi = act == NVC_ACT_RELU2 ? NVC_EPI_RELU2 : NVC_EPI_NONE, f32 = out_dtype == NVC_DT_F32;
   cudaStream_t st = nvc_stream(stream);
-  // 256-wide tiles bring fewer bytes per column; 128-wide ones spread few tiles better (below two 256-wide tiles per SM)
+  // Wide tiles bring fewer bytes per column, narrow ones spread few tiles over more SMs.  256 columns from two tiles per SM on (of M_cap's), and with long
+  // k-loops where waves of tiles times a k-block's (128 + BN) x 128 bytes are fewer.  How many row tiles there will be is the device's to know: M_cap holds the
+  // rows, groups x 127 of padding and up to 127 of rounding; a group of up to 112 rows on average fills one tile, a larger one half a tile more than its rows.
+  // us, 128 / 256 columns wide: 16 groups of 4 rows, 3 072 x 1 024 24 / 27; 4 of 200, 4 096 x 2 048 23.6 / 21.2, of 400 40 / 33; 24 of 375, 768 x 2 048 42 / 35;
+  // 64 columns only where they are one wave of a long k-loop: 8 groups of 4 to 60 rows, 768 x 2 048 13.0 / 10.3
+  const double rows = std::max((double)M_cap - 127.0 * groups - 64.0, 1.0), per = rows / groups;
+  const double m_tiles = groups * (per <= 112.0 ? std::min(per, 1.0) : per / BM + 0.5);
+  auto cost = [&](int bn) { return std::max(std::ceil(m_tiles * ((Nout + bn - 1) / bn) / ctx->num_sms - 0.08), 1.0) * (128 + bn); };
+  if ((long long)(M_cap / BM) * ((Nout + 63) / 64) <= ctx->num_sms && K >= 2048)
+    return launch<64>(ctx, A, lda, W, C, ldc, f32, M_cap, Nout, K, tile_group, groups, epi, zero, st);
   const long long wide = (long long)(M_cap / BM) * ((Nout + 255) / 256);
-  if (wide >= 2LL * ctx->num_sms) return launch<256>(ctx, A, lda, W, C, ldc, f32, M_cap, Nout, K, tile_group, groups, epi, zero, st);
+  if (wide >= 2LL * ctx->num_sms || (K >= 1024 && cost(256) < 0.97 * cost(128))) return launch<256>(ctx, A, lda, W, C, ldc, f32, M_cap, Nout, K, tile_group, groups, epi, zero, st);
   return launch<128>(ctx, A, lda, W, C, ldc, f32, M_cap, Nout, K, tile_group, groups, epi, zero, st);
 }
 

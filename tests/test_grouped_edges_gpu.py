@@ -1,4 +1,4 @@
-"""The grouped product on its persistent grid: few and many tiles (both tile widths), more tiles than SMs, column counts around the tiles, groups
+"""The grouped product on its persistent grid: few and many tiles (all three tile widths), more tiles than SMs, column counts around the tiles, groups
 without rows and groups without a product, against 64-bit sums (bf16 operands: exact products, fp32 sums of up to 1 024 terms stay within 1e-5 of the
 largest value; a bf16 result within half of its last place more).  Rows that no group computes are zeros; the rows behind the groups keep the
 marks of the sort and the gather."""
@@ -17,7 +17,8 @@ def ops():
 
 
 @pytest.mark.parametrize("tokens,E,E_real,top,N,K", [(1, 3, 3, 1, 16, 64), (64, 16, 16, 2, 400, 128), (300, 5, 3, 2, 256, 192), (2500, 6, 6, 2, 1040, 64),
-                                                     (4000, 9, 8, 1, 3072, 128), (129, 1, 1, 1, 128, 1024)])
+                                                     (4000, 9, 8, 1, 3072, 128), (129, 1, 1, 1, 128, 1024),
+                                                     (200, 8, 8, 2, 1536, 448), (64, 8, 8, 1, 768, 1024), (40, 4, 4, 2, 176, 640)])      # 128 and 64 columns, rings that wrap
 @pytest.mark.parametrize("dt,act", [(torch.float32, 0), (torch.bfloat16, 1)])
 def test_grouped_product(ctx, ops, tokens, E, E_real, top, N, K, dt, act):
     g = torch.Generator(device=DEV).manual_seed(tokens + N)
