@@ -155,7 +155,8 @@ template <typename T, int kKind>
 cudaError_t launch_act_mul_rows(nvc_ctx* ctx, cudaStream_t st, const T* in, int ldi, T* out, int ldo, int N, int F, int Fp, float p0, float p1) {
   const int lanes = F / (int)(16 / sizeof(T)), passes = (lanes + 511) / 512;
   const int threads = ((lanes + passes - 1) / passes + 31) & ~31;
-  if (passes == 1 && N >= 32 * ctx->num_sms)
+  // narrow rows from half of that on: a CTA of one warp per row is bound by the rate at which CTAs start (fp32 4 000 x 100: 4.5 us, so 1.9)
+  if (passes == 1 && N >= (lanes <= 32 ? 16 : 32) * ctx->num_sms)
     return nvc_launch(ctx, act_mul_rows_kernel<T, kKind, 4>, dim3((unsigned)(((int64_t)N + 3) / 4)), dim3(threads), 0, st, in, ldi, out, ldo, N, F, Fp, p0, p1);
   return nvc_launch(ctx, act_mul_rows_kernel<T, kKind, 1>, dim3((unsigned)N), dim3(threads), 0, st, in, ldi, out, ldo, N, F, Fp, p0, p1);
 }

@@ -38,7 +38,7 @@ def test_gate_rows(ctx, rows, groups, size, dt):
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,F", [(4736, 8), (4737, 24), (4739, 264), (4738, 1536), (4741, 2056), (9001, 768)])
+@pytest.mark.parametrize("rows,F", [(4736, 8), (4737, 24), (4739, 264), (4738, 1536), (4741, 2056), (9001, 768), (2371, 100), (2369, 256), (2367, 256)])
 @pytest.mark.parametrize("kind", [1, 2, 3, 4, 5])
 def test_units_of_many_rows(ctx, rows, F, kind, dt):
     """Four rows per CTA: the numbers of one row per CTA, the last rows included, and a neighbour's buffer untouched."""
