@@ -554,7 +554,10 @@ int launch_prep(nvc_ctx* ctx, const nvc_qkv_prep* p, int N, void* stream) {
   const bool vec = wmax <= 128 && ((p->dim | p->vdim | p->q_off | p->k_off | p->v_off | p->ldi | p->ldq | p->ldk | p->ldv | p->rot_dims) & 3) == 0 &&
                    (!p->rot_half || (p->rot_dims & 7) == 0) && (p->blend == NVC_BLEND_NONE || ((p->ldvf & 3) == 0 && al16(p->v_first))) && al16(p->in) &&
                    al16(p->bias) && al16(p->q_norm) && al16(p->k_norm) && al16(p->rot_table) && al16(p->q_out) && al16(p->k_out) && al16(p->v_out);
-  if (vec) {
+  // a token whose heads fit in one warp, in a small grid: a warp per head is quicker (2 + 1 + 1 heads of 32, 1 - 256 rows: 1.7 - 1.9 us, one warp for all 1.9 - 2.3; 1 000 rows
+  // 2.8 and 2.7)
+  const bool tiny = N <= 512 && p->q_heads + 2 * p->kv_heads <= (wmax <= 64 ? 8 : 4);
+  if (vec && !tiny) {
     // a CTA per token, or several when a token has more than 8 warps of heads
     const int lanes = wmax <= 64 ? 16 : 32, per = 4 * (32 / lanes), groups = (p->q_heads + 2 * p->kv_heads + per - 1) / per, warps = std::min(groups, 8);
     NVC_CUDA_CHECK(ctx, nvc_launch(ctx, lanes == 16 ? prep_heads_kernel<TQ, TKV, 16> : prep_heads_kernel<TQ, TKV, 32>,

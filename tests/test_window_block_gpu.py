@@ -47,20 +47,21 @@ def test_portions_with_window_sink_gate_and_factor(ctx, ops, q_lens, old, window
     assert float((got - want).abs().max()) <= 2e-2 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("N", [13, 600])                     # tokens of few heads: a warp per head up to 512 rows
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,d,vd,rot,half,norm", [(16, 8, 128, 128, 64, False, "weight"), (3, 1, 64, 64, 64, True, "weight"), (5, 2, 68, 124, 24, True, "unit"),
                                                     (4, 2, 8, 60, 4, False, None), (1, 1, 128, 4, 128, True, "unit"), (7, 7, 100, 100, 0, False, "weight")])
-def test_preparation_of_heads_in_registers(ctx, ops, dt, H, G, d, vd, rot, half, norm):
+def test_preparation_of_heads_in_registers(ctx, ops, dt, H, G, d, vd, rot, half, norm, N):
     g = torch.Generator().manual_seed(H * d + vd)
-    N, eps, pad = 13, 1e-5, 4
+    eps, pad, rows = 1e-5, 4, N + 7
     qw, kw, vw = H * d, G * d, G * vd
     x, bias, first = torch.randn(N, pad + qw + kw + vw, generator=g), torch.randn(pad + qw + kw + vw, generator=g), torch.randn(N, vw, generator=g)
     qn, kn = ((1 + 0.3 * torch.randn(d, generator=g)).to(DEV) for _ in range(2)) if norm == "weight" else (None, None)
     pos = torch.randint(0, 300, (N,), generator=g)
-    slots = torch.randperm(20, generator=g)[:N].to(torch.int32)
+    slots = torch.randperm(rows, generator=g)[:N].to(torch.int32)
     slots[3] = -1
     lam = torch.tensor([0.3], device=DEV)
-    q, kc, vc = torch.zeros(N, qw, dtype=dt, device=DEV), torch.full((20, kw), 9.0, dtype=dt, device=DEV), torch.full((20, vw), 9.0, dtype=dt, device=DEV)
+    q, kc, vc = torch.zeros(N, qw, dtype=dt, device=DEV), torch.full((rows, kw), 9.0, dtype=dt, device=DEV), torch.full((rows, vw), 9.0, dtype=dt, device=DEV)
     ops.qkv_prep(ctx, x.to(DEV), pad, pad + qw, pad + qw + kw, H, G, d, vd, q, kc, vc, bias=bias.to(DEV), q_norm=qn, k_norm=kn, eps=eps, rot_dims=rot, rot_half=half,
                  rot_table=ops.rotary_table(ctx, 5000.0, rot, 300) if rot else None, positions=i32(pos.tolist()), k_scale=0.5, blend=2, lam=lam, v_first=first.to(DEV),
                  slot_mapping=slots.to(DEV), v_scale=1.5, unit_norm=norm == "unit")
@@ -86,6 +87,6 @@ def test_preparation_of_heads_in_registers(ctx, ops, dt, H, G, d, vd, rot, half,
     v = 1.5 * (0.7 * xb[:, qw + kw:] + 0.3 * first.double())
     for got, want in ((q.cpu(), heads(xb[:, :qw], H, qn)), (kc.cpu()[at], 0.5 * heads(xb[:, qw:qw + kw], G, kn)[ok]), (vc.cpu()[at], v[ok])):
         assert ((got.double() - want).abs() <= tol * (1 + want.abs())).all()
-    rest = torch.ones(20, dtype=torch.bool)
+    rest = torch.ones(rows, dtype=torch.bool)
     rest[at] = False
     assert (kc.cpu()[rest] == 9).all() and (vc.cpu()[rest] == 9).all()
