@@ -17,7 +17,7 @@
 // four steps, and the chunk kernel works with the running sums L_t of each channel: the token-by-token products take
 // exp(L_t - L_j) inside their sums, the keys and queries that meet the state carry exp(L_t), those that enter it exp(L_n - L_j).
 // Both states live in fp32 in pools of state slots; a sequence whose first new token sits at position 0 starts from zeros.
-// All arithmetic is fp32: FMA code, or products of three bf16 parts per number (scan_mma.cuh).
+// All arithmetic is fp32: FMA code, or products of 16-bit parts of numbers (scan_mma.cuh).
 #include <type_traits>
 
 #include "conv_tile.cuh"
@@ -35,6 +35,9 @@ struct DeltaArgs {
 };
 
 __device__ __forceinline__ float softplus_f32(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+
+// log decay of a head, -exp(A_log) softplus(x), rounded once: a portion's decays are products of up to hundreds of them
+__device__ __forceinline__ float log_decay_f64(float a_log, double x) { return (float)(-exp((double)a_log) * (fmax(x, 0.0) + log1p(exp(-fabs(x))))); }
 
 // grid (row tiles, units): a warp per (row, unit), the row's sequence by a search.  Decode steps, and shapes that delta_prep_tile_kernel does not take
 // TAPS: the convolution's taps when they are 2 .. 4 (all inputs of a channel are in flight at once), 0: any number of them
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(128) delta_prep_tile_kernel(const DeltaArgs a)
       const int n = n0 + e / p.heads, h = e % p.heads;
       const float* in = p.in + (int64_t)n * p.ldi;
       float* gb = p.gb_out + ((int64_t)n * p.heads + h) * 2;
-      if (!p.channel_a) gb[0] = -expf(__ldg(p.A_log + h)) * softplus_f32(in[p.a_off + h] + __ldg(p.dt_bias + h));       // log of the decay
+      if (!p.channel_a) gb[0] = log_decay_f64(__ldg(p.A_log + h), (double)in[p.a_off + h] + __ldg(p.dt_bias + h));
       gb[1] = sigmoid_f32(in[p.b_off + h]);
     }
     return;
@@ -680,28 +683,15 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 3) delta_chunk_kernel(c
 // column with forward substitution in fp32 by the preparing warp that computed the block.  B, U and O never leave a state warp's registers.
 constexpr int kHT = 16;                  // tokens of a half
 constexpr int kHP = kHT + 8;             // row stride of a half's planes
-__host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 5 * kMT * 4; }
-
-// decays between the tokens of a thread's numbers in a 16 x 16 block, from running sums in two parts
-struct Decays {
-  float th[2], tl[2], jh[4], jl[4];
-  __device__ __forceinline__ void load(const float* Lh, const float* Ll, int t0, int j0, int lane) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) { th[i] = Lh[t0 + (lane >> 2) + 8 * i]; tl[i] = Ll[t0 + (lane >> 2) + 8 * i]; }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { jh[i] = Lh[j0 + 2 * (lane & 3) + (i & 1) + 4 * (i & 2)]; jl[i] = Ll[j0 + 2 * (lane & 3) + (i & 1) + 4 * (i & 2)]; }
-  }
-  // number e of tile y
-  __device__ __forceinline__ float operator()(int y, int e) const { return ex2((th[e >> 1] - jh[2 * y + (e & 1)]) + (tl[e >> 1] - jl[2 * y + (e & 1)])); }
-};
+__host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 4 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 9 * kMT * 4; }
 
 template <int KS>
-__global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, const int vecv) {
+__global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaArgs a, const int vecv) {
   constexpr int DZ = 16 * KS, DP = DZ + 8;
-  constexpr float kLog2e = 1.4426950408889634f;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int which;
-  __shared__ __align__(16) float nts[2][kHT * kDA];       // A of a half, transposed, for its inversion
+  __shared__ RankScratch ranks;
+  __shared__ float4 swap[4][3][4][32];                    // of a pair: products with the queries, with the keys, U
+  __shared__ __align__(16) float nts[2][2][kHT * kDA];    // A of a half, transposed, for its inversion
   pdl_trigger();
   const nvc_delta_prep& p = a.p;
   const int slices = (p.vdim + kMC - 1) / kMC, h = blockIdx.x / slices, v0 = (blockIdx.x % slices) * kMC;
@@ -709,212 +699,256 @@ __global__ void __launch_bounds__(256, 1) delta_mma_kernel(const DeltaArgs a, co
   const int hk = h / (p.heads / p.kv_heads);
   const int dim = p.dim, cols = min(kMC, p.vdim - v0);
   pdl_wait();
-  const int b = sequence_of_rank(p.cu_seqlens, p.B, blockIdx.y, &which);
+  const int b = sequence_of_rank(p.cu_seqlens, p.B, blockIdx.y, ranks);
   const int r0 = p.cu_seqlens[b], r1 = p.cu_seqlens[b + 1], chunks = (r1 - r0 + kMT - 1) / kMT;
   if (chunks == 0) return;
   const bool fresh = p.positions[r0] == 0;
   const int slot = p.state_slots[b];
-  struct Buffer { Planes Q, K, P, X0, X1, A10; float *V, *beta, *Lh, *Ll, *from, *to; };
+  struct Buffer { Planes Q, K, P, X0, X1, A10; float *V, *beta, *Lh, *Ll, *from, *fk, *fq, *tk, *dq, *dk; };
   auto buffer = [&](int i) {
-    uint8_t* q = smem + (i & 1) * delta_buf(DZ);
-    uint8_t* x = q + 2 * kMT * DP * 6 + kMT * kMP * 6;
+    uint8_t* q = smem + (i % kBuffers) * delta_buf(DZ);
+    uint8_t* x = q + 2 * kMT * DP * 4 + kMT * kMP * 6;
     float* v = reinterpret_cast<float*>(x + 3 * kHT * kHP * 6);
-    float* l = v + kMT * kMV;               // beta; running sums in two parts; decay from the chunk's start to a token, from a token to its end
-    return Buffer{planes(q, kMT, DP), planes(q + kMT * DP * 6, kMT, DP), planes(q + 2 * kMT * DP * 6, kMT, kMP), planes(x, kHT, kHP),
-                  planes(x + kHT * kHP * 6, kHT, kHP), planes(x + 2 * kHT * kHP * 6, kHT, kHP), v, l, l + kMT, l + 2 * kMT, l + 3 * kMT, l + 4 * kMT};
+    // beta; running sums in two parts; decay from the chunk's start to a token, and the same times the inverse scales of its key and query;
+    // decay from a token to the chunk's end times its key's inverse scale; the inverse scales
+    float* l = v + kMT * kMV;
+    return Buffer{planes(q, kMT, DP), planes(q + kMT * DP * 4, kMT, DP), planes(q + 2 * kMT * DP * 4, kMT, kMP), planes(x, kHT, kHP),
+                  planes(x + kHT * kHP * 6, kHT, kHP), planes(x + 2 * kHT * kHP * 6, kHT, kHP), v, l, l + kMT, l + 2 * kMT,
+                  l + 3 * kMT, l + 4 * kMT, l + 5 * kMT, l + 6 * kMT, l + 7 * kMT, l + 8 * kMT};
   };
-  if (w >= 4) {
+  if (w >= kPrep0) {
     // ------------------------------------------------ preparing warps
-    const int pw = w - 4;
-    RowTile<DZ> q, k;
+    registers_give<kPrepRegs>();
+    const int pw = w & 3, group = (w - kPrep0) >> 2;
+    RowTile<DZ> x;                            // queries, then keys
     RowTile<kMC> v;
-    float2 gb = make_float2(0.f, 0.f);        // (log2 decay, beta) of a token; none behind the end
+    float2 gb = make_float2(0.f, 0.f);        // (log decay, beta) of a token; none behind the end
     auto fetch = [&](int i) {
       const int64_t row = r0 + i * kMT;
       const int n = r1 - (int)row;
-      q.load(p.q_out + row * p.ldq + hk * dim, p.ldq, dim, n, a.vec, pw, lane);
-      k.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, n, a.vec, pw, lane);
+      x.load(p.q_out + row * p.ldq + hk * dim, p.ldq, dim, n, a.vec, pw, lane);
       v.load(p.v_out + row * p.ldv + h * p.vdim + v0, p.ldv, cols, n, vecv, pw, lane);
       if (pw == 3) {
         const float* x = p.gb_out + ((row + lane) * p.heads + h) * 2;
-        gb = lane < n ? make_float2(x[0] * kLog2e, x[1]) : make_float2(0.f, 0.f);
+        gb = lane < n ? make_float2(x[0], x[1]) : make_float2(0.f, 0.f);
       }
     };
-    fetch(0);
-    for (int i = 0; i < chunks; ++i) {
+    if (group < chunks) fetch(group);
+    for (int i = group; i < chunks; i += 2) {
       const Buffer bf = buffer(i);
-      if (i >= 2) bar_sync(kEmpty + (i & 1), 256);
-      q.split_to(bf.Q, pw, lane);
-      k.split_to(bf.K, pw, lane);
+      if (i >= kBuffers) bar_sync(kEmpty + i % (2 * kBuffers), kBufThreads);
+      x.split_to(bf.Q, bf.dq, pw, lane);
+      {
+        const int64_t row = r0 + i * kMT;
+        x.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, r1 - (int)row, a.vec, pw, lane);
+      }
       v.store_to(bf.V, kMV, pw, lane);
+      float from = 0.f, to = 0.f;
       if (pw == 3) {
-        // running sums in 64 bits: over 32 tokens they reach 40 and more, and what is exponentiated are their differences
-        double l = (double)gb.x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double up = __shfl_up_sync(0xffffffffu, l, o);
-          if (lane >= o) l += up;
-        }
-        const float hi = (float)l;
+        const LogSum sum(gb.x, lane);
+        const float hi = (float)sum.l;
         bf.Lh[lane] = hi;
-        bf.Ll[lane] = (float)(l - (double)hi);
-        bf.from[lane] = ex2(hi);
-        bf.to[lane] = ex2((float)(__shfl_sync(0xffffffffu, l, 31) - l));
+        bf.Ll[lane] = (float)(sum.l - (double)hi);
+        bf.from[lane] = from = sum.from();
+        to = sum.to();
         bf.beta[lane] = gb.y;
       }
-      if (i + 1 < chunks) fetch(i + 1);
-      bar_sync(kPrepare, 128);
+      x.split_to(bf.K, bf.dk, pw, lane);
+      bar_sync(kPrepare + group, 128);
+      if (pw == 3) {
+        bf.fk[lane] = from * bf.dk[lane];
+        bf.fq[lane] = from * bf.dq[lane];
+        bf.tk[lane] = to * bf.dk[lane];
+      }
       // warps 0 and 1: the diagonal blocks of A and their inverses; 2: P (16, 0) and A_10; 3: P (0, 0) and P (16, 16)
-      float x[2][4];
-      if (pw < 2) {
-        const int t0 = kHT * pw;
-        Decays f;
-        f.load(bf.Lh, bf.Ll, t0, t0, lane);
-        token_products<KS>(x, bf.K, t0, bf.K, t0, lane);
-        float* nt = nts[pw];
-#pragma unroll
-        for (int y = 0; y < 2; ++y)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = g + 4 * (e & 2), j = 8 * y + 2 * tq + (e & 1);
-            nt[j * kDA + t] = j < t ? bf.beta[t0 + t] * (f(y, e) * x[y][e]) : 0.f;
-          }
-        __syncwarp();
-        const int col = lane & 15;            // a column of the inverse per lane (both halves of the warp do the same)
-        float z[kHT];
-#pragma unroll
-        for (int t = 0; t < kHT; ++t) z[t] = t == col ? 1.f : 0.f;
-#pragma unroll
-        for (int j = 0; j + 1 < kHT; ++j)
-#pragma unroll
-          for (int t4 = (j + 1) / 4 * 4; t4 < kHT; t4 += 4) {
-            const float4 m = *reinterpret_cast<const float4*>(nt + j * kDA + t4);
-            if (t4 > j) z[t4] = fmaf(-m.x, z[j], z[t4]);
-            if (t4 + 1 > j) z[t4 + 1] = fmaf(-m.y, z[j], z[t4 + 1]);
-            if (t4 + 2 > j) z[t4 + 2] = fmaf(-m.z, z[j], z[t4 + 2]);
-            z[t4 + 3] = fmaf(-m.w, z[j], z[t4 + 3]);
-          }
-        const Planes X = pw ? bf.X1 : bf.X0;
-#pragma unroll
-        for (int t = 0; t < kHT / 2; ++t) {                 // rows 0 .. 7 by the left lanes, 8 .. 15 by the right ones
-          const float mine = lane < kHT ? z[t] : z[t + kHT / 2], right = __shfl_down_sync(0xffffffffu, mine, 1);
-          if (!(lane & 1)) store_pair(X, t + (lane & kHT) / 2, col, mine, right);
-        }
-      } else {
 #pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-          const bool isa = pw == 2 && half;
-          const int t0 = pw == 2 ? kHT : kHT * half, j0 = pw == 2 ? 0 : kHT * half;
+      for (int part = 0; part < (pw < 2 ? 1 : 2); ++part) {
+        const bool isa = pw < 2 || (pw == 2 && part);
+        const int t0 = pw == 2 || (pw == 3 ? part : pw) ? kHT : 0, j0 = pw == 2 ? 0 : t0;
+        float z[2][4];
+        token_products<KS>(z, isa ? bf.K : bf.Q, t0, bf.K, j0, lane);
+        {
           Decays f;
           f.load(bf.Lh, bf.Ll, t0, j0, lane);
-          const float b0 = isa ? bf.beta[t0 + g] : 1.f, b1 = isa ? bf.beta[t0 + g + 8] : 1.f;
-          token_products<KS>(x, isa ? bf.K : bf.Q, t0, bf.K, j0, lane);
+          Down d;
+          d.load(isa ? bf.dk : bf.dq, bf.dk, t0, j0, lane);
+          const float be[2] = {isa ? bf.beta[t0 + g] : 1.f, isa ? bf.beta[t0 + g + 8] : 1.f};
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int t = t0 + g + 4 * (e & 2), j = j0 + 8 * y + 2 * tq + (e & 1);
+              z[y][e] = j < t + !isa ? be[e >> 1] * (f(y, e) * d(y, e, z[y][e])) : 0.f;
+            }
+        }
+        if (pw >= 2) {
           const Planes M = isa ? bf.A10 : bf.P;
 #pragma unroll
           for (int y = 0; y < 2; ++y)
 #pragma unroll
-            for (int e = 0; e < 4; e += 2) {
-              const int t = t0 + g + 4 * e, j = j0 + 8 * y + 2 * tq;
-              const float be = e ? b1 : b0;
-              store_pair(M, isa ? t - kHT : t, j, j <= t ? be * (f(y, e) * x[y][e]) : 0.f, j + 1 <= t ? be * (f(y, e + 1) * x[y][e + 1]) : 0.f);
+            for (int e = 0; e < 4; e += 2) store_pair(M, (isa ? 0 : t0) + g + 4 * e, j0 + 8 * y + 2 * tq, z[y][e], z[y][e + 1]);
+        } else {
+          float* nt = nts[group][pw];
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) nt[(8 * y + 2 * tq + (e & 1)) * kDA + g + 4 * (e & 2)] = z[y][e];
+          __syncwarp();
+          const int col = lane & 15;          // a column of the inverse per lane (both halves of the warp do the same)
+          float c[kHT];
+#pragma unroll
+          for (int t = 0; t < kHT; ++t) c[t] = t == col ? 1.f : 0.f;
+#pragma unroll
+          for (int j = 0; j + 1 < kHT; ++j)
+#pragma unroll
+            for (int t4 = (j + 1) / 4 * 4; t4 < kHT; t4 += 4) {
+              const float4 m = *reinterpret_cast<const float4*>(nt + j * kDA + t4);
+              if (t4 > j) c[t4] = fmaf(-m.x, c[j], c[t4]);
+              if (t4 + 1 > j) c[t4 + 1] = fmaf(-m.y, c[j], c[t4 + 1]);
+              if (t4 + 2 > j) c[t4 + 2] = fmaf(-m.z, c[j], c[t4 + 2]);
+              c[t4 + 3] = fmaf(-m.w, c[j], c[t4 + 3]);
             }
+          const Planes X = pw ? bf.X1 : bf.X0;
+          const int odd = lane & 1;
+#pragma unroll
+          for (int t = 0; t < kHT / 2; t += 2) {            // rows 0 .. 7 by the left lanes, 8 .. 15 by the right ones; an even lane writes row t, an odd one t + 1
+            const float a0 = lane < kHT ? c[t] : c[t + kHT / 2], a1 = lane < kHT ? c[t + 1] : c[t + 1 + kHT / 2];
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+            store_pair(X, t + odd + (lane & kHT) / 2, col & ~1, odd ? got : a0, odd ? a1 : got);
+          }
         }
       }
-      if (i == 0) advance_conv_state(p, r0, r1, fresh, slot, blockIdx.x, gridDim.x, threadIdx.x - 128, 128);      // nothing here reads that state
-      bar_arrive(kFull + (i & 1), 256);
+      if (i == 0) advance_conv_state(p, r0, r1, fresh, slot, blockIdx.x, gridDim.x, threadIdx.x - 32 * kPrep0, 128);      // nothing here reads that state
+      bar_arrive(kFull + i % kBuffers, kBufThreads);
+      if (i + 2 < chunks) fetch(i + 2);
     }
     return;
   }
   // -------------------------------------------------- state warps
-  const int c = w * 16 + g;
-  float* sp = a.state + (((int64_t)slot * p.heads + h) * dim) * p.vdim + v0;
-  float S[2 * KS][4];
-  load_state<KS>(S, sp, p.vdim, dim, c, cols, fresh, lane);
+  registers_take<kStateRegs>();
+  constexpr int KH = KS / 2;                  // blocks of 16 channels of a half
+  const int pair = w & 3, half = w >> 2, c = pair * 16 + g, d0 = half * (DZ / 2);
+  float* sp = a.state + (((int64_t)slot * p.heads + h) * dim + d0) * p.vdim + v0;
+  float S[2 * KH][4];
+  load_state<KH>(S, sp, p.vdim, dim - d0, c, cols, fresh, lane);
+  float4(*const xch)[4][32] = swap[pair];
+  auto put = [&](int k, const float (&x)[4][4]) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) xch[k][t][lane] = make_float4(x[t][0], x[t][1], x[t][2], x[t][3]);
+  };
+  auto add = [&](int k, float (&x)[4][4]) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float4 y = xch[k][t][lane];
+      x[t][0] += y.x; x[t][1] += y.y; x[t][2] += y.z; x[t][3] += y.w;
+    }
+  };
   using Two = float(*)[2][4];
   for (int i = 0; i < chunks; ++i) {
     const Buffer bf = buffer(i);
     const int64_t row = r0 + i * kMT;
     const int n = min(kMT, r1 - (int)row);
-    bar_sync(kFull + (i & 1), 256);
-    float u[4][4], o[4][4];                   // right sides, then U; outputs
+    const ColumnScale sc = column_scale(S);
+    bar_sync(kFull + i % kBuffers, kBufThreads);
+    float u[4][4] = {}, o[4][4] = {};         // products with the keys, then right sides, then U; with the queries, then outputs
     {
-      float kr[4][4] = {}, qr[4][4] = {}, kx[4][4] = {}, qx[4][4] = {};
+      float us[4][4] = {}, os[4][4] = {};
 #pragma unroll
-      for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) u[t][e] = o[t][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        FragA s;
-        FragB x[4];
-        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1]);
-        load_b(x, bf.K, 0, 16 * ks, lane);
-        if (ks < KS / 2) mma_high(kx, s, x);
-        else mma_high(u, s, x);
-        mma_small(kr, s, x);
-        load_b(x, bf.Q, 0, 16 * ks, lane);
-        if (ks < KS / 2) mma_high(qx, s, x);
-        else mma_high(o, s, x);
-        mma_small(qr, s, x);
+      for (int ks = 0; ks < KH; ++ks) {
+        HalfA s;
+        HalfB x[4];
+        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1], sc.c0.up, sc.c1.up);
+        load_b(x, bf.K, 0, d0 + 16 * ks, lane);
+        mma_high(u, s, x);
+        mma_small(us, s, x);
+        load_b(x, bf.Q, 0, d0 + 16 * ks, lane);
+        mma_high(o, s, x);
+        mma_small(os, s, x);
       }
 #pragma unroll
       for (int t = 0; t < 4; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int tt = 8 * t + 2 * tq + (e & 1);
-          const float f = bf.from[tt];
-          u[t][e] = bf.beta[tt] * (bf.V[tt * kMV + c + 4 * (e & 2)] - f * ((u[t][e] + kx[t][e]) + kr[t][e]));
-          o[t][e] = f * ((o[t][e] + qx[t][e]) + qr[t][e]);
+          u[t][e] = (u[t][e] + us[t][e]) * sc.down(e);
+          o[t][e] = (o[t][e] + os[t][e]) * sc.down(e);
         }
     }
-    FragA f;
-    auto solve = [&](float (&x)[2][4], const Planes& X) {     // x <- x X^T;  f: its parts
-      frag_of_tiles(f, x[0], x[1]);
+    // the left warp of a pair solves for U, the right one takes the outputs
+    if (half == 0) {
+      put(0, o);
+      bar_sync(kPair + pair, 64);
+      add(1, u);
 #pragma unroll
-      for (int t = 0; t < 2; ++t)
+      for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[t][e] = 0.f;
-      add_tokens(x, f, X, 0, 0, lane);
-      frag_of_tiles(f, x[0], x[1]);
-    };
-    solve(*reinterpret_cast<Two>(u), bf.X0);
-    {
+        for (int e = 0; e < 4; ++e) {
+          const int tt = 8 * t + 2 * tq + (e & 1);
+          u[t][e] = bf.beta[tt] * (bf.V[tt * kMV + c + 4 * (e & 2)] - bf.fk[tt] * u[t][e]);
+        }
+      FragA f;
+      auto solve = [&](float (&x)[2][4], const Planes& X) {     // x <- x X^T
+        frag_of_tiles(f, x[0], x[1]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[t][e] = 0.f;
+        add_tokens(x, f, X, 0, 0, lane);
+      };
+      solve(*reinterpret_cast<Two>(u), bf.X0);
+      frag_of_tiles(f, u[0], u[1]);
       float m[2][4] = {};
       add_tokens(m, f, bf.A10, 0, 0, lane);
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) u[2 + t][e] -= m[t][e];
+      solve(*reinterpret_cast<Two>(u + 2), bf.X1);
+      put(2, u);
+      bar_sync(kPair + pair, 64);
+    } else {
+      put(1, u);
+      bar_sync(kPair + pair, 64);
+      add(0, o);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o[t][e] *= bf.fq[8 * t + 2 * tq + (e & 1)];
+          u[t][e] = 0.f;
+        }
+      bar_sync(kPair + pair, 64);
+      add(2, u);
+      FragA f;
+      frag_of_tiles(f, u[0], u[1]);
+      add_tokens(o, f, bf.P, 0, 0, lane);
+      frag_of_tiles(f, u[2], u[3]);
+      add_tokens(*reinterpret_cast<Two>(o + 2), f, bf.P, 16, 16, lane);
     }
-    add_tokens(o, f, bf.P, 0, 0, lane);
-    solve(*reinterpret_cast<Two>(u + 2), bf.X1);
-    add_tokens(*reinterpret_cast<Two>(o + 2), f, bf.P, 16, 16, lane);
     // ---- the state behind the chunk
-    FragA us[2];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) u[t][e] *= bf.to[8 * t + 2 * tq + (e & 1)];
-    frag_of_tiles(us[0], u[0], u[1]);
-    frag_of_tiles(us[1], u[2], u[3]);
-    state_update<KS>(S, bf.from[kMT - 1], us, bf.K, lane);
-    if (i + 2 < chunks) bar_arrive(kEmpty + (i & 1), 256);
-    float* op = a.o + row * a.ldo + h * p.vdim + v0;
+      for (int e = 0; e < 4; ++e) u[t][e] *= bf.tk[8 * t + 2 * tq + (e & 1)];
+    state_update<KH>(S, bf.from[kMT - 1], u, bf.K, d0, lane);
+    if (i + kBuffers < chunks) bar_arrive(kEmpty + (i + kBuffers) % (2 * kBuffers), kBufThreads);
+    if (half == 1) {
+      float* op = a.o + (row + 2 * tq) * a.ldo + h * p.vdim + v0 + c;
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
+      for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int tt = 8 * t + 2 * tq + (e & 1), cc = c + 4 * (e & 2);
-        if (tt < n && cc < cols) op[(int64_t)tt * a.ldo + cc] = o[t][e];
-      }
+        for (int e = 0; e < 4; ++e) {
+          const int tt = 8 * t + (e & 1), cc = 4 * (e & 2);
+          if (tt + 2 * tq < n && c + cc < cols) op[(int64_t)tt * a.ldo + cc] = o[t][e];
+        }
+    }
   }
-  store_state<KS>(S, sp, p.vdim, dim, c, cols, lane);
+  store_state<KH>(S, sp, p.vdim, dim - d0, c, cols, lane);
 }
 
 template <int KS>
 cudaError_t launch_delta_mma(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) {
   const nvc_delta_prep& p = a.p;
-  constexpr int smem = 2 * delta_buf(16 * KS);
+  constexpr int smem = kBuffers * delta_buf(16 * KS);
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(delta_mma_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -922,7 +956,7 @@ cudaError_t launch_delta_mma(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) 
     attr_set = true;
   }
   const int vecv = (p.vdim & 3) == 0 && (p.ldv & 3) == 0 && (reinterpret_cast<uintptr_t>(p.v_out) & 15) == 0;
-  return nvc_launch(ctx, delta_mma_kernel<KS>, dim3(p.heads * ((p.vdim + kMC - 1) / kMC), p.B), dim3(256), smem, st, a, vecv);
+  return nvc_launch(ctx, delta_mma_kernel<KS>, dim3(p.heads * ((p.vdim + kMC - 1) / kMC), p.B), dim3(kScanThreads), smem, st, a, vecv);
 }
 
 template <int C, int NW, bool CH>

@@ -17,7 +17,7 @@
 //                              S      <- decay^n S + sum_j decay^(n - 1 - j) k_j v_j^T n: tokens of the chunk
 //                            Powers of the decay come from a table built by repeated multiplication (exact for 0 and 1).
 //   decay_mma_kernel         the same chunks of 32 tokens on the tensor pipe, without the normaliser of the gated memory: up to 128 channels
-// All arithmetic is fp32 (FMA code, or products of three bf16 parts per number: scan_mma.cuh); they differ by rounding only.
+// All arithmetic is fp32 (FMA code, or products of 16-bit parts of numbers: scan_mma.cuh); they differ by rounding only.
 //
 // nvc_decay_scan is the same pair of kernels with what other linear recurrences of this shape need (kVar):
 //   a decay per token and head, given as its logarithm: S_t = exp(l_t) S_(t-1) + k_t v_t^T.  Inside a chunk only differences of the
@@ -452,15 +452,16 @@ __global__ void __launch_bounds__(NW * 32, 2) retention_chunk_kernel(const RetAr
 // ---- kFixed and kVar with keys of up to 128 numbers: the same chunks of 32 tokens with every product on the tensor pipe (scan_mma.cuh says how the
 // warps share the work).  With (.)^T for a state warp's 16 value columns,
 //   O^T = exp(L_t) S^T Q^T + V^T A^T,    S^T <- exp(L_n) S^T + (w_j v_j)^T K.
-__host__ __device__ constexpr int decay_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + kMT * kMV * 4 + 3 * kMT * 4; }      // bytes of a chunk's buffer
+__host__ __device__ constexpr int decay_buf(int dz) { return 2 * kMT * (dz + 8) * 4 + kMT * kMP * 6 + kMT * kMV * 4 + 7 * kMT * 4; }      // bytes of a chunk's buffer
 
 template <int KS, int MODE>
-__global__ void __launch_bounds__(256, 1) decay_mma_kernel(const RetArgs a, const int B, const int vec, const int vecv) {
+__global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArgs a, const int B, const int vec, const int vecv) {
   constexpr bool VAR = MODE == kVar;
   constexpr int DZ = 16 * KS, DP = DZ + 8;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int which;
+  __shared__ RankScratch ranks;
   __shared__ float gp[kMT + 1];               // decay^0 .. decay^32 (kFixed)
+  __shared__ float4 swap[4][2][2][2][32];     // of a pair, alternately: products with the queries of tokens 0 .. 15 and 16 .. 31
   pdl_trigger();
   const int slices = (a.vdim + kMC - 1) / kMC, h = blockIdx.x / slices, v0 = (blockIdx.x % slices) * kMC;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
@@ -468,157 +469,187 @@ __global__ void __launch_bounds__(256, 1) decay_mma_kernel(const RetArgs a, cons
   const int hq = h / (a.heads / a.qk_heads);
   if (!VAR && threadIdx.x == 0) {
     const float dec = __ldg(a.decay + h);
-    float p = 1.f;
-    for (int i = 0; i <= kMT; ++i) { gp[i] = p; p *= dec; }
+    double p = 1.0;
+    for (int i = 0; i <= kMT; ++i) { gp[i] = (float)p; p *= (double)dec; }
   }
   pdl_wait();
-  const int b = sequence_of_rank(a.cu_seqlens, B, blockIdx.y, &which);
+  const int b = sequence_of_rank(a.cu_seqlens, B, blockIdx.y, ranks);
   const int r0 = a.cu_seqlens[b], r1 = a.cu_seqlens[b + 1], chunks = (r1 - r0 + kMT - 1) / kMT;
   if (chunks == 0) return;
   __syncthreads();                            // gp
-  struct Buffer { Planes Q, K, A; float *V, *keep, *wj, *L; };
-  auto buffer = [&](int i) {                  // planes, values, decay of the state up to token t, weight of token j behind the chunk, running sums
-    uint8_t* p = smem + (i & 1) * decay_buf(DZ);
-    float* v = reinterpret_cast<float*>(p + 2 * kMT * DP * 6 + kMT * kMP * 6);
+  struct Buffer { Planes Q, K, A; float *V, *keep, *kq, *wk, *Lh, *Ll, *dq, *dk; };
+  auto buffer = [&](int i) {                  // planes, values, decay of the state up to token t, the same times its query's inverse scale, weight of token j
+                                              // behind the chunk times its key's inverse scale, running sums in two parts, inverse scales
+    uint8_t* p = smem + (i % kBuffers) * decay_buf(DZ);
+    float* v = reinterpret_cast<float*>(p + 2 * kMT * DP * 4 + kMT * kMP * 6);
     float* k = v + kMT * kMV;
-    return Buffer{planes(p, kMT, DP), planes(p + kMT * DP * 6, kMT, DP), planes(p + 2 * kMT * DP * 6, kMT, kMP), v, k, k + kMT, k + 2 * kMT};
+    return Buffer{planes(p, kMT, DP), planes(p + kMT * DP * 4, kMT, DP), planes(p + 2 * kMT * DP * 4, kMT, kMP), v, k, k + kMT, k + 2 * kMT, k + 3 * kMT,
+                  k + 4 * kMT, k + 5 * kMT, k + 6 * kMT};
   };
-  if (w >= 4) {
+  if (w >= kPrep0) {
     // ------------------------------------------------ preparing warps
-    const int pw = w - 4;
-    RowTile<DZ> q, k;
+    registers_give<kPrepRegs>();
+    const int pw = w & 3, group = (w - kPrep0) >> 2;
+    RowTile<DZ> x;                            // queries, then keys
     RowTile<kMC> v;
     float l = 0.f;
     auto fetch = [&](int i) {
       const int64_t row = r0 + i * kMT;
       const int n = r1 - (int)row;
-      q.load(a.q + row * a.ldq + hq * dim, a.ldq, dim, n, vec, pw, lane);
-      k.load(a.k + row * a.ldk + hq * dim, a.ldk, dim, n, vec, pw, lane);
+      x.load(a.q + row * a.ldq + hq * dim, a.ldq, dim, n, vec, pw, lane);
       v.load(a.v + row * a.ldv + h * a.vdim + v0, a.ldv, cols, n, vecv, pw, lane);
       if (VAR && pw == 3) l = lane < n ? a.log_decay[(row + lane) * a.ldl + h] : 0.f;
     };
-    fetch(0);
-    for (int i = 0; i < chunks; ++i) {
+    if (group < chunks) fetch(group);
+    for (int i = group; i < chunks; i += 2) {
       const Buffer bf = buffer(i);
       const int n = min(kMT, r1 - r0 - i * kMT);
-      if (i >= 2) bar_sync(kEmpty + (i & 1), 256);
-      q.split_to(bf.Q, pw, lane);
-      k.split_to(bf.K, pw, lane);
-      v.store_to(bf.V, kMV, pw, lane);
-      if (pw == 3) {
-        if (VAR) {                            // inclusive running sums of the chunk's log decays (a fixed order: lane by lane)
-          float s = l;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const float up = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += up;
-          }
-          bf.L[lane] = s;
-          bf.keep[lane] = expf(s);
-          const float last = __shfl_sync(0xffffffffu, s, n - 1);
-          bf.wj[lane] = lane < n ? expf(last - s) : 0.f;
-        } else {
-          bf.keep[lane] = gp[min(lane, n - 1) + 1];
-          bf.wj[lane] = lane < n ? gp[n - 1 - lane] : 0.f;
-        }
+      if (i >= kBuffers) bar_sync(kEmpty + i % (2 * kBuffers), kBufThreads);
+      x.split_to(bf.Q, bf.dq, pw, lane);
+      {
+        const int64_t row = r0 + i * kMT;
+        x.load(a.k + row * a.ldk + hq * dim, a.ldk, dim, n, vec, pw, lane);
       }
-      if (i + 1 < chunks) fetch(i + 1);
-      bar_sync(kPrepare, 128);
+      v.store_to(bf.V, kMV, pw, lane);
+      float keep = 0.f, wj = 0.f;
+      if (pw == 3) {
+        if (VAR) {
+          const LogSum sum(l, lane);
+          const float hi = (float)sum.l;
+          bf.Lh[lane] = hi;
+          bf.Ll[lane] = (float)(sum.l - (double)hi);
+          keep = sum.from();
+          wj = sum.to();
+        } else {
+          keep = gp[min(lane, n - 1) + 1];
+          wj = lane < n ? gp[n - 1 - lane] : 0.f;
+        }
+        bf.keep[lane] = keep;
+      }
+      x.split_to(bf.K, bf.dk, pw, lane);
+      bar_sync(kPrepare + group, 128);
       if (pw < 3) {                           // A[t][j]: the blocks (0, 0), (16, 0), (16, 16)
         const int t0 = pw ? 16 : 0, j0 = pw == 2 ? 16 : 0;
-        float x[2][4];
-        token_products<KS>(x, bf.Q, t0, bf.K, j0, lane);
+        float z[2][4];
+        Decays f;
+        if (VAR) f.load(bf.Lh, bf.Ll, t0, j0, lane);
+        Down d;
+        d.load(bf.dq, bf.dk, t0, j0, lane);
+        token_products<KS>(z, bf.Q, t0, bf.K, j0, lane);
 #pragma unroll
         for (int y = 0; y < 2; ++y)
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
             const int t = t0 + g + 4 * e, j = j0 + 8 * y + 2 * tq;
-            const float y0 = j <= t ? (VAR ? expf(bf.L[t] - bf.L[j]) : gp[t - j]) * x[y][e] : 0.f;
-            const float y1 = j + 1 <= t ? (VAR ? expf(bf.L[t] - bf.L[j + 1]) : gp[t - j - 1]) * x[y][e + 1] : 0.f;
+            const float y0 = j <= t ? (VAR ? f(y, e) : gp[t - j]) * d(y, e, z[y][e]) : 0.f;
+            const float y1 = j + 1 <= t ? (VAR ? f(y, e + 1) : gp[t - j - 1]) * d(y, e + 1, z[y][e + 1]) : 0.f;
             store_pair(bf.A, t, j, y0, y1);
           }
+      } else {
+        bf.kq[lane] = keep * bf.dq[lane];
+        bf.wk[lane] = wj * bf.dk[lane];
       }
-      bar_arrive(kFull + (i & 1), 256);
+      bar_arrive(kFull + i % kBuffers, kBufThreads);
+      if (i + 2 < chunks) fetch(i + 2);
     }
     return;
   }
   // -------------------------------------------------- state warps
-  const int c = w * 16 + g;
+  registers_take<kStateRegs>();
+  constexpr int KH = KS / 2;                  // blocks of 16 channels of a half
+  const int pair = w & 3, half = w >> 2, c = pair * 16 + g, d0 = half * (DZ / 2);
   const float sw = a.skip ? __ldg(a.skip_w + h) : 0.f;
-  float* sp = a.state + (((int64_t)a.state_slots[b] * a.heads + h) * dim) * a.vdim + v0;
-  float S[2 * KS][4];
-  load_state<KS>(S, sp, a.vdim, dim, c, cols, a.positions[r0] == 0, lane);
+  float* sp = a.state + (((int64_t)a.state_slots[b] * a.heads + h) * dim + d0) * a.vdim + v0;
+  float S[2 * KH][4];
+  load_state<KH>(S, sp, a.vdim, dim - d0, c, cols, a.positions[r0] == 0, lane);
   for (int i = 0; i < chunks; ++i) {
     const Buffer bf = buffer(i);
-    const int64_t row = r0 + i * kMT;
-    const int n = min(kMT, r1 - (int)row);
-    float xs[4][4];                           // the skip term
+    const int64_t row = r0 + i * kMT + kMT / 2 * half + 2 * tq;        // a warp of a pair takes the outputs of one half of the tokens
+    const int n = r1 - (int)row;
+    float xs[2][4];                           // the skip term
     if (a.skip) {
-      const float* xp = a.skip + row * a.lds + h * a.vdim + v0;
+      const float* xp = a.skip + row * a.lds + h * a.vdim + v0 + c;
 #pragma unroll
-      for (int t = 0; t < 4; ++t)
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int tt = 8 * t + 2 * tq + (e & 1), cc = c + 4 * (e & 2);
-          xs[t][e] = (tt < n && cc < cols) ? xp[(int64_t)tt * a.lds + cc] : 0.f;
+          const int tt = 8 * t + (e & 1), cc = 4 * (e & 2);
+          xs[t][e] = (tt < n && c + cc < cols) ? xp[(int64_t)tt * a.lds + cc] : 0.f;
         }
     }
-    bar_sync(kFull + (i & 1), 256);
+    const ColumnScale sc = column_scale(S);
+    bar_sync(kFull + i % kBuffers, kBufThreads);
     // ---- the state's share of the outputs
-    float o[4][4];
+    float o[2][4];
     {
-      float rest[4][4] = {}, x[2][4][4] = {};
+      float x[4][4] = {}, y[4][4] = {}, rest[4][4] = {};       // large products in sums of 32 terms
 #pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        FragA s;
-        FragB f[4];
-        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1]);
-        load_b(f, bf.Q, 0, 16 * ks, lane);
-        mma_high(x[ks & 1], s, f);
+      for (int ks = 0; ks < KH; ++ks) {
+        HalfA s;
+        HalfB f[4];
+        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1], sc.c0.up, sc.c1.up);
+        load_b(f, bf.Q, 0, d0 + 16 * ks, lane);
+        if (ks & 1) mma_high(y, s, f);
+        else mma_high(x, s, f);
         mma_small(rest, s, f);
       }
 #pragma unroll
       for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[t][e] = ((x[0][t][e] + x[1][t][e]) + rest[t][e]) * bf.keep[8 * t + 2 * tq + (e & 1)];
+        for (int e = 0; e < 4; ++e) x[t][e] = ((x[t][e] + y[t][e]) + rest[t][e]) * sc.down(e);
+      float4(*const mine)[32] = swap[pair][i & 1][half], (*const other)[32] = swap[pair][i & 1][half ^ 1];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        other[t][lane] = half ? make_float4(x[t][0], x[t][1], x[t][2], x[t][3]) : make_float4(x[2 + t][0], x[2 + t][1], x[2 + t][2], x[2 + t][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[t][e] = half ? x[2 + t][e] : x[t][e];
+      }
+      bar_sync(kPair + pair, 64);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float4 y = mine[t][lane];
+        o[t][0] += y.x; o[t][1] += y.y; o[t][2] += y.z; o[t][3] += y.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[t][e] *= bf.kq[kMT / 2 * half + 8 * t + 2 * tq + (e & 1)];
+      }
     }
     // ---- the chunk's own share; tokens 0 .. 15 see nothing of 16 .. 31
-    FragA u[2];
+    float u[4][4];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      float v[2][4], wv[2][4];
+      float v[2][4];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int t = 16 * s + 2 * tq + (e & 1) + 2 * (e & 4);
         v[e >> 2][e & 3] = bf.V[t * kMV + c + 4 * (e & 2)];
-        wv[e >> 2][e & 3] = v[e >> 2][e & 3] * bf.wj[t];
+        u[2 * s + (e >> 2)][e & 3] = v[e >> 2][e & 3] * bf.wk[t];
       }
-      FragA f;
-      frag_of_tiles(f, v[0], v[1]);
-      frag_of_tiles(u[s], wv[0], wv[1]);
-      if (s == 0) add_tokens(o, f, bf.A, 0, 0, lane);
-      else add_tokens(*reinterpret_cast<float(*)[2][4]>(o + 2), f, bf.A, 16, 16, lane);
+      if (s <= half) {
+        FragA f;
+        frag_of_tiles(f, v[0], v[1]);
+        add_tokens(o, f, bf.A, kMT / 2 * half, 16 * s, lane);
+      }
     }
     // ---- the state behind the chunk
-    state_update<KS>(S, bf.keep[n - 1], u, bf.K, lane);
-    if (i + 2 < chunks) bar_arrive(kEmpty + (i & 1), 256);
-    float* op = a.o + row * a.ldo + h * a.vdim + v0;
+    state_update<KH>(S, bf.keep[min(kMT, r1 - r0 - i * kMT) - 1], u, bf.K, d0, lane);
+    if (i + kBuffers < chunks) bar_arrive(kEmpty + (i + kBuffers) % (2 * kBuffers), kBufThreads);
+    float* op = a.o + row * a.ldo + h * a.vdim + v0 + c;
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
+    for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int tt = 8 * t + 2 * tq + (e & 1), cc = c + 4 * (e & 2);
+        const int tt = 8 * t + (e & 1), cc = 4 * (e & 2);
         if (a.skip) o[t][e] += sw * xs[t][e];
-        if (tt < n && cc < cols) op[(int64_t)tt * a.ldo + cc] = o[t][e];
+        if (tt < n && c + cc < cols) op[(int64_t)tt * a.ldo + cc] = o[t][e];
       }
   }
-  store_state<KS>(S, sp, a.vdim, dim, c, cols, lane);
+  store_state<KH>(S, sp, a.vdim, dim - d0, c, cols, lane);
 }
 
 template <int KS, int MODE>
 cudaError_t launch_decay_mma(nvc_ctx* ctx, const RetArgs& a, int B, cudaStream_t st) {
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  constexpr int smem = 2 * decay_buf(16 * KS);
+  constexpr int smem = kBuffers * decay_buf(16 * KS);
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(decay_mma_kernel<KS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -627,7 +658,7 @@ cudaError_t launch_decay_mma(nvc_ctx* ctx, const RetArgs& a, int B, cudaStream_t
   }
   const int vec = (a.dim & 3) == 0 && (a.ldq & 3) == 0 && (a.ldk & 3) == 0 && al16(a.q) && al16(a.k);
   const int vecv = (a.vdim & 3) == 0 && (a.ldv & 3) == 0 && al16(a.v);
-  return nvc_launch(ctx, decay_mma_kernel<KS, MODE>, dim3(a.heads * ((a.vdim + kMC - 1) / kMC), B), dim3(256), smem, st, a, B, vec, vecv);
+  return nvc_launch(ctx, decay_mma_kernel<KS, MODE>, dim3(a.heads * ((a.vdim + kMC - 1) / kMC), B), dim3(kScanThreads), smem, st, a, B, vec, vecv);
 }
 
 template <int C, int NW, int MODE>
@@ -652,7 +683,7 @@ int run_scan(nvc_ctx* ctx, const RetArgs& a, int B, int max_qlen, void* stream) 
     // wide slices while they fill the GPU; keys of more than 256 numbers leave room for 32 columns only
     cudaError_t ce;
     // the tensor pipe keeps 16 columns x all channels of the state in a warp's registers, which is what ends it at 128 channels; at 128 x 64
-    // over eight prompts of 245 to 1 050 tokens, 32 heads: 168 us, the FMA form 640
+    // over eight prompts of 245 to 1 050 tokens, 32 heads: 120 us, the FMA form 640
     if constexpr (MODE != kMemory) {
       // portions of up to 16 tokens over states that do not fit in L2: the FMA kernel's slices of 128 columns read them better (256 portions of 10 tokens, 16 heads of
       // 128 x 128, 1 GB of states: 581 us, here 642; 64 portions: 161, here 121; heads of 64 x 64: 282, here 258)

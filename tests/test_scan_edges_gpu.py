@@ -188,3 +188,30 @@ def test_state_space_preparation_in_tiles_of_rows(ctx, ops, H, vdim, Gs, state, 
         return [torch.cat(t) for t in zip(*out)] + [st]
     for got, want in zip(run(0, B, 1 << 20), run(0, B, 400)):
         assert close(got, want.to(F64))
+
+
+@pytest.mark.parametrize("dim,vdim,n", [(128, 64, 250), (64, 33, 33), (20, 130, 97)])
+def test_scans_over_rows_and_columns_of_any_size(ctx, ops, dim, vdim, n):
+    """Rows and state columns are scaled to fp16's range one by one: queries, keys and values of sizes from 1e-12 to 1e12, rows of zeros among them, give the
+    result of the same numbers at size 1, times their sizes.  Powers of two, so that the scaling itself is exact: the results agree bit by bit."""
+    H, G = 2, 1
+    g = torch.Generator().manual_seed(dim)
+    q, k, v = rows([n], g, G, dim) * dim ** -0.5, rows([n], g, G, dim) * dim ** -0.5, rows([n], g, H, vdim)
+    k[n // 2] = 0.0
+    q[n // 3] = 0.0
+    ld = -rows([n], g, H).abs()
+    sq = 2.0 ** torch.randint(-40, 41, (n, 1, 1), generator=g).to(DEV)
+    sv = 2.0 ** torch.randint(-40, 41, (1, 1, vdim), generator=g).to(DEV)
+    state = torch.randn(1, H, dim, vdim, generator=g).to(DEV)
+    cu, pos, slot = i32([0, n]), i32(list(range(3, 3 + n))), i32([0])
+
+    def run(q, v, state, sk=1.0):
+        state = state.clone()
+        o = ops.decay_scan(ctx, (q * 1.0).view(-1, G * dim), (k * sk).view(-1, G * dim), (v / sk).reshape(-1, H * vdim), state, slot, cu, pos, H, G, dim, vdim,
+                           log_decay=ld, max_qlen=n)
+        return o.view(n, H, vdim), state
+    o0, s0 = run(q, v, state)
+    o1, s1 = run(q * sq, v * sv, state * sv)
+    assert torch.equal(o1, o0 * sq * sv) and torch.equal(s1, s0 * sv)
+    o2, s2 = run(q, v, state, sk=2.0 ** 37)
+    assert torch.equal(o2, o0) and torch.equal(s2, s0)
