@@ -18,7 +18,7 @@ namespace widemma {
 constexpr int kSdTok = 16;                            // tokens per warp tile
 template <int DK> constexpr int shared_decode_smem() {
   constexpr int ring = kWarps * kStages * (kSdTok * DK * 2 + kSdTok * 4);
-  constexpr int merge = (2 * kWarps * 16 + 2 * 16 + kWarps * 16 * DK) * 4;
+  constexpr int merge = merge_floats<DK>() * 4;
   return ring > merge ? ring : merge;
 }
 
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) attn_shared_decode_kernel(cons
   float* sm_m = reinterpret_cast<float*>(smem);       // [kWarps][16]
   float* sm_l = sm_m + kWarps * 16;
   float* cta_ml = sm_l + kWarps * 16;                 // [2][16]
-  float* sm_o = cta_ml + 32;                          // [kWarps][16][DK]
+  float* sm_o = cta_ml + 32;                          // [kWarps][16][merge_ld]
 #pragma unroll
   for (int t = 0; t < NR; ++t) {
 #pragma unroll
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(kWarps * 32, 4) attn_shared_decode_kernel(cons
 #pragma unroll
       for (int mt = 0; mt < KS; ++mt) {
         if (mt < mt_n) {
-          sm_o[(warp * 16 + row) * DK + mt * 16 + quad] = o[mt][t][c];
-          sm_o[(warp * 16 + row) * DK + mt * 16 + quad + 8] = o[mt][t][2 + c];
+          sm_o[(warp * 16 + row) * merge_ld<DK>() + mt * 16 + quad] = o[mt][t][c];
+          sm_o[(warp * 16 + row) * merge_ld<DK>() + mt * 16 + quad + 8] = o[mt][t][2 + c];
         }
       }
     }

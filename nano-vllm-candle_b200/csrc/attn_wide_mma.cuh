@@ -67,10 +67,12 @@ __host__ __device__ __forceinline__ int first_visible(int pos, int window, int c
 // tanh from one exp2 and one division: absolute error of a few 1e-7, exact limits at both ends
 __device__ __forceinline__ float tanh_exp2(float x) { return 1.0f - __fdividef(2.0f, fast_exp2(x * (2.0f * kLog2e)) + 1.0f); }
 
+template <int DVM> __host__ __device__ constexpr int merge_ld() { return DVM + 4; }      // floats per row of partial outputs: the four rows that a quad's lanes write fall into different banks
+template <int DVM> __host__ __device__ constexpr int merge_floats() { return 2 * kWarps * 16 + 32 + kWarps * 16 * merge_ld<DVM>(); }
 // a ring stage: keys, values (unless shared), one factor per key
 template <int DKM, int DVM> constexpr int smem_bytes(bool shared) {
   const int ring = kStages * kCtaTok * ((DKM + (shared ? 0 : DVM)) * 2 + 4);
-  constexpr int merge = (2 * kWarps * 16 + 2 * 16 + kWarps * 16 * DVM) * 4;
+  constexpr int merge = merge_floats<DVM>() * 4;
   return ring > merge ? ring : merge;
 }
 
@@ -232,65 +234,121 @@ __device__ __forceinline__ void softmax_step(uint32_t stK, uint32_t stV, uint32_
 }
 
 // The closing merge of a CTA whose warps hold partial results of the same rows in shared memory - per warp and row the running maximum
-// and sum (sm_m, sm_l: [kWarps][16]) and DVM output numbers (sm_o: [kWarps][16][DVM]); cta_ml: 2 x 16 floats of scratch - and, with
+// and sum (sm_m, sm_l: [kWarps][16]) and DVM output numbers (sm_o: [kWarps][16][merge_ld]); cta_ml: 2 x 16 floats of scratch - and, with
 // splits > 1, of the cluster's CTAs through distributed shared memory.  Row r0 + rr of the sequence is token (r0 + rr) / hg of its portion
 // and head g hg + (r0 + rr) % hg.  Sink, gate and factor are applied on the way out.
+//
+// A merge is latency and nothing else: a row's factors are computed once (and not per output number), four numbers go together, and what comes from the
+// other CTAs is requested at once.  Number by number, with a chain over the CTAs, it was 5 us of a decode step's 18.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void fma4_acc(float4& o, const float4& x, float f) {
+  o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+}
+
 template <int DVM, bool kSig>
-__device__ __forceinline__ void merge_store(const Args& a, const float* sm_m, const float* sm_l, float* cta_ml, float* sm_o, int nrows, int r0, int hg,
-                                            int g, int row_begin) {
+__device__ __forceinline__ void merge_store(const Args& a, float* sm_m, const float* sm_l, float* cta_ml, float* sm_o, int nrows, int r0, int hg, int g,
+                                            int row_begin) {
+  constexpr int LD = merge_ld<DVM>();
   float* cta_m = cta_ml;
   float* cta_l = cta_ml + 16;
-  const auto finish = [&](int rr, int d, float M, float L, float O) {     // one output number from the merged partials
+  const int tid = threadIdx.x;
+  const uint32_t q4 = (uint32_t)a.dv >> 2;
+  const auto finish = [&](int rr, int d, float M, float L, float4 O) {     // four output numbers from the merged partials
     const int row = r0 + rr, t = row / hg, h = g * hg + row - t * hg;
-    if (a.sink) {
-      const float sk = __ldg(a.sink + h) * kLog2e, M2 = fmaxf(M, sk);
-      const float f = M == -INFINITY ? 0.f : fast_exp2(M - M2);
-      L = L * f + fast_exp2(sk - M2);
-      O *= f;
-    }
-    float y = kSig ? O * a.out_scale : (L > 0.f ? O / L * a.out_scale : 0.f);
-    if (a.gate) y *= sigmoid_f32(a.gate[(int64_t)(row_begin + t) * a.ldg + (a.gate_per_head ? (int64_t)h : (int64_t)h * a.dv + d)]);
-    a.out[(int64_t)(row_begin + t) * a.ldo + (int64_t)h * a.dv + d] = __bfloat16_as_ushort(__float2bfloat16_rn(y));
-  };
-  for (int idx = threadIdx.x; idx < nrows * a.dv; idx += kWarps * 32) {
-    const int rr = idx / a.dv, d = idx - rr * a.dv;
-    float M = -INFINITY, L = 0.f, O = 0.f;
+    float f = a.out_scale;
     if constexpr (!kSig) {
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm_m[w * 16 + rr]);
+      if (a.sink) {
+        const float sk = __ldg(a.sink + h) * kLog2e, M2 = fmaxf(M, sk), e = M == -INFINITY ? 0.f : fast_exp2(M - M2);
+        L = L * e + fast_exp2(sk - M2);
+        O.x *= e; O.y *= e; O.z *= e; O.w *= e;
+      }
+      f = L > 0.f ? 1.f / L * a.out_scale : 0.f;
     }
+    float y[4] = {O.x * f, O.y * f, O.z * f, O.w * f};
+    if (a.gate) {
+      const float* gp = a.gate + (int64_t)(row_begin + t) * a.ldg;
+      if (a.gate_per_head) {
+        const float s = sigmoid_f32(gp[h]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] *= s;
+      } else {
+        gp += (int64_t)h * a.dv + d;
+        float4 z;
+        if ((reinterpret_cast<uintptr_t>(gp) & 15) == 0) z = *reinterpret_cast<const float4*>(gp);
+        else z = make_float4(gp[0], gp[1], gp[2], gp[3]);
+        y[0] *= sigmoid_f32(z.x); y[1] *= sigmoid_f32(z.y); y[2] *= sigmoid_f32(z.z); y[3] *= sigmoid_f32(z.w);
+      }
+    }
+    nvc_bf16* out = a.out + (int64_t)(row_begin + t) * a.ldo + (int64_t)h * a.dv + d;
+    if ((reinterpret_cast<uintptr_t>(out) & 3) == 0) {
+      reinterpret_cast<uint32_t*>(out)[0] = pack_bf16(y[0], y[1]);
+      reinterpret_cast<uint32_t*>(out)[1] = pack_bf16(y[2], y[3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[i] = __bfloat16_as_ushort(__float2bfloat16_rn(y[i]));
+    }
+  };
+  // ---- the warps of the CTA: the rows' factors take the place of their maxima
+  if (!kSig && tid < 16) {
+    float M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm_m[w * 16 + tid]);
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float mw = sm_m[w * 16 + rr];
-      const float wt = kSig ? 1.f : (mw == -INFINITY ? 0.f : fast_exp2(mw - M));
-      L += sm_l[w * 16 + rr] * wt;
-      O += sm_o[(w * 16 + rr) * DVM + d] * wt;
+      const float mw = sm_m[w * 16 + tid], f = mw == -INFINITY ? 0.f : fast_exp2(mw - M);
+      L = fmaf(sm_l[w * 16 + tid], f, L);
+      sm_m[w * 16 + tid] = f;
     }
-    if (a.splits == 1) {
-      finish(rr, d, M, L, O);
-    } else {
-      sm_o[rr * DVM + d] = O;                         // warp 0's partial of the same number: this thread alone reads and writes it
-      if (d == 0) { cta_m[rr] = M; cta_l[rr] = L; }
-    }
+    cta_m[tid] = M;
+    cta_l[tid] = L;
+  }
+  __syncthreads();
+  for (uint32_t idx = tid; idx < nrows * q4; idx += kWarps * 32) {
+    const int rr = idx / q4, d = 4 * (idx - rr * q4);
+    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) fma4_acc(O, *reinterpret_cast<const float4*>(sm_o + (w * 16 + rr) * LD + d), kSig ? 1.f : sm_m[w * 16 + rr]);
+    if (a.splits == 1) finish(rr, d, kSig ? 0.f : cta_m[rr], kSig ? 0.f : cta_l[rr], O);
+    else *reinterpret_cast<float4*>(sm_o + rr * LD + d) = O;       // warp 0's partial of the same numbers: this thread alone reads and writes it
   }
   if (a.splits == 1) return;
-  // ---- merge the CTAs of the cluster: each takes a share of the output numbers and reads the others' partials
+  // ---- the CTAs of the cluster: each takes a share of the output numbers and reads the others' partials
   ptx::cluster_sync_all();
   const uint32_t rank = ptx::cluster_ctarank();
-  for (int idx = rank * (kWarps * 32) + threadIdx.x; idx < nrows * a.dv; idx += a.splits * kWarps * 32) {
-    const int rr = idx / a.dv, d = idx - rr * a.dv;
-    float M = -INFINITY, L = 0.f, O = 0.f;
-    for (int c = 0; c < a.splits; ++c) {
-      const float oc = ld_cluster_f(ptx::mapa_u32(smem_u32(sm_o + rr * DVM + d), c));
-      if constexpr (kSig) {
-        O += oc;
-      } else {
-        const float mc = ld_cluster_f(ptx::mapa_u32(smem_u32(cta_m + rr), c)), lc = ld_cluster_f(ptx::mapa_u32(smem_u32(cta_l + rr), c));
-        const float Mn = fmaxf(M, mc), Mb = Mn == -INFINITY ? 0.f : Mn;
-        const float f0 = fast_exp2(M - Mb), f1 = fast_exp2(mc - Mb);          // -inf: 0
-        L = L * f0 + lc * f1;
-        O = O * f0 + oc * f1;
-        M = Mn;
+  float* all_m = sm_o + 16 * LD;                      // [16][16], [16][16] behind warp 0's partials, which alone are read from outside
+  float* all_l = all_m + 256;
+  static_assert(16 * LD >= 512, "room for the CTAs' maxima and sums");
+  if constexpr (!kSig) {
+    for (int i = tid; i < 16 * a.splits; i += kWarps * 32) {
+      all_m[i] = ld_cluster_f(ptx::mapa_u32(smem_u32(cta_m + (i & 15)), i >> 4));
+      all_l[i] = ld_cluster_f(ptx::mapa_u32(smem_u32(cta_l + (i & 15)), i >> 4));
+    }
+    __syncthreads();
+  }
+  for (uint32_t idx = rank + a.splits * tid; idx < nrows * q4; idx += a.splits * kWarps * 32) {
+    const int rr = idx / q4, d = 4 * (idx - rr * q4);
+    const uint32_t at = smem_u32(sm_o + rr * LD + d);
+    float M = -INFINITY, L = 0.f;
+    if constexpr (!kSig)
+      for (int c = 0; c < a.splits; ++c) M = fmaxf(M, all_m[c * 16 + rr]);
+    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c0 = 0; c0 < a.splits; c0 += 4) {        // four at a time; a cluster of two reads each of its CTAs' numbers once and the last ones again, with a factor of 0
+      float4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = ld_cluster_f4(ptx::mapa_u32(at, min(c0 + i, a.splits - 1)));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float f = c0 + i < a.splits ? 1.f : 0.f;
+        if constexpr (!kSig) {
+          const int e = min(c0 + i, a.splits - 1) * 16 + rr;
+          f = c0 + i < a.splits && all_m[e] != -INFINITY ? fast_exp2(all_m[e] - M) : 0.f;
+          L = fmaf(all_l[e], f, L);
+        }
+        fma4_acc(O, x[i], f);
       }
     }
     finish(rr, d, M, L, O);
@@ -536,7 +594,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3) attn_wide_mma_kernel(const Arg
   float* sm_m = reinterpret_cast<float*>(smem);       // [kWarps][16]
   float* sm_l = sm_m + kWarps * 16;
   float* cta_m = sm_l + kWarps * 16;                  // [2][16]: the CTA's own merge (splits > 1)
-  float* sm_o = cta_m + 32;                           // [kWarps][16][DVM]
+  float* sm_o = cta_m + 32;                           // [kWarps][16][merge_ld]
   if (tq == 0) {
     sm_m[warp * 16 + quad] = m0;
     sm_m[warp * 16 + quad + 8] = m1;
@@ -546,8 +604,8 @@ __global__ void __launch_bounds__(kWarps * 32, 3) attn_wide_mma_kernel(const Arg
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
     const int d = nt * 8 + 2 * tq;
-    float* p0 = sm_o + (warp * 16 + quad) * DVM + d;
-    float* p1 = sm_o + (warp * 16 + quad + 8) * DVM + d;
+    float* p0 = sm_o + (warp * 16 + quad) * merge_ld<DVM>() + d;
+    float* p1 = sm_o + (warp * 16 + quad + 8) * merge_ld<DVM>() + d;
     p0[0] = o[nt][0]; p0[1] = o[nt][1];
     p1[0] = o[nt][2]; p1[1] = o[nt][3];
   }
@@ -600,12 +658,15 @@ inline int attn_wide_mma_launch(nvc_ctx* ctx, const void* q, const void* k_cache
   if (s.kv_heads > 65535 || B > 65535) return NVC_ENOTIMPL;
   const bool shared = k_cache == v_cache && ldk == ldv && s.vdim <= s.dim && (s.kv_heads == 1 || s.vdim == s.dim);
   // few rows and few CTAs: clusters of up to 8 (16 for decode over shared rows) share the keys of a chunk, as long as a CTA keeps at least
-  // 128 of them
+  // 64 of them, a tile per warp (1 sequence of 700, latent rows: 14.3 -> 12.3 us against 128 of them; 8 x 8 heads, window of 256: 16.4 -> 14.4).  Up to three CTAs
+  // per SM; clusters of two and four over shared rows up to four, which is what an SM holds of them (64 sequences of 24 heads 24.6 -> 20.5; clusters of eight lose
+  // there: 36 of 24 heads 18.4 -> 21.7)
   int splits = 1;
-  const int max_splits = attn_shared_decode_takes(s, shared, cu_seqlens, block_size) ? 16 : 8;
+  const bool shared_decode = attn_shared_decode_takes(s, shared, cu_seqlens, block_size);
   if (max_total < 64) {
     const int64_t keys = s.window > 0 ? s.window : (s.chunk > 0 ? s.chunk : (int64_t)bt_stride * block_size);
-    while (splits < max_splits && (int64_t)gx * B * s.kv_heads * splits * 2 <= 3 * ctx->num_sms && keys >= 256 * splits) splits *= 2;
+    while (splits < (shared_decode ? 16 : 8) && (int64_t)gx * B * s.kv_heads * splits * 2 <= (shared_decode && splits < 4 ? 4 : 3) * ctx->num_sms && keys >= 128 * splits)
+      splits *= 2;
     gx *= splits;
   }
   widemma::Args a{reinterpret_cast<const nvc_bf16*>(q), reinterpret_cast<const nvc_bf16*>(k_cache), reinterpret_cast<const nvc_bf16*>(v_cache),

@@ -84,6 +84,71 @@ __global__ void latent_norm_store_kernel(const float* __restrict__ in, int ldi, 
   }
 }
 
+// four neighbouring numbers in the storage format
+__device__ __forceinline__ void st_f4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st_f4(__nv_bfloat16* p, const float4& v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
+__device__ __forceinline__ float4 scale4(const float4& x, float r, const float4& w) { return make_float4(x.x * r * w.x, x.y * r * w.y, x.z * r * w.z, x.w * r * w.w); }
+__device__ __forceinline__ float dot4(const float4& x) { return x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w; }
+
+// The same where the rows allow 16-byte accesses, n0 <= 128 V and latent and rotated part fit in 128 numbers: a warp requests all of its row at once, keeps
+// it in registers, and finds weights, slot and angles already there.  The general kernel reads the row twice, number by number, and the slot, the second part
+// and the angles one behind the other: 64 rows of 512 + 96 + 32 took 4.4 us, here 2.9; 2 400 rows 6.5, here 3.3.
+template <typename T, int V>
+__global__ void __launch_bounds__(128) latent_norm_store_row_kernel(const float* __restrict__ in, int ldi, int n0, int off1, int n1, const float* __restrict__ w0,
+                                                                    const float* __restrict__ w1, float eps, T* __restrict__ out0, int ld0, T* __restrict__ cache,
+                                                                    int ldc, const int32_t* __restrict__ slots, int rot_dim, int rot_dims, int rot_half,
+                                                                    const float* __restrict__ rot_table, const int32_t* __restrict__ positions, int N) {
+  pdl_trigger();
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= N) return;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int j = 4 * lane, jr = j - n1, half = rot_dims >> 1;          // this lane's numbers of the second part; of its rotated part
+  const bool rotated = jr >= 0 && jr < rot_dims;
+  // what no kernel of the step writes: weights, the slot, the angles
+  float4 w[V], wl = zero, c0 = zero, c1 = zero;
+#pragma unroll
+  for (int v = 0; v < V; ++v) w[v] = j + 128 * v < n0 ? __ldg(reinterpret_cast<const float4*>(w0 + j + 128 * v)) : zero;
+  const int slot = cache ? slots[row] : -1;
+  if (cache) {
+    if (j < n1) wl = __ldg(reinterpret_cast<const float4*>(w1 + j));
+    if (rotated) {
+      const float4* cs = reinterpret_cast<const float4*>(rot_table + (int64_t)positions[row] * rot_dims + (rot_half ? 2 * (jr < half ? jr : jr - half) : jr));
+      c0 = __ldg(cs);
+      if (rot_half) c1 = __ldg(cs + 1);
+    }
+  }
+  pdl_wait();
+  const float* x = in + (int64_t)row * ldi;
+  float4 a[V], k = zero;
+#pragma unroll
+  for (int v = 0; v < V; ++v) a[v] = j + 128 * v < n0 ? *reinterpret_cast<const float4*>(x + j + 128 * v) : zero;
+  if (slot >= 0 && j < n1 + rot_dim) k = *reinterpret_cast<const float4*>(x + off1 + j);
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < V; ++v) ss += dot4(a[v]);
+  const float r0 = 1.0f / sqrtf(warp_sum(ss) / (float)n0 + eps);
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+    if (j + 128 * v < n0) st_f4(out0 + (int64_t)row * ld0 + j + 128 * v, scale4(a[v], r0, w[v]));
+  if (slot < 0) return;
+  const float r1 = 1.0f / sqrtf(warp_sum(j < n1 ? dot4(k) : 0.f) / (float)n1 + eps);
+  // (i, i + half) by exchange, neighbouring pairs inside the lane
+  const int from = lane + (jr < half ? half >> 2 : -(half >> 2));
+  const float4 z = make_float4(__shfl_sync(0xffffffffu, k.x, from), __shfl_sync(0xffffffffu, k.y, from), __shfl_sync(0xffffffffu, k.z, from),
+                               __shfl_sync(0xffffffffu, k.w, from));
+  if (j < n1) {
+    k = scale4(k, r1, wl);
+  } else if (rotated) {
+    if (rot_half) {
+      const float s = jr < half ? -1.f : 1.f;
+      k = make_float4(k.x * c0.x + s * z.x * c0.y, k.y * c0.z + s * z.y * c0.w, k.z * c1.x + s * z.z * c1.y, k.w * c1.z + s * z.w * c1.w);
+    } else {
+      k = make_float4(k.x * c0.x - k.y * c0.y, k.y * c0.x + k.x * c0.y, k.z * c0.z - k.w * c0.w, k.w * c0.z + k.z * c0.w);
+    }
+  }
+  if (j < n1 + rot_dim) st_f4(cache + (int64_t)slot * ldc + j, k);
+}
+
 // NVC_ACT_GELU_TANH_MUL: out[n, j] = gelu_tanh(in[n, j]) * in[n, Fp + j];  NVC_ACT_RELU2: out[n, j] = relu(in[n, j])^2;
 // NVC_ACT_SILU_MUL: silu(in[n, j]) * in[n, Fp + j];  NVC_ACT_GELU_TANH: gelu_tanh(in[n, j]);  NVC_ACT_GLU_CLAMP: g sigmoid(p1 g) (u + 1), g = min(in[n, j], p0), u = clamp(in[n, Fp + j], +-p0)
 __device__ __forceinline__ float act_unit(int kind, float g, float u, float p0, float p1) {
@@ -213,6 +278,17 @@ int nvc_latent_norm_store_rot(nvc_ctx* ctx, const float* in, int ldi, int n0, in
   NVC_REQUIRE(ctx, N >= 0 && n0 > 0 && n1 >= 0 && off1 >= n0 && ldi >= off1 + n1 + rot_dim && ld0 >= n0 && (!cache || ldc >= n1 + rot_dim),
               NVC_EINVAL, "bad sizes");
   if (N == 0) return NVC_OK;
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const bool vec = n0 <= 1024 && ((n0 | off1 | n1 | rot_dim | rot_dims | ldi | ld0 | ldc) & 3) == 0 && (!rot_half || rot_dims % 8 == 0) && al16(in) && al16(w0) &&
+                   al16(out0) && (!cache || (n1 > 0 && n1 + rot_dim <= 128 && al16(w1) && al16(cache) && (rot_dims == 0 || al16(rot_table))));
+  if (vec) {
+    NVC_DISPATCH_DT(dtype, T,
+                    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, n0 <= 512 ? latent_norm_store_row_kernel<T, 4> : latent_norm_store_row_kernel<T, 8>, dim3((N + 3) / 4), dim3(128), 0,
+                                                   nvc_stream(stream), in, ldi, n0, off1, n1, w0, w1, eps, reinterpret_cast<T*>(out0), ld0,
+                                                   reinterpret_cast<T*>(cache), ldc, slot_mapping, rot_dim, rot_dims, rot_half, rot_table, positions, N)));
+    ctx->launches++;
+    return NVC_OK;
+  }
   NVC_DISPATCH_DT(dtype, T,
                   NVC_CUDA_CHECK(ctx, nvc_launch(ctx, latent_norm_store_kernel<T>, dim3((N + 3) / 4), dim3(128), 0, nvc_stream(stream), in,
                                                  ldi, n0, off1, n1, w0, w1, eps, reinterpret_cast<T*>(out0), ld0,
