@@ -33,8 +33,8 @@ __global__ void __launch_bounds__(128) gate_rows_kernel(const float* __restrict_
   uint32_t n = min(u0, units - 1) / (uint32_t)groups, k = min(u0, units - 1) - n * groups;
   const uint32_t n0 = n, k0 = k;
   auto gated = [&](float4 v, const float4& z) {
-    if (act == NVC_GATE_SILU) { v.x *= z.x * sigmoid_f32(z.x); v.y *= z.y * sigmoid_f32(z.y); v.z *= z.z * sigmoid_f32(z.z); v.w *= z.w * sigmoid_f32(z.w); }
-    else { v.x *= sigmoid_f32(z.x); v.y *= sigmoid_f32(z.y); v.z *= sigmoid_f32(z.z); v.w *= sigmoid_f32(z.w); }
+    if (act == NVC_GATE_SILU) { v.x *= z.x * sigmoid_to<T>(z.x); v.y *= z.y * sigmoid_to<T>(z.y); v.z *= z.z * sigmoid_to<T>(z.z); v.w *= z.w * sigmoid_to<T>(z.w); }
+    else { v.x *= sigmoid_to<T>(z.x); v.y *= sigmoid_to<T>(z.y); v.z *= sigmoid_to<T>(z.z); v.w *= sigmoid_to<T>(z.w); }
     return v;
   };
   float4 x[L][V], z[L][V];
