@@ -1,6 +1,6 @@
 """Latent attention's decode step at its edges: the preparation's 16-byte rows against its general form, and decode attention over shared rows where clusters of
 1 to 16 CTAs share a sequence's keys, down to empty shares.  Bounds: fp32 sums in another order differ by a few 2^-24 of the norm (1e-6 here), a bf16 result
-by one rounding more (2^-8 of the value); attention keeps weights of 8 bits over fp32 sums (1e-2 of the largest output)."""
+may round to the neighbouring number, up to 2^-7 of its value away; attention keeps weights of 8 bits over fp32 sums (1e-2 of the largest output)."""
 import importlib
 
 import pytest
@@ -35,7 +35,7 @@ def test_rows_of_the_latent_preparation(ctx, ops, dtype, n0, n1, rot_dim, rot_di
         cache = torch.full((10, n1 + rot_dim), 7.0, device=DEV, dtype=dtype)
         out = ops.latent_norm_store_rot(ctx, rows, n0, off, n1, w0, w1, 1e-6, cache, slots, rot_dim, rot_dims, half, table, pos if rot_dims else None, dtype)
         got.append((out.float(), cache.float()))
-    tol = 1e-6 if dtype == torch.float32 else 2.0 ** -8
+    tol = 1e-6 if dtype == torch.float32 else 2.0 ** -7
     for a, b in zip(*got):
         assert float(((a - b).abs() - tol * b.abs()).max()) <= 1e-6 * float(b.abs().max())
 

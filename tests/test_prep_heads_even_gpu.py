@@ -1,5 +1,6 @@
 """Preparation of projection rows whose warps hold heads of one kind, against the general kernel (an odd row stride takes it).  Bounds: the square sum's order
-differs, a few 2^-24 of the norm, so 1e-6 of the largest number; a bf16 result by one rounding more, 2^-8 of its value."""
+differs, a few 2^-24 of the norm, so 1e-6 of the largest number; a bf16 result may round to
+the neighbouring number, which is up to 2^-7 of its value away (8 significant bits)."""
 import importlib
 
 import pytest
@@ -34,6 +35,6 @@ def test_heads_of_one_kind_per_warp(ctx, dtype, N, rot, half, H, G, d, vd):
                          k_norm=kn if normed else None, rot_dims=rot, rot_half=half, rot_table=table, positions=pos if rot else None, k_scale=0.5, v_scale=2.0,
                          slot_mapping=slots)
             got.append([t.float() for t in (q, k, v)])
-        tol = 1e-6 if dtype == torch.float32 else 2.0 ** -8
+        tol = 1e-6 if dtype == torch.float32 else 2.0 ** -7
         for a, b in zip(*got):
             assert float(((a - b).abs() - tol * b.abs()).max()) <= 1e-6 * float(b.abs().max())
