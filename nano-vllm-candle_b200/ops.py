@@ -15,12 +15,14 @@ from ._lib import check
 BF16 = torch.bfloat16
 
 
+# A call's own cost counts where its kernels are short (a decode step of one layer): every entry point declares its argument types, so that addresses
+# go in as plain integers, and the current stream's handle is asked for without building a Stream object around it.
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _req(t: torch.Tensor, dtype, name: str):
