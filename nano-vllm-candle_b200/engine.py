@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes as C
 import json
 import os
+import sys
 from dataclasses import dataclass, field
 from typing import Dict, Iterable, List, Optional, Sequence as Seq, Tuple
 
@@ -176,7 +177,21 @@ def _i32(a) -> np.ndarray:
 
 
 def _p(a: np.ndarray):
-    return a.ctypes.data_as(C.c_void_p)
+    """The address of an array that the caller holds on to (a.ctypes builds two objects around it)."""
+    return a.__array_interface__["data"][0]
+
+
+# Logits leave the GPU as they are wanted by the caller: in an array of its own.  Into fresh pageable memory the driver copies twice, page by page (8 x 32 768
+# numbers: 107 us of a 274 us step); into page-locked memory the GPU writes once (24 us).  The memory comes from the process's tensor library, where one is
+# in use, and goes back to its pool with the array; arrays below 64 KiB or above 32 MiB - which a pool should not hold on to - stay pageable.
+_PINNED_BYTES = range(1 << 16, (1 << 25) + 1)
+
+
+def _logits_array(rows: int, cols: int) -> np.ndarray:
+    torch = sys.modules.get("torch")
+    if torch is None or not torch.cuda.is_initialized() or rows * cols * 4 not in _PINNED_BYTES:
+        return np.empty((rows, cols), dtype=np.float32)
+    return torch.empty((rows, cols), dtype=torch.float32, pin_memory=True).numpy()
 
 
 class Qwen3ModelRunner:
@@ -305,7 +320,7 @@ class Qwen3ModelRunner:
     def last_logits(self, B: int) -> np.ndarray:
         """fp32 logits [B, vocab / tp_size] of this rank's vocab shard for the last step."""
         v_l = self.cfg.vocab_size // self.ctx.tp_size
-        out = np.empty((B, v_l), dtype=np.float32)
+        out = _logits_array(B, v_l)
         check(self.l.nvc_runner_last_logits(self.handle, _p(out), B), "nvc_runner_last_logits", self.ctx.h)
         return out
 
@@ -451,7 +466,7 @@ class ModelRunner(Qwen3ModelRunner):
         check(self.l.nvc_runner_set_state_slots(self.handle, _p(a), len(a)), "nvc_runner_set_state_slots", self.ctx.h)
 
     def last_logits(self, B: int) -> np.ndarray:
-        out = np.empty((B, self.vocab_size // self.ctx.tp_size), dtype=np.float32)
+        out = _logits_array(B, self.vocab_size // self.ctx.tp_size)
         check(self.l.nvc_runner_last_logits(self.handle, _p(out), B), "nvc_runner_last_logits", self.ctx.h)
         return out
 

@@ -1,0 +1,21 @@
+"""Arrays for logits: page-locked between 64 KiB and 32 MiB, plain outside, and always the caller's own."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 7), (1, 16384), (3, 32768), (64, 131072), (65, 131073)])
+def test_logits_arrays_are_the_callers_own(ctx, rows, cols):
+    engine = importlib.import_module("nano-vllm-candle_b200.engine")
+    torch.zeros(1, device="cuda:0")
+    a, b = engine._logits_array(rows, cols), engine._logits_array(rows, cols)
+    for x in (a, b):
+        assert x.shape == (rows, cols) and x.dtype == np.float32 and x.flags.c_contiguous and x.flags.writeable
+        assert torch.from_numpy(x).is_pinned() == ((1 << 16) <= rows * cols * 4 <= (1 << 25))
+    assert not np.shares_memory(a, b)
+    a[:], b[:] = 1.0, 2.0
+    assert a[0, 0] == 1.0 and a[-1, -1] == 1.0
