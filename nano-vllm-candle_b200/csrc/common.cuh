@@ -127,6 +127,8 @@ static inline cudaError_t nvc_launch(const nvc_ctx* ctx, void (*kernel)(KArgs...
 
 // Programmatic dependent launch (griddepcontrol): wait = all prerequisite grids have completed
 // and their memory is visible; trigger = the next grid in the stream may be scheduled.
+// What an earlier kernel writes is read through plain pointers where the load stands right behind the wait: through `const T* __restrict__` it is a load of
+// data that never changes, which the compiler may move in front of the wait, memory clobber or not (seen on sm_100a: an eighth of the numbers were stale).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

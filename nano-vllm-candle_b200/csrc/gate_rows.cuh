@@ -23,8 +23,8 @@ __device__ __forceinline__ void gate_store(__nv_bfloat16* p, const float4& v) {
 // w: gsize numbers per group, wstride apart (0: the same for every group).  gsize is a multiple of 4 and at most 4 W V.
 // W lanes per unit.
 template <typename T, int W, int V, int L>
-__global__ void __launch_bounds__(128) gate_rows_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, int ldg, const float* __restrict__ w,
-                                                        int wstride, T* __restrict__ out, int ldout, int groups, int gsize, int norm, int gate_first, float eps,
+__global__ void __launch_bounds__(128) gate_rows_kernel(const float* o, int ldo, const float* g, int ldg, const float* __restrict__ w,
+                                                        int wstride, T* out, int ldout, int groups, int gsize, int norm, int gate_first, float eps,
                                                         int act, float out_scale, uint32_t units) {
   pdl_trigger();
   pdl_wait();

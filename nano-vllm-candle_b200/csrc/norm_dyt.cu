@@ -94,8 +94,8 @@ __device__ __forceinline__ float dot4(const float4& x) { return x.x * x.x + x.y 
 // it in registers, and finds weights, slot and angles already there.  The general kernel reads the row twice, number by number, and the slot, the second part
 // and the angles one behind the other: 64 rows of 512 + 96 + 32 took 4.4 us, here 2.9; 2 400 rows 6.5, here 3.3.
 template <typename T, int V>
-__global__ void __launch_bounds__(128) latent_norm_store_row_kernel(const float* __restrict__ in, int ldi, int n0, int off1, int n1, const float* __restrict__ w0,
-                                                                    const float* __restrict__ w1, float eps, T* __restrict__ out0, int ld0, T* __restrict__ cache,
+__global__ void __launch_bounds__(128) latent_norm_store_row_kernel(const float* in, int ldi, int n0, int off1, int n1, const float* __restrict__ w0,
+                                                                    const float* __restrict__ w1, float eps, T* out0, int ld0, T* cache,
                                                                     int ldc, const int32_t* __restrict__ slots, int rot_dim, int rot_dims, int rot_half,
                                                                     const float* __restrict__ rot_table, const int32_t* __restrict__ positions, int N) {
   pdl_trigger();
