@@ -151,13 +151,17 @@ __global__ void __launch_bounds__(128) latent_norm_store_row_kernel(const float*
 
 // NVC_ACT_GELU_TANH_MUL: out[n, j] = gelu_tanh(in[n, j]) * in[n, Fp + j];  NVC_ACT_RELU2: out[n, j] = relu(in[n, j])^2;
 // NVC_ACT_SILU_MUL: silu(in[n, j]) * in[n, Fp + j];  NVC_ACT_GELU_TANH: gelu_tanh(in[n, j]);  NVC_ACT_GLU_CLAMP: g sigmoid(p1 g) (u + 1), g = min(in[n, j], p0), u = clamp(in[n, Fp + j], +-p0)
+// T: what the result is stored as; the gates of a bf16 result take the hardware's exponential and reciprocal (typed.cuh; silu, 10 112 x 1 536, cold cache:
+// 19.5 -> 14.4 us, 64 tokens' 2 176 rows 6.4 -> 5.2)
+template <typename T> __device__ __forceinline__ float act_sigmoid(float x) { return sizeof(T) == 2 ? sigmoid_to<T>(x) : sigmoid_f32(x); }
+template <typename T>
 __device__ __forceinline__ float act_unit(int kind, float g, float u, float p0, float p1) {
   if (kind == NVC_ACT_GELU_TANH_MUL) return gelu_tanh_f32(g) * u;
   if (kind == NVC_ACT_GELU_TANH) return gelu_tanh_f32(g);
-  if (kind == NVC_ACT_SILU_MUL) return g * sigmoid_f32(g) * u;
+  if (kind == NVC_ACT_SILU_MUL) return g * act_sigmoid<T>(g) * u;
   if (kind == NVC_ACT_GLU_CLAMP) {
     const float gc = fminf(g, p0);
-    return gc * sigmoid_f32(p1 * gc) * (fminf(fmaxf(u, -p0), p0) + 1.0f);
+    return gc * act_sigmoid<T>(p1 * gc) * (fminf(fmaxf(u, -p0), p0) + 1.0f);
   }
   const float t = fmaxf(g, 0.f);
   return t * t;
@@ -175,7 +179,7 @@ __global__ void act_mul_kernel(const T* __restrict__ in, int ldi, T* __restrict_
     if (n >= N) return;
     const T* x = in + n * ldi;
     T* y = out + n * ldo;
-    for (int j = threadIdx.x; j < F; j += blockDim.x) st_f(y + j, act_unit(kind, ld_f(x + j), two ? ld_f(x + Fp + j) : 0.f, p0, p1));
+    for (int j = threadIdx.x; j < F; j += blockDim.x) st_f(y + j, act_unit<T>(kind, ld_f(x + j), two ? ld_f(x + Fp + j) : 0.f, p0, p1));
   }
 }
 
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(512) act_mul_rows_kernel(const T* in, int ldi,
       for (int k = 0; k < PER; ++k) {
         float f = 0.f;
         if constexpr (two) f = ld_f(u[r] + k);
-        st_f(o + k, act_unit(kKind, ld_f(g[r] + k), f, p0, p1));
+        st_f(o + k, act_unit<T>(kKind, ld_f(g[r] + k), f, p0, p1));
       }
       if (n0 + r < N) *reinterpret_cast<uint4*>(out + (n0 + r) * ldo + j) = *reinterpret_cast<const uint4*>(o);
     }

@@ -45,3 +45,19 @@ def test_gates_behind_a_gather(ctx, ops, N):
     ids = torch.randint(0, 500, (40, N), device=DEV, dtype=torch.int32)
     z, w = torch.randn(N, 2048, device=DEV), torch.randn(128, device=DEV)
     chain(lambda i: [ops.head_gate_w(ctx, ops.embed_gather_f32(ctx, ids[i], table), z, w, 16, 128, True, 1e-5, "silu", 1.0, out_dtype=torch.bfloat16)])
+
+
+@pytest.mark.parametrize("N,E,top", [(40, 16, 2), (4000, 16, 2), (4000, 24, 3), (3000, 64, 5)])
+def test_experts_passes_behind_one_another(ctx, ops, N, E, top):
+    H = 1024
+    table = torch.randn(500, E, device=DEV)
+    ids = torch.randint(0, 500, (40, N), device=DEV, dtype=torch.int32)
+    x, corr = torch.randn(N, H, device=DEV).to(torch.bfloat16), torch.zeros(E, device=DEV)
+    rows_f32 = torch.randn(((N * top + E * 127 + 127) // 128) * 128, H, device=DEV)
+
+    def step(i):
+        idx, w = ops.moe_route_logits_ex(ctx, ops.embed_gather_f32(ctx, ids[i], table), corr, E, top, 1.0, ops.ROUTE_SOFTMAX, True)
+        offsets, src, pos, groups = ops.moe_sort_padded(ctx, idx, E)
+        rows = ops.gather_rows(ctx, x, src, offsets[E:])
+        return idx, w, offsets, src, pos, groups, rows, ops.moe_combine(ctx, rows_f32, pos, w)
+    chain(step, 20)
