@@ -1,0 +1,34 @@
+"""Products over a few hundred to a few thousand rows take the tile width and split that fill the last wave: every choice against fp32, at rows and columns around
+the tiles' edges.  Bound: bf16 results round by 2^-9 of the value (2^-8 is allowed, one more ulp for the sum); fp32 sums of K products of size K^-1/2 differ by less than 1e-4 of the largest."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV, BF16 = "cuda:0", torch.bfloat16
+
+
+@pytest.mark.parametrize("M", [257, 300, 511, 513, 700, 1100, 1300, 2600])
+@pytest.mark.parametrize("N,K", [(1024, 2048), (1024, 3072), (1040, 1024), (2048, 6144), (4096, 1024), (2064, 2048), (272, 512)])
+def test_widths_and_splits(ctx, M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a = torch.randn(M, K, generator=g, device=DEV).to(BF16)
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).to(BF16)
+    want = a.float() @ w.float().T
+    out = torch.full((M + 1, N), 7.0, device=DEV, dtype=BF16)
+    ctx.gemm(a, w, out=out[:M])
+    top = float(want.abs().max())
+    assert float(((out[:M].float() - want).abs() - 2.0 ** -8 * want.abs()).max()) <= 1e-4 * top
+    assert bool((out[M] == 7.0).all())
+    f32 = ctx.gemm(a, w, out_dtype=torch.float32)
+    assert float((f32 - want).abs().max()) <= 1e-4 * top
+
+
+@pytest.mark.parametrize("M,I,K", [(300, 3072, 1024), (512, 6144, 2048), (1100, 1552, 1024), (700, 400, 2048)])
+def test_widths_of_gated_products(ctx, M, I, K):
+    g = torch.Generator(device=DEV).manual_seed(M + I)
+    a = torch.randn(M, K, generator=g, device=DEV).to(BF16)
+    gu = (torch.randn(2 * I, K, generator=g, device=DEV) * K ** -0.5).to(BF16)
+    z = a.float() @ gu.float().T
+    want = torch.nn.functional.silu(z[:, :I]) * z[:, I:]
+    got = ctx.gemm_silu_mul(a, ctx.interleave_gate_up(gu))
+    assert float(((got.float() - want).abs() - 2.0 ** -8 * want.abs()).max()) <= 1e-4 * float(want.abs().max())
