@@ -84,7 +84,7 @@ cudaError_t launch_v2(nvc_ctx* ctx, int QT, int nh, int kv, int B, cudaStream_t 
   const long long items = (long long)QT * nh * B;
   if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
   const int grid = (int)(items < 2LL * ctx->num_sms ? items : 2LL * ctx->num_sms);
-  v2::Sched sc{v2::make_fastdiv(nh * B), v2::make_fastdiv(nh), v2::make_fastdiv(nh / kv), QT, (int)items};
+  v2::Sched sc{v2::make_fastdiv(nh * B), v2::make_fastdiv(nh), v2::make_fastdiv(nh / kv), QT, (int)items, B};
   return nvc_launch(ctx, v2::prefill_attn_v2_kernel<kPaged, kMode>, dim3(grid), dim3(v2::kThreads), v2::kSmemBytes, st, tq, tk, tv,
                     cu_seqlens, sc, scale_log2e, out, ldo, pk);
 }
