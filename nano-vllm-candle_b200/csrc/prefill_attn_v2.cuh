@@ -86,18 +86,22 @@ __device__ __forceinline__ Item item_of(int it, const Sched& sc) {
   return x;
 }
 
-// The items of one CTA: every gridDim.x-th of them.  Up to kListed sequences only the q tiles that exist are counted: a batch of ragged lengths is up to half empty
-// tiles, which a plain enumeration deals out as if they were work - some CTAs got twice the others' tiles (8 prompts of 245 - 1 050, window 256: 50 -> 38 us;
-// 16 of 100 - 1 060, causal: 46 -> 37).  Lane i of every warp knows how many q tiles sequences i and i + 32 have; a level (one q tile index, the highest first) is a ballot.
+// The items of one CTA: one of every gridDim.x, back and forth, since items shrink along the list: whoever gets the largest of one round gets the smallest of the
+// next (always the same place gave some CTAs 31 kv tiles of 18.6 in the mean, so 25).  Up to kListed sequences only the q tiles that exist are counted: a batch of
+// ragged lengths is up to half empty tiles, which a plain enumeration deals out as if they were work.  Lane i of every warp knows how many q tiles sequences i and
+// i + 32 have; a level (one q tile index, the highest first) is a ballot.  8 prompts of 245 - 1 050 tokens, window 256, gate, heads' preparation included: listed
+// 75 -> 73 us; this order, an item's numbers ahead and the gate by rows 73 -> 65 (kernel 47 -> 39).  A causal attention block over 16 of 100 - 1 060: 157 -> 153 -> 150.
 constexpr int kListed = 64;
 struct Walk {
   uint32_t tiles;          // of sequence lane (low half) and lane + 32 (high half); listed: the batch has up to kListed sequences
   int level, at;           // the next item: number `at` of the items from this level on (not listed: of all)
+  int step;                // to the one behind it
   bool listed;
   __device__ __forceinline__ void start(const int32_t* cu, const Sched& sc, int lane) {
     listed = sc.B <= kListed;
     level = sc.QT - 1;
     at = blockIdx.x;
+    step = 2 * (int)(gridDim.x - blockIdx.x) - 1;
     tiles = 0;
     if (listed) {
       if (lane < sc.B) tiles = (uint32_t)(cu[lane + 1] - cu[lane] + 127) >> 7;
@@ -109,7 +113,8 @@ struct Walk {
     if (!listed) {
       if (at >= sc.num_items) return false;
       x = item_of(at, sc);
-      at += gridDim.x;
+      at += step;
+      step = 2 * (int)gridDim.x - step;
       return true;
     }
     for (;; --level) {
@@ -130,7 +135,8 @@ struct Walk {
       x.b = __ffs(__ballot_sync(0xffffffffu, mine)) - 1 + (low ? 0 : 32);
       x.h = at - i * sc.nh.d;
       x.kvh = sc.group.div(x.h);
-      at += gridDim.x;
+      at += step;
+      step = 2 * (int)gridDim.x - step;
       return true;
     }
   }
@@ -175,11 +181,14 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
   // keys 0 .. q0 + i, or the last `window` of them; j0 = the first kv tile, n_tiles are counted from there; n_tiles = 0 marks
   // a q tile past the end of its sequence (skipped by every role)
   struct Geo { int seq_start, seq_len, kv_len, q0, j0, n_tiles; };
-  auto geo_of = [&](const Item& x) {
+  // (an item's numbers are requested one item ahead, and looked at when it begins: computing with them at once made every role wait for them)
+  struct Raw { int start, end, kv; };
+  auto raw_of = [&](const Item& x) { return Raw{__ldg(cu_seqlens + x.b), __ldg(cu_seqlens + x.b + 1), kPaged ? __ldg(pk.context_lens + x.b) : 0}; };
+  auto geo_of = [&](const Item& x, const Raw& raw) {
     Geo g;
-    g.seq_start = __ldg(cu_seqlens + x.b);
-    g.seq_len = __ldg(cu_seqlens + x.b + 1) - g.seq_start;
-    g.kv_len = kPaged ? __ldg(pk.context_lens + x.b) : g.seq_len;
+    g.seq_start = raw.start;
+    g.seq_len = raw.end - raw.start;
+    g.kv_len = kPaged ? raw.kv : g.seq_len;
     g.q0 = g.kv_len - g.seq_len + x.qt * 128;
     g.j0 = kMode != kPlain && pk.window > 0 ? max(g.q0 - pk.window + 1, 0) / kKT : 0;
     g.n_tiles = x.qt * 128 >= g.seq_len ? 0 : (min(g.kv_len, g.q0 + 128) + kKT - 1) / kKT - g.j0;
@@ -275,15 +284,20 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
     Walk walk;
     walk.start(cu_seqlens, sc, lane);
     Item xn;
-    Geo gn;
+    Raw rn;
     bool more = walk.next(xn, sc);
-    if (more) gn = geo_of(xn);
+    if (more) rn = raw_of(xn);
     while (more) {
       const Item x = xn;
-      const Geo ge = gn;
-      more = walk.next(xn, sc);
-      if (more) gn = geo_of(xn);                      // the next item's geometry: its loads fly under this item
-      if (ge.n_tiles == 0) continue;
+      const Geo ge = geo_of(x, rn);
+      auto advance = [&] {                            // the next item's numbers are asked for while this one's work is under way
+        more = walk.next(xn, sc);
+        if (more) rn = raw_of(xn);
+      };
+      if (ge.n_tiles == 0) {
+        advance();
+        continue;
+      }
       // Q: the previous item's last S MMA has read it (first item: the barrier is fresh, the wait falls through)
       ptx::mbar_wait(q_empty, (n_done & 1) ^ 1u);
       if (ptx::elect_one()) {
@@ -292,6 +306,7 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
         ptx::tma_load_3d(base + kOffQ + 16384, &tma_q, q_full, 64, x.h, ge.seq_start + x.qt * 128);
       }
       __syncwarp();
+      advance();
       if constexpr (kSep) {
         load_kv(x, ge, 0, g, false);
         for (int j = 0; j < ge.n_tiles; ++j) {
@@ -336,18 +351,24 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
     Walk walk;
     walk.start(cu_seqlens, sc, lane);
     Item xn;
-    Geo gn;
+    Raw rn;
     bool more = walk.next(xn, sc);
-    if (more) gn = geo_of(xn);
+    if (more) rn = raw_of(xn);
     while (more) {
       const Item x = xn;
-      const Geo ge = gn;
-      more = walk.next(xn, sc);
-      if (more) gn = geo_of(xn);                      // the next item's geometry: its loads fly under this item
-      if (ge.n_tiles == 0) continue;
+      const Geo ge = geo_of(x, rn);
+      auto advance = [&] {                            // the next item's numbers are asked for while this one's work is under way
+        more = walk.next(xn, sc);
+        if (more) rn = raw_of(xn);
+      };
+      if (ge.n_tiles == 0) {
+        advance();
+        continue;
+      }
       const int n = ge.n_tiles;
       ptx::mbar_wait(q_full, n_done & 1);
       issue_s(g, n == 1);
+      advance();
       for (int j = 0; j < n; ++j) {
         // S is double-buffered: S(j+1) is computed while the softmax threads work on S(j)
         if (j + 1 < n) issue_s(g + j + 1, j + 2 == n);
@@ -384,15 +405,20 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
     Walk walk;
     walk.start(cu_seqlens, sc, lane);
     Item xn;
-    Geo gn;
+    Raw rn;
     bool more = walk.next(xn, sc);
-    if (more) gn = geo_of(xn);
+    if (more) rn = raw_of(xn);
     while (more) {
       const Item x = xn;
-      const Geo ge = gn;
-      more = walk.next(xn, sc);
-      if (more) gn = geo_of(xn);                      // the next item's geometry: its loads fly under this item
-      if (ge.n_tiles == 0) continue;
+      const Geo ge = geo_of(x, rn);
+      auto advance = [&] {                            // the next item's numbers are asked for while this one's work is under way
+        more = walk.next(xn, sc);
+        if (more) rn = raw_of(xn);
+      };
+      if (ge.n_tiles == 0) {
+        advance();
+        continue;
+      }
       const int n = ge.n_tiles;
       const float bias = kMode == kSigmoid && pk.bias ? __ldg(pk.bias + x.h) * 1.4426950408889634f : 0.f;
       // rows past the sequence are not stored; their gate row is clamped to the last real one
@@ -554,10 +580,56 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
         ptx::mbar_arrive(p_full(gi));
       }
       // ---- O / l -> bf16 rows of the output
+      advance();
+      const bool gate = (kMode == kSigmoid || kMode == kGated) && pk.gate;
+      const int rows0 = x.qt * 128 + quad * 32, sub = lane >> 3, q4 = lane & 7;
+      float4 z[8];                                     // 32 columns of the gate's rows, 8 lanes per row
+      auto gate_rows = [&](int c) {                    // rows past the sequence are not stored; their gate row is clamped to the last real one
+        const float* gp = pk.gate + (int64_t)ge.seq_start * pk.ldg + x.h * 128 + q4 * 4 + c * 32;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) z[k] = *reinterpret_cast<const float4*>(gp + (int64_t)min(rows0 + 4 * k + sub, ge.seq_len - 1) * pk.ldg);
+      };
+      if (gate) gate_rows(0);
       ptx::mbar_wait(o_full, kMode == kSigmoid ? (n_done & 1) : ((g + n - 1) & 1));
       ptx::tcgen05_fence_after();
       if (kPaged && kMode != kSigmoid && pk.sink) l += exp2f(__ldg(pk.sink + x.h) * 1.4426950408889634f - m);   // the sink: in the denominator, without a value
       const float inv = kMode == kSigmoid ? 1.0f : (kMode == kGated ? pk.out_scale / l : 1.0f / l);
+      if (gate) {
+        // With a gate (fp32 rows): 32 columns of the warp's rows at a time through its staging buffer as fp32, so that 8 lanes per row read the gate and write the
+        // result, 128 and 64 contiguous bytes.  A thread reading its own row's gate touched 32 lines per instruction: 12 000 cycles per item, of 25 000.
+        uint8_t* buf = gen + kOffStage + quad * 4096;
+        nvc_bf16* op = out + (int64_t)ge.seq_start * ldo + x.h * 128 + q4 * 4;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          ptx::tmem_ld_32x32b_x32(tmem_o + lane_addr + c * 32, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<float4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+                make_float4(__uint_as_float(v[4 * i]) * inv, __uint_as_float(v[4 * i + 1]) * inv, __uint_as_float(v[4 * i + 2]) * inv, __uint_as_float(v[4 * i + 3]) * inv);
+          __syncwarp();
+          float4 now[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) now[k] = z[k];
+          if (c < 3) gate_rows(c + 1);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int row = 4 * k + sub;
+            const float4 y = *reinterpret_cast<const float4*>(buf + row * 128 + ((q4 ^ (row & 7)) << 4));
+            auto gated = [](float a, float b) { return a * fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * b)); };
+            if (rows0 + row < ge.seq_len)
+              *reinterpret_cast<uint2*>(op + (int64_t)(rows0 + row) * ldo + c * 32) =
+                  make_uint2(pack_bf16(gated(y.x, now[k].x), gated(y.y, now[k].y)), pack_bf16(gated(y.z, now[k].z), gated(y.w, now[k].w)));
+          }
+          __syncwarp();
+        }
+        ptx::tcgen05_fence_before();
+        ptx::mbar_arrive(o_free);
+        g += n;
+        ++n_done;
+        continue;
+      }
       // this warp's 32 rows x 128 head dims leave through its staging buffer: 8 lanes per row, 128 contiguous bytes each
       RowStage st = make_row_stage(gen + kOffStage + quad * 4096, out, 0, NVC_EPI_NONE, (int64_t)ldo,
                                    ge.seq_start + x.qt * 128 + quad * 32, ge.seq_start + ge.seq_len, x.h * 128, 128, nh * 128);
@@ -569,16 +641,6 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
         float f[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) * inv;
-        if ((kMode == kSigmoid || kMode == kGated) && grow) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float4 z = *reinterpret_cast<const float4*>(grow + c * 32 + i);
-            f[i] *= fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * z.x));
-            f[i + 1] *= fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * z.y));
-            f[i + 2] *= fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * z.z));
-            f[i + 3] *= fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * z.w));
-          }
-        }
         st.emit32(lane, 0, NVC_EPI_NONE, f);
       }
       st.finish(lane);

@@ -90,3 +90,24 @@ def test_preparation_of_heads_in_registers(ctx, ops, dt, H, G, d, vd, rot, half,
     rest = torch.ones(rows, dtype=torch.bool)
     rest[at] = False
     assert (kc.cpu()[rest] == 9).all() and (vc.cpu()[rest] == 9).all()
+
+
+@pytest.mark.parametrize("gate", [False, True])
+@pytest.mark.parametrize("B", [64, 65])                     # up to 64 sequences the q tiles that exist are listed; several items per CTA, every length of a last tile
+def test_ragged_batches_of_many_portions(ctx, ops, B, gate):
+    g = torch.Generator().manual_seed(B)
+    H, G, d, block, window = 8, 2, 128, 64, 200
+    q_lens = [(1 + 37 * i * i) % 450 + (i % 5 == 0) for i in range(B)]
+    N, need = sum(q_lens), [max(1, (n + block - 1) // block) for n in q_lens]
+    pages = torch.randperm(sum(need), generator=g).tolist()
+    tables = [[pages.pop() for _ in range(n)] + [-1] * (max(need) - n) for n in need]
+    q, k, v = (torch.randn(n, w * d, generator=g).bfloat16() for n, w in ((N, H), (sum(need) * block, G), (sum(need) * block, G)))
+    cu = [0]
+    for n in q_lens:
+        cu.append(cu[-1] + n)
+    z = torch.randn(N, H * d, generator=g).to(DEV) if gate else None
+    run = lambda dt: ops.attn_paged_wide(ctx, q.to(DEV, dt), k.to(DEV, dt), v.to(DEV, dt), i32(tables), i32(q_lens), i32(cu), max(q_lens), block, H, G, d, d,  # noqa: E731
+                                         d ** -0.5, window=window, gate=z).float()
+    got, want = run(torch.bfloat16), run(torch.float32)
+    assert torch.isfinite(got).all()
+    assert float((got - want).abs().max()) <= 2e-2 * max(1.0, float(want.abs().max()))
