@@ -420,8 +420,8 @@ __device__ __forceinline__ void argmax_finish_row(float bv, int bi, int r, int r
                                                   float* __restrict__ val, int index_offset) {
   __shared__ float sv[32];
   __shared__ int si[32];
-  __shared__ float cv[4];
-  __shared__ int ci[4];
+  __shared__ float cv[8];
+  __shared__ int ci[8];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -461,12 +461,16 @@ __device__ __forceinline__ void argmax_finish_row(float bv, int bi, int r, int r
   }
 }
 
-// widest cluster (4 / 2 / 1 CTAs per row) that keeps the grid within one resident wave of two 1024-thread CTAs per SM
-static int argmax_cluster_width(const nvc_ctx* ctx, int B, int V) {
+// widest cluster (8 / 4 / 2 / 1 CTAs per row) that keeps the grid within one resident wave of two 1024-thread CTAs per SM.  A GPC of 18 SMs holds four clusters of
+// eight and has four places left: eight of nine places count; and a row has to be long enough (`long_row`) to pay for the wider merge.
+// Rows of 151 936 drawn from, 4 -> 8: 1 row 15.1 -> 9.6 us, 8 15.1 -> 12.5, 32 26.3 -> 17.1; 4 rows of 65 536 8.7 -> 6.7, 32 14.5 -> 10.3.  Greedy over 151 936: 1 row
+// 4.0 -> 3.4, 24 5.9 -> 5.2, 32 6.35 -> 5.3, but 37 (a second wave) 6.5 -> 7.6, and 8 rows of 65 536 3.25 -> 3.5.
+static int argmax_cluster_width(const nvc_ctx* ctx, int B, int V, int long_row) {
+  if (V >= long_row && 9 * B <= 2 * ctx->num_sms) return 8;
   return (V >= 16384 && 4 * B <= 2 * ctx->num_sms) ? 4 : (V >= 16384 && 2 * B <= 2 * ctx->num_sms) ? 2 : 1;
 }
 
-// A row is shared by the `csz` CTAs of a cluster (csz = 1, 2 or 4: at batch 64 one CTA per row would leave 84 SMs idle):
+// A row is shared by the `csz` CTAs of a cluster (csz = 1, 2, 4 or 8: at batch 64 one CTA per row would leave 84 SMs idle):
 // CTA r scans the r-th slice of the row, stores its (value, index) into CTA 0's shared memory over DSMEM, and CTA 0
 // merges after one cluster barrier.  The "last maximal index" rule is order-independent, so the split does not show.
 __global__ void __launch_bounds__(1024)
@@ -502,7 +506,7 @@ extern "C" int nvc_argmax_last(nvc_ctx* ctx, const float* logits, int ld, int32_
   NVC_REQUIRE(ctx, B >= 0 && V > 0 && ld >= V, NVC_EINVAL, "bad sizes");
   NVC_REQUIRE(ctx, ld % 4 == 0, NVC_ESHAPE, "ld must be a multiple of 4");
   if (B == 0) return NVC_OK;
-  const int csz = argmax_cluster_width(ctx, B, V);
+  const int csz = argmax_cluster_width(ctx, B, V, 131072);
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, argmax_last_kernel, dim3(B * csz), dim3(1024), 0, nvc_stream(stream), csz,
                                          logits, ld, idx, val, V, index_offset, csz));
   NVC_CUDA_CHECK(ctx, cudaGetLastError());
@@ -561,17 +565,16 @@ __device__ __forceinline__ bool gumbel_may_reach(float l, float rT, uint32_t bit
 }
 
 __global__ void __launch_bounds__(1024)
-sample_gumbel_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ temperatures,
-                     const uint64_t* __restrict__ streams, uint64_t seed, int32_t* __restrict__ idx,
+sample_gumbel_kernel(const float* __restrict__ logits, int ld, const float* temperatures, const uint64_t* streams, uint64_t seed, int32_t* __restrict__ idx,
                      float* __restrict__ val, int V, int index_offset, int csz, int screen) {
   pdl_trigger();
   pdl_wait();
   __shared__ int s_thr;
   const int b = blockIdx.x / csz, rank = blockIdx.x - b * csz;     // a row is shared by a cluster, as in the argmax
   const float* row = logits + (int64_t)b * ld;
-  const float T = fmaxf(__ldg(temperatures + b), 1e-6f);          // llm_engine.rs:104
+  const float T = fmaxf(temperatures[b], 1e-6f);          // llm_engine.rs:104
   const float rT = 1.0f / T;
-  const uint64_t stream = __ldg(streams + b);
+  const uint64_t stream = streams[b];
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   const uint32_t s_lo = (uint32_t)stream, s_hi = (uint32_t)(stream >> 32);
   float bv = -INFINITY;
@@ -623,7 +626,7 @@ extern "C" int nvc_sample_gumbel(nvc_ctx* ctx, const float* logits, int ld, cons
   NVC_REQUIRE(ctx, ld % 4 == 0 && V % 4 == 0 && index_offset % 4 == 0 && index_offset >= 0, NVC_ESHAPE,
               "ld, V and index_offset must be multiples of 4");
   if (B == 0) return NVC_OK;
-  const int csz = argmax_cluster_width(ctx, B, V);
+  const int csz = argmax_cluster_width(ctx, B, V, 65536);
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, sample_gumbel_kernel, dim3(B * csz), dim3(1024), 0, nvc_stream(stream), csz,
                                          logits, ld, temperatures, streams, seed, idx, val, V, index_offset, csz,
                                          g_nvc_debug[6] == 1 ? 0 : 1));

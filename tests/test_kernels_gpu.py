@@ -216,8 +216,26 @@ def test_argmax_last_index(ctx, B, V):
     assert torch.equal(val.cpu(), logits.max(dim=1).values)
 
 
+@pytest.mark.parametrize("B,V", [(32, 131072), (33, 131072), (3, 163843), (3, 65543), (5, 20480), (4, 6), (4, 3)])
+def test_argmax_widest_clusters_and_what_never_wins(ctx, B, V):
+    """clusters of 8 (up to 32 rows of 131 072 numbers or more) and 4, with and without a ragged end; a NaN never wins, and of a row of -inf the last one does"""
+    g = torch.Generator().manual_seed(V)
+    logits = torch.randn(B, (V + 3) // 4 * 4, generator=g)[:, :V]
+    logits[0] = -float("inf")
+    logits[1, torch.rand(V, generator=g) < 0.5] = float("nan")
+    logits[1, V // 3] = 9.0
+    logits[1, V // 2] = float("inf")
+    logits[2, V // 7] = logits[2, V - 1] = 9.0
+    dev = torch.full((B, (V + 3) // 4 * 4), float("inf"), device="cuda")[:, :V]
+    dev.copy_(logits)
+    idx, val = ctx.argmax_last(dev)
+    clean = torch.where(logits.isnan(), torch.full_like(logits, -float("inf")), logits)
+    assert idx.cpu().tolist() == [int((row == row.max()).nonzero().max()) for row in clean]
+    assert torch.equal(val.cpu(), clean.max(dim=1).values)
+
+
 # ----------------------------------------------------------------------------- K8s sampling
-@pytest.mark.parametrize("B,V,offset", [(5, 2048, 0), (3, 151936, 0), (4, 18992, 37984), (100, 32768, 0), (64, 151936, 0)])
+@pytest.mark.parametrize("B,V,offset", [(5, 2048, 0), (3, 151936, 0), (32, 65536, 4), (4, 18992, 37984), (100, 32768, 0), (64, 151936, 0)])
 def test_sample_gumbel_matches_oracle(ctx, B, V, offset):
     """Device Gumbel-max draw against oracle/sampling_oracle.py (same Philox counters).  The noise
     bits are exact; logf differs from numpy's float64 log by ulps, so the device's token must be
