@@ -17,7 +17,7 @@
 // four steps, and the chunk kernel works with the running sums L_t of each channel: the token-by-token products take
 // exp(L_t - L_j) inside their sums, the keys and queries that meet the state carry exp(L_t), those that enter it exp(L_n - L_j).
 // Both states live in fp32 in pools of state slots; a sequence whose first new token sits at position 0 starts from zeros.
-// All arithmetic is fp32: FMA code, or products of 16-bit parts of numbers (scan_mma.cuh).
+// All arithmetic is fp32: FMA code, or products of three bf16 parts per number (scan_mma.cuh).
 #include <type_traits>
 
 #include "conv_tile.cuh"
@@ -683,11 +683,14 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 3) delta_chunk_kernel(c
 // column with forward substitution in fp32 by the preparing warp that computed the block.  B, U and O never leave a state warp's registers.
 constexpr int kHT = 16;                  // tokens of a half
 constexpr int kHP = kHT + 8;             // row stride of a half's planes
-__host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 4 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 9 * kMT * 4; }
+__host__ __device__ constexpr int delta_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + 3 * kHT * kHP * 6 + kMT * kMV * 4 + 5 * kMT * 4; }
+
+// three chunks under way where 227 KB hold them: up to 64 channels
+__host__ __device__ constexpr int delta_buffers(int ks) { return ks <= 4 ? kBuffers : 2; }
 
 template <int KS>
 __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaArgs a, const int vecv) {
-  constexpr int DZ = 16 * KS, DP = DZ + 8;
+  constexpr int DZ = 16 * KS, DP = DZ + 8, NB = delta_buffers(KS);
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ RankScratch ranks;
   __shared__ float4 swap[4][3][4][32];                    // of a pair: products with the queries, with the keys, U
@@ -704,21 +707,17 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
   if (chunks == 0) return;
   const bool fresh = p.positions[r0] == 0;
   const int slot = p.state_slots[b];
-  struct Buffer { Planes Q, K, P, X0, X1, A10; float *V, *beta, *Lh, *Ll, *from, *fk, *fq, *tk, *dq, *dk; };
+  struct Buffer { Planes Q, K, P, X0, X1, A10; float *V, *beta, *Lh, *Ll, *from, *to; };
   auto buffer = [&](int i) {
-    uint8_t* q = smem + (i % kBuffers) * delta_buf(DZ);
-    uint8_t* x = q + 2 * kMT * DP * 4 + kMT * kMP * 6;
+    uint8_t* q = smem + (i % NB) * delta_buf(DZ);
+    uint8_t* x = q + 2 * kMT * DP * 6 + kMT * kMP * 6;
     float* v = reinterpret_cast<float*>(x + 3 * kHT * kHP * 6);
-    // beta; running sums in two parts; decay from the chunk's start to a token, and the same times the inverse scales of its key and query;
-    // decay from a token to the chunk's end times its key's inverse scale; the inverse scales
-    float* l = v + kMT * kMV;
-    return Buffer{planes(q, kMT, DP), planes(q + kMT * DP * 4, kMT, DP), planes(q + 2 * kMT * DP * 4, kMT, kMP), planes(x, kHT, kHP),
-                  planes(x + kHT * kHP * 6, kHT, kHP), planes(x + 2 * kHT * kHP * 6, kHT, kHP), v, l, l + kMT, l + 2 * kMT,
-                  l + 3 * kMT, l + 4 * kMT, l + 5 * kMT, l + 6 * kMT, l + 7 * kMT, l + 8 * kMT};
+    float* l = v + kMT * kMV;               // beta; running sums in two parts; decay from the chunk's start to a token, from a token to its end
+    return Buffer{planes(q, kMT, DP), planes(q + kMT * DP * 6, kMT, DP), planes(q + 2 * kMT * DP * 6, kMT, kMP), planes(x, kHT, kHP),
+                  planes(x + kHT * kHP * 6, kHT, kHP), planes(x + 2 * kHT * kHP * 6, kHT, kHP), v, l, l + kMT, l + 2 * kMT, l + 3 * kMT, l + 4 * kMT};
   };
   if (w >= kPrep0) {
     // ------------------------------------------------ preparing warps
-    registers_give<kPrepRegs>();
     const int pw = w & 3, group = (w - kPrep0) >> 2;
     RowTile<DZ> x;                            // queries, then keys
     RowTile<kMC> v;
@@ -736,30 +735,24 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
     if (group < chunks) fetch(group);
     for (int i = group; i < chunks; i += 2) {
       const Buffer bf = buffer(i);
-      if (i >= kBuffers) bar_sync(kEmpty + i % (2 * kBuffers), kBufThreads);
-      x.split_to(bf.Q, bf.dq, pw, lane);
+      if (i >= NB) bar_sync(kEmpty + i % (2 * NB), kBufThreads);
+      x.split_to(bf.Q, pw, lane);
       {
         const int64_t row = r0 + i * kMT;
         x.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, r1 - (int)row, a.vec, pw, lane);
       }
       v.store_to(bf.V, kMV, pw, lane);
-      float from = 0.f, to = 0.f;
       if (pw == 3) {
         const LogSum sum(gb.x, lane);
         const float hi = (float)sum.l;
         bf.Lh[lane] = hi;
         bf.Ll[lane] = (float)(sum.l - (double)hi);
-        bf.from[lane] = from = sum.from();
-        to = sum.to();
+        bf.from[lane] = sum.from();
+        bf.to[lane] = sum.to();
         bf.beta[lane] = gb.y;
       }
-      x.split_to(bf.K, bf.dk, pw, lane);
+      x.split_to(bf.K, pw, lane);
       bar_sync(kPrepare + group, 128);
-      if (pw == 3) {
-        bf.fk[lane] = from * bf.dk[lane];
-        bf.fq[lane] = from * bf.dq[lane];
-        bf.tk[lane] = to * bf.dk[lane];
-      }
       // warps 0 and 1: the diagonal blocks of A and their inverses; 2: P (16, 0) and A_10; 3: P (0, 0) and P (16, 16)
 #pragma unroll 1
       for (int part = 0; part < (pw < 2 ? 1 : 2); ++part) {
@@ -770,15 +763,13 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
         {
           Decays f;
           f.load(bf.Lh, bf.Ll, t0, j0, lane);
-          Down d;
-          d.load(isa ? bf.dk : bf.dq, bf.dk, t0, j0, lane);
           const float be[2] = {isa ? bf.beta[t0 + g] : 1.f, isa ? bf.beta[t0 + g + 8] : 1.f};
 #pragma unroll
           for (int y = 0; y < 2; ++y)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int t = t0 + g + 4 * (e & 2), j = j0 + 8 * y + 2 * tq + (e & 1);
-              z[y][e] = j < t + !isa ? be[e >> 1] * (f(y, e) * d(y, e, z[y][e])) : 0.f;
+              z[y][e] = j < t + !isa ? be[e >> 1] * (f(y, e) * z[y][e]) : 0.f;
             }
         }
         if (pw >= 2) {
@@ -819,13 +810,12 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
         }
       }
       if (i == 0) advance_conv_state(p, r0, r1, fresh, slot, blockIdx.x, gridDim.x, threadIdx.x - 32 * kPrep0, 128);      // nothing here reads that state
-      bar_arrive(kFull + i % kBuffers, kBufThreads);
+      bar_arrive(kFull + i % NB, kBufThreads);
       if (i + 2 < chunks) fetch(i + 2);
     }
     return;
   }
   // -------------------------------------------------- state warps
-  registers_take<kStateRegs>();
   constexpr int KH = KS / 2;                  // blocks of 16 channels of a half
   const int pair = w & 3, half = w >> 2, c = pair * 16 + g, d0 = half * (DZ / 2);
   float* sp = a.state + (((int64_t)slot * p.heads + h) * dim + d0) * p.vdim + v0;
@@ -848,16 +838,15 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
     const Buffer bf = buffer(i);
     const int64_t row = r0 + i * kMT;
     const int n = min(kMT, r1 - (int)row);
-    const ColumnScale sc = column_scale(S);
-    bar_sync(kFull + i % kBuffers, kBufThreads);
+    bar_sync(kFull + i % NB, kBufThreads);
     float u[4][4] = {}, o[4][4] = {};         // products with the keys, then right sides, then U; with the queries, then outputs
     {
       float us[4][4] = {}, os[4][4] = {};
 #pragma unroll
       for (int ks = 0; ks < KH; ++ks) {
-        HalfA s;
-        HalfB x[4];
-        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1], sc.c0.up, sc.c1.up);
+        FragA s;
+        FragB x[4];
+        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1]);
         load_b(x, bf.K, 0, d0 + 16 * ks, lane);
         mma_high(u, s, x);
         mma_small(us, s, x);
@@ -869,8 +858,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
       for (int t = 0; t < 4; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          u[t][e] = (u[t][e] + us[t][e]) * sc.down(e);
-          o[t][e] = (o[t][e] + os[t][e]) * sc.down(e);
+          u[t][e] += us[t][e];
+          o[t][e] += os[t][e];
         }
     }
     // the left warp of a pair solves for U, the right one takes the outputs
@@ -883,7 +872,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int tt = 8 * t + 2 * tq + (e & 1);
-          u[t][e] = bf.beta[tt] * (bf.V[tt * kMV + c + 4 * (e & 2)] - bf.fk[tt] * u[t][e]);
+          u[t][e] = bf.beta[tt] * (bf.V[tt * kMV + c + 4 * (e & 2)] - bf.from[tt] * u[t][e]);
         }
       FragA f;
       auto solve = [&](float (&x)[2][4], const Planes& X) {     // x <- x X^T
@@ -913,7 +902,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
       for (int t = 0; t < 4; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          o[t][e] *= bf.fq[8 * t + 2 * tq + (e & 1)];
+          o[t][e] *= bf.from[8 * t + 2 * tq + (e & 1)];
           u[t][e] = 0.f;
         }
       bar_sync(kPair + pair, 64);
@@ -928,9 +917,9 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) u[t][e] *= bf.tk[8 * t + 2 * tq + (e & 1)];
+      for (int e = 0; e < 4; ++e) u[t][e] *= bf.to[8 * t + 2 * tq + (e & 1)];
     state_update<KH>(S, bf.from[kMT - 1], u, bf.K, d0, lane);
-    if (i + kBuffers < chunks) bar_arrive(kEmpty + (i + kBuffers) % (2 * kBuffers), kBufThreads);
+    if (i + NB < chunks) bar_arrive(kEmpty + (i + NB) % (2 * NB), kBufThreads);
     if (half == 1) {
       float* op = a.o + (row + 2 * tq) * a.ldo + h * p.vdim + v0 + c;
 #pragma unroll
@@ -948,7 +937,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
 template <int KS>
 cudaError_t launch_delta_mma(nvc_ctx* ctx, const DeltaArgs& a, cudaStream_t st) {
   const nvc_delta_prep& p = a.p;
-  constexpr int smem = kBuffers * delta_buf(16 * KS);
+  constexpr int smem = delta_buffers(KS) * delta_buf(16 * KS);
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(delta_mma_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -17,7 +17,7 @@
 //                              S      <- decay^n S + sum_j decay^(n - 1 - j) k_j v_j^T n: tokens of the chunk
 //                            Powers of the decay come from a table built by repeated multiplication (exact for 0 and 1).
 //   decay_mma_kernel         the same chunks of 32 tokens on the tensor pipe, without the normaliser of the gated memory: up to 128 channels
-// All arithmetic is fp32 (FMA code, or products of 16-bit parts of numbers: scan_mma.cuh); they differ by rounding only.
+// All arithmetic is fp32 (FMA code, or products of three bf16 parts per number: scan_mma.cuh); they differ by rounding only.
 //
 // nvc_decay_scan is the same pair of kernels with what other linear recurrences of this shape need (kVar):
 //   a decay per token and head, given as its logarithm: S_t = exp(l_t) S_(t-1) + k_t v_t^T.  Inside a chunk only differences of the
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(NW * 32, 2) retention_chunk_kernel(const RetAr
 // ---- kFixed and kVar with keys of up to 128 numbers: the same chunks of 32 tokens with every product on the tensor pipe (scan_mma.cuh says how the
 // warps share the work).  With (.)^T for a state warp's 16 value columns,
 //   O^T = exp(L_t) S^T Q^T + V^T A^T,    S^T <- exp(L_n) S^T + (w_j v_j)^T K.
-__host__ __device__ constexpr int decay_buf(int dz) { return 2 * kMT * (dz + 8) * 4 + kMT * kMP * 6 + kMT * kMV * 4 + 7 * kMT * 4; }      // bytes of a chunk's buffer
+__host__ __device__ constexpr int decay_buf(int dz) { return 2 * kMT * (dz + 8) * 6 + kMT * kMP * 6 + kMT * kMV * 4 + 4 * kMT * 4; }      // bytes of a chunk's buffer
 
 template <int KS, int MODE>
 __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArgs a, const int B, const int vec, const int vecv) {
@@ -477,18 +477,15 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
   const int r0 = a.cu_seqlens[b], r1 = a.cu_seqlens[b + 1], chunks = (r1 - r0 + kMT - 1) / kMT;
   if (chunks == 0) return;
   __syncthreads();                            // gp
-  struct Buffer { Planes Q, K, A; float *V, *keep, *kq, *wk, *Lh, *Ll, *dq, *dk; };
-  auto buffer = [&](int i) {                  // planes, values, decay of the state up to token t, the same times its query's inverse scale, weight of token j
-                                              // behind the chunk times its key's inverse scale, running sums in two parts, inverse scales
+  struct Buffer { Planes Q, K, A; float *V, *keep, *wj, *Lh, *Ll; };
+  auto buffer = [&](int i) {                  // planes, values, decay of the state up to token t, weight of token j behind the chunk, running sums in two parts
     uint8_t* p = smem + (i % kBuffers) * decay_buf(DZ);
-    float* v = reinterpret_cast<float*>(p + 2 * kMT * DP * 4 + kMT * kMP * 6);
+    float* v = reinterpret_cast<float*>(p + 2 * kMT * DP * 6 + kMT * kMP * 6);
     float* k = v + kMT * kMV;
-    return Buffer{planes(p, kMT, DP), planes(p + kMT * DP * 4, kMT, DP), planes(p + 2 * kMT * DP * 4, kMT, kMP), v, k, k + kMT, k + 2 * kMT, k + 3 * kMT,
-                  k + 4 * kMT, k + 5 * kMT, k + 6 * kMT};
+    return Buffer{planes(p, kMT, DP), planes(p + kMT * DP * 6, kMT, DP), planes(p + 2 * kMT * DP * 6, kMT, kMP), v, k, k + kMT, k + 2 * kMT, k + 3 * kMT};
   };
   if (w >= kPrep0) {
     // ------------------------------------------------ preparing warps
-    registers_give<kPrepRegs>();
     const int pw = w & 3, group = (w - kPrep0) >> 2;
     RowTile<DZ> x;                            // queries, then keys
     RowTile<kMC> v;
@@ -505,49 +502,42 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
       const Buffer bf = buffer(i);
       const int n = min(kMT, r1 - r0 - i * kMT);
       if (i >= kBuffers) bar_sync(kEmpty + i % (2 * kBuffers), kBufThreads);
-      x.split_to(bf.Q, bf.dq, pw, lane);
+      x.split_to(bf.Q, pw, lane);
       {
         const int64_t row = r0 + i * kMT;
         x.load(a.k + row * a.ldk + hq * dim, a.ldk, dim, n, vec, pw, lane);
       }
       v.store_to(bf.V, kMV, pw, lane);
-      float keep = 0.f, wj = 0.f;
       if (pw == 3) {
         if (VAR) {
           const LogSum sum(l, lane);
           const float hi = (float)sum.l;
           bf.Lh[lane] = hi;
           bf.Ll[lane] = (float)(sum.l - (double)hi);
-          keep = sum.from();
-          wj = sum.to();
+          bf.keep[lane] = sum.from();
+          bf.wj[lane] = sum.to();
         } else {
-          keep = gp[min(lane, n - 1) + 1];
-          wj = lane < n ? gp[n - 1 - lane] : 0.f;
+          bf.keep[lane] = gp[min(lane, n - 1) + 1];
+          bf.wj[lane] = lane < n ? gp[n - 1 - lane] : 0.f;
         }
-        bf.keep[lane] = keep;
       }
-      x.split_to(bf.K, bf.dk, pw, lane);
+      x.split_to(bf.K, pw, lane);
       bar_sync(kPrepare + group, 128);
       if (pw < 3) {                           // A[t][j]: the blocks (0, 0), (16, 0), (16, 16)
         const int t0 = pw ? 16 : 0, j0 = pw == 2 ? 16 : 0;
         float z[2][4];
+        token_products<KS>(z, bf.Q, t0, bf.K, j0, lane);
         Decays f;
         if (VAR) f.load(bf.Lh, bf.Ll, t0, j0, lane);
-        Down d;
-        d.load(bf.dq, bf.dk, t0, j0, lane);
-        token_products<KS>(z, bf.Q, t0, bf.K, j0, lane);
 #pragma unroll
         for (int y = 0; y < 2; ++y)
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
             const int t = t0 + g + 4 * e, j = j0 + 8 * y + 2 * tq;
-            const float y0 = j <= t ? (VAR ? f(y, e) : gp[t - j]) * d(y, e, z[y][e]) : 0.f;
-            const float y1 = j + 1 <= t ? (VAR ? f(y, e + 1) : gp[t - j - 1]) * d(y, e + 1, z[y][e + 1]) : 0.f;
+            const float y0 = j <= t ? (VAR ? f(y, e) : gp[t - j]) * z[y][e] : 0.f;
+            const float y1 = j + 1 <= t ? (VAR ? f(y, e + 1) : gp[t - j - 1]) * z[y][e + 1] : 0.f;
             store_pair(bf.A, t, j, y0, y1);
           }
-      } else {
-        bf.kq[lane] = keep * bf.dq[lane];
-        bf.wk[lane] = wj * bf.dk[lane];
       }
       bar_arrive(kFull + i % kBuffers, kBufThreads);
       if (i + 2 < chunks) fetch(i + 2);
@@ -555,7 +545,6 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
     return;
   }
   // -------------------------------------------------- state warps
-  registers_take<kStateRegs>();
   constexpr int KH = KS / 2;                  // blocks of 16 channels of a half
   const int pair = w & 3, half = w >> 2, c = pair * 16 + g, d0 = half * (DZ / 2);
   const float sw = a.skip ? __ldg(a.skip_w + h) : 0.f;
@@ -566,18 +555,6 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
     const Buffer bf = buffer(i);
     const int64_t row = r0 + i * kMT + kMT / 2 * half + 2 * tq;        // a warp of a pair takes the outputs of one half of the tokens
     const int n = r1 - (int)row;
-    float xs[2][4];                           // the skip term
-    if (a.skip) {
-      const float* xp = a.skip + row * a.lds + h * a.vdim + v0 + c;
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int tt = 8 * t + (e & 1), cc = 4 * (e & 2);
-          xs[t][e] = (tt < n && c + cc < cols) ? xp[(int64_t)tt * a.lds + cc] : 0.f;
-        }
-    }
-    const ColumnScale sc = column_scale(S);
     bar_sync(kFull + i % kBuffers, kBufThreads);
     // ---- the state's share of the outputs
     float o[2][4];
@@ -585,9 +562,9 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
       float x[4][4] = {}, y[4][4] = {}, rest[4][4] = {};       // large products in sums of 32 terms
 #pragma unroll
       for (int ks = 0; ks < KH; ++ks) {
-        HalfA s;
-        HalfB f[4];
-        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1], sc.c0.up, sc.c1.up);
+        FragA s;
+        FragB f[4];
+        frag_of_tiles(s, S[2 * ks], S[2 * ks + 1]);
         load_b(f, bf.Q, 0, d0 + 16 * ks, lane);
         if (ks & 1) mma_high(y, s, f);
         else mma_high(x, s, f);
@@ -596,7 +573,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
 #pragma unroll
       for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[t][e] = ((x[t][e] + y[t][e]) + rest[t][e]) * sc.down(e);
+        for (int e = 0; e < 4; ++e) x[t][e] = (x[t][e] + y[t][e]) + rest[t][e];
       float4(*const mine)[32] = swap[pair][i & 1][half], (*const other)[32] = swap[pair][i & 1][half ^ 1];
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
@@ -610,8 +587,19 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
         const float4 y = mine[t][lane];
         o[t][0] += y.x; o[t][1] += y.y; o[t][2] += y.z; o[t][3] += y.w;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[t][e] *= bf.kq[kMT / 2 * half + 8 * t + 2 * tq + (e & 1)];
+        for (int e = 0; e < 4; ++e) o[t][e] *= bf.keep[kMT / 2 * half + 8 * t + 2 * tq + (e & 1)];
       }
+    }
+    float xs[2][4];                           // the skip term
+    if (a.skip) {
+      const float* xp = a.skip + row * a.lds + h * a.vdim + v0 + c;
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int tt = 8 * t + (e & 1), cc = 4 * (e & 2);
+          xs[t][e] = (tt < n && c + cc < cols) ? xp[(int64_t)tt * a.lds + cc] : 0.f;
+        }
     }
     // ---- the chunk's own share; tokens 0 .. 15 see nothing of 16 .. 31
     float u[4][4];
@@ -622,7 +610,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
       for (int e = 0; e < 8; ++e) {
         const int t = 16 * s + 2 * tq + (e & 1) + 2 * (e & 4);
         v[e >> 2][e & 3] = bf.V[t * kMV + c + 4 * (e & 2)];
-        u[2 * s + (e >> 2)][e & 3] = v[e >> 2][e & 3] * bf.wk[t];
+        u[2 * s + (e >> 2)][e & 3] = v[e >> 2][e & 3] * bf.wj[t];
       }
       if (s <= half) {
         FragA f;
@@ -683,7 +671,7 @@ int run_scan(nvc_ctx* ctx, const RetArgs& a, int B, int max_qlen, void* stream) 
     // wide slices while they fill the GPU; keys of more than 256 numbers leave room for 32 columns only
     cudaError_t ce;
     // the tensor pipe keeps 16 columns x all channels of the state in a warp's registers, which is what ends it at 128 channels; at 128 x 64
-    // over eight prompts of 245 to 1 050 tokens, 32 heads: 120 us, the FMA form 640
+    // over eight prompts of 245 to 1 050 tokens, 32 heads: 146 us, the FMA form 640
     if constexpr (MODE != kMemory) {
       // portions of up to 16 tokens over states that do not fit in L2: the FMA kernel's slices of 128 columns read them better (256 portions of 10 tokens, 16 heads of
       // 128 x 128, 1 GB of states: 581 us, here 642; 64 portions: 161, here 121; heads of 64 x 64: 282, here 258)

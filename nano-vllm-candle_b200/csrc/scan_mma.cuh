@@ -1,25 +1,21 @@
-// Products of fp32 numbers on the tensor pipe for the chunked recurrences (retention.cu, delta_rule.cu): mma.sync m16n8k16, exact products of 16-bit
-// parts, fp32 sums.  Two ways to take a number apart:
-//   fp16, two parts    for the long contractions.  A row (a token's query or key, a state's column) is scaled by a power of two so that its largest number
-//                      lies in 2^13 .. 2^14; the two parts then keep 22 bits and a sign of every number down to 2^-15 of that one, and 2^-39 of it below.
-//                      Three products (four, and a third part of one side, where the state is updated).
-//   bf16, three parts  (8 + 8 + 8 bits, no scale) for what is solved and summed inside a chunk: six products, those left out are below 2^-24 of
-//                      the whole.
+// Products of fp32 numbers on the tensor pipe for the chunked recurrences (retention.cu, delta_rule.cu).
+//
+// An fp32 number is the exact sum of three bf16 numbers (8 + 8 + 8 bits: high, middle, low), and a product of two numbers is the sum of nine
+// products of parts.  The six largest are taken (mma.sync m16n8k16, exact products, fp32 sums); the three that are left out are below
+// 2^-24 of the whole.  That holds for every number by itself, whatever its neighbours are.  (Two fp16 parts under one scale per row or state column, three
+// products: 177 us for the delta rule where this takes 222, but 22 bits of the row's largest number for all of them: a channel 2^11 below its
+// neighbours came out with errors of 5e-6 to 5e-5, one 2^20 below with none of its digits.)
 // The pipe's own sums round towards zero, relative to the sum: the large products, which make that sum, are added up in short chains of their own (16 - 64 terms)
-// that ordinary fp32 adds take over, the small ones apart from them (the observation and the remedy are Ootomo and Yokota's, "Recovering single precision
-// accuracy from Tensor Cores", 2022).  Three bf16 parts everywhere, with chains of 64: outputs of the delta rule over 128 channels off by 1.4 - 1.7e-7, its
-// state behind eight prompts by 1.56e-7; this: 1.4e-7 and 1.52e-7.  Half the products, two thirds of the shared memory.
+// that ordinary fp32 adds take over, the small ones apart from them, or in front of them (the observation and the remedy are Ootomo and Yokota's, "Recovering
+// single precision accuracy from Tensor Cores", 2022).  Against 64 bits, relative, over eight prompts of 245 to 1 050 tokens: delta rule of 16 heads of
+// 128 x 128, outputs 1.1e-7, state 0.97e-7; 32 heads of 128 x 64 with a decay per token, 0.91e-7 and 0.63e-7.
 #pragma once
 #include "scan_common.cuh"
 
 namespace {
 
-template <int P> struct PartsA { uint32_t r[P][4]; };      // a 16 x 16 operand in its parts
-template <int P> struct PartsB { uint32_t r[P][2]; };      // a 16 x 8 operand
-using FragA = PartsA<3>;      // bf16
-using FragB = PartsB<3>;
-using HalfA = PartsA<2>;      // fp16, scaled
-using HalfB = PartsB<2>;
+struct FragA { uint32_t r[3][4]; };        // a 16 x 16 operand in its three parts
+struct FragB { uint32_t r[3][2]; };        // a 16 x 8 operand
 
 // the three parts of two numbers, two bf16 to a register
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& low) {
@@ -31,51 +27,12 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint3
   y -= __uint_as_float(mid & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(low) : "f"(y), "f"(x));
 }
-// the two fp16 parts of two scaled numbers
-__device__ __forceinline__ void split_half(float x, float y, uint32_t& hi, uint32_t& low) {
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y), "f"(x));
-  float fx, fy;
-  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(fx), "=f"(fy) : "r"(hi));
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(low) : "f"(y - fy), "f"(x - fx));
-}
-// what two parts leave of two scaled numbers: the third ones
-__device__ __forceinline__ uint32_t split_rest(float x, float y, uint32_t hi, uint32_t low) {
-  float hx, hy, lx, ly;
-  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(hx), "=f"(hy) : "r"(hi));
-  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(lx), "=f"(ly) : "r"(low));
-  uint32_t r;
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"((y - hy) - ly), "f"((x - hx) - lx));
-  return r;
-}
-// The power of two that takes a row whose largest absolute value is m to 2^13 .. 2^14, and its inverse.  Exact for every row above 2^-112 (below it the
-// scale stays, and an infinity or a NaN goes through as it is).
-struct Pow2 {
-  float up, down;
-  __device__ __forceinline__ explicit Pow2(uint32_t bits_of_m) {
-    const uint32_t e = max(bits_of_m >> 23, 14u);
-    up = __uint_as_float((267u - e) << 23);
-    down = __uint_as_float((e - 13u) << 23);
-  }
-};
-__device__ __forceinline__ float abs_max(float m, float x) { return fmaxf(m, fabsf(x)); }
 // two neighbouring 16 x 8 accumulator tiles as the left operand of the next product (the register layouts agree)
 __device__ __forceinline__ void frag_of_tiles(FragA& a, const float (&t0)[4], const float (&t1)[4]) {
   split_pair(t0[0], t0[1], a.r[0][0], a.r[1][0], a.r[2][0]);
   split_pair(t0[2], t0[3], a.r[0][1], a.r[1][1], a.r[2][1]);
   split_pair(t1[0], t1[1], a.r[0][2], a.r[1][2], a.r[2][2]);
   split_pair(t1[2], t1[3], a.r[0][3], a.r[1][3], a.r[2][3]);
-}
-// the same scaled, rows g by up0 and rows g + 8 by up1
-__device__ __forceinline__ void frag_of_tiles(HalfA& a, const float (&t0)[4], const float (&t1)[4], float up0, float up1) {
-  split_half(t0[0] * up0, t0[1] * up0, a.r[0][0], a.r[1][0]);
-  split_half(t0[2] * up1, t0[3] * up1, a.r[0][1], a.r[1][1]);
-  split_half(t1[0] * up0, t1[1] * up0, a.r[0][2], a.r[1][2]);
-  split_half(t1[2] * up1, t1[3] * up1, a.r[0][3], a.r[1][3]);
-}
-__device__ __forceinline__ void mma_f16_acc(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 __device__ __forceinline__ void mma_bf16_acc(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -97,24 +54,6 @@ __device__ __forceinline__ void mma_high(float (&acc)[NT][4], const FragA& a, co
 #pragma unroll
   for (int t = 0; t < NT; ++t) mma_bf16_acc(acc[t], a.r[0], b[t].r[0]);
 }
-template <int NT>
-__device__ __forceinline__ void mma_least(float (&acc)[NT][4], const HalfA& a, const HalfB (&b)[NT]) {
-#pragma unroll
-  for (int t = 0; t < NT; ++t) mma_f16_acc(acc[t], a.r[1], b[t].r[1]);
-}
-template <int NT>
-__device__ __forceinline__ void mma_small(float (&acc)[NT][4], const HalfA& a, const HalfB (&b)[NT]) {
-#pragma unroll
-  for (int t = 0; t < NT; ++t) mma_f16_acc(acc[t], a.r[1], b[t].r[0]);
-#pragma unroll
-  for (int t = 0; t < NT; ++t) mma_f16_acc(acc[t], a.r[0], b[t].r[1]);
-}
-template <int NT>
-__device__ __forceinline__ void mma_high(float (&acc)[NT][4], const HalfA& a, const HalfB (&b)[NT]) {
-#pragma unroll
-  for (int t = 0; t < NT; ++t) mma_f16_acc(acc[t], a.r[0], b[t].r[0]);
-}
-
 __device__ __forceinline__ void ldsm4(uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w, uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr));
 }
@@ -134,34 +73,31 @@ __device__ __forceinline__ Planes planes(const void* p, int rows, int ld) {
   return Planes{(uint32_t)__cvta_generic_to_shared(p), ld, rows * ld * 2};
 }
 // rows r0 .. r0 + 15, columns c0 .. c0 + 15 as the left operand
-template <int P>
-__device__ __forceinline__ void load_a(PartsA<P>& a, const Planes& m, int r0, int c0, int lane) {
+__device__ __forceinline__ void load_a(FragA& a, const Planes& m, int r0, int c0, int lane) {
   const uint32_t p = m.at(r0 + (lane & 15), c0 + (lane >> 4) * 8);
 #pragma unroll
-  for (int i = 0; i < P; ++i) ldsm4(a.r[i][0], a.r[i][1], a.r[i][2], a.r[i][3], p + i * m.plane);
+  for (int i = 0; i < 3; ++i) ldsm4(a.r[i][0], a.r[i][1], a.r[i][2], a.r[i][3], p + i * m.plane);
 }
 // the matrix holds the right operand's columns as rows: rows n0 .. n0 + 15 (two operands of eight columns), columns k0 .. k0 + 15
-template <int P>
-__device__ __forceinline__ void load_b2(PartsB<P>& x, PartsB<P>& y, const Planes& m, int n0, int k0, int lane) {
+__device__ __forceinline__ void load_b2(FragB& x, FragB& y, const Planes& m, int n0, int k0, int lane) {
   const uint32_t p = m.at(n0 + (lane & 7) + ((lane >> 4) << 3), k0 + ((lane >> 3) & 1) * 8);
 #pragma unroll
-  for (int i = 0; i < P; ++i) ldsm4(x.r[i][0], x.r[i][1], y.r[i][0], y.r[i][1], p + i * m.plane);
+  for (int i = 0; i < 3; ++i) ldsm4(x.r[i][0], x.r[i][1], y.r[i][0], y.r[i][1], p + i * m.plane);
 }
 // the matrix holds the right operand as it is: rows k0 .. k0 + 15, columns n0 .. n0 + 15
-template <int P>
-__device__ __forceinline__ void load_b2_t(PartsB<P>& x, PartsB<P>& y, const Planes& m, int k0, int n0, int lane) {
+__device__ __forceinline__ void load_b2_t(FragB& x, FragB& y, const Planes& m, int k0, int n0, int lane) {
   const uint32_t p = m.at(k0 + (lane & 7) + ((lane >> 3) & 1) * 8, n0 + (lane >> 4) * 8);
 #pragma unroll
-  for (int i = 0; i < P; ++i) ldsm4_t(x.r[i][0], x.r[i][1], y.r[i][0], y.r[i][1], p + i * m.plane);
+  for (int i = 0; i < 3; ++i) ldsm4_t(x.r[i][0], x.r[i][1], y.r[i][0], y.r[i][1], p + i * m.plane);
 }
 // NT operands of eight columns side by side (NT even)
-template <int NT, int P>
-__device__ __forceinline__ void load_b(PartsB<P> (&x)[NT], const Planes& m, int n0, int k0, int lane) {
+template <int NT>
+__device__ __forceinline__ void load_b(FragB (&x)[NT], const Planes& m, int n0, int k0, int lane) {
 #pragma unroll
   for (int t = 0; t < NT; t += 2) load_b2(x[t], x[t + 1], m, n0 + 8 * t, k0, lane);
 }
-template <int NT, int P>
-__device__ __forceinline__ void load_b_t(PartsB<P> (&x)[NT], const Planes& m, int k0, int n0, int lane) {
+template <int NT>
+__device__ __forceinline__ void load_b_t(FragB (&x)[NT], const Planes& m, int k0, int n0, int lane) {
 #pragma unroll
   for (int t = 0; t < NT; t += 2) load_b2_t(x[t], x[t + 1], m, k0, n0 + 8 * t, lane);
 }
@@ -172,13 +108,13 @@ __device__ __forceinline__ void store_pair(const Planes& m, int r, int c, float 
 #pragma unroll
   for (int i = 0; i < 3; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(m.at(r, c) + i * m.plane), "r"(v[i]));
 }
-// four neighbouring numbers (c a multiple of 4), scaled, into two planes of fp16 parts
-__device__ __forceinline__ void store_quad(const Planes& m, int r, int c, const float4& x, float up) {
-  uint32_t u[2], v[2];
-  split_half(x.x * up, x.y * up, u[0], u[1]);
-  split_half(x.z * up, x.w * up, v[0], v[1]);
+// four neighbouring numbers (c a multiple of 4)
+__device__ __forceinline__ void store_quad(const Planes& m, int r, int c, const float4& x) {
+  uint32_t u[3], v[3];
+  split_pair(x.x, x.y, u[0], u[1], u[2]);
+  split_pair(x.z, x.w, v[0], v[1], v[2]);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(m.at(r, c) + i * m.plane), "r"(u[i]), "r"(v[i]));
+  for (int i = 0; i < 3; ++i) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(m.at(r, c) + i * m.plane), "r"(u[i]), "r"(v[i]));
 }
 constexpr int kMT = 32;                 // tokens per chunk
 constexpr int kMC = 64;                 // value columns per CTA: 16 for each of its four state warps
@@ -188,29 +124,25 @@ constexpr int kMP = kMT + 8;            // row stride of the token-by-token plan
 constexpr int kBuffers = 3, kScanThreads = 512, kPrep0 = 8;       // threads, first preparing warp
 
 // What the chunked recurrences on the tensor pipe have in common.  One CTA of sixteen warps per (sequence, head, 64 value columns), one CTA per SM:
-//   warps 8 .. 15 prepare the chunks of 32 tokens, in two groups that take every other chunk: rows from global memory into planes of fp16 parts in
+//   warps 8 .. 15 prepare the chunks of 32 tokens, in two groups that take every other chunk: rows from global memory into planes of bf16 parts in
 //                 shared memory, decays, the token-by-token products
 //   warps 0 .. 7  carry the state, 16 value columns of one half of the channels each.  It is kept TRANSPOSED in the warp's accumulator registers
 //                 (16 columns x 64 channels: 32 numbers per thread at 128 channels), where it is at once the left operand of its products
 //                 with the chunk's rows and the accumulator of its own update: it never travels.  The two warps of a pair (w, w + 4) add what their halves
 //                 of the channels give to the chunk's rows by way of shared memory.
-// The chain of a sequence's chunks is what takes the time, and its length is a warp's instructions times the four to five cycles that each of them
-// waits: a chunk of the delta rule takes 8 300 cycles, of which the state warps alone would take 6 300 and the preparing ones 4 700.  Eight warps (four and
-// four, bf16 parts) took 12 600.  Over eight prompts of 245 to 1 050 tokens: delta rule, 16 heads of 128 x 128, 238 -> 180 us; 32 heads of 128 x 64, a decay
-// per token, 160 -> 120.
-// Named barriers: a buffer is filled / free for its next chunk; a group of preparing warps; a pair.  (Chunks i and i + 3 share a buffer but not the group
-// that fills it, so each group waits for a free buffer at barriers of its own: chunk i at kEmpty + i % 6.)
+// The tensor pipe is what takes the time: 51 - 54 % of all cycles in the mean over the SMs, with some 700 products per SM quarter and chunk, and the warps that
+// wait for it or for one another are the rest.  Over eight prompts of 245 to 1 050 tokens, against four and four warps: delta rule, 16 heads of 128 x 128,
+// 240 -> 222 us; 32 heads of 128 x 64, a decay per token, 154 -> 146.  Not kept: the pair's sums exchanged behind the state's update instead of in front
+// of it (146 -> 150), both warps of a pair solving for the chunk's U instead of one that hands it on (222 -> 232), two buffers instead of three (no change).
+// 128 registers per thread: at 128 channels a few numbers are spilled (8 - 56 bytes loaded per thread); moving registers from the preparing warps to the
+// state's (144 and 112: 277 -> 281 us for the delta rule with its preparation) only moves the spills there.
+// Named barriers: a buffer is filled / free for its next chunk; a group of preparing warps; a pair.  (Of three buffers, chunks i and i + 3 share one but not
+// the group that fills it, so each group waits for a free buffer at barriers of its own: chunk i at kEmpty + i % 6; of two, at kEmpty + i % 4.)
 enum { kFull = 1, kEmpty = kFull + kBuffers, kPrepare = kEmpty + 2 * kBuffers, kPair = kPrepare + 2 };
 static_assert(kPair + 4 <= 16, "barriers");
 constexpr int kBufThreads = 384;        // the state warps and one group
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-
-// Registers move from the preparing warps to the state's: 256 x 144 + 256 x 112 of the 512 x 128 that the block is launched with.
-constexpr int kStateRegs = 144, kPrepRegs = 112;
-static_assert(256 * kStateRegs + 256 * kPrepRegs <= 128 * kScanThreads, "more registers than the block is launched with");
-template <int N> __device__ __forceinline__ void registers_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void registers_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // four neighbouring numbers of a row of `dim` (zeros behind it, or everywhere)
 __device__ __forceinline__ float4 load_quad(const float* row, int c, int dim, bool in, bool vec) {
@@ -247,25 +179,9 @@ struct RowTile {
       }
     }
   }
-  // into planes of scaled fp16 parts; down[row]: the inverse of the row's scale
-  __device__ __forceinline__ void split_to(const Planes& m, float* down, int pw, int lane) const {
-    uint32_t top[kPasses];
+  __device__ __forceinline__ void split_to(const Planes& m, int pw, int lane) const {
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
-      const float y = abs_max(abs_max(abs_max(fabsf(x[i].x), x[i].y), x[i].z), x[i].w);
-      if constexpr (kLanes == 32) top[i] = __reduce_max_sync(0xffffffffu, __float_as_uint(y));       // bits of numbers >= 0 are in their order
-      else {
-        top[i] = __float_as_uint(y);
-#pragma unroll
-        for (int o = kLanes / 2; o > 0; o >>= 1) top[i] = max(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
-      const Pow2 f(top[i]);
-      store_quad(m, row(i, pw, lane), 4 * (lane % kLanes), x[i], f.up);
-      if (lane % kLanes == 0) down[row(i, pw, lane)] = f.down;
-    }
+    for (int i = 0; i < kPasses; ++i) store_quad(m, row(i, pw, lane), 4 * (lane % kLanes), x[i]);
   }
   __device__ __forceinline__ void store_to(float* dst, int ld, int pw, int lane) const {
 #pragma unroll
@@ -306,8 +222,8 @@ __device__ __forceinline__ void token_products(float (&out)[2][4], const Planes&
   for (int ks = 0; ks < KS; ks += 2) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-      HalfA a;
-      HalfB b[2];
+      FragA a;
+      FragB b[2];
       load_a(a, X, x0, (ks + p) * 16, lane);
       load_b(b, Y, y0, (ks + p) * 16, lane);
       float y[2][4] = {};
@@ -363,18 +279,6 @@ struct Decays {
     return exp_parts(d, ((a - d) - b) + (tl[e >> 1] - jl[2 * y + (e & 1)]));
   }
 };
-// the inverse scales of a thread's numbers in such a block
-struct Down {
-  float t[2], j[4];
-  __device__ __forceinline__ void load(const float* X, const float* Y, int t0, int j0, int lane) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) t[i] = X[t0 + (lane >> 2) + 8 * i];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) j[i] = Y[j0 + 2 * (lane & 3) + (i & 1) + 4 * (i & 2)];
-  }
-  __device__ __forceinline__ float operator()(int y, int e, float x) const { return x * t[e >> 1] * j[2 * y + (e & 1)]; }
-};
-
 // The state of a warp: tile i holds channels 8 i + 2 tq (+ 1), columns g (0, 1) and g + 8 (2, 3) of the warp's 16 (g = lane / 4, tq = lane % 4)
 template <int KS>
 __device__ __forceinline__ void load_state(float (&S)[2 * KS][4], const float* sp, int64_t ld, int dim, int c, int cols, bool fresh, int lane) {
@@ -396,50 +300,18 @@ __device__ __forceinline__ void store_state(const float (&S)[2 * KS][4], float* 
       if (d < dim && cc < cols) sp[(int64_t)d * ld + cc] = S[i][e];
     }
 }
-// the scales of a warp's 16 columns by their largest absolute values: m0 (columns g) and m1 (columns g + 8) of this thread's numbers
-struct ColumnScale {
-  Pow2 c0, c1;
-  __device__ __forceinline__ static uint32_t whole(float m) {
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    return __float_as_uint(fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)));
-  }
-  __device__ __forceinline__ ColumnScale(float m0, float m1) : c0(whole(m0)), c1(whole(m1)) {}
-  __device__ __forceinline__ float down(int e) const { return e & 2 ? c1.down : c0.down; }
-};
-template <int N>
-__device__ __forceinline__ ColumnScale column_scale(const float (&x)[N][4]) {
-  float m[2] = {0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) m[e >> 1] = abs_max(m[e >> 1], x[i][e]);
-  return ColumnScale(m[0], m[1]);
-}
-// S <- gn S + u K  (u: 16 columns x 32 tokens, with the inverse scales of K's rows in it; the channels from d0 on)
+// S <- gn S + u K  (u: 16 columns x 32 tokens; the channels from d0 on)
 template <int KS>
 __device__ __forceinline__ void state_update(float (&S)[2 * KS][4], float gn, const float (&u)[4][4], const Planes& K, int d0, int lane) {
-  const ColumnScale f = column_scale(u);
-  HalfA a[2];
-  frag_of_tiles(a[0], u[0], u[1], f.c0.up, f.c1.up);
-  frag_of_tiles(a[1], u[2], u[3], f.c0.up, f.c1.up);
-  uint32_t rest[2][4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t)
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-      rest[t >> 1][2 * (t & 1) + e] = split_rest(u[t][2 * e] * (e ? f.c1.up : f.c0.up), u[t][2 * e + 1] * (e ? f.c1.up : f.c0.up), a[t >> 1].r[0][2 * (t & 1) + e], a[t >> 1].r[1][2 * (t & 1) + e]);
+  FragA a[2];
+  frag_of_tiles(a[0], u[0], u[1]);
+  frag_of_tiles(a[1], u[2], u[3]);
 #pragma unroll
   for (int i = 0; i < 2 * KS; i += 4) {
     float r[4][4] = {};
-    HalfB x[2][4];
+    FragB x[2][4];
 #pragma unroll
     for (int s = 0; s < 2; ++s) load_b_t(x[s], K, 16 * s, d0 + 8 * i, lane);
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) mma_f16_acc(r[t], rest[s], x[s][t].r[0]);
-    mma_least(r, a[0], x[0]);
-    mma_least(r, a[1], x[1]);
     mma_small(r, a[0], x[0]);                 // the small products first, so that only the large ones meet a large sum
     mma_small(r, a[1], x[1]);
     mma_high(r, a[0], x[0]);
@@ -447,7 +319,7 @@ __device__ __forceinline__ void state_update(float (&S)[2 * KS][4], float gn, co
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) S[i + t][e] = fmaf(gn, S[i + t][e], r[t][e] * f.down(e));
+      for (int e = 0; e < 4; ++e) S[i + t][e] = fmaf(gn, S[i + t][e], r[t][e]);
   }
 }
 // out += f M^T: 16 columns x 8 NT tokens from 16 tokens of a token-by-token matrix

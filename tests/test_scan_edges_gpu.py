@@ -215,3 +215,62 @@ def test_scans_over_rows_and_columns_of_any_size(ctx, ops, dim, vdim, n):
     assert torch.equal(o1, o0 * sq * sv) and torch.equal(s1, s0 * sv)
     o2, s2 = run(q, v, state, sk=2.0 ** 37)
     assert torch.equal(o2, o0) and torch.equal(s2, s0)
+
+
+def spread(dim, e, g):
+    """2^a per channel, a between -e and e in any order"""
+    return (2.0 ** (torch.rand(dim, generator=g) * 2 * e - e)).to(DEV)
+
+
+def off(got, want, dims):
+    """the largest relative error of the vectors along `dims`"""
+    return float(((got.to(F64) - want).norm(dim=dims) / want.norm(dim=dims)).max())
+
+
+# Channels far apart in size inside one row: queries are large where keys, and so the state's rows, are small, and every channel has its share of a result.  Each
+# channel of the state and each token's outputs have to come out with the error of fp32 sums, as above but of its own size and not of its neighbours': 2e-6.
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("e", [0, 11, 20])
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 64), (100, 33)])
+def test_decayed_scan_over_channels_far_apart(ctx, ops, dim, vdim, e, fixed):
+    n, H, G = 77, 2, 1
+    g = torch.Generator().manual_seed(dim + e)
+    f = spread(dim, e, g)
+    q, k, v = rows([n], g, G, dim) * dim ** -0.5 * f, rows([n], g, G, dim) * dim ** -0.5 / f, rows([n], g, H, vdim)
+    ld, decay = -rows([n], g, H).abs() * 0.1, torch.tensor([0.9, 0.99], device=DEV)
+    state = torch.randn(1, H, dim, vdim, generator=g).to(DEV) / f[:, None]
+    S = state[0].to(F64)
+    o = ops.decay_scan(ctx, q.view(-1, G * dim), k.view(-1, G * dim), v.view(-1, H * vdim), state, i32([0]), i32([0, n]), i32(list(range(3, 3 + n))), H, G, dim, vdim,
+                       decay=decay if fixed else None, log_decay=None if fixed else ld, max_qlen=n)
+    keep, want = decay.to(F64).expand(n, H) if fixed else ld.to(F64).exp(), []
+    for t in range(n):
+        S = S * keep[t][:, None, None] + k[t].to(F64).expand(H, dim)[:, :, None] * v[t].to(F64)[:, None]
+        want.append(torch.einsum("hdv,hd->hv", S, q[t].to(F64).expand(H, dim)))
+    assert off(state[0], S, -1) <= 2e-6
+    assert off(o.view(n, H, vdim), torch.stack(want), -1) <= 2e-6
+
+
+@pytest.mark.parametrize("e", [0, 11, 20])
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 64), (100, 33)])
+def test_delta_rule_over_channels_far_apart(ctx, ops, dim, vdim, e):
+    n, H, G, taps = 77, 2, 1, 2
+    g = torch.Generator().manual_seed(dim + e)
+    C = 2 * G * dim + H * vdim
+    f = spread(dim, e, g)
+    w = torch.randn(taps, C, generator=g).to(DEV)
+    w[:, :dim] *= f
+    w[:, dim:2 * dim] /= f
+    state = torch.randn(1, H, dim, vdim, generator=g).to(DEV) / f[:, None] * float(f.min())
+    S = state[0].to(F64)
+    o, q, k, v, gb = ops.delta_rule(ctx, rows([n], g, C + 2 * H), (0, G * dim, 2 * G * dim, C, C + H), H, G, dim, vdim, taps, w, torch.zeros(1, taps - 1, C, device=DEV),
+                                    state, i32([0]), i32([0, n]), i32(list(range(3, 3 + n))), torch.full((H,), -2.0, device=DEV), torch.full((H,), -1.0, device=DEV),
+                                    max_qlen=n)
+    q, k, v = q.to(F64).view(-1, G, dim).expand(-1, H, dim), k.to(F64).view(-1, G, dim).expand(-1, H, dim), v.to(F64).view(-1, H, vdim)
+    gb, want = gb.to(F64).view(-1, H, 2), []
+    for t in range(n):
+        S = S * gb[t, :, 0].exp()[:, None, None]
+        u = gb[t, :, 1][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None]
+        want.append(torch.einsum("hdv,hd->hv", S, q[t]))
+    assert off(state[0], S, -1) <= 2e-6
+    assert off(o.view(n, H, vdim), torch.stack(want), -1) <= 2e-6
