@@ -75,7 +75,7 @@ __device__ __forceinline__ void conv_tile(float4 (&y)[TT], const float* in, int6
 }
 
 __device__ __forceinline__ float4 silu4(const float4& a) {
-  return make_float4(a.x * sigmoid_to<float>(a.x), a.y * sigmoid_to<float>(a.y), a.z * sigmoid_to<float>(a.z), a.w * sigmoid_to<float>(a.w));
+  return make_float4(a.x * sigmoid_f32(a.x), a.y * sigmoid_f32(a.y), a.z * sigmoid_f32(a.z), a.w * sigmoid_f32(a.w));
 }
 
 }  // namespace
