@@ -259,16 +259,15 @@ __device__ __forceinline__ void merge_store(const Args& a, float* sm_m, const fl
   const uint32_t q4 = (uint32_t)a.dv >> 2;
   const auto finish = [&](int rr, int d, float M, float L, float4 O) {     // four output numbers from the merged partials
     const int row = r0 + rr, t = row / hg, h = g * hg + row - t * hg;
-    float f = a.out_scale;
     if constexpr (!kSig) {
       if (a.sink) {
         const float sk = __ldg(a.sink + h) * kLog2e, M2 = fmaxf(M, sk), e = M == -INFINITY ? 0.f : fast_exp2(M - M2);
         L = L * e + fast_exp2(sk - M2);
         O.x *= e; O.y *= e; O.z *= e; O.w *= e;
       }
-      f = L > 0.f ? 1.f / L * a.out_scale : 0.f;
     }
-    float y[4] = {O.x * f, O.y * f, O.z * f, O.w * f};
+    const auto scaled = [&](float x) { return kSig ? x * a.out_scale : (L > 0.f ? x / L * a.out_scale : 0.f); };
+    float y[4] = {scaled(O.x), scaled(O.y), scaled(O.z), scaled(O.w)};
     if (a.gate) {
       const float* gp = a.gate + (int64_t)(row_begin + t) * a.ldg;
       if (a.gate_per_head) {
@@ -336,16 +335,17 @@ __device__ __forceinline__ void merge_store(const Args& a, float* sm_m, const fl
     if constexpr (!kSig)
       for (int c = 0; c < a.splits; ++c) M = fmaxf(M, all_m[c * 16 + rr]);
     float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c0 = 0; c0 < a.splits; c0 += 4) {        // four at a time; a cluster of two reads each of its CTAs' numbers once and the last ones again, with a factor of 0
+    for (int c0 = 0; c0 < a.splits; c0 += 4) {        // four at a time; a cluster of two asks for its last CTA's numbers again and leaves them out
       float4 x[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[i] = ld_cluster_f4(ptx::mapa_u32(at, min(c0 + i, a.splits - 1)));
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float f = c0 + i < a.splits ? 1.f : 0.f;
+        if (c0 + i >= a.splits) break;                // (left out, not taken times 0: an infinity would come out as a NaN)
+        float f = 1.f;
         if constexpr (!kSig) {
-          const int e = min(c0 + i, a.splits - 1) * 16 + rr;
-          f = c0 + i < a.splits && all_m[e] != -INFINITY ? fast_exp2(all_m[e] - M) : 0.f;
+          const int e = (c0 + i) * 16 + rr;
+          f = all_m[e] != -INFINITY ? fast_exp2(all_m[e] - M) : 0.f;
           L = fmaf(all_l[e], f, L);
         }
         fma4_acc(O, x[i], f);

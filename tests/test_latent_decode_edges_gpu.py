@@ -59,3 +59,35 @@ def test_shared_decode_by_clusters(ctx, ops, heads, lens, table, window):
         w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), 1)[:, :-1]
         want = (w @ k[:, :R]).reshape(-1)
         assert float((o[b].double() - want).abs().max()) <= 1e-2 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("window,length", [(100, 300), (200, 300), (300, 420), (0, 1000)])       # 1, 2, 4 and 8 CTAs share the keys
+def test_an_infinite_value_comes_out_as_one(ctx, ops, window, length, sigmoid):
+    """Equal scores give every visible key a weight above 0, so an infinite value makes its column's result infinite and no other number anything but finite."""
+    H, G, D, bs, B = 4, 2, 64, 16, 2
+    g = torch.Generator(device=DEV).manual_seed(window)
+    pages = 1024 // bs
+    k, v = (torch.randn(B * pages * bs, G * D, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    tables = torch.arange(B * pages, device=DEV, dtype=torch.int32).view(B, pages)
+    v[length - 20, 7], v[pages * bs + length - 90, D + 33] = float("inf"), -float("inf")
+    o = ops.attn_paged_wide(ctx, torch.zeros(B, H * D, device=DEV, dtype=torch.bfloat16), k, v, tables, i32([length, length]), None, 1, bs, H, G, D, D, D ** -0.5, window=window,
+                            sigmoid=sigmoid).float().view(B, H, D)
+    want = torch.zeros_like(o)
+    want[0, :2, 7], want[1, 2:, 33] = float("inf"), -float("inf")
+    assert torch.equal(torch.where(o.isfinite(), torch.zeros_like(o), o), want)
+
+
+@pytest.mark.parametrize("lens", [[28, 56, 60, 104, 112, 120, 224, 480], [28, 56, 28, 56, 28, 56] * 6])
+def test_results_are_sums_over_sums_rounded_once(ctx, ops, lens):
+    """Equal scores and whole values: sums and weights are exact, so a result is one division, rounded to bf16, whoever shares the keys.  (About a
+    hundredth of these quotients lie in the middle between two bf16 numbers, where a product with a rounded reciprocal falls to either side.)"""
+    D, R, bs, B, H = 128, 96, 16, len(lens), 8
+    g = torch.Generator(device=DEV).manual_seed(5)
+    pages = 704 // bs
+    cache = (torch.rand(B * pages * bs, D, generator=g, device=DEV) * torch.randint(2, 129, (D,), generator=g, device=DEV)).floor().to(torch.bfloat16)
+    tables = torch.arange(B * pages, device=DEV, dtype=torch.int32).view(B, pages)
+    o = ops.attn_paged_wide(ctx, torch.zeros(B, H * D, device=DEV, dtype=torch.bfloat16), cache, cache, tables, i32(lens), None, 1, bs, H, 1, D, R, D ** -0.5)
+    for b, n in enumerate(lens):
+        total = cache[b * pages * bs:b * pages * bs + n, :R].float().sum(0)
+        assert torch.equal(o[b].view(H, R), (total / torch.full_like(total, n)).to(torch.bfloat16).expand(H, R))
