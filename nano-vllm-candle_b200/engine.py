@@ -16,6 +16,8 @@ import ctypes as C
 import json
 import os
 import sys
+import weakref
+from collections import deque
 from dataclasses import dataclass, field
 from typing import Dict, Iterable, List, Optional, Sequence as Seq, Tuple
 
@@ -183,15 +185,27 @@ def _p(a: np.ndarray):
 
 # Logits leave the GPU as they are wanted by the caller: in an array of its own.  Into fresh pageable memory the driver copies twice, page by page (8 x 32 768
 # numbers: 107 us of a 274 us step); into page-locked memory the GPU writes once (24 us).  The memory comes from the process's tensor library, where one is
-# in use, and goes back to its pool with the array; arrays below 64 KiB or above 32 MiB - which a pool should not hold on to - stay pageable.
+# in use, and goes back to its pool with the array.  Pageable memory, as ever: arrays below 64 KiB or above 32 MiB, all but four at a time - a caller who keeps
+# the logits of many steps must not lock the machine's memory, and the pool holds on to what it once gave - and where no page-locked memory can be had.
 _PINNED_BYTES = range(1 << 16, (1 << 25) + 1)
+_pinned_permits = deque([None] * 4)      # taken and given back in one step each, so safe among threads and in a finalizer
 
 
 def _logits_array(rows: int, cols: int) -> np.ndarray:
     torch = sys.modules.get("torch")
     if torch is None or not torch.cuda.is_initialized() or rows * cols * 4 not in _PINNED_BYTES:
         return np.empty((rows, cols), dtype=np.float32)
-    return torch.empty((rows, cols), dtype=torch.float32, pin_memory=True).numpy()
+    try:
+        _pinned_permits.pop()
+    except IndexError:
+        return np.empty((rows, cols), dtype=np.float32)
+    try:
+        out = torch.empty((rows, cols), dtype=torch.float32, device="cpu", pin_memory=True).numpy()
+        weakref.finalize(out, _pinned_permits.append, None).atexit = False
+        return out
+    except RuntimeError:                 # no page-locked memory left
+        _pinned_permits.append(None)
+        return np.empty((rows, cols), dtype=np.float32)
 
 
 class Qwen3ModelRunner:
@@ -318,7 +332,8 @@ class Qwen3ModelRunner:
               "nvc_runner_set_sampling", self.ctx.h)
 
     def last_logits(self, B: int) -> np.ndarray:
-        """fp32 logits [B, vocab / tp_size] of this rank's vocab shard for the last step."""
+        """fp32 logits [B, vocab / tp_size] of this rank's vocab shard for the last step.  The array is the caller's own; up to four that live at a time lie in
+        page-locked memory (64 KiB to 32 MiB each), the others in pageable memory, whose copy is slower."""
         v_l = self.cfg.vocab_size // self.ctx.tp_size
         out = _logits_array(B, v_l)
         check(self.l.nvc_runner_last_logits(self.handle, _p(out), B), "nvc_runner_last_logits", self.ctx.h)
