@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_wide_simt_kernel(const W
       float dot = 0.f;
       for (int d = 0; d < s.dim; ++d) dot = fmaf(q_s[d], ld_f(kp + d), dot);
       sc = dot * s.scale;
-      if (s.key_scale) sc *= __ldg(s.key_scale + slot);
+      if (s.key_scale) sc *= s.key_scale[slot];
       if (s.softcap > 0.f) sc = s.softcap * tanhf(sc / s.softcap);
     }
     float p;

@@ -412,10 +412,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3) attn_wide_mma_kernel(const Arg
     for (int ks = 0; ks < KS; ++ks) {
       const int d = ks * 16 + 2 * tq;
       const bool in = ks < ks_n;
-      qa[ks][0] = va && in ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d)) : 0u;
-      qa[ks][1] = vb && in ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d)) : 0u;
-      qa[ks][2] = va && in ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d + 8)) : 0u;
-      qa[ks][3] = vb && in ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d + 8)) : 0u;
+      qa[ks][0] = va && in ? *reinterpret_cast<const uint32_t*>(qrow0 + d) : 0u;
+      qa[ks][1] = vb && in ? *reinterpret_cast<const uint32_t*>(qrow1 + d) : 0u;
+      qa[ks][2] = va && in ? *reinterpret_cast<const uint32_t*>(qrow0 + d + 8) : 0u;
+      qa[ks][3] = vb && in ? *reinterpret_cast<const uint32_t*>(qrow1 + d + 8) : 0u;
     }
   }
   float o[NT][4];

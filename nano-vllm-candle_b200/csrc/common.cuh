@@ -127,8 +127,9 @@ static inline cudaError_t nvc_launch(const nvc_ctx* ctx, void (*kernel)(KArgs...
 
 // Programmatic dependent launch (griddepcontrol): wait = all prerequisite grids have completed
 // and their memory is visible; trigger = the next grid in the stream may be scheduled.
-// What an earlier kernel writes is read through plain pointers where the load stands right behind the wait: through `const T* __restrict__` it is a load of
-// data that never changes, which the compiler may move in front of the wait, memory clobber or not (seen on sm_100a: an eighth of the numbers were stale).
+// What an earlier kernel writes is read through plain pointers, without __ldg: through `const T* __restrict__`, or __ldg, it is a load of data that never
+// changes, which the compiler may move in front of the wait, memory clobber or not (seen on sm_100a: an eighth of the numbers were stale).  Those forms
+// are for the static operands alone (weights, tables, positions, slots, block tables, lengths), and __restrict__ for what a kernel writes.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -204,10 +205,11 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-__device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
+// 16 bytes that are read once: coherent, since an earlier kernel of the stream writes them
+__device__ __forceinline__ uint4 ld_once_u4(const void* p) {
   uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
   return r;
 }
 

@@ -16,7 +16,7 @@ extern int g_nvc_debug[8];   // prefill_attn.cu: [6] == 1 switches the sampling 
 // K0 embed gather: out[n,:] = table[ids[n],:]        (src/models/qwen3.rs:465-468)
 // one warp per 512-byte slice of a row; 16 B per lane.
 // ------------------------------------------------------------------------------------
-__global__ void embed_gather_kernel(const int32_t* __restrict__ ids, const uint4* __restrict__ table,
+__global__ void embed_gather_kernel(const int32_t* ids, const uint4* __restrict__ table,
                                     uint4* __restrict__ out, int N, int vec_per_row) {
   pdl_trigger();
   pdl_wait();
@@ -25,7 +25,7 @@ __global__ void embed_gather_kernel(const int32_t* __restrict__ ids, const uint4
   if (i >= total) return;
   int n = (int)(i / vec_per_row);
   int c = (int)(i - (int64_t)n * vec_per_row);
-  int id = __ldg(ids + n);
+  int id = ids[n];
   out[i] = __ldg(table + (int64_t)id * vec_per_row + c);
 }
 
@@ -54,7 +54,7 @@ extern "C" int nvc_embed_gather(nvc_ctx* ctx, const int32_t* ids, const nvc_bf16
 // ------------------------------------------------------------------------------------
 template <bool kLoop>
 __global__ void __launch_bounds__(1024)
-fused_add_rmsnorm_kernel(const uint4* __restrict__ x, const float4* __restrict__ res_in,
+fused_add_rmsnorm_kernel(const uint4* x, const float4* res_in,
                          float4* __restrict__ res_out, const uint4* __restrict__ w, float eps,
                          uint4* __restrict__ out, int H) {
   __shared__ float red[32];
@@ -71,7 +71,7 @@ fused_add_rmsnorm_kernel(const uint4* __restrict__ x, const float4* __restrict__
   if (!kLoop) {
     const int v = threadIdx.x;
     if (v < nvec) {
-      unpack8(ldg_nc_u4(x + vbase + v), s);
+      unpack8(ld_once_u4(x + vbase + v), s);
       if (res_in) {
         float4 a = res_in[(vbase + v) * 2], b = res_in[(vbase + v) * 2 + 1];
         s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
@@ -86,7 +86,7 @@ fused_add_rmsnorm_kernel(const uint4* __restrict__ x, const float4* __restrict__
     }
   } else {
     for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      unpack8(ldg_nc_u4(x + vbase + v), s);
+      unpack8(ld_once_u4(x + vbase + v), s);
       if (res_in) {
         float4 a = res_in[(vbase + v) * 2], b = res_in[(vbase + v) * 2 + 1];
         s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
@@ -124,7 +124,7 @@ fused_add_rmsnorm_kernel(const uint4* __restrict__ x, const float4* __restrict__
         float4 a = res_out[(vbase + v) * 2], b = res_out[(vbase + v) * 2 + 1];
         s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w; s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
       } else {
-        unpack8(ldg_nc_u4(x + vbase + v), s);
+        unpack8(ld_once_u4(x + vbase + v), s);
         if (res_in) {
           float4 a = res_in[(vbase + v) * 2], b = res_in[(vbase + v) * 2 + 1];
           s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
@@ -298,7 +298,7 @@ extern "C" int nvc_qk_norm_rope_store(nvc_ctx* ctx, nvc_bf16* qkv, const nvc_bf1
 // Algorithmic bytes per token: 2 * kv * hd * 2 read + the same written.
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-store_kvcache_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, int ld_vec,
+store_kvcache_kernel(const uint4* k, const uint4* v, int ld_vec,
                      uint4* __restrict__ k_cache, uint4* __restrict__ v_cache,
                      const int32_t* __restrict__ slot_mapping, int N, int row_vec) {
   pdl_trigger();
@@ -309,8 +309,8 @@ store_kvcache_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, i
   const int c = (int)(i - (int64_t)n * row_vec);
   const int slot = __ldg(slot_mapping + n);
   if (slot < 0) return;
-  k_cache[(int64_t)slot * row_vec + c] = ldg_nc_u4(k + (int64_t)n * ld_vec + c);
-  v_cache[(int64_t)slot * row_vec + c] = ldg_nc_u4(v + (int64_t)n * ld_vec + c);
+  k_cache[(int64_t)slot * row_vec + c] = ld_once_u4(k + (int64_t)n * ld_vec + c);
+  v_cache[(int64_t)slot * row_vec + c] = ld_once_u4(v + (int64_t)n * ld_vec + c);
 }
 
 extern "C" int nvc_store_kvcache(nvc_ctx* ctx, const nvc_bf16* k, const nvc_bf16* v, int ld,
@@ -337,7 +337,7 @@ extern "C" int nvc_store_kvcache(nvc_ctx* ctx, const nvc_bf16* k, const nvc_bf16
 // Algorithmic bytes per token: I * (4 read + 2 written).
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-silu_and_mul_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, int N, int ivec) {
+silu_and_mul_kernel(const uint4* x, uint4* __restrict__ out, int N, int ivec) {
   pdl_trigger();
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -345,8 +345,8 @@ silu_and_mul_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, int N,
   const int n = (int)(i / ivec);
   const int c = (int)(i - (int64_t)n * ivec);
   float g[8], u[8];
-  unpack8(ldg_nc_u4(x + (int64_t)n * 2 * ivec + c), g);
-  unpack8(ldg_nc_u4(x + (int64_t)n * 2 * ivec + ivec + c), u);
+  unpack8(ld_once_u4(x + (int64_t)n * 2 * ivec + c), g);
+  unpack8(ld_once_u4(x + (int64_t)n * 2 * ivec + ivec + c), u);
 #pragma unroll
   for (int j = 0; j < 8; ++j) g[j] = (g[j] / (1.0f + __expf(-g[j]))) * u[j];
   out[i] = pack8(g);
@@ -372,7 +372,7 @@ extern "C" int nvc_silu_and_mul(nvc_ctx* ctx, const nvc_bf16* x, nvc_bf16* out, 
 // K7 last-token row gather (hidden bf16 + residual f32)
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const uint4* __restrict__ x, const float4* __restrict__ res, const int32_t* __restrict__ rows,
+gather_rows_kernel(const uint4* x, const float4* res, const int32_t* rows,
                    uint4* __restrict__ x_out, float4* __restrict__ res_out, int B, int hvec) {
   pdl_trigger();
   pdl_wait();
@@ -380,7 +380,7 @@ gather_rows_kernel(const uint4* __restrict__ x, const float4* __restrict__ res, 
   if (i >= (int64_t)B * hvec) return;
   const int b = (int)(i / hvec);
   const int c = (int)(i - (int64_t)b * hvec);
-  const int64_t r = __ldg(rows + b);
+  const int64_t r = rows[b];
   x_out[i] = x[r * hvec + c];
   if (res != nullptr) {
     res_out[i * 2] = res[(r * hvec + c) * 2];
@@ -474,7 +474,7 @@ static int argmax_cluster_width(const nvc_ctx* ctx, int B, int V, int long_row) 
 // CTA r scans the r-th slice of the row, stores its (value, index) into CTA 0's shared memory over DSMEM, and CTA 0
 // merges after one cluster barrier.  The "last maximal index" rule is order-independent, so the split does not show.
 __global__ void __launch_bounds__(1024)
-argmax_last_kernel(const float* __restrict__ logits, int ld, int32_t* __restrict__ idx, float* __restrict__ val,
+argmax_last_kernel(const float* logits, int ld, int32_t* __restrict__ idx, float* __restrict__ val,
                    int V, int index_offset, int csz) {
   pdl_trigger();
   pdl_wait();
@@ -488,7 +488,7 @@ argmax_last_kernel(const float* __restrict__ logits, int ld, int32_t* __restrict
   const float4* row4 = reinterpret_cast<const float4*>(row);
 #pragma unroll 4
   for (int j = rank * per + threadIdx.x; j < j1; j += blockDim.x) {
-    const float4 f = __ldg(row4 + j);
+    const float4 f = row4[j];
     const int base = j << 2;
     argmax_combine(bv, bi, f.x, base);
     argmax_combine(bv, bi, f.y, base + 1);
@@ -496,7 +496,7 @@ argmax_last_kernel(const float* __restrict__ logits, int ld, int32_t* __restrict
     argmax_combine(bv, bi, f.w, base + 3);
   }
   if (rank == csz - 1)
-    for (int j = (v4 << 2) + threadIdx.x; j < V; j += blockDim.x) argmax_combine(bv, bi, __ldg(row + j), j);
+    for (int j = (v4 << 2) + threadIdx.x; j < V; j += blockDim.x) argmax_combine(bv, bi, row[j], j);
   argmax_finish_row(bv, bi, r, rank, csz, idx, val, index_offset);
 }
 
@@ -565,7 +565,7 @@ __device__ __forceinline__ bool gumbel_may_reach(float l, float rT, uint32_t bit
 }
 
 __global__ void __launch_bounds__(1024)
-sample_gumbel_kernel(const float* __restrict__ logits, int ld, const float* temperatures, const uint64_t* streams, uint64_t seed, int32_t* __restrict__ idx,
+sample_gumbel_kernel(const float* logits, int ld, const float* temperatures, const uint64_t* streams, uint64_t seed, int32_t* __restrict__ idx,
                      float* __restrict__ val, int V, int index_offset, int csz, int screen) {
   pdl_trigger();
   pdl_wait();
@@ -591,7 +591,7 @@ sample_gumbel_kernel(const float* __restrict__ logits, int ld, const float* temp
     const int j = j0 + threadIdx.x;
     const bool first = j0 == jbeg;
     if (j < j1) {
-      const float4 f = __ldg(row4 + j);
+      const float4 f = row4[j];
       const uint4 n = philox4x32_10(make_uint4((uint32_t)((index_offset >> 2) + j), s_lo, s_hi, 0u), key);
       bool exact = first || !screen;
       if (!exact) {
@@ -636,7 +636,7 @@ extern "C" int nvc_sample_gumbel(nvc_ctx* ctx, const float* logits, int ld, cons
 }
 
 // (max, idx) of a vocab shard as one 8-byte record per sequence (TP argmax exchange)
-__global__ void pack_argmax_pairs_kernel(const float* __restrict__ val, const int32_t* __restrict__ idx,
+__global__ void pack_argmax_pairs_kernel(const float* val, const int32_t* idx,
                                          float2* __restrict__ pairs, int B) {
   pdl_trigger();
   pdl_wait();

@@ -42,7 +42,7 @@ struct GroupedCfg {
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, void* __restrict__ C, int ldc, int out_f32, int M, int N,
-                    int num_kb, int num_tiles, int n_tiles, int epi, int zero, const int32_t* __restrict__ tile_group) {
+                    int num_kb, int num_tiles, int n_tiles, int epi, int zero, const int32_t* tile_group) {
   using cfg = GroupedCfg<BN>;
   pdl_trigger();
   extern __shared__ uint8_t smem_raw[];

@@ -24,7 +24,7 @@ constexpr int kMaxDPerLane = 16;               // D <= 512
 
 template <typename T>
 __global__ void __launch_bounds__(32 * kWarps)
-latent_attn_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache, int ldc, const int32_t* __restrict__ block_tables,
+latent_attn_kernel(const T* q, int ldq, const T* cache, int ldc, const int32_t* __restrict__ block_tables,
                    int bt_stride, const int32_t* __restrict__ context_lens, const int32_t* __restrict__ cu_seqlens, int heads, int D,
                    int head_stride, int block_size, float scale, T* __restrict__ out, int ldo) {
   extern __shared__ float sm[];

@@ -31,7 +31,7 @@ template <int DP> constexpr int smem_bytes() {
 
 template <int DP>
 __global__ void __launch_bounds__(kWarps * 32)
-latent_attn_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* __restrict__ cache, int ldc,
+latent_attn_mma_kernel(const nvc_bf16* q, int ldq, const nvc_bf16* cache, int ldc,
                        const int32_t* __restrict__ block_tables, int bt_stride, const int32_t* __restrict__ context_lens,
                        const int32_t* __restrict__ cu_seqlens, int heads, int head_stride, int block_size, float scale_log2e,
                        nvc_bf16* __restrict__ out, int ldo, float* __restrict__ part, int num_splits) {
@@ -98,10 +98,10 @@ latent_attn_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* 
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks) {
         const int d = ks * 16 + 2 * tq;
-        qa[ks][0] = va ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d)) : 0u;
-        qa[ks][1] = vb ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d)) : 0u;
-        qa[ks][2] = va ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d + 8)) : 0u;
-        qa[ks][3] = vb ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d + 8)) : 0u;
+        qa[ks][0] = va ? *reinterpret_cast<const uint32_t*>(qrow0 + d) : 0u;
+        qa[ks][1] = vb ? *reinterpret_cast<const uint32_t*>(qrow1 + d) : 0u;
+        qa[ks][2] = va ? *reinterpret_cast<const uint32_t*>(qrow0 + d + 8) : 0u;
+        qa[ks][3] = vb ? *reinterpret_cast<const uint32_t*>(qrow1 + d + 8) : 0u;
       }
     }
     float o[NT][4];
@@ -280,10 +280,10 @@ latent_attn_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* 
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
       const int d = ks * 16 + 2 * tq;
-      qa[ks][0] = va ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d)) : 0u;
-      qa[ks][1] = vb ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d)) : 0u;
-      qa[ks][2] = va ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d + 8)) : 0u;
-      qa[ks][3] = vb ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d + 8)) : 0u;
+      qa[ks][0] = va ? *reinterpret_cast<const uint32_t*>(qrow0 + d) : 0u;
+      qa[ks][1] = vb ? *reinterpret_cast<const uint32_t*>(qrow1 + d) : 0u;
+      qa[ks][2] = va ? *reinterpret_cast<const uint32_t*>(qrow0 + d + 8) : 0u;
+      qa[ks][3] = vb ? *reinterpret_cast<const uint32_t*>(qrow1 + d + 8) : 0u;
     }
   }
   for (int i = 0; i < n_tiles; ++i) {
@@ -418,7 +418,7 @@ latent_attn_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* 
 
 // merges the splits of every row: out = sum_s O_s 2^(M_s - M) / sum_s L_s 2^(M_s - M)
 template <int DP>
-__global__ void latent_attn_combine_kernel(const float* __restrict__ part, int S, int chunks, const int32_t* __restrict__ cu_seqlens,
+__global__ void latent_attn_combine_kernel(const float* part, int S, int chunks, const int32_t* __restrict__ cu_seqlens,
                                            int heads, int head_stride, nvc_bf16* __restrict__ out, int ldo) {
   pdl_trigger();
   pdl_wait();

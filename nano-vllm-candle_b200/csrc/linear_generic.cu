@@ -18,8 +18,8 @@ constexpr int TM = 64, TN = 64, TK = 16;
 
 template <typename T, typename TC>
 __global__ void __launch_bounds__(256)
-linear_kernel(const T* __restrict__ A, int lda, int64_t sa, const int32_t* __restrict__ a_rows, const T* __restrict__ W, int ldw,
-              int64_t sw, TC* __restrict__ C, int ldc, int64_t sc, const int32_t* __restrict__ offsets, int groups, int M, int N,
+linear_kernel(const T* A, int lda, int64_t sa, const int32_t* a_rows, const T* __restrict__ W, int ldw,
+              int64_t sw, TC* __restrict__ C, int ldc, int64_t sc, const int32_t* offsets, int groups, int M, int N,
               int K, int act) {
   __shared__ float As[TK][TM + 4];
   __shared__ float Ws[TK][TN + 4];
@@ -110,9 +110,9 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b
 // BT x BT output tile, 2 * BT threads: BT / 32 x 2 warps of 32 x BT / 2
 template <typename TC, int BT>
 __global__ void __launch_bounds__(2 * BT)
-linear_mma_kernel(const __nv_bfloat16* __restrict__ A, int lda, int64_t sa, const int32_t* __restrict__ a_rows,
+linear_mma_kernel(const __nv_bfloat16* A, int lda, int64_t sa, const int32_t* a_rows,
                   const __nv_bfloat16* __restrict__ W, int ldw, int64_t sw, TC* __restrict__ C, int ldc, int64_t sc,
-                  const int32_t* __restrict__ offsets, int groups, int M, int N, int K, int act) {
+                  const int32_t* offsets, int groups, int M, int N, int K, int act) {
   __shared__ __align__(128) uint8_t sA[2][BT * MROW];
   __shared__ __align__(128) uint8_t sW[2][BT * MROW];
   pdl_trigger();

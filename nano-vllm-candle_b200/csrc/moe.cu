@@ -108,7 +108,7 @@ __global__ void moe_topk_kernel(const float* z, int ldz, const float* __restrict
 }
 
 template <typename T>
-__global__ void moe_route_kernel(const T* __restrict__ h, int ldh, const float* __restrict__ wr, const float* __restrict__ corr,
+__global__ void moe_route_kernel(const T* h, int ldh, const float* __restrict__ wr, const float* __restrict__ corr,
                                  const float* __restrict__ wsg, int E, int top, float scale, int32_t* __restrict__ idx,
                                  float* __restrict__ wout, float* __restrict__ gate, int N, int H) {
   extern __shared__ float hs[];   // [warps][H]
@@ -253,8 +253,8 @@ moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align
 
 // out[r] = in[src_rows[r]] for r < *num_rows (a device count), zeros where src_rows[r] < 0, `two` (a pair of bf16) behind them when fill is set;
 // 16 bytes per thread
-__global__ void gather_rows_kernel(const uint4* __restrict__ in, int ld_in, const int32_t* __restrict__ src_rows,
-                                   const int32_t* __restrict__ num_rows, uint4* __restrict__ out, int ld_out, int rows_cap, int per_row,
+__global__ void gather_rows_kernel(const uint4* in, int ld_in, const int32_t* src_rows,
+                                   const int32_t* num_rows, uint4* __restrict__ out, int ld_out, int rows_cap, int per_row,
                                    int rows_per_cta, int fill, uint32_t two) {
   pdl_trigger();
   pdl_wait();
@@ -296,8 +296,8 @@ __global__ void __launch_bounds__(256) gather_rows_warp_kernel(const uint4* in, 
 
 // experts from E_real on are identity experts: their pairs read the token's own row x[n] instead of a row of y
 template <typename TY, typename TX>
-__global__ void moe_combine_identity_kernel(const TY* __restrict__ y, int ldy, const int32_t* __restrict__ pos, const float* __restrict__ w,
-                                            const int32_t* __restrict__ idx, int top, int E_real, const TX* __restrict__ x, int ldx,
+__global__ void moe_combine_identity_kernel(const TY* y, int ldy, const int32_t* pos, const float* w,
+                                            const int32_t* idx, int top, int E_real, const TX* x, int ldx,
                                             float* __restrict__ out, int ldo, int H) {
   pdl_trigger();
   pdl_wait();
@@ -314,8 +314,8 @@ __global__ void moe_combine_identity_kernel(const TY* __restrict__ y, int ldy, c
 }
 
 template <typename TY, typename TS>
-__global__ void moe_combine_kernel(const TY* __restrict__ y, int ldy, const int32_t* __restrict__ pos, const float* __restrict__ w,
-                                   int top, const TS* __restrict__ shared, int lds, const float* __restrict__ gate,
+__global__ void moe_combine_kernel(const TY* y, int ldy, const int32_t* pos, const float* w,
+                                   int top, const TS* shared, int lds, const float* gate,
                                    float* __restrict__ out, int ldo, int H) {
   pdl_trigger();
   pdl_wait();
@@ -367,7 +367,7 @@ __global__ void moe_combine_f4_kernel(const float4* y, int ldy4, const int32_t* 
 
 // one CTA per (token, choice): the token's row times the pair's router weight, written where the sort put the pair
 template <typename T>
-__global__ void moe_scatter_scaled_kernel(const T* __restrict__ h, int ldh, const int32_t* __restrict__ pos, const float* __restrict__ topk_w,
+__global__ void moe_scatter_scaled_kernel(const T* h, int ldh, const int32_t* pos, const float* topk_w,
                                           T* __restrict__ out, int ldo, int top, int H) {
   pdl_trigger();
   pdl_wait();

@@ -41,10 +41,10 @@ __device__ __forceinline__ float sq4(const float4& v) { return v.x * v.x + v.y *
 // one CTA per output row; the branch rows and the summed row stay in shared memory between the passes
 // VEC: H, ld and ldo are multiples of 4 and every pointer is 16-byte aligned: four numbers per access
 template <typename T, bool VEC>
-__global__ void rms_norm_blend_kernel(const float* __restrict__ res_in, const float* __restrict__ bias, const float* __restrict__ y0,
-                                      const float* __restrict__ w0, float c0, const float* __restrict__ y1, const float* __restrict__ w1,
+__global__ void rms_norm_blend_kernel(const float* res_in, const float* __restrict__ bias, const float* y0,
+                                      const float* __restrict__ w0, float c0, const float* y1, const float* __restrict__ w1,
                                       float c1, float* __restrict__ res_out, int ld, const float* __restrict__ w, T* __restrict__ out, int ldo,
-                                      float eps, const int32_t* __restrict__ rows, int H) {
+                                      float eps, const int32_t* rows, int H) {
   extern __shared__ __align__(16) float sm[];          // [3][H]: y0, y1, s
   __shared__ float part[33];
   pdl_trigger();
@@ -143,7 +143,7 @@ __global__ void rms_norm_blend_kernel(const float* __restrict__ res_in, const fl
 // one CTA per (row, group).  VEC: gsize and the three row strides are multiples of 4 and every pointer is 16-byte aligned (out: 8 bytes in
 // bf16): four numbers per access
 template <typename T, bool VEC>
-__global__ void group_norm_gate_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ gate, int ldg,
+__global__ void group_norm_gate_kernel(const float* o, int ldo, const float* gate, int ldg,
                                        const float* __restrict__ weight, T* __restrict__ out, int ldout, int gsize, int gate_first, float eps,
                                        int act) {
   extern __shared__ __align__(16) float sm[];          // [gsize]

@@ -10,7 +10,7 @@
 namespace {
 
 template <typename T>
-__global__ void embed_gather_f32_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, int ldt,
+__global__ void embed_gather_f32_kernel(const int32_t* ids, const T* __restrict__ table, int ldt,
                                         float* __restrict__ out, int ldo, int N, int H) {
   pdl_trigger();
   pdl_wait();
@@ -22,10 +22,10 @@ __global__ void embed_gather_f32_kernel(const int32_t* __restrict__ ids, const T
 
 // one CTA per output row
 template <typename T>
-__global__ void dyt_norm_kernel(const float* __restrict__ res_in, const float* __restrict__ a0, const float* __restrict__ a1,
-                                const float* __restrict__ a2, float* __restrict__ res_out, int ld, const float* __restrict__ w,
+__global__ void dyt_norm_kernel(const float* res_in, const float* a0, const float* a1,
+                                const float* a2, float* __restrict__ res_out, int ld, const float* __restrict__ w,
                                 const float* __restrict__ b, const float* __restrict__ alpha, T* __restrict__ out, int ldo,
-                                const int32_t* __restrict__ rows, int H) {
+                                const int32_t* rows, int H) {
   pdl_trigger();
   const float al = w ? __ldg(alpha) : 0.f;
   pdl_wait();
@@ -43,7 +43,7 @@ __global__ void dyt_norm_kernel(const float* __restrict__ res_in, const float* _
 
 // one warp per row: segment 0 = columns [0, n0) -> out0; segment 1 = columns [off1, off1 + n1) -> the cache row of the slot
 template <typename T>
-__global__ void latent_norm_store_kernel(const float* __restrict__ in, int ldi, int n0, int off1, int n1,
+__global__ void latent_norm_store_kernel(const float* in, int ldi, int n0, int off1, int n1,
                                          const float* __restrict__ w0, const float* __restrict__ w1, float eps,
                                          T* __restrict__ out0, int ld0, T* __restrict__ cache, int ldc,
                                          const int32_t* __restrict__ slots, int rot_dim, int rot_dims, int rot_half,
@@ -168,7 +168,7 @@ __device__ __forceinline__ float act_unit(int kind, float g, float u, float p0, 
 
 // rows_per_cta rows per CTA, the threads walk along a row: no division per element
 template <typename T>
-__global__ void act_mul_kernel(const T* __restrict__ in, int ldi, T* __restrict__ out, int ldo, int N, int F, int Fp, int kind, float p0,
+__global__ void act_mul_kernel(const T* in, int ldi, T* __restrict__ out, int ldo, int N, int F, int Fp, int kind, float p0,
                                float p1, int rows_per_cta) {
   pdl_trigger();
   pdl_wait();

@@ -12,7 +12,7 @@
 namespace {
 
 template <typename T>
-__global__ void embed_gather_scaled_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, int ldt, float scale,
+__global__ void embed_gather_scaled_kernel(const int32_t* ids, const T* __restrict__ table, int ldt, float scale,
                                            float* __restrict__ out, int ldo, int N, int H) {
   pdl_trigger();
   pdl_wait();
@@ -39,10 +39,10 @@ __global__ void softcap_kernel(float* __restrict__ x, int ld, float cap, int V) 
 
 // one CTA per output row; the summed row stays in shared memory between the two passes
 template <typename T>
-__global__ void rms_norm_pair_kernel(const float* __restrict__ res_in, const float* __restrict__ a0, const float* __restrict__ a1,
+__global__ void rms_norm_pair_kernel(const float* res_in, const float* a0, const float* a1,
                                      float* __restrict__ res_out, int ld, const float* __restrict__ w0, T* __restrict__ out0,
                                      const float* __restrict__ w1, T* __restrict__ out1, int ldo, float eps,
-                                     const int32_t* __restrict__ rows, int H) {
+                                     const int32_t* rows, int H) {
   extern __shared__ float row[];
   __shared__ float part[32];
   pdl_trigger();
@@ -79,9 +79,9 @@ __global__ void rms_norm_pair_kernel(const float* __restrict__ res_in, const flo
 
 // one CTA per output row: y is normed and added to the residual row, the sum is normed again; the row stays in shared memory
 template <typename T>
-__global__ void rms_norm_sandwich_kernel(const float* __restrict__ res_in, const float* __restrict__ y, const float* __restrict__ wy,
+__global__ void rms_norm_sandwich_kernel(const float* res_in, const float* y, const float* __restrict__ wy,
                                          float* __restrict__ res_out, int ld, const float* __restrict__ w, T* __restrict__ out, int ldo,
-                                         float eps, float woff, const int32_t* __restrict__ rows, int H) {
+                                         float eps, float woff, const int32_t* rows, int H) {
   extern __shared__ float row[];
   __shared__ float part[33];
   pdl_trigger();
@@ -159,9 +159,9 @@ __device__ __forceinline__ float block_sum(float v, float* part) {
 }
 
 template <typename T, int V>
-__global__ void rms_norm_sandwich_vec_kernel(const float* __restrict__ res_in, const float* __restrict__ y, const float* __restrict__ wy,
+__global__ void rms_norm_sandwich_vec_kernel(const float* res_in, const float* y, const float* __restrict__ wy,
                                              float* __restrict__ res_out, int ld, const float* __restrict__ w, T* __restrict__ out, int ldo,
-                                             float eps, float woff, const int32_t* __restrict__ rows, int H) {
+                                             float eps, float woff, const int32_t* rows, int H) {
   __shared__ float part[33];
   pdl_trigger();
   pdl_wait();
@@ -218,7 +218,7 @@ __global__ void rms_norm_sandwich_vec_kernel(const float* __restrict__ res_in, c
 
 // one warp per (row, head); vec: vdim and every stride are multiples of 4 and the pointers 16-byte aligned (16-byte accesses)
 template <typename T>
-__global__ void head_gate_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, int ldg,
+__global__ void head_gate_kernel(const float* o, int ldo, const float* g, int ldg,
                                  const float* __restrict__ wgt, T* __restrict__ out, int ldout, int heads, int vdim, int norm, float eps, int act,
                                  float out_scale, int N, int vec) {
   pdl_trigger();

@@ -134,7 +134,7 @@ __device__ __forceinline__ void row_epilogue(float (&s)[8], const Epilogue& ep, 
 // LL one-shot.  grid = N rows, block = H / 8 threads rounded up to a warp.  x = this rank's partial [N, H] bf16.
 template <int TP>
 __global__ void __launch_bounds__(1024)
-nvls_ll_allreduce_rmsnorm_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ uc_ll, uint8_t* __restrict__ mc_ll,
+nvls_ll_allreduce_rmsnorm_kernel(const uint4* x, uint8_t* __restrict__ uc_ll, uint8_t* __restrict__ mc_ll,
                                  size_t ll_buf_bytes, uint32_t* __restrict__ state, int my_rank, Epilogue ep, int H) {
   __shared__ float red[32];
   __shared__ uint32_t s_epoch, s_clear;

@@ -47,7 +47,7 @@ __device__ __forceinline__ uint4 ld_peer_u4(const void* p) {     // peer memory:
 template <int TP>
 __global__ void __launch_bounds__(1024)
 p2p_allreduce_rmsnorm_kernel(uint8_t* const* __restrict__ peers, uint32_t* __restrict__ state, int my_rank,
-                             size_t slot_off, const float4* __restrict__ res_in, float4* __restrict__ res_out,
+                             size_t slot_off, const float4* res_in, float4* __restrict__ res_out,
                              const uint4* __restrict__ w, float eps, uint4* __restrict__ out, int H) {
   __shared__ float red[32];
   __shared__ uint32_t s_epoch;

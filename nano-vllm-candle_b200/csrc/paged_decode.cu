@@ -35,20 +35,20 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 __global__ void __launch_bounds__(128)
-paged_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+paged_decode_combine_kernel(const float* part_o, const float* part_ml,
                             nvc_bf16* __restrict__ out, int nh, int num_splits) {
   pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const int64_t p0 = ((int64_t)b * nh + head) * num_splits;
   float M = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) M = fmaxf(M, __ldg(part_ml + (p0 + s) * 2));
+  for (int s = 0; s < num_splits; ++s) M = fmaxf(M, part_ml[(p0 + s) * 2]);
   float L = 0.f, O = 0.f;
   if (M != -INFINITY) {
     for (int s = 0; s < num_splits; ++s) {
-      const float w = fast_exp2(__ldg(part_ml + (p0 + s) * 2) - M);
-      L += __ldg(part_ml + (p0 + s) * 2 + 1) * w;
-      O += __ldg(part_o + (p0 + s) * 128 + d) * w;
+      const float w = fast_exp2(part_ml[(p0 + s) * 2] - M);
+      L += part_ml[(p0 + s) * 2 + 1] * w;
+      O += part_o[(p0 + s) * 128 + d] * w;
     }
   }
   const float o = L > 0.f ? O / L : 0.f;

@@ -71,8 +71,8 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 // kTeams: four warps, a one-dimensional grid of at least half as many CTAs as units; no splits, up to 128 sequences.
 template <int kWarps, bool kTeams = false>
 __global__ void __launch_bounds__(kWarps * 32, kWarps == 4 ? 2 : 4)
-paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16* __restrict__ k_cache,
-                        const nvc_bf16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_blocks,
+paged_decode_mma_kernel(const nvc_bf16* q, int ldq, const nvc_bf16* k_cache,
+                        const nvc_bf16* v_cache, const int32_t* __restrict__ block_tables, int max_blocks,
                         const int32_t* __restrict__ context_lens, int nh, int kv, int group_total, int gchunk,
                         int block_size, float scale_log2e, nvc_bf16* __restrict__ out, float* __restrict__ part_o,
                         float* __restrict__ part_ml, int num_splits, int B) {
@@ -247,10 +247,10 @@ paged_decode_mma_kernel(const nvc_bf16* __restrict__ q, int ldq, const nvc_bf16*
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const int d = ks * 16 + 2 * tq;
-      qa[ks][0] = r0 ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d)) : 0u;
-      qa[ks][1] = r1 ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d)) : 0u;
-      qa[ks][2] = r0 ? __ldg(reinterpret_cast<const uint32_t*>(qrow0 + d + 8)) : 0u;
-      qa[ks][3] = r1 ? __ldg(reinterpret_cast<const uint32_t*>(qrow1 + d + 8)) : 0u;
+      qa[ks][0] = r0 ? *reinterpret_cast<const uint32_t*>(qrow0 + d) : 0u;
+      qa[ks][1] = r1 ? *reinterpret_cast<const uint32_t*>(qrow1 + d) : 0u;
+      qa[ks][2] = r0 ? *reinterpret_cast<const uint32_t*>(qrow0 + d + 8) : 0u;
+      qa[ks][3] = r1 ? *reinterpret_cast<const uint32_t*>(qrow1 + d + 8) : 0u;
     }
   }
   if (pre < 1) issue(0);

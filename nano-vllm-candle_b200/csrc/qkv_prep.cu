@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(1024) prep_token_kernel(const PrepArgs a, cons
 // one warp per (token, head) of a query projection laid out [heads][dim | rot_dim]: the unrotated part goes to out_a, the rotated
 // part (turned by the token's position) to out_b
 template <typename T>
-__global__ void head_split_rot_kernel(const float* __restrict__ in, int ldi, int heads, int dim, int rot_dim, int rot_dims, int rot_half,
+__global__ void head_split_rot_kernel(const float* in, int ldi, int heads, int dim, int rot_dim, int rot_dims, int rot_half,
                                       const float* __restrict__ rot_table, const int32_t* __restrict__ positions, T* __restrict__ out_a,
                                       int ld_a, int hs_a, T* __restrict__ out_b, int ld_b, int hs_b, int off_b, int N) {
   pdl_trigger();
@@ -562,7 +562,7 @@ __global__ void head_split_rot_kernel(const float* __restrict__ in, int ldi, int
 // one CTA per token: the sums of squares of the whole query and the whole key projection in one pass (the key rows leave for the cache
 // on the way), then the queries.  VEC: every offset, width and stride is a multiple of 4 and the pointers are 16-byte aligned.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) qk_norm_fold_store_kernel(const float* __restrict__ in, int ldi, int q_off, int qw, int k_off, int kw,
+__global__ void __launch_bounds__(256) qk_norm_fold_store_kernel(const float* in, int ldi, int q_off, int qw, int k_off, int kw,
                                                                  const float* __restrict__ wqk, float eps, const int32_t* __restrict__ positions,
                                                                  float temp_coef, int temp_every, T* __restrict__ q_out, int ldq,
                                                                  T* __restrict__ cache, int ldc, float* __restrict__ key_scale,

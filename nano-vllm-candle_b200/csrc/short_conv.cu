@@ -8,7 +8,7 @@ namespace {
 constexpr int kMaxTaps = 16;
 
 // thread = (sequence, channel): reads the taps - 1 inputs that end the sequence so far, then writes them
-__global__ void conv_advance_kernel(const nvc_short_conv cv, const float* __restrict__ in, int ldi, int off, const float* __restrict__ bias, int C,
+__global__ void conv_advance_kernel(const nvc_short_conv cv, const float* in, int ldi, int off, const float* __restrict__ bias, int C,
                                     const int32_t* __restrict__ positions) {
   pdl_trigger();
   pdl_wait();
