@@ -12,7 +12,7 @@ namespace {
 constexpr int kMaxPerLane = 8;   // experts <= 256
 
 // top-k by repeated arg-max over the choice scores c (ties -> the lower expert index); expert e lives in lane e % 32,
-// slot e / 32.  Writes idx / weights of token n: s_chosen / (sum of the chosen s + 1e-20) * scale.
+// slot e / 32.  Writes idx / weights of token n: s_chosen / (sum of the chosen s + 1e-20) * scale.  idx names an expert whatever the scores are.
 template <int PER>
 __device__ __forceinline__ void topk_write(float (&s)[PER], float (&c)[PER], int lane, int E, int top, float scale,
                                            int32_t* __restrict__ idx, float* __restrict__ wout, int64_t n, bool normalize = true) {
@@ -33,6 +33,7 @@ __device__ __forceinline__ void topk_write(float (&s)[PER], float (&c)[PER], int
       const int oe = __shfl_xor_sync(0xffffffffu, be, o);
       if (ov > bv || (ov == bv && oe < be)) { bv = ov; be = oe; }
     }
+    if (be >= E) be = 0;                      // only NaNs are left, which compare with nothing: expert 0, with the weight NaN
     // the owner lane publishes the unbiased score and retires the expert
     float sv = 0.f;
 #pragma unroll
@@ -243,6 +244,8 @@ moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align
         const int at = off[x] + cnt[warp * E + x] + __popc(peers & ((1u << lane) - 1));
         src_rows[at] = p / top;
         pos[p] = at;
+      } else if (p < p_end) {
+        pos[p] = 0;                                      // no expert, no place: a row that exists, so that what reads it stays in bounds
       }
       __syncwarp();
       if (x >= 0 && lane == 31 - __clz(peers)) cnt[warp * E + x] += __popc(peers);   // the last peer advances the group
