@@ -720,28 +720,34 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
     // ------------------------------------------------ preparing warps
     const int pw = w & 3, group = (w - kPrep0) >> 2;
     RowTile<DZ> x;                            // queries, then keys
-    RowTile<kMC> v;
     float2 gb = make_float2(0.f, 0.f);        // (log decay, beta) of a token; none behind the end
     auto fetch = [&](int i) {
       const int64_t row = r0 + i * kMT;
       const int n = r1 - (int)row;
       x.load(p.q_out + row * p.ldq + hk * dim, p.ldq, dim, n, a.vec, pw, lane);
-      v.load(p.v_out + row * p.ldv + h * p.vdim + v0, p.ldv, cols, n, vecv, pw, lane);
       if (pw == 3) {
         const float* x = p.gb_out + ((row + lane) * p.heads + h) * 2;
         gb = lane < n ? make_float2(x[0], x[1]) : make_float2(0.f, 0.f);
       }
     };
+    auto keys = [&](int i) {
+      const int64_t row = r0 + i * kMT;
+      x.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, r1 - (int)row, a.vec, pw, lane);
+      return buffer(i).K;
+    };
+    if (group) {                              // the first chunk is prepared by both groups: this one takes its keys
+      const Planes K = keys(0);
+      x.split_to(K, pw, lane);
+      bar_arrive(kPrepare, 256);
+    }
     if (group < chunks) fetch(group);
     for (int i = group; i < chunks; i += 2) {
       const Buffer bf = buffer(i);
       if (i >= NB) bar_sync(kEmpty + i % (2 * NB), kBufThreads);
+      const int64_t row = r0 + i * kMT;
+      fetch_values(bf.V, p.v_out + row * p.ldv + h * p.vdim + v0, p.ldv, cols, r1 - (int)row, vecv, pw, lane);
       x.split_to(bf.Q, pw, lane);
-      {
-        const int64_t row = r0 + i * kMT;
-        x.load(p.k_out + row * p.ldk + hk * dim, p.ldk, dim, r1 - (int)row, a.vec, pw, lane);
-      }
-      v.store_to(bf.V, kMV, pw, lane);
+      if (i > 0) keys(i);
       if (pw == 3) {
         const LogSum sum(gb.x, lane);
         const float hi = (float)sum.l;
@@ -751,8 +757,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
         bf.to[lane] = sum.to();
         bf.beta[lane] = gb.y;
       }
-      x.split_to(bf.K, pw, lane);
-      bar_sync(kPrepare + group, 128);
+      if (i > 0) x.split_to(bf.K, pw, lane);
+      bar_sync(kPrepare + group, i > 0 ? 128 : 256);
       // warps 0 and 1: the diagonal blocks of A and their inverses; 2: P (16, 0) and A_10; 3: P (0, 0) and P (16, 16)
 #pragma unroll 1
       for (int part = 0; part < (pw < 2 ? 1 : 2); ++part) {
@@ -810,6 +816,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_mma_kernel(const DeltaA
         }
       }
       if (i == 0) advance_conv_state(p, r0, r1, fresh, slot, blockIdx.x, gridDim.x, threadIdx.x - 32 * kPrep0, 128);      // nothing here reads that state
+      values_wait();
       bar_arrive(kFull + i % NB, kBufThreads);
       if (i + 2 < chunks) fetch(i + 2);
     }

@@ -488,26 +488,36 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
     // ------------------------------------------------ preparing warps
     const int pw = w & 3, group = (w - kPrep0) >> 2;
     RowTile<DZ> x;                            // queries, then keys
-    RowTile<kMC> v;
     float l = 0.f;
     auto fetch = [&](int i) {
       const int64_t row = r0 + i * kMT;
       const int n = r1 - (int)row;
       x.load(a.q + row * a.ldq + hq * dim, a.ldq, dim, n, vec, pw, lane);
-      v.load(a.v + row * a.ldv + h * a.vdim + v0, a.ldv, cols, n, vecv, pw, lane);
       if (VAR && pw == 3) l = lane < n ? a.log_decay[(row + lane) * a.ldl + h] : 0.f;
     };
+    auto keys = [&](int i) {
+      const int64_t row = r0 + i * kMT;
+      x.load(a.k + row * a.ldk + hq * dim, a.ldk, dim, r1 - (int)row, vec, pw, lane);
+      return buffer(i).K;
+    };
+    if (group) {                              // the first chunk is prepared by both groups: this one takes its keys
+      const Planes K = keys(0);
+      x.split_to(K, pw, lane);
+      bar_arrive(kPrepare, 256);
+    }
     if (group < chunks) fetch(group);
     for (int i = group; i < chunks; i += 2) {
       const Buffer bf = buffer(i);
       const int n = min(kMT, r1 - r0 - i * kMT);
       if (i >= kBuffers) bar_sync(kEmpty + i % (2 * kBuffers), kBufThreads);
+      const int64_t row = r0 + i * kMT;
+      fetch_values(bf.V, a.v + row * a.ldv + h * a.vdim + v0, a.ldv, cols, n, vecv, pw, lane);
       x.split_to(bf.Q, pw, lane);
-      {
-        const int64_t row = r0 + i * kMT;
-        x.load(a.k + row * a.ldk + hq * dim, a.ldk, dim, n, vec, pw, lane);
+      if (i > 0) {
+        keys(i);
+        x.split_to(bf.K, pw, lane);
       }
-      v.store_to(bf.V, kMV, pw, lane);
+      bar_sync(kPrepare + group, i > 0 ? 128 : 256);
       if (pw == 3) {
         if (VAR) {
           const LogSum sum(l, lane);
@@ -521,12 +531,11 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
           bf.wj[lane] = lane < n ? gp[n - 1 - lane] : 0.f;
         }
       }
-      x.split_to(bf.K, pw, lane);
-      bar_sync(kPrepare + group, 128);
-      if (pw < 3) {                           // A[t][j]: the blocks (0, 0), (16, 0), (16, 16)
-        const int t0 = pw ? 16 : 0, j0 = pw == 2 ? 16 : 0;
-        float z[2][4];
-        token_products<KS>(z, bf.Q, t0, bf.K, j0, lane);
+      const int t0 = pw ? 16 : 0, j0 = pw == 2 ? 16 : 0;       // A[t][j]: the blocks (0, 0), (16, 0), (16, 16)
+      float z[2][4];
+      if (pw < 3) token_products<KS>(z, bf.Q, t0, bf.K, j0, lane);
+      if (VAR) bar_sync(kPrepare + group, 128);               // the decays, which warp 3 has summed meanwhile
+      if (pw < 3) {
         Decays f;
         if (VAR) f.load(bf.Lh, bf.Ll, t0, j0, lane);
 #pragma unroll
@@ -539,6 +548,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) decay_mma_kernel(const RetArg
             store_pair(bf.A, t, j, y0, y1);
           }
       }
+      values_wait();
       bar_arrive(kFull + i % kBuffers, kBufThreads);
       if (i + 2 < chunks) fetch(i + 2);
     }
@@ -671,7 +681,7 @@ int run_scan(nvc_ctx* ctx, const RetArgs& a, int B, int max_qlen, void* stream) 
     // wide slices while they fill the GPU; keys of more than 256 numbers leave room for 32 columns only
     cudaError_t ce;
     // the tensor pipe keeps 16 columns x all channels of the state in a warp's registers, which is what ends it at 128 channels; at 128 x 64
-    // over eight prompts of 245 to 1 050 tokens, 32 heads: 146 us, the FMA form 640
+    // over eight prompts of 245 to 1 050 tokens, 32 heads: 141 us, the FMA form 640
     if constexpr (MODE != kMemory) {
       // portions of up to 16 tokens over states that do not fit in L2: the FMA kernel's slices of 128 columns read them better (256 portions of 10 tokens, 16 heads of
       // 128 x 128, 1 GB of states: 581 us, here 642; 64 portions: 161, here 121; heads of 64 x 64: 282, here 258)

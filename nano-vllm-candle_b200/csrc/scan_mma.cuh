@@ -3,12 +3,12 @@
 // An fp32 number is the exact sum of three bf16 numbers (8 + 8 + 8 bits: high, middle, low), and a product of two numbers is the sum of nine
 // products of parts.  The six largest are taken (mma.sync m16n8k16, exact products, fp32 sums); the three that are left out are below
 // 2^-24 of the whole.  That holds for every number by itself, whatever its neighbours are.  (Two fp16 parts under one scale per row or state column, three
-// products: 177 us for the delta rule where this takes 222, but 22 bits of the row's largest number for all of them: a channel 2^11 below its
+// products: 177 us for the delta rule where this takes 213, but 22 bits of the row's largest number for all of them: a channel 2^11 below its
 // neighbours came out with errors of 5e-6 to 5e-5, one 2^20 below with none of its digits.)
 // The pipe's own sums round towards zero, relative to the sum: the large products, which make that sum, are added up in short chains of their own (16 - 64 terms)
 // that ordinary fp32 adds take over, the small ones apart from them, or in front of them (the observation and the remedy are Ootomo and Yokota's, "Recovering
 // single precision accuracy from Tensor Cores", 2022).  Against 64 bits, relative, over eight prompts of 245 to 1 050 tokens: delta rule of 16 heads of
-// 128 x 128, outputs 1.1e-7, state 0.97e-7; 32 heads of 128 x 64 with a decay per token, 0.91e-7 and 0.63e-7.
+// 128 x 128, outputs 1.2e-7, state 0.96e-7; 32 heads of 128 x 64 with a decay per token, 0.97e-7 and 0.63e-7.
 #pragma once
 #include "scan_common.cuh"
 
@@ -124,18 +124,21 @@ constexpr int kMP = kMT + 8;            // row stride of the token-by-token plan
 constexpr int kBuffers = 3, kScanThreads = 512, kPrep0 = 8;       // threads, first preparing warp
 
 // What the chunked recurrences on the tensor pipe have in common.  One CTA of sixteen warps per (sequence, head, 64 value columns), one CTA per SM:
-//   warps 8 .. 15 prepare the chunks of 32 tokens, in two groups that take every other chunk: rows from global memory into planes of bf16 parts in
-//                 shared memory, decays, the token-by-token products
+//   warps 8 .. 15 prepare the chunks of 32 tokens, in two groups that take every other chunk (and the first one together, so that a short portion does
+//                 not wait for its keys behind its queries): rows from global memory into planes of bf16 parts in shared memory, decays, the
+//                 token-by-token products
 //   warps 0 .. 7  carry the state, 16 value columns of one half of the channels each.  It is kept TRANSPOSED in the warp's accumulator registers
 //                 (16 columns x 64 channels: 32 numbers per thread at 128 channels), where it is at once the left operand of its products
 //                 with the chunk's rows and the accumulator of its own update: it never travels.  The two warps of a pair (w, w + 4) add what their halves
 //                 of the channels give to the chunk's rows by way of shared memory.
-// The tensor pipe is what takes the time: 51 - 54 % of all cycles in the mean over the SMs, with some 700 products per SM quarter and chunk, and the warps that
-// wait for it or for one another are the rest.  Over eight prompts of 245 to 1 050 tokens, against four and four warps: delta rule, 16 heads of 128 x 128,
-// 240 -> 222 us; 32 heads of 128 x 64, a decay per token, 154 -> 146.  Not kept: the pair's sums exchanged behind the state's update instead of in front
-// of it (146 -> 150), both warps of a pair solving for the chunk's U instead of one that hands it on (222 -> 232), two buffers instead of three (no change).
-// 128 registers per thread: at 128 channels a few numbers are spilled (8 - 56 bytes loaded per thread); moving registers from the preparing warps to the
-// state's (144 and 112: 277 -> 281 us for the delta rule with its preparation) only moves the spills there.
+// The tensor pipe is what takes the time: half of all cycles in the mean over the SMs, with some 700 products per SM quarter and chunk, and the warps that
+// wait for it or for one another are the rest.  Against four and four warps, whose preparation asks for queries, keys and values at once (us): eight prompts of 245 to
+// 1 050 tokens, delta rule of 16 heads of 128 x 128 238 -> 212, of 8 heads of 64 x 128 158 -> 133; 32 heads of 128 x 64 with a decay per token 152 -> 141; 64
+// portions of 20 tokens 123 -> 116, delta rule 176 -> 178, of 64 x 128 64 -> 73.  Not kept: the pair's sums exchanged behind the state's update instead of in front
+// of it (ssm 146 -> 150), both warps of a pair solving for the chunk's U instead of one that hands it on (delta 222 -> 232), two buffers instead of three at 128
+// channels (no change), queries and keys of every chunk at once (213 -> 223, for want of registers).
+// 128 registers per thread: a few numbers are spilled (8 - 52 bytes loaded per thread); moving registers from the preparing warps to the state's
+// (144 and 112: 277 -> 281 us for the delta rule with its preparation) only moves the spills there.
 // Named barriers: a buffer is filled / free for its next chunk; a group of preparing warps; a pair.  (Of three buffers, chunks i and i + 3 share one but not
 // the group that fills it, so each group waits for a free buffer at barriers of its own: chunk i at kEmpty + i % 6; of two, at kEmpty + i % 4.)
 enum { kFull = 1, kEmpty = kFull + kBuffers, kPrepare = kEmpty + 2 * kBuffers, kPair = kPrepare + 2 };
@@ -189,6 +192,23 @@ struct RowTile {
   }
 };
 
+// 32 rows of up to kMC values into shared memory by a group of preparing warps; they are there behind values_wait() of every thread
+__device__ __forceinline__ void fetch_values(float* dst, const float* src, int64_t ld, int cols, int n, bool vec, int pw, int lane) {
+  using Tile = RowTile<kMC>;
+  if (vec && cols == kMC) {
+#pragma unroll
+    for (int i = 0; i < Tile::kPasses; ++i) {
+      const int r = Tile::row(i, pw, lane), c = 4 * (lane % Tile::kLanes);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * kMV + c)), "l"(src + min(r, n - 1) * ld + c), "r"(r < n ? 16 : 0) : "memory");
+    }
+  } else {
+    Tile v;
+    v.load(src, ld, cols, n, vec, pw, lane);
+    v.store_to(dst, kMV, pw, lane);
+  }
+}
+__device__ __forceinline__ void values_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The sequence of a block when the longest are to start first (one wave of CTAs rarely holds them all): the one with `rank` longer ones.
 // Sequences beyond 256 keep their order.  All threads of the CTA call it; every sequence is compared by two of them.
 struct RankScratch { int len[256], longer[256], found; };
@@ -213,32 +233,48 @@ __device__ __forceinline__ int sequence_of_rank(const int32_t* cu, int B, int ra
   return s.found;
 }
 
-// Token-by-token products: rows x0 .. x0 + 15 of X against rows y0 .. y0 + 15 of Y, two tiles of eight columns; KS blocks of 16 channels,
-// alternately with sums of their own (at most 64 terms each)
+// Token-by-token products: rows x0 .. x0 + 15 of X against rows y0 .. y0 + 15 of Y, two tiles of eight columns; KS blocks of 16 channels, two side by side with
+// sums of their own (at most 32 terms each).  A chain of products on one accumulator waits for each of them, so the two blocks' products alternate: one block behind the other
+// took 3 100 cycles per 16 x 16 tokens of 128 channels.
 template <int KS>
 __device__ __forceinline__ void token_products(float (&out)[2][4], const Planes& X, int x0, const Planes& Y, int y0, int lane) {
-  float x[2][2][4] = {}, rest[2][2][4] = {};
-#pragma unroll 2
-  for (int ks = 0; ks < KS; ks += 2) {
+  constexpr int pa[5] = {2, 0, 1, 1, 0}, pb[5] = {0, 2, 1, 0, 1};
+  float rest[2][2][4] = {};
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      FragA a;
-      FragB b[2];
-      load_a(a, X, x0, (ks + p) * 16, lane);
-      load_b(b, Y, y0, (ks + p) * 16, lane);
-      float y[2][4] = {};
-      mma_high(y, a, b);
-      mma_small(rest[p], a, b);
+  for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int t = 0; t < 2; ++t)
+    for (int i = 0; i < 4; ++i) out[t][i] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[p][t][i] += y[t][i];
+  for (int half = 0; half < 2; ++half) {
+    float x[2][2][4] = {};
+#pragma unroll
+    for (int ks = half * (KS / 2); ks < (half + 1) * (KS / 2); ks += 2) {
+      FragA a[2];
+      FragB b[2][2];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        load_a(a[p], X, x0, (ks + p) * 16, lane);
+        load_b(b[p], Y, y0, (ks + p) * 16, lane);
+      }
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (i == 0) mma_bf16_acc(x[p][t], a[p].r[0], b[p][t].r[0]);
+            else mma_bf16_acc(rest[p][t], a[p].r[pa[i - 1]], b[p][t].r[pb[i - 1]]);
+          }
     }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[t][i] += x[0][t][i] + x[1][t][i];
   }
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) out[t][i] = (x[0][t][i] + x[1][t][i]) + (rest[0][t][i] + rest[1][t][i]);
+    for (int i = 0; i < 4; ++i) out[t][i] += rest[0][t][i] + rest[1][t][i];
 }
 
 // Decays are differences of running sums of log decays over a chunk's tokens, kept in 64 bits and handed on in two parts: sums of 32 tokens reach 30 and
