@@ -16,7 +16,6 @@ import ctypes as C
 import json
 import os
 import sys
-import weakref
 from collections import deque
 from dataclasses import dataclass, field
 from typing import Dict, Iterable, List, Optional, Sequence as Seq, Tuple
@@ -188,7 +187,15 @@ def _p(a: np.ndarray):
 # in use, and goes back to its pool with the array.  Pageable memory, as ever: arrays below 64 KiB or above 32 MiB, all but four at a time - a caller who keeps
 # the logits of many steps must not lock the machine's memory, and the pool holds on to what it once gave - and where no page-locked memory can be had.
 _PINNED_BYTES = range(1 << 16, (1 << 25) + 1)
-_pinned_permits = deque([None] * 4)      # taken and given back in one step each, so safe among threads and in a finalizer
+_pinned_permits = deque([None] * 4)      # taken and given back in one step each, so safe among threads and while memory is collected
+
+
+class _Permit:
+    """Belongs to a page-locked tensor whose memory an array lies in: given back when both are gone."""
+    __slots__ = ()
+
+    def __del__(self, give=_pinned_permits.append):
+        give(None)
 
 
 def _logits_array(rows: int, cols: int) -> np.ndarray:
@@ -199,13 +206,13 @@ def _logits_array(rows: int, cols: int) -> np.ndarray:
         _pinned_permits.pop()
     except IndexError:
         return np.empty((rows, cols), dtype=np.float32)
+    permit = _Permit()
     try:
         out = torch.empty((rows, cols), dtype=torch.float32, device="cpu", pin_memory=True).numpy()
-        weakref.finalize(out, _pinned_permits.append, None).atexit = False
-        return out
     except RuntimeError:                 # no page-locked memory left
-        _pinned_permits.append(None)
         return np.empty((rows, cols), dtype=np.float32)
+    out.base._permit = permit            # the tensor that the array, and every view of it, holds on to
+    return out
 
 
 class Qwen3ModelRunner:
