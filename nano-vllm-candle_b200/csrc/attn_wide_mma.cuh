@@ -335,20 +335,22 @@ __device__ __forceinline__ void merge_store(const Args& a, float* sm_m, const fl
     if constexpr (!kSig)
       for (int c = 0; c < a.splits; ++c) M = fmaxf(M, all_m[c * 16 + rr]);
     float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c0 = 0; c0 < a.splits; c0 += 4) {        // four at a time; a cluster of two asks for its last CTA's numbers again and leaves them out
+    // four at a time; a cluster of two asks for its last CTA's numbers again and takes zeros in their place (not the numbers times 0: an infinity would come out as
+    // a NaN; and no branch, which would put every CTA's factor behind the one before)
+    for (int c0 = 0; c0 < a.splits; c0 += 4) {
       float4 x[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[i] = ld_cluster_f4(ptx::mapa_u32(at, min(c0 + i, a.splits - 1)));
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        if (c0 + i >= a.splits) break;                // (left out, not taken times 0: an infinity would come out as a NaN)
+        const bool in = c0 + i < a.splits;
         float f = 1.f;
         if constexpr (!kSig) {
-          const int e = (c0 + i) * 16 + rr;
-          f = all_m[e] != -INFINITY ? fast_exp2(all_m[e] - M) : 0.f;
+          const int e = min(c0 + i, a.splits - 1) * 16 + rr;
+          f = in && all_m[e] != -INFINITY ? fast_exp2(all_m[e] - M) : 0.f;
           L = fmaf(all_l[e], f, L);
         }
-        fma4_acc(O, x[i], f);
+        fma4_acc(O, in ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f), f);
       }
     }
     finish(rr, d, M, L, O);
