@@ -659,16 +659,21 @@ inline int attn_wide_mma_launch(nvc_ctx* ctx, const void* q, const void* k_cache
   int gx = max_total >= 64 ? std::max((max_total + 63) / 64, 4) : (max_total + 15) / 16;
   if (s.kv_heads > 65535 || B > 65535) return NVC_ENOTIMPL;
   const bool shared = k_cache == v_cache && ldk == ldv && s.vdim <= s.dim && (s.kv_heads == 1 || s.vdim == s.dim);
-  // few rows and few CTAs: clusters of up to 8 (16 for decode over shared rows) share the keys of a chunk, as long as a CTA keeps at least
-  // 64 of them, a tile per warp (1 sequence of 700, latent rows: 14.3 -> 12.3 us against 128 of them; 8 x 8 heads, window of 256: 16.4 -> 14.4).  Up to three CTAs
-  // per SM; clusters of two and four over shared rows up to four, which is what an SM holds of them (64 sequences of 24 heads 24.6 -> 20.5; clusters of eight lose
-  // there: 36 of 24 heads 18.4 -> 21.7)
+  // few rows and few CTAs: clusters of up to 8 (16 for decode over shared rows) share the keys of a chunk.  A merge costs 1 - 1.5 us and more in wide clusters, so
+  // keys are shared from 256 of them on, as long as a CTA of the next width keeps 64 (over shared rows 96, in clusters of sixteen 128) of them.  Up to three CTAs
+  // per SM; clusters of two and four over shared rows up to four, which is what an SM holds of them.  416 measured shapes, 1 to 64 sequences
+  // (profiles/decode_cluster_splits.txt): 0.5 % over the best width for each in the mean over shared rows, 3 % over separate ones; against twice as many
+  // keys per CTA everywhere 10 - 13 % less where the two differ, against half as many 9 - 15 % (16 sequences of 200 - 1 500, 8 heads over shared rows: 6.6 us in
+  // clusters of eight, 9.0 in clusters of sixteen; 1 of 100, 8 heads of 64: 5.7 alone, 6.8 in a cluster of two).
   int splits = 1;
   const bool shared_decode = attn_shared_decode_takes(s, shared, cu_seqlens, block_size);
   if (max_total < 64) {
     const int64_t keys = s.window > 0 ? s.window : (s.chunk > 0 ? s.chunk : (int64_t)bt_stride * block_size);
-    while (splits < (shared_decode ? 16 : 8) && (int64_t)gx * B * s.kv_heads * splits * 2 <= (shared_decode && splits < 4 ? 4 : 3) * ctx->num_sms && keys >= 128 * splits)
-      splits *= 2;
+    for (int next = 2; next <= (shared_decode ? 16 : 8); next *= 2) {
+      const int64_t per_cta = shared_decode ? (next == 16 ? 128 : 96) : 64;
+      if ((int64_t)gx * B * s.kv_heads * next > (shared_decode && next <= 4 ? 4 : 3) * ctx->num_sms || keys < std::max<int64_t>(256, per_cta * next)) break;
+      splits = next;
+    }
     gx *= splits;
   }
   widemma::Args a{reinterpret_cast<const nvc_bf16*>(q), reinterpret_cast<const nvc_bf16*>(k_cache), reinterpret_cast<const nvc_bf16*>(v_cache),
