@@ -98,7 +98,7 @@ struct Walk {
   int step;                // to the one behind it
   bool listed;
   __device__ __forceinline__ void start(const int32_t* cu, const Sched& sc, int lane) {
-    listed = sc.B <= kListed;
+    listed = sc.B <= kListed && sc.num_items > (int)gridDim.x;      // one item per CTA needs no list, and no second latency in front of it
     level = sc.QT - 1;
     at = blockIdx.x;
     step = 2 * (int)(gridDim.x - blockIdx.x) - 1;
