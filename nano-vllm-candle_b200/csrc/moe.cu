@@ -275,12 +275,12 @@ __global__ void gather_rows_kernel(const uint4* in, int ld_in, const int32_t* sr
 }
 
 // The same for rows of 512 numbers and more: a warp per row, four accesses per lane in flight, no division (10 000 x 1 024, cold cache: 8.5 -> 7.0 us)
-__global__ void __launch_bounds__(256) gather_rows_warp_kernel(const uint4* in, int ld_in, const int32_t* src_rows,
+__global__ void __launch_bounds__(128) gather_rows_warp_kernel(const uint4* in, int ld_in, const int32_t* src_rows,
                                                                const int32_t* num_rows, uint4* out, int ld_out, int rows_cap, int per_row,
                                                                int fill, uint32_t two) {
   pdl_trigger();
   pdl_wait();
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const bool behind = r >= min(rows_cap, *num_rows);
   if (r >= rows_cap || (behind && !fill)) return;
   const int src = behind ? -1 : src_rows[r];
@@ -464,7 +464,7 @@ static int gather(nvc_ctx* ctx, const nvc_bf16* in, int ld_in, const int32_t* sr
   if (rows_cap == 0) return NVC_OK;
   const int per_row = width / 8;                                   // 16-byte chunks per row
   if (per_row >= 64) {
-    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, gather_rows_warp_kernel, dim3((rows_cap + 7) / 8), dim3(256), 0, nvc_stream(stream), reinterpret_cast<const uint4*>(in),
+    NVC_CUDA_CHECK(ctx, nvc_launch(ctx, gather_rows_warp_kernel, dim3((rows_cap + 3) / 4), dim3(128), 0, nvc_stream(stream), reinterpret_cast<const uint4*>(in),
                                    ld_in / 8, src_rows, num_rows, reinterpret_cast<uint4*>(out), ld_out / 8, rows_cap, per_row, fill, (uint32_t)value * 0x10001u));
     ctx->launches++;
     return NVC_OK;
