@@ -98,7 +98,8 @@ struct Walk {
   int step;                // to the one behind it
   bool listed;
   __device__ __forceinline__ void start(const int32_t* cu, const Sched& sc, int lane) {
-    listed = sc.B <= kListed && sc.num_items > (int)gridDim.x;      // one item per CTA needs no list, and no second latency in front of it
+    // one item per CTA needs no list, and no second latency in front of it; a list counts up to 65 535 tiles of a sequence
+    listed = sc.B <= kListed && sc.num_items > (int)gridDim.x && sc.QT <= 0xffff;
     level = sc.QT - 1;
     at = blockIdx.x;
     step = 2 * (int)(gridDim.x - blockIdx.x) - 1;
@@ -111,7 +112,7 @@ struct Walk {
   // the whole warp calls it
   __device__ __forceinline__ bool next(Item& x, const Sched& sc) {
     if (!listed) {
-      if (at >= sc.num_items) return false;
+      if ((uint32_t)at >= (uint32_t)sc.num_items) return false;       // (unsigned: the step behind one of 2^31 - 1 items)
       x = item_of(at, sc);
       at += step;
       step = 2 * (int)gridDim.x - step;
