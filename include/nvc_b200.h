@@ -525,7 +525,8 @@ int nvc_rms_norm_sandwich(nvc_ctx* ctx, const float* res_in, const float* y, con
  *   [ rmsnorm(in[n, off1 : off1 + n1]) * w1 | rot(in[n, off1 + n1 : off1 + n1 + rot_dim]) ]
  * where rot turns the first rot_dims numbers of the part by the angles of positions[n] ((cos, sin) table of
  * nvc_rotary_table_init_sync; pairs (2i, 2i + 1), or (i, i + rot_dims / 2) when rot_half) and leaves the rest.  cache == NULL:
- * only the query latent (a layer that reads another layer's rows). */
+ * only the query latent (a layer that reads another layer's rows).  slot_mapping, positions, weights and table are static operands (launch order, above):
+ * rows that allow 16-byte accesses are prepared by a kernel that reads them in front of its wait. */
 int nvc_latent_norm_store_rot(nvc_ctx* ctx, const float* in, int ldi, int n0, int off1, int n1, const float* w0, const float* w1,
                               float eps, void* out0, int ld0, void* cache, int ldc, const int32_t* slot_mapping, int rot_dim,
                               int rot_dims, int rot_half, const float* rot_table, const int32_t* positions, int dtype, int N,

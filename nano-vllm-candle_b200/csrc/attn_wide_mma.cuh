@@ -663,8 +663,8 @@ inline int attn_wide_mma_launch(nvc_ctx* ctx, const void* q, const void* k_cache
   // keys are shared from 256 of them on, as long as a CTA of the next width keeps 64 (over shared rows 96, in clusters of sixteen 128) of them.  Up to three CTAs
   // per SM; clusters of two and four over shared rows up to four, which is what an SM holds of them.  416 measured shapes, 1 to 64 sequences
   // (profiles/decode_cluster_splits.txt): 0.5 % over the best width for each in the mean over shared rows, 3 % over separate ones; against twice as many
-  // keys per CTA everywhere 10 - 13 % less where the two differ, against half as many 9 - 15 % (16 sequences of 200 - 1 500, 8 heads over shared rows: 6.6 us in
-  // clusters of eight, 9.0 in clusters of sixteen; 1 of 100, 8 heads of 64: 5.7 alone, 6.8 in a cluster of two).
+  // keys per CTA everywhere 10 - 13 % less where the two differ, against half as many 9 - 15 % (16 sequences of 200 - 1 500, 8 heads over shared rows: 6.1 us in
+  // clusters of eight, 8.4 in clusters of sixteen; 1 of 100, 8 heads of 64: 5.9 alone, 6.8 in a cluster of two).
   int splits = 1;
   const bool shared_decode = attn_shared_decode_takes(s, shared, cu_seqlens, block_size);
   if (max_total < 64) {

@@ -657,7 +657,9 @@ static void choose_schedule(const nvc_ctx* ctx, int M, int N, int kb, bool gated
   // a whole one.  Narrower tiles, or more splits, fill it (us, 256-wide / the choice: 512 x 4 096 x 1 024 11.2 / 8.5, 700 x 1 024 x 2 048 10.9 / 9.2,
   // 1 300 x 2 048 x 6 144 36.7 / 29.1, 2 100 x 1 024 x 3 072 19.5 / 15.7, 2 600 x 4 096 x 12 288 227 / 196, 6 555 x 1 024 x 2 048 25.7 / 23.1; gated
   // 512 x 12 288 x 2 048 27.1 / 23.9).  The model, in us, is fitted to 1 750 configurations of 13 shapes (residual 7 %: so a choice has to promise 7 %), for 1 to 4 waves;
-  // beyond, quantisation is lost in the power cap's noise.  Against 256-wide tiles it gains 6.5 % in the mean over these shapes; the best of all widths 8.8 %.
+  // beyond, quantisation is lost in the power cap's noise.  Against 256-wide tiles it gains 6.7 % in the mean over 195 products of these shapes, at most
+  // 30 and never loses; the best of all widths gains 8.5 % (profiles/gemm_pair_prefill_widths.txt).  Another split regroups a product's sums: results of 257 rows and
+  // more differ from those of 256-wide tiles by their rounding, and may differ between batches of different sizes, as they did among 256-wide tiles.
   if (wide) return;
   auto waves_of = [&](int nt, int S) { return ceil((double)(m_tiles * ((N + nt - 1) / nt)) / avail(S)); };
   auto model = [&](int nt, int S) {

@@ -91,8 +91,8 @@ __device__ __forceinline__ float4 scale4(const float4& x, float r, const float4&
 __device__ __forceinline__ float dot4(const float4& x) { return x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w; }
 
 // The same where the rows allow 16-byte accesses, n0 <= 128 V and latent and rotated part fit in 128 numbers: a warp requests all of its row at once, keeps
-// it in registers, and finds weights, slot and angles already there.  The general kernel reads the row twice, number by number, and the slot, the second part
-// and the angles one behind the other: 64 rows of 512 + 96 + 32 took 4.4 us, here 2.9; 2 400 rows 6.5, here 3.3.
+// it in registers, and finds weights, slot and angles (static operands) already there.  The general kernel reads the row twice, number by number, and the slot, the
+// second part and the angles one behind the other: 64 rows of 512 + 96 + 32 took 4.5 us, here 2.1; 2 400 rows of 512 + 112 + 16 5.9, here 3.0 (calls in a row).
 template <typename T, int V>
 __global__ void __launch_bounds__(128) latent_norm_store_row_kernel(const float* in, int ldi, int n0, int off1, int n1, const float* __restrict__ w0,
                                                                     const float* __restrict__ w1, float eps, T* out0, int ld0, T* cache,

@@ -597,7 +597,8 @@ prefill_attn_v2_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
       const float inv = kMode == kSigmoid ? 1.0f : (kMode == kGated ? pk.out_scale / l : 1.0f / l);
       if (gate) {
         // With a gate (fp32 rows): 32 columns of the warp's rows at a time through its staging buffer as fp32, so that 8 lanes per row read the gate and write the
-        // result, 128 and 64 contiguous bytes.  A thread reading its own row's gate touched 32 lines per instruction: 12 000 cycles per item, of 25 000.
+        // result, 128 and 64 contiguous bytes.  A thread reading its own row's gate touched 32 lines per instruction: 12 000 cycles per item, of 25 000.  (The mode
+        // with windows and gates spills 8 bytes per thread at its 168 registers, 48 read back.)
         uint8_t* buf = gen + kOffStage + quad * 4096;
         nvc_bf16* op = out + (int64_t)ge.seq_start * ldo + x.h * 128 + q4 * 4;
 #pragma unroll 1
