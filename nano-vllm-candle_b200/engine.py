@@ -488,6 +488,7 @@ class ModelRunner(Qwen3ModelRunner):
         check(self.l.nvc_runner_set_state_slots(self.handle, _p(a), len(a)), "nvc_runner_set_state_slots", self.ctx.h)
 
     def last_logits(self, B: int) -> np.ndarray:
+        """As Qwen3ModelRunner.last_logits: the caller's own array, page-locked for up to four that live at a time."""
         out = _logits_array(B, self.vocab_size // self.ctx.tp_size)
         check(self.l.nvc_runner_last_logits(self.handle, _p(out), B), "nvc_runner_last_logits", self.ctx.h)
         return out

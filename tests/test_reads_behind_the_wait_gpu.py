@@ -39,6 +39,23 @@ def test_latent_rows_behind_a_gather(ctx, ops, N):
     chain(step)
 
 
+@pytest.mark.parametrize("pad", [0, 1])                 # rows that allow 16-byte accesses, and rows that do not
+def test_latent_rows_with_slots_of_the_moment(ctx, ops, pad):
+    """Slots and positions are static operands: another library's kernel may write them right in front of the call, which plain stream order covers."""
+    N = 300
+    table, ids = torch.randn(500, 640 + pad, device=DEV), torch.randint(0, 500, (40, N), device=DEV, dtype=torch.int32)
+    w0, w1, tab = torch.randn(512, device=DEV), torch.randn(96, device=DEV), ops.rotary_table(ctx, 10000.0, 32, 1024)
+    slots, pos = torch.arange(N, device=DEV, dtype=torch.int32), torch.zeros(N, device=DEV, dtype=torch.int32)
+
+    def step(i):
+        cache = torch.zeros(2 * N, 128, device=DEV, dtype=torch.bfloat16)
+        x = ops.embed_gather_f32(ctx, ids[i], table)
+        slots.copy_((torch.arange(N, device=DEV, dtype=torch.int32) * 7 + 11 * i) % (2 * N - 1))
+        pos.copy_(slots + i)
+        return ops.latent_norm_store_rot(ctx, x, 512, 512, 96, w0, w1, 1e-6, cache, slots, 32, 32, True, tab, pos, torch.bfloat16), cache
+    chain(step)
+
+
 @pytest.mark.parametrize("N", [64, 3000])
 def test_gates_behind_a_gather(ctx, ops, N):
     table = torch.randn(500, 2048, device=DEV)
