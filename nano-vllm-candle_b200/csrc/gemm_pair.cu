@@ -10,7 +10,7 @@
 // cycles (64 B/clk) against 48 KB (96 B/clk) for the 1-CTA 128 x 256 tile.
 //
 // Two schedules share the kernel:
-//  * S = 1, persistent: min(tiles, #pairs) clusters of 2 walk the tiles (n fastest); two
+//  * S = 1, persistent: min(tiles, #pairs) clusters of 2 walk the tiles (column tiles fastest, or bands of row tiles: see launch_pair); two
 //    256-column accumulators in tensor memory (all 512 columns) so the epilogue of tile i
 //    overlaps the main loop of tile i+1.
 //  * S > 1, split-K inside a cluster of 2S CTAs (decode, M <= 256: too few tiles to fill 148
@@ -184,12 +184,18 @@ __device__ __forceinline__ void pair_reduce(const float4* __restrict__ ws_cluste
   }
 }
 
+// Tile number -> row tile, column tile: bands of `band` row tiles, the row tiles of a band fastest (band 1: column tiles fastest).
+__device__ __forceinline__ int2 tile_at(int tile, int m_tiles, int n_tiles, int band) {
+  const int b = tile / (band * n_tiles), rest = tile - b * band * n_tiles, rows = min(band, m_tiles - b * band), n = rest / rows;
+  return make_int2(b * band + rest - n * rows, n);
+}
+
 // kClamp: the variant with the clamped gated epilogue
 template <int NT, bool kClamp = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total, int kb_per_split,
-                 int num_tiles, int n_tiles, int prefetch_w, int epi, float4* __restrict__ ws,
+                 int num_tiles, int n_tiles, int band, int prefetch_w, int epi, float4* __restrict__ ws,
                  long long* __restrict__ trace, const QkEpi qk) {
   using cfg = PairCfg<NT>;
   constexpr int kStages = cfg::kStages;
@@ -221,6 +227,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const uint16_t pair_mask = (uint16_t)(3u << leader_rank);
   const int cluster_id = blockIdx.x / csize;
   const int num_clusters = gridDim.x / csize;
+  const int m_tiles = num_tiles / n_tiles;
   const int kb_begin = p * kb_per_split;
   const int num_kb = min(kb_per_split, k_blocks_total - kb_begin);
 
@@ -256,7 +263,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   constexpr int kPrefetchKb = 16;
   if (warp == 0 && prefetch_w && cluster_id < num_tiles) {
     if (ptx::elect_one()) {
-      const int n_tile = cluster_id % n_tiles;
+      const int n_tile = tile_at(cluster_id, m_tiles, n_tiles, band).y;
       const int n = min(num_kb, kPrefetchKb);
       for (int kb = 0; kb < n; ++kb) {
 #pragma unroll
@@ -276,7 +283,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t leader_full0 = ptx::mapa_u32(full_bar(0), leader_rank);
     uint32_t it = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
-      const int m_tile = tile / n_tiles, n_tile = tile - m_tile * n_tiles;
+      const int2 at = tile_at(tile, m_tiles, n_tiles, band);
+      const int m_tile = at.x, n_tile = at.y;
       const int a_row = m_tile * kTileM + h * kHalf;
       const int b_row = n_tile * NT + h * cfg::kBoxRowsB;
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
@@ -346,7 +354,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t leader_tmem_empty0 = ptx::mapa_u32(tmem_empty_bar(0), leader_rank);
     int ti = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters, ++ti) {
-      const int m_tile = tile / n_tiles, n_tile = tile - m_tile * n_tiles;
+      const int2 at = tile_at(tile, m_tiles, n_tiles, band);
+      const int m_tile = at.x, n_tile = at.y;
       const int acc = ti & 1, use = ti >> 1;
       const int grow = m_tile * kTileM + h * kHalf + r;
       const bool row_ok = grow < M;
@@ -478,7 +487,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if (S > 1) {
     // ------------------------------------------------------------ split-K exchange (one tile per cluster)
     const int tile = cluster_id;
-    const int m_tile = tile / n_tiles, n_tile = tile - m_tile * n_tiles;
+    const int2 at = tile_at(tile, m_tiles, n_tiles, band);
+    const int m_tile = at.x, n_tile = at.y;
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -554,6 +564,17 @@ int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, voi
     const int waves = (tiles + avail - 1) / avail;
     clusters = (tiles + waves - 1) / waves;
   }
+  // Bands of row tiles.  Column tiles fastest, every row of tiles streams all weights: nothing while L2 holds them, but 3 977 x 24 576 x 4 096 reads its 201 MB
+  // 16 times, 4 TB/s beside the tensor cores under one power cap.  Weights of more than 32 MB are walked in bands whose activations take at most 48 MB
+  // of L2, 16 row tiles at most (sustained, new operands per call, us, column tiles fastest / bands of 4 / 8 / 16: 3 977 x 24 576 x 4 096 804 / 609 / 587 / 578,
+  // 1 300 x 24 576 x 4 096 293 / 235 / 222 / 224, 8 192 x 8 192 x 8 192 924 / 852 / 833 / 846, 1 300 x 4 096 x 12 288 134 / 131 / 126 / 127,
+  // 4 200 x 6 144 x 4 096 175 / 172 / 171 / 169; weights that fit gain nothing: 16 000 x 6 144 x 1 024 158.9 / 159.7 / 159.6 / 159.3)
+  int band = 1;
+  if ((int64_t)N * K * 2 > (32 << 20)) {
+    const int64_t most = (48 << 20) / ((int64_t)kTileM * K * 2);
+    band = (int)(most < 1 ? 1 : (most > 16 ? 16 : most));
+    band = (m_tiles + (m_tiles + band - 1) / band - 1) / ((m_tiles + band - 1) / band);    // bands of equal height
+  }
   dim3 grid(clusters * 2 * S);
   // L2 prefetch of the first weight k-blocks before the dependency wait + 16 k-blocks ahead of the ring: pays for short,
   // latency-bound k-loops (decode at K <= 3072: 1 - 3 %), costs 4 - 9 % on the long ones (Qwen3-8B at batch 256, K >= 4096:
@@ -562,7 +583,7 @@ int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, voi
   const int prefetch_w = (M <= kTileM && kb_total <= 48) ? 1 : 0;
   auto* kernel = nvc_epi_glu_clamp(epi) ? gemm_pair_kernel<NT, true> : gemm_pair_kernel<NT>;
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes, stream, 2 * S,
-                                         ta, tb, C, ldc, out_f32, M, N, kb_total, kb_per, tiles, n_tiles,
+                                         ta, tb, C, ldc, out_f32, M, N, kb_total, kb_per, tiles, n_tiles, band,
                                          prefetch_w, epi, reinterpret_cast<float4*>(ctx->gemm_ws), trace,
                                          qk));
   NVC_CUDA_CHECK(ctx, cudaGetLastError());

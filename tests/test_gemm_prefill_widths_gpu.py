@@ -51,3 +51,19 @@ def test_every_width_with_every_split(ctx, M, N, K, NT, S):
     want = torch.nn.functional.silu(z[:, :N // 32 * 16]) * z[:, N // 32 * 16:]
     got = ctx.gemm_silu_mul(a, ctx.interleave_gate_up(gu), **forced)
     assert float(((got.float() - want).abs() - 2.0 ** -8 * want.abs()).max()) <= 1e-4 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 17424, 1024), (1100, 16400, 1024), (4400, 16400, 1024), (2100, 1552, 12288), (600, 256, 65600), (515, 4112, 4160)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_bands_of_row_tiles(ctx, M, N, K, f32):
+    """Weights above 32 MB are walked in bands of row tiles: the same sums as the same weights in pieces below it, bit by bit."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a = torch.randn(M, K, generator=g, device=DEV).to(BF16)
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).to(BF16)
+    dt = torch.float32 if f32 else BF16
+    cut = N // 32 * 16
+    assert N * K * 2 > 32 << 20 >= (N - cut) * K * 2 >= cut * K * 2
+    out = torch.full((M + 1, N), 7.0, device=DEV, dtype=dt)
+    ctx.gemm(a, w, out_dtype=dt, out=out[:M], force_bn=512, force_splits=1)
+    pieces = torch.cat([ctx.gemm(a, p.contiguous(), out_dtype=dt, force_bn=512, force_splits=1) for p in (w[:cut], w[cut:])], 1)
+    assert torch.equal(out[:M], pieces) and bool((out[M] == 7.0).all())
