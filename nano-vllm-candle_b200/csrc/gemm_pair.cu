@@ -19,8 +19,8 @@
 //    publishes the 16-column chunks it does not own; CTA (p, h) sums chunk c, c % S == p, in
 //    split order 0..S-1: deterministic, no atomics).  Distributed shared memory was measured
 //    first and is too slow for 128 KB partial tiles (~17 B/clk per SM).
-// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer (leader
-// only), warps 2-5 epilogue (tcgen05.ld -> bf16/f32 -> 16-byte stores).
+// Roles per CTA (192 or 320 threads): warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer (leader
+// only), warps 2-5 or 2-9 epilogue (tcgen05.ld -> bf16/f32 -> 16-byte stores).
 #include "common.cuh"
 #include "ptx.cuh"
 #include "internal.h"
@@ -34,7 +34,12 @@ extern int g_nvc_debug[8];
 namespace {
 
 constexpr int kTileM = 256, kHalf = 128, BK = 64;
-constexpr int kThreads = 192;
+// What a kernel's epilogue does: bf16 or fp32 rows, as they are or through an element-wise unit; rows through a gated unit (clamped, silu, tanh-gelu: known to the compiler,
+// where one branch more between them costs the loop 13 %); norm and rotation of query and key heads; fp32 rows of a product with its operands swapped.
+// The last two read the accumulators with eight warps, four for either half of the columns, the others with four: where the k-loop is short the epilogue is what a tile
+// takes (one warp per quadrant / two, us: heads of 128, 9 000 x 4 096 x 1 024 90 / 72, 6 555 rows 68 / 58; 100 x 151 936 x 1 024 swapped 82 / 74), but rows
+// through a staging buffer are done behind the next tile's main loop and four more warps only cost (300 x 4 096 x 1 024 14.4 / 16.4, 4 000 x 12 288 x 2 048 gated 125 / 127).
+enum Mode { kRows, kClampedRows, kSilu, kGelu, kHeads, kSwapped };
 constexpr int kBytesA = kHalf * BK * 2;            // 16 KB: this CTA's 128 rows of the activation tile
 constexpr int kTmemCols = 512;
 constexpr int kRingBudget = 200 * 1024;
@@ -44,7 +49,7 @@ constexpr int kRingBudget = 200 * 1024;
 // smaller tiles when 256-wide ones quantise badly onto the 74 pairs (96 tiles = two waves of which the second is 30 %
 // full; 128 tiles of 192 = two full waves of 3/4 the work each).  (Wide tiles, NT in (256, 512] as two MMAs per k-step
 // into one accumulator stage, measured no gain - 8B gate_up at batch 256: 53.1 vs 53.6 us - and are gone.)
-template <int NT>
+template <int NT, int kMode = kRows>
 struct PairCfg {
   static_assert(NT == 64 || (NT >= 128 && NT <= 256 && NT % 32 == 0), "tile width");
   static constexpr int NH = NT;                          // N of one tcgen05.mma
@@ -52,16 +57,19 @@ struct PairCfg {
   static constexpr int kBytesB = (NT / 2) * BK * 2;      // this CTA's rows of the weight tile per k-block
   static constexpr int kStageBytes = kBytesA + kBytesB;
   // NT = 64 is the swapped-operand lm_head (NVC_EPI_TRANSPOSE): 20 KB stages, a deeper ring keeps as many bytes in flight
-  static constexpr int kMaxStages = NT == 64 ? 10 : 6;
+  static constexpr int kMaxStages = NT == 64 ? 10 : (kMode == kHeads ? 5 : 6);
+  static constexpr int kSides = kMode >= kHeads ? 2 : 1;   // warps per quadrant of tensor memory in the epilogue
+  static constexpr int kThreads = 64 + 128 * kSides;       // TMA, MMA, epilogue
   static constexpr int kStages = kRingBudget / kStageBytes < kMaxStages ? kRingBudget / kStageBytes : kMaxStages;
   static constexpr int kAccStages = 2;
   static constexpr int kNumBars = 2 * kStages + 4;       // full[], empty[], tmem_full[2], tmem_empty[2]
-  static constexpr int kOffStage = (kStages * kStageBytes + kNumBars * 8 + 16 + 127) & ~127;   // 4 epilogue warps x row staging
-  // 4 KB per warp (32 rows x 128 B, RowStage); 8 KB for 256-wide tiles, whose QK-norm epilogue parks whole heads (32 rows x 256 B)
-  static constexpr int kStageBuf = NT == 256 ? 8192 : 4096;
-  static constexpr int kSmemBytes = kOffStage + 4 * kStageBuf + 1024;
+  static constexpr int kOffStage = (kStages * kStageBytes + kNumBars * 8 + 16 + 127) & ~127;   // epilogue warps x row staging
+  // 4 KB per warp (32 rows x 128 B, RowStage); 8 KB where the QK-norm epilogue parks whole heads (32 rows x 256 B)
+  static constexpr int kStageBuf = kMode == kSwapped ? 0 : (kMode == kHeads ? 8192 : 4096);
+  static constexpr int kSmemBytes = kOffStage + 4 * kSides * kStageBuf + 1024;
   static_assert(kSmemBytes <= 232448, "shared memory per CTA");
   static constexpr int kChunks = NT / 16;                // 16-column accumulator chunks of a tile
+  static constexpr int kUnits = NT / 32, kSplit = (kUnits + kSides - 1) / kSides;      // units of 32 columns; the first four epilogue warps take those in front of kSplit
   static constexpr int kPartF4 = kChunks * 4 * kHalf;    // float4s of one CTA's partial tile in the split-K workspace
   static_assert(kStageBytes % 1024 == 0 && (kBoxRowsB % 8) == 0, "swizzle atoms");
   // tensor-memory column of accumulator chunk c (accumulator stage 0)
@@ -114,7 +122,7 @@ template <int NT, int S>
 __device__ __forceinline__ void pair_publish(float4* __restrict__ my_ws, uint32_t taddr, int p, int r) {
   using cfg = PairCfg<NT>;
 #pragma unroll 1
-  for (int u = 0; u < cfg::kChunks / 2; ++u) {
+  for (int u = 0; u < cfg::kUnits; ++u) {
     if (u % S == p) continue;           // my units stay in tensor memory
     uint32_t v[32];
     ptx::tmem_ld_32x32b_x16(taddr + cfg::chunk_col(2 * u), v);
@@ -130,9 +138,9 @@ __device__ __forceinline__ void pair_publish(float4* __restrict__ my_ws, uint32_
 template <int NT, int S, bool kClamp>
 __device__ __forceinline__ void pair_reduce(const float4* __restrict__ ws_cluster, uint32_t taddr, int p, int h, int r,
                                             void* __restrict__ C, int out_f32, int epi, int64_t ldc, int row0, int M,
-                                            int n_base, int N, uint8_t* stage_buf) {
+                                            int n_base, int N) {
   using cfg = PairCfg<NT>;
-  constexpr int kUnits = cfg::kChunks / 2;
+  constexpr int kUnits = cfg::kUnits;
   // G units per batch: 16-24 independent 16-byte L2 loads in flight per thread (one round trip per batch)
   constexpr int G = S == 2 ? 3 : 1;
   constexpr int kOwnedMax = (kUnits + S - 1) / S;
@@ -190,14 +198,16 @@ __device__ __forceinline__ int2 tile_at(int tile, int m_tiles, int n_tiles, int 
   return make_int2(b * band + rest - n * rows, n);
 }
 
-// kClamp: the variant with the clamped gated epilogue
-template <int NT, bool kClamp = false>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int NT, int kMode = kRows>
+__global__ void __launch_bounds__((PairCfg<NT, kMode>::kThreads), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total, int kb_per_split,
-                 int num_tiles, int n_tiles, int band, int prefetch_w, int epi, float4* __restrict__ ws,
+                 int num_tiles, int n_tiles, int band, int prefetch_w, int epilogue, float4* __restrict__ ws,
                  long long* __restrict__ trace, const QkEpi qk) {
-  using cfg = PairCfg<NT>;
+  using cfg = PairCfg<NT, kMode>;
+  constexpr bool kClamp = kMode == kClampedRows;
+  const int epi = kMode == kSilu ? NVC_EPI_SILU_MUL : (kMode == kGelu ? NVC_EPI_GELU_TANH_MUL : epilogue);
+  if (kMode == kRows) __builtin_assume(epi != NVC_EPI_SILU_MUL && epi != NVC_EPI_GELU_TANH_MUL);
   constexpr int kStages = cfg::kStages;
   constexpr int kStageBytes = cfg::kStageBytes;
   // optional phase timestamps of CTA 0 (tools/gemm_microbench.py); NULL in production
@@ -243,7 +253,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       for (int a = 0; a < 2; ++a) {
         ptx::mbar_init(tmem_full_bar(a), 1);    // leader's commit after the last k-block of a tile (multicast)
-        ptx::mbar_init(tmem_empty_bar(a), 8);   // 4 epilogue warps x 2 CTAs, on the leader's barrier
+        ptx::mbar_init(tmem_empty_bar(a), 8 * cfg::kSides);   // epilogue warps x 2 CTAs, on the leader's barrier
       }
       ptx::fence_barrier_init();
     }
@@ -350,6 +360,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     // ------------------------------------------------------------ epilogue, persistent schedule
     const int q = warp & 3;                 // TMEM lane quadrant this warp may access
     const int r = q * 32 + lane;
+    const int side = cfg::kSides == 1 ? 0 : (warp - 2) >> 2;       // which columns of the tile
+    const int u0 = side ? cfg::kSplit : 0, u1 = side ? cfg::kUnits : cfg::kSplit;
+    uint8_t* stage_buf = smem_gen + cfg::kOffStage + (warp - 2) * cfg::kStageBuf;
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t leader_tmem_empty0 = ptx::mapa_u32(tmem_empty_bar(0), leader_rank);
     int ti = 0;
@@ -363,27 +376,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       ptx::tcgen05_fence_after();
       if (tr && threadIdx.x == 64 && ti == 0) trace[81] = clock64();
       if (tr && threadIdx.x == 64 && tile + num_clusters >= num_tiles) trace[86] = clock64();   // last tile: exposed epilogue
-      if constexpr (NT == 256) {
-        if (epi == NVC_EPI_QK_NORM_ROPE) {
-          // ---- K2 as the epilogue of the QKV projection: two heads of 128 columns per tile
+      if constexpr (kMode == kHeads) {
+        {
+          // ---- K2 as the epilogue of the QKV projection: two heads of 128 columns per tile, one for either four warps
           const int row_base = m_tile * kTileM + h * kHalf + q * 32;            // first row of this warp
-          const uint32_t stage = smem_u32(smem_gen + cfg::kOffStage + q * cfg::kStageBuf);   // [32 rows][16 chunks of 16 B], chunk ^= row & 7
+          const uint32_t stage = smem_u32(stage_buf);   // [32 rows][16 chunks of 16 B], chunk ^= row & 7
           const int l = lane & 7, sub = lane >> 3;
           const unsigned mask8 = 0xffu << (lane & 24);
           const int my_row = row_base + lane;
           const int pos_lane = my_row < M ? __ldg(qk.positions + my_row) : 0;
           const int slot_lane = (my_row < M && qk.slot_mapping != nullptr) ? __ldg(qk.slot_mapping + my_row) : -1;
           nvc_bf16* Cb = reinterpret_cast<nvc_bf16*>(C);
-#pragma unroll 1
-          for (int hh = 0; hh < 2; ++hh) {
-            const int head = n_tile * 2 + hh;                                   // head index in the fused [q | k | v] row
-            if (head * 128 >= N) break;
+          const int head = n_tile * 2 + side;                                   // head index in the fused [q | k | v] row
+          if (head * 128 < N) {
             // park the head's 128 accumulator columns as bf16 (what the plain epilogue would have stored)
 #pragma unroll 1
             for (int c4 = 0; c4 < 4; ++c4) {
               uint32_t v[32];
-              ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256 + hh * 128 + c4 * 32), v);
-              ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256 + hh * 128 + c4 * 32 + 16), v + 16);
+              ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256 + side * 128 + c4 * 32), v);
+              ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256 + side * 128 + c4 * 32 + 16), v + 16);
               ptx::tmem_ld_wait();
               float f[32];
 #pragma unroll
@@ -432,7 +443,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 }
               }
             }
-            __syncwarp();                       // the staging buffer is reused by the next head
+            __syncwarp();                       // the staging buffer is reused by the next tile
           }
           ptx::tcgen05_fence_before();
           __syncwarp();
@@ -440,12 +451,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           continue;
         }
       }
-      if (epi == NVC_EPI_TRANSPOSE) {
+      if constexpr (kMode == kSwapped) {
         // accumulator row `grow` (a weight row) is column `grow` of the fp32 C; the warp's 32 rows are 128 contiguous bytes of
         // every C row (token) they touch
         float* Ct = reinterpret_cast<float*>(C) + grow;
 #pragma unroll 1
-        for (int c = 0; c < cfg::kChunks; c += 2) {
+        for (int c = 2 * u0; c < 2 * u1; c += 2) {
           uint32_t v[32];
           ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256) + cfg::chunk_col(c), v);
           ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256) + cfg::chunk_col(c + 1), v + 16);
@@ -462,10 +473,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (lane == 0) mbar_arrive_cluster(leader_tmem_empty0 + 8u * acc);
         continue;
       }
-      RowStage st = make_row_stage<kClamp>(smem_gen + cfg::kOffStage + q * cfg::kStageBuf, C, out_f32, epi, ldc,
-                                   m_tile * kTileM + h * kHalf + q * 32, M, n_tile * NT, NT, N);
+      RowStage st = make_row_stage<kClamp>(stage_buf, C, out_f32, epi, ldc,
+                                   m_tile * kTileM + h * kHalf + q * 32, M, n_tile * NT + u0 * 32, (u1 - u0) * 32, N);
 #pragma unroll 1
-      for (int c = 0; c < cfg::kChunks; c += 2) {       // two 16-column chunks per tensor-memory round trip
+      for (int c = 2 * u0; c < 2 * u1; c += 2) {       // two 16-column chunks per tensor-memory round trip
         uint32_t v[32];
         ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256) + cfg::chunk_col(c), v);
         ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)(acc * 256) + cfg::chunk_col(c + 1), v + 16);
@@ -484,7 +495,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   }
 
-  if (S > 1) {
+  if (cfg::kSides == 1 && S > 1) {
     // ------------------------------------------------------------ split-K exchange (one tile per cluster)
     const int tile = cluster_id;
     const int2 at = tile_at(tile, m_tiles, n_tiles, band);
@@ -507,10 +518,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     if (tr && threadIdx.x == 64) trace[85] = clock64();
     if (warp >= 2) {
       const int row0 = m_tile * kTileM + h * kHalf + q * 32;          // first row of this warp
-      uint8_t* stage_buf = smem_gen + cfg::kOffStage + q * cfg::kStageBuf;
-      if (S == 2) pair_reduce<NT, 2, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N, stage_buf);
-      else if (S == 3) pair_reduce<NT, 3, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N, stage_buf);
-      else pair_reduce<NT, 4, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N, stage_buf);
+      if (S == 2) pair_reduce<NT, 2, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N);
+      else if (S == 3) pair_reduce<NT, 3, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N);
+      else pair_reduce<NT, 4, kClamp>(ws_cluster, taddr, p, h, r, C, out_f32, epi, ldc, row0, M, n_tile * NT, N);
       if (tr && threadIdx.x == 64) trace[83] = clock64();
     }
   }
@@ -541,10 +551,10 @@ int make_tma_2d(nvc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t inner
 
 #define NVC_PAIR_WIDTHS(X) X(64) X(128) X(160) X(192) X(224) X(256)
 
-template <int NT>
+template <int NT, int kMode = kRows>
 int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M, int N,
                 int K, int S, int epi, cudaStream_t stream, long long* trace, const QkEpi& qk = QkEpi{}, int ldw = 0) {
-  using cfg = PairCfg<NT>;
+  using cfg = PairCfg<NT, kMode>;
   if (ldw == 0) ldw = K;
   CUtensorMap ta, tb;
   int rc = make_tma_2d(ctx, &ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, kHalf);
@@ -581,8 +591,13 @@ int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, voi
   // qkv 18.4 -> 16.8 us, o_proj 14.6 -> 13.9, gate_up 49.6 -> 47.4, down 30.3 -> 28.4 without it) - the prefetches compete
   // with the ring's own TMA loads for the same L2 / HBM queues (profiles/r02_pair_prefetch_ab.txt)
   const int prefetch_w = (M <= kTileM && kb_total <= 48) ? 1 : 0;
-  auto* kernel = nvc_epi_glu_clamp(epi) ? gemm_pair_kernel<NT, true> : gemm_pair_kernel<NT>;
-  NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes, stream, 2 * S,
+  auto* kernel = gemm_pair_kernel<NT, kMode>;
+  if constexpr (kMode == kRows) {              // of the same size and threads
+    if (nvc_epi_glu_clamp(epi)) kernel = gemm_pair_kernel<NT, kClampedRows>;
+    else if (epi == NVC_EPI_SILU_MUL) kernel = gemm_pair_kernel<NT, kSilu>;
+    else if (epi == NVC_EPI_GELU_TANH_MUL) kernel = gemm_pair_kernel<NT, kGelu>;
+  }
+  NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, kernel, grid, dim3(cfg::kThreads), cfg::kSmemBytes, stream, 2 * S,
                                          ta, tb, C, ldc, out_f32, M, N, kb_total, kb_per, tiles, n_tiles, band,
                                          prefetch_w, epi, reinterpret_cast<float4*>(ctx->gemm_ws), trace,
                                          qk));
@@ -596,15 +611,17 @@ int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, voi
 // Co-resident clusters of 2S CTAs (S = 1..4), measured once per context: the schedule model needs
 // them (cluster placement is per GPC: B200 holds 74 / 33 / 22 / 15 clusters of 2 / 4 / 6 / 8 CTAs).
 extern "C" int nvc_gemm_pair_init(nvc_ctx* ctx) {
-#define X(NT) \
-  NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_pair_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<NT>::kSmemBytes)); \
-  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_pair_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<NT>::kSmemBytes)));
-  NVC_PAIR_WIDTHS(X)
+#define X(NT, MODE) \
+  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_pair_kernel<NT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<NT, MODE>::kSmemBytes)));
+#define Y(NT) X(NT, kRows) X(NT, kClampedRows) X(NT, kSilu) X(NT, kGelu)
+  NVC_PAIR_WIDTHS(Y)
+  X(256, kHeads) X(64, kSwapped) X(128, kSwapped)
+#undef Y
 #undef X
   for (int S = 1; S <= 4; ++S) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * S * 64);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(PairCfg<256>::kThreads);
     cfg.dynamicSmemBytes = PairCfg<256>::kSmemBytes;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -720,8 +737,8 @@ extern "C" int nvc_gemm_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc
 extern "C" int nvc_gemm_pair_swapped(nvc_ctx* ctx, const nvc_bf16* X, int ldx, const nvc_bf16* W, float* C, int ldc, int M,
                                      int N, int K, void* stream, long long* trace) {
   if (M < 1 || M > 128 || K % BK != 0) return NVC_ENOTIMPL;
-  if (M <= 64) return launch_pair<64>(ctx, W, K, X, C, ldc, 1, N, M, K, 1, NVC_EPI_TRANSPOSE, nvc_stream(stream), trace, QkEpi{}, ldx);
-  return launch_pair<128>(ctx, W, K, X, C, ldc, 1, N, M, K, 1, NVC_EPI_TRANSPOSE, nvc_stream(stream), trace, QkEpi{}, ldx);
+  if (M <= 64) return launch_pair<64, kSwapped>(ctx, W, K, X, C, ldc, 1, N, M, K, 1, NVC_EPI_TRANSPOSE, nvc_stream(stream), trace, QkEpi{}, ldx);
+  return launch_pair<128, kSwapped>(ctx, W, K, X, C, ldc, 1, N, M, K, 1, NVC_EPI_TRANSPOSE, nvc_stream(stream), trace, QkEpi{}, ldx);
 }
 
 // K3 + K2 in one launch for the fused QKV projection of a prefill-sized step (src/models/qwen3.rs:205-234): returns
@@ -754,7 +771,7 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
   qk.eps = eps;
   qk.nh = nh;
   qk.kv = kv;
-  return launch_pair<256>(ctx, A, lda, W, C, ldc, 0, M, N, K, 1, NVC_EPI_QK_NORM_ROPE, nvc_stream(stream), nullptr, qk);
+  return launch_pair<256, kHeads>(ctx, A, lda, W, C, ldc, 0, M, N, K, 1, NVC_EPI_QK_NORM_ROPE, nvc_stream(stream), nullptr, qk);
 }
 
 // Public form: the fused QKV projection followed by K2, one launch when the shape takes the persistent pair schedule
