@@ -750,13 +750,12 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
                                 int nh, int kv, void* stream) {
   auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   if (N != (nh + 2 * kv) * 128 || K % BK != 0 || lda < K || (lda | ldc) % 8 || !al16(A) || !al16(W) || !al16(C)) return NVC_ENOTIMPL;
-  // The fusion saves a pass over the rows and lengthens the epilogue, of which all but the last wave's runs under the next tile's main loop.
-  // K >= 2 048: it wins from about 1 500 rows on (one call against two kernels: 1 500 x 6 144 x 4 096 57 / 63 us, 3 000 x 4 096 x 2 048 51 / 62,
-  // 4 096 x 6 144 x 4 096 167 / 191, 6 555 x 4 096 x 2 048 115 / 151; 1 000 rows 54 / 52).  Shorter k-loops hide less of it: below 8 192 rows it wins
-  // where the last wave is at least 2/5 full (6 555 x 4 096 x 1 024, 5.6 waves: 90 / 104; 5 500, 4.8: 65 / 70) and loses else (6 000, 5.2: 97 / 89;
-  // 3 500, 3.03: 62 / 58; 4 096, 3.5: even; 4 100 - 4 608, 3.7 - 3.9: 46 / 47 - 50)
-  const int pairs = ctx->num_sms / 2, rem = ((M + 255) / 256) * ((N + 255) / 256) % pairs, last = rem ? rem : pairs;
-  if (K >= 2048 ? M < 1500 : M < 8192 && (M <= 4096 || 5 * last < 2 * pairs)) return NVC_ENOTIMPL;
+  // The fusion saves a pass over the rows and lengthens the epilogue, of which all but the last wave's runs under the next tile's main loop; but it is bound to 256-wide
+  // tiles without splits.  It wins wherever these fill the chip: from two waves on, and at one or two waves that are 85 % full (one call against two kernels, us:
+  // 3 000 x 4 096 x 1 024, 2.6 waves: 30.5 / 36.6; 6 555 rows, 5.6: 50 / 72; 2 600 x 4 096 x 2 048, 2.4: 42.8 / 46.3; 2 000 x 4 096 x 1 024, 1.73: 23.3 / 27.8; 1 000, 0.86:
+  // 16.1 / 18.2; 700 x 6 144 x 2 560, 0.97: 30.7 / 33.6; it loses at 1 300 x 4 096 x 2 048, 1.3: 31.2 / 29.7, and 500 x 6 144 x 4 096, 0.65: 34.7 / 28.9)
+  const int pairs = ctx->num_sms / 2, tiles = ((M + 255) / 256) * ((N + 255) / 256), waves = (tiles + pairs - 1) / pairs;
+  if (M <= kTileM || (waves <= 2 && 20 * tiles < 17 * waves * pairs)) return NVC_ENOTIMPL;
   int nt = 256, S = 1;
   choose_schedule(ctx, M, N, K / BK, false, true, &nt, &S);
   if (nt != 256 || S != 1) return NVC_ENOTIMPL;

@@ -11,7 +11,8 @@ BF16 = torch.bfloat16
 
 
 @pytest.mark.parametrize("M,nh,kv,K", [(1500, 4, 2, 2048), (1501, 32, 8, 4096), (3001, 16, 8, 2048), (5500, 16, 8, 1024), (6000, 16, 8, 1024), (6555, 16, 8, 1024),
-                                       (8191, 8, 4, 512), (2400, 5, 1, 2048),
+                                       (8191, 8, 4, 512), (2400, 5, 1, 2048), (1000, 16, 8, 1024), (2000, 16, 8, 1024), (3000, 16, 8, 1024), (700, 32, 8, 2560), (2600, 16, 8, 2048),
+                                       (257, 58, 2, 256),
                                        (5120, 66, 4, 512)])      # 740 tiles: ten full waves on 74 pairs of SMs
 def test_fused_projection_between_its_thresholds(ctx, nvc, M, nh, kv, K):
     g = torch.Generator().manual_seed(M + K)
