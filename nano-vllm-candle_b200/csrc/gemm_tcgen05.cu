@@ -8,7 +8,7 @@
 // 128B-swizzled TMA box), so one mbarrier round trip (~130 cycles) is amortised over 4*KPS MMAs.
 //   warp 0   : TMA producer for the activation sub-tiles (only the rows that exist when M < 128)
 //   warp 2   : TMA producer for the weight sub-tiles, then joins the epilogue
-//   warp 1   : allocates TMEM; one elected lane issues tcgen05.mma (M=128, N=BN, K=16);
+//   warp 1   : allocates TMEM; one elected lane issues tcgen05.mma (M=128, or 64 for up to 64 rows, N=BN, K=16);
 //              tcgen05.commit frees the stage / publishes the accumulator
 //   warps 2-5: epilogue - tcgen05.ld 32 lanes x 16 columns, convert, 16-byte stores
 // All role loops are executed by the whole warp with one elected lane issuing, which keeps the
@@ -38,9 +38,9 @@ constexpr int kThreads = 192;
 constexpr int kEpilogueThreads = 128;
 constexpr int kSmemBudget = 200 * 1024;
 
-template <int BN, int KPS>
+template <int BN, int KPS, int RM = BM>
 struct Cfg {
-  static constexpr int kBytesA = BM * BK * 2;                 // one A sub-tile
+  static constexpr int kBytesA = RM * BK * 2;                 // one A sub-tile
   static constexpr int kBytesB = BN * BK * 2;                 // one W sub-tile
   static constexpr int kStageBytes = KPS * (kBytesA + kBytesB);
   static constexpr int kStages = kSmemBudget / kStageBytes < 8 ? kSmemBudget / kStageBytes : 8;
@@ -60,13 +60,17 @@ __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
 }
 
 // kExt: the variant with the element-wise and the clamped epilogues; the plain variant compiles them out
-template <int BN, int KPS, bool kExt = false>
+// RM: rows of a product, 128 or, for up to 64 rows of activations, 64.  A product of K 16 takes the time its left operand takes to be read, some 35 cycles at 128 rows
+// however few columns there are, so a decode product of K 1 024 spent 1.2 us on rows that do not exist; and with half the bytes per k-block of activations the ring holds
+// half as many weights again in front of the dependency (64 rows, us, 128 / 64: 6 144 x 1 024 gated 5.75 / 5.1, 2 048 x 1 024 4.45 / 3.8, 12 288 x 2 048 gated 13.9 / 13.2,
+// 2 048 x 6 144 9.7 / 8.9, 3 072 x 2 048 gated 6.9 / 5.6; 1 row 6 144 x 1 024 gated 5.5 / 4.8)
+template <int BN, int KPS, bool kExt = false, int RM = BM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                          void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total,
                          int k_blocks_per_split, int a_box_rows, int prefetch_w, int ks_cluster, int epi, float* __restrict__ ws,
                          int* __restrict__ counters, long long* __restrict__ trace) {
-  using cfg = Cfg<BN, KPS>;
+  using cfg = Cfg<BN, KPS, RM>;
   // optional phase timestamps of CTA (0,0,0) (tools/gemm_microbench.py); NULL in production
   const bool tr = trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
   pdl_trigger();   // the next kernel may start its own prologue
@@ -172,7 +176,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = ptx::umma_idesc_bf16(BM, BN, 0, 0);
+    constexpr uint32_t idesc = ptx::umma_idesc_bf16(RM, BN, 0, 0);
     constexpr uint32_t desc_hi = ptx::umma_desc_hi_sw128(1024);
     const uint32_t a_lo0 = ptx::umma_desc_lo(smem_base, 16);
     const uint32_t b_lo0 = ptx::umma_desc_lo(smem_base + KPS * cfg::kBytesA, 16);
@@ -209,9 +213,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   if (warp >= 2) {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;                 // TMEM lane quadrant this warp may access
-    const int r = q * 32 + lane;            // row inside the tile
+    // row inside the tile; a product of 64 rows has 16 lanes of every quadrant
+    const int r = RM == BM ? q * 32 + lane : q * 16 + (lane & 15);
     const int grow = m_tile * BM + r;
-    const bool row_ok = grow < M;
+    const bool row_ok = grow < M && (RM == BM || lane < 16);
     ptx::mbar_wait(tmem_full_bar, 0);
     ptx::tcgen05_fence_after();
     if (tr && threadIdx.x == 64) trace[81] = clock64();
@@ -249,6 +254,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         uint32_t v[16];
         ptx::tmem_ld_32x32b_x16(taddr + c * 16, v);
         ptx::tmem_ld_wait();
+        if (RM == BM || lane < 16)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           ptx::st_shared_f4(smem_base + (uint32_t)(((c * 4 + j) * BM + r) * 16), __uint_as_float(v[4 * j]),
@@ -394,10 +400,10 @@ int make_tma_2d(nvc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t inner
   return NVC_OK;
 }
 
-template <int BN, int KPS>
+template <int BN, int KPS, int RM = BM>
 int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
            int N, int K, int splits, int ks_cluster, int epi, cudaStream_t stream, long long* trace) {
-  using cfg = Cfg<BN, KPS>;
+  using cfg = Cfg<BN, KPS, RM>;
   CUtensorMap ta, tb;
   // a single partial m-tile only needs the rows that exist (rounded to the 8-row swizzle atom)
   const int a_rows = M >= BM ? BM : (M + 7) / 8 * 8;
@@ -415,8 +421,8 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   NVC_REQUIRE(ctx, !ks || (size_t)BN * BM * 4 <= (size_t)cfg::kStages * cfg::kStageBytes, NVC_EINVAL, "ring too small for the partial tile");
   const bool ext = nvc_epi_unary(epi) || nvc_epi_glu_clamp(epi);
   NVC_REQUIRE(ctx, !ext || has_ext(BN), NVC_EINVAL, "no element-wise epilogue on this tile");
-  auto kernel = gemm_bf16_tcgen05_kernel<BN, KPS, false>;
-  if constexpr (has_ext(BN)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true>; }
+  auto kernel = gemm_bf16_tcgen05_kernel<BN, KPS, false, RM>;
+  if constexpr (has_ext(BN)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true, RM>; }
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
                                           stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
                                           kb_per, a_rows,
@@ -433,6 +439,7 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 // (BN, KPS) instantiations.  KPS > 1 (several k-blocks per mbarrier round trip) is for short,
 // latency-bound CTAs (decode); KPS = 1 keeps the deepest ring for long compute-bound k-loops.  The last two are reached by force_bn only.
 #define NVC_GEMM_CONFIGS(X) X(256, 1) X(128, 1) X(128, 2) X(64, 2) X(64, 4) X(32, 4) X(16, 4) X(96, 2)
+#define NVC_GEMM_FEW_ROWS(X) X(256, 1) X(128, 2) X(64, 4) X(32, 4)      // with products of 64 rows: what the choice may take for up to 64
 
 // Tile choice, fitted to tools/gemm_microbench.py (CUDA-graph timing + CTA phase traces) on B200:
 //  * a CTA ingests ~60 B/clk through TMA when the operands stream from HBM, so a k-block costs
@@ -445,6 +452,27 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
                    int* ks_out) {
   *splits_out = 1;
   *ks_out = 0;
+  if (M <= 64) {
+    // Decode on products of 64 rows, in us: fitted to 1 675 configurations of 28 products (N 256 - 24 576, K 512 - 12 288) over 1 - 64 rows, those within 15 % of a product's
+    // best (residual 4.3 %).  What it picks is 0.6 % slower than the best in the mean, 7 % at most; beside what was picked and run with 128 rows 9.8 % faster, nowhere slower.
+    // A cluster's start waits for all of its SMs, the longer the fuller the chip: the cube.
+    const int rows = ((M + 7) / 8) * 8, kb = K / BK;
+    double best = 1e30;
+    for (int bn : {32, 64, 128, 256})
+      for (int S : {1, 2, 4}) {
+        if (S > 1 && (!allow_split || !g_nvc_gemm_ks || kb / S < 4)) continue;
+        if (bn / 2 >= N) continue;
+        const int ctas = (N + bn - 1) / bn * S, cap = S == 1 ? ctx->num_sms : S * (ctx->pair_clusters[S / 2] > 0 ? ctx->pair_clusters[S / 2] : ctx->num_sms / (S == 2 ? 2 : 5));
+        const double fill = ctas < cap ? (double)ctas / cap : 1.0;
+        double t = ceil((double)ctas / cap) * (2.17 + (kb + S - 1) / S * (0.0331 + 0.00077 * bn + 0.00018 * rows));
+        if (S > 1) t += 0.69 + 0.73 * fill * fill * fill + 0.00021 * rows * bn * (S - 1) / S;
+        if (t < best) { best = t; *bn_out = bn; *splits_out = S; }
+      }
+    if (best > 1e29) *bn_out = 32;
+    *kps_out = *bn_out == 256 ? 1 : (*bn_out == 128 ? 2 : 4);
+    *ks_out = *splits_out > 1 ? 1 : 0;
+    return;
+  }
   if (M <= BM) {
     // Decode (one m-tile).  Cycle model fitted to CTA phase traces (tools/gemm_microbench.py --trace-decode):
     // the TMA unit of an SM moves ~90 B/clk plus ~30 cycles per box (two loads + one L2 prefetch per k-block),
@@ -511,6 +539,13 @@ extern "C" int nvc_gemm_init(nvc_ctx* ctx) {
     NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, true>,                                    \
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS>::kSmemBytes));
   NVC_GEMM_CONFIGS(X)
+#undef X
+#define X(BN, KPS)                                                                                                       \
+  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, false, 64>,                                \
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS, 64>::kSmemBytes))); \
+  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, true, 64>,                                 \
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS, 64>::kSmemBytes)));
+  NVC_GEMM_FEW_ROWS(X)
 #undef X
   return NVC_OK;
 }
@@ -588,6 +623,11 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   }
   cudaStream_t st = nvc_stream(stream);
   const int f32 = out_dtype == NVC_DT_F32;
+  if (M <= 64 && (splits == 1 || ks)) {
+#define X(BN, KPS) if (bn == BN && kps == KPS) return launch<BN, KPS, 64>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
+    NVC_GEMM_FEW_ROWS(X)
+#undef X
+  }
 #define X(BN, KPS) \
   if (bn == BN && kps == KPS) return launch<BN, KPS>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
   NVC_GEMM_CONFIGS(X)

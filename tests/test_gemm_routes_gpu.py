@@ -57,3 +57,24 @@ def test_narrow_products_over_many_rows(ctx, M, N, K):
     got = ctx.gemm(a, w, out=buf[:, :N])
     assert float((got - ctx.gemm(a, w, out_dtype=torch.float32, force_bn=512)).abs().max()) < 1e-3
     assert bool(torch.isnan(buf[:, N:]).all())
+
+
+@pytest.mark.parametrize("M", [1, 7, 15, 16, 17, 33, 63, 64, 65])
+@pytest.mark.parametrize("N,K", [(16, 512), (48, 256), (1024, 3072), (2048, 1024), (2064, 2048), (6144, 2560), (4096, 4096), (19456, 512), (1040, 6144)])
+def test_few_rows(ctx, M, N, K):
+    """Up to 64 rows run on products of 64 rows, every tile width and split of their choice; 65 do not.  Sums of K exact products of size K^-1/2 in fp32, in another order:
+    1e-4 of the largest; bf16 results one more rounding, 2^-8 of the value.  Rows and columns around the result keep their marks."""
+    ops = __import__("importlib").import_module("nano-vllm-candle_b200.ops")
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g, device="cuda").to(BF16), (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    want = a.double() @ w.double().T
+    top = float(want.abs().max())
+    buf = torch.full((M + 1, N + 16), 7.0, device="cuda")
+    ctx.gemm(a, w, out_dtype=torch.float32, out=buf[:M, :N])
+    assert float((buf[:M, :N] - want).abs().max()) <= 1e-4 * top and bool((buf[M] == 7.0).all()) and bool((buf[:, N:] == 7.0).all())
+    near = lambda got, ref: float(((got.double() - ref).abs() - 2.0 ** -8 * ref.abs()).max()) <= 1e-4 * float(ref.abs().max())  # noqa: E731
+    assert near(ctx.gemm(a, w), want)
+    assert near(ops.gemm_act(ctx, a, w, ops.ACT_RELU2), want.clamp(min=0) ** 2)
+    if N % 32 == 0:
+        gu = torch.cat([w[:N // 2], w[N // 2:]])
+        assert near(ctx.gemm_silu_mul(a, ctx.interleave_gate_up(gu)), torch.nn.functional.silu(want[:, :N // 2]) * want[:, N // 2:])
