@@ -74,8 +74,19 @@ __device__ __forceinline__ void conv_tile(float4 (&y)[TT], const float* in, int6
   }
 }
 
-__device__ __forceinline__ float4 silu4(const float4& a) {
-  return make_float4(a.x * sigmoid_f32(a.x), a.y * sigmoid_f32(a.y), a.z * sigmoid_f32(a.z), a.w * sigmoid_f32(a.w));
+// x sigmoid(x) without a division's branch and range checks, which are most of a convolved number's instructions: with t = exp(-|x|) the sigmoid is 1 / (1 + t) or
+// t / (1 + t), its divisor lies in [1, 2], and one Newton step on the hardware's reciprocal (off by one unit in the last place at most) and one on the quotient round it
+// correctly (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990); what 1 + t rounds away takes part in the second.
+// Infinities and NaN come out as those of x / (1 + exp(-x)).  Against 64 bits, relative 2-norm, that division / this: x from N(0, 1) 4.54e-8 / 3.49e-8, from N(0, 1e-8)
+// 5.0e-8 / 3.9e-8; below -87, where that division had no digits left, 5.0e-8.  4 480 rows of 4 096 channels 46.2 -> 42.2 us, of 2 560 31.5 -> 28.6.
+__device__ __forceinline__ float silu_f32(float x) {
+  const float t = expf(-fabsf(x)), d = 1.0f + t, rest = t - (d - 1.0f), a = x < 0.f ? t : 1.0f;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.0f), r, r);
+  const float q = a * r;
+  return x * fmaf(fmaf(-rest, q, fmaf(-d, q, a)), r, q);
 }
+__device__ __forceinline__ float4 silu4(const float4& a) { return make_float4(silu_f32(a.x), silu_f32(a.y), silu_f32(a.z), silu_f32(a.w)); }
 
 }  // namespace

@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
 
 // Prompt portions with 16-byte rows, heads of up to 128 numbers and 1 .. 4 taps: a warp takes 8 neighbouring rows of 128 channels (conv_tile.cuh).
 // Tasks of a tile of rows: the q and k heads (a head in L lanes, its length by exchange: one root and division per row), the v channels, the
-// heads' decays and betas, and the decays per channel.  Bound by memory and the exponentials: 4 480 rows of 16 heads of 128 over 8 take 43 us
-// (150 MB: 3.5 TB/s), one warp per (row, head) that read every row once per tap 84 us.
+// heads' decays and betas, and the decays per channel.  Bound by memory and the exponentials: 4 480 rows of 16 heads of 128 over 8 take 42 us
+// (150 MB: 3.6 TB/s), one warp per (row, head) that read every row once per tap 84 us.
 template <int TAPS, int L>
 __global__ void __launch_bounds__(128) delta_prep_tile_kernel(const DeltaArgs a) {
   constexpr int TT = 8, HP = 32 / L;
