@@ -426,10 +426,13 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
                                           stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
                                           kb_per, a_rows,
-                                          // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring:
-                                          // helps the short, latency-bound k-loops of decode (K <= 3072: 5.1 vs 5.7 us), costs
-                                          // 2 - 8 % on the long ones (K 12288 at M 64: 23.2 -> 21.6 us without it) and at M >= 256
-                                          (g_nvc_gemm_prefetch && M <= BM && kb_total <= 48) ? 1 : 0,
+                                          // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring, up to 128 rows and below
+                                          // 32 MB of weights: 148 rings of 190 KB hold 28 MB, so that nearly all of W is on chip when the activations
+                                          // arrive, however long the k-loop (us, without / with: 6 144 x 1 024 gated 5.7 / 4.8, 2 560 x 4 096 8.2 / 7.7,
+                                          // 2 048 x 6 144 8.4 / 8.05, 6 144 x 2 560 8.9 / 8.5).  Larger weights stream behind the wait either way, and
+                                          // early bytes only displace each other (12 288 x 2 048 gated 12.7 / 13.1, 19 456 x 2 560 gated 21.5 / 23.7,
+                                          // 64 rows 22.05 / 25.0, 4 096 x 12 288 20.5 / 21.9; 4 096 x 4 096, the edge: 9.95 / 9.75 and at 64 rows 10.0 / 10.45)
+                                          (g_nvc_gemm_prefetch && M <= BM && (long long)N * kb_total * BK < (16ll << 20)) ? 1 : 0,
                                           ks, epi, ctx->gemm_ws, ctx->gemm_counters, trace));
   NVC_CUDA_CHECK(ctx, cudaGetLastError());
   ctx->launches++;
