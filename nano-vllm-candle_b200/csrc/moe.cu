@@ -3,6 +3,7 @@
 //   nvc_moe_route    router logits in fp32, sigmoid scores, biased top-k choice, normalised weights, shared-expert gate
 //   nvc_moe_sort     counting sort of the (token, choice) pairs by expert: group offsets, source rows, positions
 //   nvc_moe_combine  weighted sum of a token's expert rows plus the gated shared expert, fp32
+#include "ptx.cuh"
 #include "typed.cuh"
 
 namespace {
@@ -156,26 +157,32 @@ __global__ void moe_route_kernel(const T* h, int ldh, const float* __restrict__ 
   topk_write(s, c, lane, E, top, scale, idx, wout, n);
 }
 
-// Stable counting sort by expert in one CTA of 32 warps (pairs = N * top).  Warp w owns the contiguous segment w of the
+// Stable counting sort by expert in one CTA of 32 warps or a cluster of C (pairs = N * top).  Warp w owns the contiguous segment w of the
 // pairs: it counts its pairs per expert, a prefix over (expert, warp) gives every warp its first position in every
 // expert's group, and the warp then places its pairs in order (__match_any_sync ranks equal experts inside a batch of
 // 32).  Within an expert the pairs keep token order, so the layout - and every sum downstream - is deterministic.
 // One CTA's latencies are its time: a warp requests 8 x 32 of its pairs at once and keeps the first 256 for the second pass, and both prefixes go by
 // exchange (8 000 pairs, 16 experts, cold cache: 11.1 -> 10.6 us against loads one behind the other and prefixes thread by thread; 128 pairs 6.0 -> 5.3).
+// Of many pairs it is one SM's scattered 4-byte stores and matches: eight CTAs take a stretch each and read each other's counts per expert (8 000 pairs, 16 experts
+// 8.3 -> 4.6 us; 32 000 pairs, 128 experts 49.8 -> 11.0).  Counts lie in rows of an odd length: 128 of them put a column of 32 into one bank (512 pairs 11.1 -> 7.3).
+template <int C>
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align, int32_t* __restrict__ offsets,
                 int32_t* __restrict__ src_rows, int32_t* __restrict__ pos, int32_t* __restrict__ tile_group, int tiles_cap, int tail_cap, int tail) {
-  extern __shared__ int32_t sm[];   // [32][E] counts -> pairs of earlier warps, then [E + 1] offsets, then [E] sizes
+  extern __shared__ int32_t sm[];   // [32][E | 1] counts -> pairs of earlier warps, then [E + 1] offsets, [E] sizes and, of several CTAs, [E] pairs here and [E] pairs of earlier CTAs
+  const int Es = E | 1;                                  // a column of an even number of counts would lie in few banks
   int32_t* cnt = sm;
-  int32_t* off = sm + 32 * E;
+  int32_t* off = sm + 32 * Es;
   int32_t* size = off + E + 1;
+  int32_t* here = C > 1 ? size + E : size;
+  int32_t* before = here + E;
   constexpr int kBatch = 8;
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) cnt[i] = 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = C > 1 ? blockIdx.x : 0, run = rank * 32 + warp;
+  for (int i = threadIdx.x; i < 32 * Es; i += blockDim.x) cnt[i] = 0;
   pdl_wait();
-  const int seg = ((P + 31) / 32 + 31) / 32 * 32;      // pairs per warp, a multiple of 32
-  const int p_begin = min(P, warp * seg), p_end = min(P, warp * seg + seg);
+  const int seg = ((P + 32 * C - 1) / (32 * C) + 31) / 32 * 32;      // pairs per warp, a multiple of 32
+  const int p_begin = min(P, run * seg), p_end = min(P, run * seg + seg);
   int e[kBatch];
   auto load = [&](int p0) {
 #pragma unroll
@@ -190,19 +197,34 @@ moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align
     if (p0 > p_begin) load(p0);
 #pragma unroll
     for (int i = 0; i < kBatch; ++i)
-      if (e[i] >= 0) atomicAdd(&cnt[warp * E + e[i]], 1);
+      if (e[i] >= 0) atomicAdd(&cnt[warp * Es + e[i]], 1);
   }
   __syncthreads();
   for (int x = warp; x < E; x += 32) {                   // an expert's pairs in earlier warps
-    const int v = cnt[lane * E + x];
+    const int v = cnt[lane * Es + x];
     int sum = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int up = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += up;
     }
-    cnt[lane * E + x] = sum - v;
-    if (lane == 31) size[x] = sum;
+    cnt[lane * Es + x] = sum - v;
+    if (lane == 31) here[x] = sum;
+  }
+  if constexpr (C > 1) {
+    __syncwarp();                                        // the barrier is for whole warps
+    ptx::cluster_sync_all();
+    for (int x = threadIdx.x; x < E; x += blockDim.x) {
+      int all = 0, earlier = 0;
+#pragma unroll
+      for (int r = 0; r < C; ++r) {
+        const int v = ptx::ld_cluster_s32(ptx::mapa_u32(smem_u32(here + x), r));
+        all += v;
+        earlier += r < rank ? v : 0;
+      }
+      size[x] = all;
+      before[x] = earlier;
+    }
   }
   __syncthreads();
   if (warp == 0) {                                       // every group starts at a multiple of `align` rows
@@ -222,16 +244,17 @@ moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align
   __syncthreads();
   if (align > 1) {
     // rows between a group's last pair and the next group's start have no source; tiles of `align` rows -> their group
-    for (int x = warp; x < E; x += blockDim.x >> 5) {
+    for (int x = run; x < E; x += 32 * C) {
       for (int r = off[x] + size[x] + lane; r < off[x + 1]; r += 32) src_rows[r] = -1;
       if (tile_group)
         for (int t = off[x] / align + lane; t < off[x + 1] / align; t += 32) tile_group[t] = x < E_real ? x : -1;   // no product behind an identity expert
     }
     if (tile_group)
-      for (int t = off[E] / align + threadIdx.x; t < tiles_cap; t += blockDim.x) tile_group[t] = -1;
-    for (int r = off[E] + threadIdx.x; r < tail_cap; r += blockDim.x) src_rows[r] = tail;       // behind the last group
+      for (int t = off[E] / align + rank * blockDim.x + threadIdx.x; t < tiles_cap; t += C * blockDim.x) tile_group[t] = -1;
+    for (int r = off[E] + rank * blockDim.x + threadIdx.x; r < tail_cap; r += C * blockDim.x) src_rows[r] = tail;       // behind the last group
   }
-  for (int x = threadIdx.x; x <= E; x += blockDim.x) offsets[x] = off[x];
+  if (rank == 0)
+    for (int x = threadIdx.x; x <= E; x += blockDim.x) offsets[x] = off[x];
   const bool kept = p_end - p_begin <= 32 * kBatch;
   for (int p0 = p_begin; p0 < p_end; p0 += 32 * kBatch) {
     if (!kept) load(p0);
@@ -241,16 +264,20 @@ moe_sort_kernel(const int32_t* idx, int P, int top, int E, int E_real, int align
       const int p = p0 + 32 * i + lane, x = e[i];
       const unsigned peers = __match_any_sync(0xffffffffu, x);
       if (x >= 0) {
-        const int at = off[x] + cnt[warp * E + x] + __popc(peers & ((1u << lane) - 1));
+        const int at = off[x] + (C > 1 ? before[x] : 0) + cnt[warp * Es + x] + __popc(peers & ((1u << lane) - 1));
         src_rows[at] = p / top;
         pos[p] = at;
       } else if (p < p_end) {
         pos[p] = 0;                                      // no expert, no place: a row that exists, so that what reads it stays in bounds
       }
       __syncwarp();
-      if (x >= 0 && lane == 31 - __clz(peers)) cnt[warp * E + x] += __popc(peers);   // the last peer advances the group
+      if (x >= 0 && lane == 31 - __clz(peers)) cnt[warp * Es + x] += __popc(peers);   // the last peer advances the group
       __syncwarp();
     }
+  }
+  if constexpr (C > 1) {                                 // the other CTAs have read this one's counts
+    __syncwarp();
+    ptx::cluster_sync_all();
   }
 }
 
@@ -438,8 +465,13 @@ static int sort_padded(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, in
   NVC_REQUIRE(ctx, N >= 0 && top > 0 && E > 0 && E <= 320 && align >= 1, NVC_EINVAL, "bad sizes");
   NVC_REQUIRE(ctx, !tile_group || (align > 1 && (int64_t)tiles_cap * align >= (int64_t)N * top + (int64_t)E * (align - 1)), NVC_EINVAL,
               "tile_group needs align > 1 and room for every group's padding");
-  NVC_CUDA_CHECK(ctx, nvc_launch(ctx, moe_sort_kernel, dim3(1), dim3(1024), (size_t)(34 * E + 1) * sizeof(int32_t), nvc_stream(stream),
-                                 topk_idx, N * top, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, tail_cap, tail));
+  const int P = N * top;
+  // Eight CTAs cost 0.5 - 1.2 us of cluster launch and barriers and divide everything else, pairs and a quarter of the padding counted (us, one / eight CTAs:
+  // 512 pairs to 16 experts 3.2 / 4.2, 2 000 4.0 / 4.55, 4 000 5.2 / 4.6, 8 000 7.6 / 4.6; to 128 experts 512 pairs 7.3 / 6.4, 8 000 15.7 / 7.5, 32 000 44 / 11)
+  const int C = P + (int64_t)E * (align - 1) / 4 > 3000 ? 8 : 1;
+  auto kernel = C == 8 ? moe_sort_kernel<8> : moe_sort_kernel<1>;
+  NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, kernel, dim3(C), dim3(1024), (size_t)(32 * (E | 1) + (C > 1 ? 4 : 2) * E + 1) * sizeof(int32_t), nvc_stream(stream), C,
+                                         topk_idx, P, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, tail_cap, tail));
   ctx->launches++;
   return NVC_OK;
 }

@@ -226,6 +226,11 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ int ld_cluster_s32(uint32_t cluster_addr) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_addr));
+  return v;
+}
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
   float4 v;
   // volatile (ordered against the cluster barriers, which are volatile too) but no memory clobber: a batch
