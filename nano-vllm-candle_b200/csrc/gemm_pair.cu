@@ -589,8 +589,10 @@ int launch_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, voi
   // L2 prefetch of the first weight k-blocks before the dependency wait + 16 k-blocks ahead of the ring: pays for short,
   // latency-bound k-loops (decode at K <= 3072: 1 - 3 %), costs 4 - 9 % on the long ones (Qwen3-8B at batch 256, K >= 4096:
   // qkv 18.4 -> 16.8 us, o_proj 14.6 -> 13.9, gate_up 49.6 -> 47.4, down 30.3 -> 28.4 without it) - the prefetches compete
-  // with the ring's own TMA loads for the same L2 / HBM queues (profiles/r02_pair_prefetch_ab.txt)
-  const int prefetch_w = (M <= kTileM && kb_total <= 48) ? 1 : 0;
+  // with the ring's own TMA loads for the same L2 / HBM queues (profiles/r02_pair_prefetch_ab.txt).  So do those of large weights behind short k-loops, of
+  // which the wait hides little (136 - 256 rows, us, with / without: 4 096 x 2 048 11.1 / 11.4, 4 096 x 1 024 7.35 / 7.75, 3 072 x 512 5.7 / 6.0, but
+  // 6 144 x 2 560 13.8 / 13.1, 12 288 x 2 048 gated 17.1 / 15.6, 19 456 x 2 560 gated 28.9 / 27.1): below 24 MB only
+  const int prefetch_w = (M <= kTileM && kb_total <= 48 && (long long)N * kb_total * BK < (12ll << 20)) ? 1 : 0;
   auto* kernel = gemm_pair_kernel<NT, kMode>;
   if constexpr (kMode == kRows) {              // of the same size and threads
     if (nvc_epi_glu_clamp(epi)) kernel = gemm_pair_kernel<NT, kClampedRows>;
