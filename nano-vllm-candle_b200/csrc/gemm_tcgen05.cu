@@ -455,10 +455,13 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
                    int* ks_out) {
   *splits_out = 1;
   *ks_out = 0;
-  if (M <= 64) {
-    // Decode on products of 64 rows, in us: fitted to 1 675 configurations of 28 products (N 256 - 24 576, K 512 - 12 288) over 1 - 64 rows, those within 15 % of a product's
-    // best (residual 4.3 %).  What it picks is 0.6 % slower than the best in the mean, 7 % at most; beside what was picked and run with 128 rows 9.8 % faster, nowhere slower.
+  if (M <= BM) {
+    // Decode, in us: fitted to measured products of K 512 - 12 288 and N 256 - 24 576, by size of the tensor products they run on.
+    // 64 rows: 1 675 configurations of 28 products, those within 15 % of a product's best (residual 4.3 %); what it picks is 0.6 % slower than the best in the mean, 7 % at most,
+    // beside what was picked and run with 128 rows 9.8 % faster, nowhere slower.  128 rows: 28 products of 72 - 128 rows; 0.1 % and 6 % slower than the best; beside the cycle model in
+    // its place, on 16 more products too, 1.1 % faster in the mean (2 048 x 1 024 5.47 -> 4.8, 6 144 x 2 560 13.2 -> 11.7, 6 144 x 4 096 18.8 -> 17.4), at most 1.5 % slower.
     // A cluster's start waits for all of its SMs, the longer the fuller the chip: the cube.
+    const bool few = M <= 64;
     const int rows = ((M + 7) / 8) * 8, kb = K / BK;
     double best = 1e30;
     for (int bn : {32, 64, 128, 256})
@@ -467,51 +470,14 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
         if (bn / 2 >= N) continue;
         const int ctas = (N + bn - 1) / bn * S, cap = S == 1 ? ctx->num_sms : S * (ctx->pair_clusters[S / 2] > 0 ? ctx->pair_clusters[S / 2] : ctx->num_sms / (S == 2 ? 2 : 5));
         const double fill = ctas < cap ? (double)ctas / cap : 1.0;
-        double t = ceil((double)ctas / cap) * (2.17 + (kb + S - 1) / S * (0.0331 + 0.00077 * bn + 0.00018 * rows));
-        if (S > 1) t += 0.69 + 0.73 * fill * fill * fill + 0.00021 * rows * bn * (S - 1) / S;
+        double t = ceil((double)ctas / cap) * (few ? 2.17 + (kb + S - 1) / S * (0.0331 + 0.00077 * bn + 0.00018 * rows)
+                                                   : 1.65 + (kb + S - 1) / S * (0.096 + 0.00168 * bn + 0.000277 * rows));
+        if (S > 1) t += few ? 0.69 + 0.73 * fill * fill * fill + 0.00021 * rows * bn * (S - 1) / S : 1.22 + 1.02 * fill * fill * fill + 0.000164 * rows * bn * (S - 1) / S;
         if (t < best) { best = t; *bn_out = bn; *splits_out = S; }
       }
     if (best > 1e29) *bn_out = 32;
     *kps_out = *bn_out == 256 ? 1 : (*bn_out == 128 ? 2 : 4);
     *ks_out = *splits_out > 1 ? 1 : 0;
-    return;
-  }
-  if (M <= BM) {
-    // Decode (one m-tile).  Cycle model fitted to CTA phase traces (tools/gemm_microbench.py --trace-decode):
-    // the TMA unit of an SM moves ~90 B/clk plus ~30 cycles per box (two loads + one L2 prefetch per k-block),
-    // whatever the source (the L2 prefetch before the PDL wait hides HBM), and the activation rows are re-read
-    // by every n-tile, so a k-block costs (rows + BN) * 128 / 90 + 90 cycles; ~2200 cycles of prologue +
-    // first-load latency; epilogue 300 + 6 * BN, or, with split-K inside a cluster (1,1,S), ~2300 + the DSMEM
-    // exchange at ~17 B/clk.  The winners are always ONE wave of ~96-132 CTAs with the widest tile that allows it
-    // (co-resident: 148 CTAs, 74 clusters of 2, 33 clusters of 4).
-    const int rows = ((M + 7) / 8) * 8;
-    const int kb = K / BK;
-    const int bns[4] = {32, 64, 128, 256};
-    const int ss[3] = {1, 2, 4};
-    double best = 1e30;
-    int best_bn = 32, best_s = 1;
-    const double hbm_floor = (double)N * K * 2 / 3400.0 + 3000.0;     // 6.5 TB/s at 1.9 GHz
-    for (int i = 0; i < 4; ++i) {
-      for (int j = 0; j < 3; ++j) {
-        const int bn = bns[i], S = ss[j];
-        if (S > 1 && (!allow_split || !g_nvc_gemm_ks || kb / S < 4)) continue;
-        if (bn / 2 >= N) continue;
-        const int tiles = (N + bn - 1) / bn;
-        const int cap = S == 1 ? ctx->num_sms : (S == 2 ? 2 * (ctx->pair_clusters[1] > 0 ? ctx->pair_clusters[1] : ctx->num_sms / 2)
-                                                       : 4 * (ctx->pair_clusters[2] > 0 ? ctx->pair_clusters[2] : ctx->num_sms / 5));
-        const double waves = ceil((double)tiles * S / cap);
-        const double per_kb = (double)(rows + bn) * 128.0 / 90.0 + 90.0;
-        const double tail = S == 1 ? 300.0 + 6.0 * bn : 2300.0 + (double)(S - 1) * rows * (bn / S) * 4.0 / 17.0;
-        const double t = waves * (2200.0 + per_kb * ((kb + S - 1) / S) + tail);
-        // below the HBM floor every candidate takes the floor: rank those by the modeled CTA time (most slack)
-        const double key = t > hbm_floor ? t : hbm_floor * (1.0 + 1e-3 * t / hbm_floor);
-        if (key < best * 0.98 || (key < best && t < hbm_floor)) { best = key; best_bn = bn; best_s = S; }
-      }
-    }
-    *bn_out = best_bn;
-    *kps_out = best_bn == 256 ? 1 : (best_bn == 128 ? 2 : 4);
-    *splits_out = best_s;
-    *ks_out = best_s > 1 ? 1 : 0;
     return;
   }
   const int kb = K / BK;
