@@ -426,13 +426,13 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
                                           stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
                                           kb_per, a_rows,
-                                          // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring, up to 128 rows and below
+                                          // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring, up to 256 rows and below
                                           // 32 MB of weights: 148 rings of 190 KB hold 28 MB, so that nearly all of W is on chip when the activations
                                           // arrive, however long the k-loop (us, without / with: 6 144 x 1 024 gated 5.7 / 4.8, 2 560 x 4 096 8.2 / 7.7,
                                           // 2 048 x 6 144 8.4 / 8.05, 6 144 x 2 560 8.9 / 8.5).  Larger weights stream behind the wait either way, and
                                           // early bytes only displace each other (12 288 x 2 048 gated 12.7 / 13.1, 19 456 x 2 560 gated 21.5 / 23.7,
                                           // 64 rows 22.05 / 25.0, 4 096 x 12 288 20.5 / 21.9; 4 096 x 4 096, the edge: 9.95 / 9.75 and at 64 rows 10.0 / 10.45)
-                                          (g_nvc_gemm_prefetch && M <= BM && (long long)N * kb_total * BK < (16ll << 20)) ? 1 : 0,
+                                          (g_nvc_gemm_prefetch && M <= 2 * BM && (long long)N * kb_total * BK < (16ll << 20)) ? 1 : 0,
                                           ks, epi, ctx->gemm_ws, ctx->gemm_counters, trace));
   NVC_CUDA_CHECK(ctx, cudaGetLastError());
   ctx->launches++;
@@ -559,6 +559,17 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   if (force_bn == 0 && force_splits == 0 && epi == NVC_EPI_NONE && M > BM && Nout <= 256 && K <= (M <= 2 * BM ? 1536 : 2048)) {
     for (int bn : {32, 64, 128})
       if ((int64_t)((M + BM - 1) / BM) * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
+        force_bn = bn + (bn == 128 ? 2000 : 4000);
+        break;
+      }
+  }
+  // Decode batches of 129 to 256 rows with short k-loops: two row tiles of the narrowest 1-CTA tiles that stay in one wave.  Few 256-row tiles leave pairs idle or pay an exchange of
+  // partial sums, 6 us before the first k-block (200 rows, us, pair / this: 2 048 x 512 gated 5.7 / 3.65, 1 024 x 1 024 7.2 / 4.6, 4 096 x 1 024 8.0 / 6.0, 8 192 x 1 024 9.2 / 7.7,
+  // 3 584 x 1 792 11.6 / 8.3, 2 048 x 2 048 9.5 / 7.5, 4 096 x 2 048 10.8 / 8.9, 1 024 x 2 048 7.4 / 7.2; longer k-loops read the rows too often: 768 x 2 304 7.2 / 7.35,
+  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4)
+  if (force_bn == 0 && force_splits == 0 && M > BM && M <= 2 * BM && K <= 2048 && g_nvc_gemm_pair) {
+    for (int bn : {32, 64, 128})
+      if (2 * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
         force_bn = bn + (bn == 128 ? 2000 : 4000);
         break;
       }

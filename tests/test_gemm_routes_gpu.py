@@ -78,3 +78,11 @@ def test_few_rows(ctx, M, N, K):
     if N % 32 == 0:
         gu = torch.cat([w[:N // 2], w[N // 2:]])
         assert near(ctx.gemm_silu_mul(a, ctx.interleave_gate_up(gu)), torch.nn.functional.silu(want[:, :N // 2]) * want[:, N // 2:])
+
+
+@pytest.mark.parametrize("M", [129, 192, 255, 256, 257])
+@pytest.mark.parametrize("N,K", [(16, 1600), (64, 2048), (2368, 64), (2400, 512), (4736, 192), (4768, 2048), (9472, 128), (9504, 1024), (1024, 2112)])
+def test_two_row_tiles(ctx, M, N, K):
+    """129 to 256 rows over K up to 2 048 run on two row tiles of 32, 64 or 128 columns as long as these are one wave; a column tile more, a row more or a longer K does not.
+    The same bounds as for few rows."""
+    test_few_rows(ctx, M, N, K)
