@@ -451,12 +451,12 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 //  * decode (M <= 128): one wave, as many CTAs as the N dimension gives (up to ~all SMs), several
 //    k-blocks per pipeline stage; split-K through the L2 workspace costs >= 6 us (ticket atomic +
 //    reduction round trips) and never won in the sweep, so it is only used when forced.
-void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, int* bn_out, int* kps_out, int* splits_out,
+void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, bool f32, int* bn_out, int* kps_out, int* splits_out,
                    int* ks_out) {
   *splits_out = 1;
   *ks_out = 0;
-  if (M <= BM) {
-    // Decode, in us: fitted to measured products of K 512 - 12 288 and N 256 - 24 576, by size of the tensor products they run on.
+  if (M <= BM && !f32) {
+    // Decode with bf16 results, in us: fitted to measured products of K 512 - 12 288 and N 256 - 24 576, by size of the tensor products they run on.
     // 64 rows: 1 675 configurations of 28 products, those within 15 % of a product's best (residual 4.3 %); what it picks is 0.6 % slower than the best in the mean, 7 % at most,
     // beside what was picked and run with 128 rows 9.8 % faster, nowhere slower.  128 rows: 28 products of 72 - 128 rows; 0.1 % and 6 % slower than the best; beside the cycle model in
     // its place, on 16 more products too, 1.1 % faster in the mean (2 048 x 1 024 5.47 -> 4.8, 6 144 x 2 560 13.2 -> 11.7, 6 144 x 4 096 18.8 -> 17.4), at most 1.5 % slower.
@@ -478,6 +478,46 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
     if (best > 1e29) *bn_out = 32;
     *kps_out = *bn_out == 256 ? 1 : (*bn_out == 128 ? 2 : 4);
     *ks_out = *splits_out > 1 ? 1 : 0;
+    return;
+  }
+  if (M <= BM) {
+    // fp32 results keep the splits of this model: the accumulators' error grows with the length of their chains, and the model above takes longer ones where a cluster does not pay.
+    // (100 rows, error against 64 bits: 2 048 x 1 024 in fp32 2.3e-7 with these splits, 1.0e-6 without, in bf16 1.660e-3 both; 200 rows of K 2 048 4.7e-7 with, 2.1e-6 without.)
+    // Cycle model fitted to CTA phase traces (tools/gemm_microbench.py --trace-decode):
+    // the TMA unit of an SM moves ~90 B/clk plus ~30 cycles per box (two loads + one L2 prefetch per k-block),
+    // whatever the source (the L2 prefetch before the PDL wait hides HBM), and the activation rows are re-read
+    // by every n-tile, so a k-block costs (rows + BN) * 128 / 90 + 90 cycles; ~2200 cycles of prologue +
+    // first-load latency; epilogue 300 + 6 * BN, or, with split-K inside a cluster (1,1,S), ~2300 + the DSMEM
+    // exchange at ~17 B/clk.  The winners are always ONE wave of ~96-132 CTAs with the widest tile that allows it
+    // (co-resident: 148 CTAs, 74 clusters of 2, 33 clusters of 4).
+    const int rows = ((M + 7) / 8) * 8;
+    const int kb = K / BK;
+    const int bns[4] = {32, 64, 128, 256};
+    const int ss[3] = {1, 2, 4};
+    double best = 1e30;
+    int best_bn = 32, best_s = 1;
+    const double hbm_floor = (double)N * K * 2 / 3400.0 + 3000.0;     // 6.5 TB/s at 1.9 GHz
+    for (int i = 0; i < 4; ++i) {
+      for (int j = 0; j < 3; ++j) {
+        const int bn = bns[i], S = ss[j];
+        if (S > 1 && (!allow_split || !g_nvc_gemm_ks || kb / S < 4)) continue;
+        if (bn / 2 >= N) continue;
+        const int tiles = (N + bn - 1) / bn;
+        const int cap = S == 1 ? ctx->num_sms : (S == 2 ? 2 * (ctx->pair_clusters[1] > 0 ? ctx->pair_clusters[1] : ctx->num_sms / 2)
+                                                       : 4 * (ctx->pair_clusters[2] > 0 ? ctx->pair_clusters[2] : ctx->num_sms / 5));
+        const double waves = ceil((double)tiles * S / cap);
+        const double per_kb = (double)(rows + bn) * 128.0 / 90.0 + 90.0;
+        const double tail = S == 1 ? 300.0 + 6.0 * bn : 2300.0 + (double)(S - 1) * rows * (bn / S) * 4.0 / 17.0;
+        const double t = waves * (2200.0 + per_kb * ((kb + S - 1) / S) + tail);
+        // below the HBM floor every candidate takes the floor: rank those by the modeled CTA time (most slack)
+        const double key = t > hbm_floor ? t : hbm_floor * (1.0 + 1e-3 * t / hbm_floor);
+        if (key < best * 0.98 || (key < best && t < hbm_floor)) { best = key; best_bn = bn; best_s = S; }
+      }
+    }
+    *bn_out = best_bn;
+    *kps_out = best_bn == 256 ? 1 : (best_bn == 128 ? 2 : 4);
+    *splits_out = best_s;
+    *ks_out = best_s > 1 ? 1 : 0;
     return;
   }
   const int kb = K / BK;
@@ -566,8 +606,8 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   // Decode batches of 129 to 256 rows with short k-loops: two row tiles of the narrowest 1-CTA tiles that stay in one wave.  Few 256-row tiles leave pairs idle or pay an exchange of
   // partial sums, 6 us before the first k-block (200 rows, us, pair / this: 2 048 x 512 gated 5.7 / 3.65, 1 024 x 1 024 7.2 / 4.6, 4 096 x 1 024 8.0 / 6.0, 8 192 x 1 024 9.2 / 7.7,
   // 3 584 x 1 792 11.6 / 8.3, 2 048 x 2 048 9.5 / 7.5, 4 096 x 2 048 10.8 / 8.9, 1 024 x 2 048 7.4 / 7.2; longer k-loops read the rows too often: 768 x 2 304 7.2 / 7.35,
-  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4)
-  if (force_bn == 0 && force_splits == 0 && M > BM && M <= 2 * BM && K <= 2048 && g_nvc_gemm_pair) {
+  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4).  bf16 results only: pairs that split K sum fp32 results in shorter chains
+  if (force_bn == 0 && force_splits == 0 && M > BM && M <= 2 * BM && K <= 2048 && out_dtype == NVC_DT_BF16 && g_nvc_gemm_pair) {
     for (int bn : {32, 64, 128})
       if (2 * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
         force_bn = bn + (bn == 128 ? 2000 : 4000);
@@ -577,7 +617,7 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   if (force_bn == 512 || vocab_pair || (force_bn == 0 && M > BM && g_nvc_gemm_pair))
     return nvc_gemm_pair(ctx, A, lda, W, C, ldc, out_dtype == NVC_DT_F32, M, Nout, K, force_splits, epi, stream, trace);
   int bn, kps, splits, ks = 0;
-  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, &bn, &kps, &splits, &ks);
+  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, out_dtype == NVC_DT_F32, &bn, &kps, &splits, &ks);
   if (force_bn) {          // force_bn = BN + 1000 * KPS (KPS 0: the first instantiation of that BN); a digit in front of KPS has no meaning
     bn = force_bn % 1000;
     kps = (force_bn / 1000) % 10;
