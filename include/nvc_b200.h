@@ -165,7 +165,10 @@ int nvc_fused_add_rmsnorm(nvc_ctx* ctx, const nvc_bf16* x, const float* residual
  * (src/models/qwen3.rs:542-550):  C[M, Nout] = A[M, K] * W[Nout, K]^T  (W is the
  * reference's [out, in] layout), bf16 inputs, fp32 accumulation on tcgen05 / TMEM.
  * lda / ldc: row strides in elements.  K % 64 == 0, Nout % 16 == 0, lda % 8 == 0.
- * out_dtype: NVC_DT_BF16 or NVC_DT_F32. */
+ * out_dtype: NVC_DT_BF16 or NVC_DT_F32.
+ * A row's sums are grouped along K by a rule on M, Nout and K alone: a call repeats itself bit by bit, and up to
+ * 128 rows most shapes group alike whatever M is, but at some sizes of M the grouping changes, and with it the
+ * rounding of a row beside other rows. */
 enum { NVC_DT_BF16 = 0, NVC_DT_F32 = 1 };
 int nvc_gemm_bf16(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc,
                   int out_dtype, int M, int Nout, int K, void* stream);

@@ -716,6 +716,13 @@ static void choose_schedule(const nvc_ctx* ctx, int M, int N, int kb, bool gated
     }
 }
 
+// The parts of K that the schedule of up to 256 rows sums apart (sums_of of gemm_tcgen05.cu).
+extern "C" int nvc_gemm_pair_sums(const nvc_ctx* ctx, int M, int N, int K) {
+  int nt = 256, S = 1;
+  choose_schedule(ctx, M, N, K / BK, false, false, &nt, &S);
+  return S;
+}
+
 // force_splits: 0 = choose; 1..4 = in-cluster split-K factor with 256-wide tiles; 10000 * S + 1000 + NT = tile width NT
 extern "C" int nvc_gemm_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32,
                              int M, int N, int K, int force_splits, int epi, void* stream, long long* trace) {

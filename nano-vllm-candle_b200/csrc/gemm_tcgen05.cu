@@ -64,11 +64,12 @@ __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
 // however few columns there are, so a decode product of K 1 024 spent 1.2 us on rows that do not exist; and with half the bytes per k-block of activations the ring holds
 // half as many weights again in front of the dependency (64 rows, us, 128 / 64: 6 144 x 1 024 gated 5.75 / 5.1, 2 048 x 1 024 4.45 / 3.8, 12 288 x 2 048 gated 13.9 / 13.2,
 // 2 048 x 6 144 9.7 / 8.9, 3 072 x 2 048 gated 6.9 / 5.6; 1 row 6 144 x 1 024 gated 5.5 / 4.8)
+// sums: the parts of K that are summed apart and added in order by the epilogue (choose_config), each in BN columns of tensor memory of its own, up to 512 together
 template <int BN, int KPS, bool kExt = false, int RM = BM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                          void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total,
-                         int k_blocks_per_split, int a_box_rows, int prefetch_w, int ks_cluster, int epi, float* __restrict__ ws,
+                         int k_blocks_per_split, int sums, int k_blocks_per_sum, int a_box_rows, int prefetch_w, int ks_cluster, int epi, float* __restrict__ ws,
                          int* __restrict__ counters, long long* __restrict__ trace) {
   using cfg = Cfg<BN, KPS, RM>;
   // optional phase timestamps of CTA (0,0,0) (tools/gemm_microbench.py); NULL in production
@@ -95,6 +96,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   const int kb_end = min(k_blocks_total, kb_begin + k_blocks_per_split);
   const int num_kb = kb_end - kb_begin;
   const int num_it = (num_kb + KPS - 1) / KPS;       // pipeline iterations (stages consumed)
+  const uint32_t tmem_cols = cfg::kTmemCols * (sums <= 2 ? sums : 4);
 
   if (warp == 0 && lane == 0) {
     ptx::tma_prefetch_desc(&tma_a);
@@ -110,7 +112,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       ptx::fence_barrier_init();
     }
     __syncwarp();
-    ptx::tmem_alloc(tmem_slot, cfg::kTmemCols);
+    ptx::tmem_alloc(tmem_slot, tmem_cols);
     ptx::tmem_relinquish();
   }
   ptx::tcgen05_fence_before();
@@ -180,6 +182,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     constexpr uint32_t desc_hi = ptx::umma_desc_hi_sw128(1024);
     const uint32_t a_lo0 = ptx::umma_desc_lo(smem_base, 16);
     const uint32_t b_lo0 = ptx::umma_desc_lo(smem_base + KPS * cfg::kBytesA, 16);
+    uint32_t acc = tmem_base;                        // the present sum's accumulator and its k-blocks so far; one lane is elected every time
+    int in_sum = 0;
     for (int it = 0; it < num_it; ++it) {
       const int s = it % cfg::kStages;
       ptx::mbar_wait(full_bar(s), (it / cfg::kStages) & 1);
@@ -195,9 +199,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k) {
               // 16 bf16 = 32 bytes along K inside the 128-byte swizzle span: +2 in the address field
-              ptx::umma_bf16_ss(tmem_base, ptx::umma_desc(a_lo + j * (cfg::kBytesA >> 4) + 2 * k, desc_hi),
+              ptx::umma_bf16_ss(acc, ptx::umma_desc(a_lo + j * (cfg::kBytesA >> 4) + 2 * k, desc_hi),
                                 ptx::umma_desc(b_lo + j * (cfg::kBytesB >> 4) + 2 * k, desc_hi), idesc,
-                                (it | j | k) != 0 ? 1u : 0u);
+                                (in_sum | k) != 0 ? 1u : 0u);
+            }
+            if (++in_sum == k_blocks_per_sum) {
+              in_sum = 0;
+              acc += BN;
             }
           }
         }
@@ -228,12 +236,33 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 #pragma unroll 1
         for (int c = 0; c < BN / 16; c += 2) {          // two 16-column chunks per tensor-memory round trip
           uint32_t v[32];
+          float f[32];
           ptx::tmem_ld_32x32b_x16(taddr + c * 16, v);
           ptx::tmem_ld_32x32b_x16(taddr + c * 16 + 16, v + 16);
-          ptx::tmem_ld_wait();
-          float f[32];
+          if (sums > 1) {                               // every sum in one round trip, added in order and from zero as a cluster does (-0 becomes 0)
+            uint32_t v1[32], v2[32], v3[32];
+            ptx::tmem_ld_32x32b_x16(taddr + BN + c * 16, v1);
+            ptx::tmem_ld_32x32b_x16(taddr + BN + c * 16 + 16, v1 + 16);
+            if (sums > 2) {
+              ptx::tmem_ld_32x32b_x16(taddr + 2 * BN + c * 16, v2);
+              ptx::tmem_ld_32x32b_x16(taddr + 2 * BN + c * 16 + 16, v2 + 16);
+            }
+            if (sums > 3) {
+              ptx::tmem_ld_32x32b_x16(taddr + 3 * BN + c * 16, v3);
+              ptx::tmem_ld_32x32b_x16(taddr + 3 * BN + c * 16 + 16, v3 + 16);
+            }
+            ptx::tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+            for (int j = 0; j < 32; ++j) {
+              f[j] = 0.f + __uint_as_float(v[j]) + __uint_as_float(v1[j]);
+              if (sums > 2) f[j] += __uint_as_float(v2[j]);
+              if (sums > 3) f[j] += __uint_as_float(v3[j]);
+            }
+          } else {
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+          }
           if (row_ok) emit32<kExt, kExt>(C, out_f32, epi, (int64_t)grow * ldc, n_tile * BN + c * 16, N, f);
         }
       } else {
@@ -379,7 +408,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   if (ks_cluster) ptx::cluster_sync_all();   // nobody exits while a peer may still read its smem
   if (warp == 1) {
     ptx::tcgen05_fence_after();
-    ptx::tmem_dealloc(tmem_base, cfg::kTmemCols);
+    ptx::tmem_dealloc(tmem_base, tmem_cols);
   }
   if (tr && threadIdx.x == 0) trace[83] = clock64();
 }
@@ -402,7 +431,7 @@ int make_tma_2d(nvc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t inner
 
 template <int BN, int KPS, int RM = BM>
 int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
-           int N, int K, int splits, int ks_cluster, int epi, cudaStream_t stream, long long* trace) {
+           int N, int K, int splits, int ks_cluster, int sums, int epi, cudaStream_t stream, long long* trace) {
   using cfg = Cfg<BN, KPS, RM>;
   CUtensorMap ta, tb;
   // a single partial m-tile only needs the rows that exist (rounded to the 8-row swizzle atom)
@@ -414,6 +443,9 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   const int kb_total = K / BK;
   const int kb_per = (kb_total + splits - 1) / splits;
   const int eff_splits = (kb_total + kb_per - 1) / kb_per;   // no empty splits
+  const int kb_sum = (kb_total + sums - 1) / sums;
+  sums = (kb_total + kb_sum - 1) / kb_sum;
+  NVC_REQUIRE(ctx, sums == 1 || (eff_splits == 1 && BN >= 32 && sums <= 4 && sums * BN <= 512), NVC_EINVAL, "these sums do not fit the tensor memory of one CTA");
   const int n_tiles = (N + BN - 1) / BN;
   dim3 grid(n_tiles, (M + BM - 1) / BM, eff_splits);
   // ks_cluster: the eff_splits CTAs of one output tile form a cluster (1,1,S) and reduce over DSMEM
@@ -425,7 +457,7 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   if constexpr (has_ext(BN)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true, RM>; }
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
                                           stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
-                                          kb_per, a_rows,
+                                          kb_per, sums, kb_sum, a_rows,
                                           // first ring lap of W before the dependency wait + L2 prefetch ahead of the ring, up to 256 rows and below
                                           // 32 MB of weights: 148 rings of 190 KB hold 28 MB, so that nearly all of W is on chip when the activations
                                           // arrive, however long the k-loop (us, without / with: 6 144 x 1 024 gated 5.7 / 4.8, 2 560 x 4 096 8.2 / 7.7,
@@ -444,80 +476,62 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
 #define NVC_GEMM_CONFIGS(X) X(256, 1) X(128, 1) X(128, 2) X(64, 2) X(64, 4) X(32, 4) X(16, 4) X(96, 2)
 #define NVC_GEMM_FEW_ROWS(X) X(256, 1) X(128, 2) X(64, 4) X(32, 4)      // with products of 64 rows: what the choice may take for up to 64
 
-// Tile choice, fitted to tools/gemm_microbench.py (CUDA-graph timing + CTA phase traces) on B200:
-//  * a CTA ingests ~60 B/clk through TMA when the operands stream from HBM, so a k-block costs
-//    max(2*BN [tcgen05 floor], (rows + BN) * 128 / 60 [TMA]) cycles, plus ~2500 cycles of
-//    prologue + first-load latency + epilogue per CTA;
-//  * decode (M <= 128): one wave, as many CTAs as the N dimension gives (up to ~all SMs), several
-//    k-blocks per pipeline stage; split-K through the L2 workspace costs >= 6 us (ticket atomic +
-//    reduction round trips) and never won in the sweep, so it is only used when forced.
-void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, bool f32, int* bn_out, int* kps_out, int* splits_out,
-                   int* ks_out) {
+// In how many parts the K of a product of up to 128 rows is summed: 1, 2 or 4 runs of k-blocks, added in order.  The parts belong to a result's bits, so they do not follow the tile that runs
+// the product: one CTA with an accumulator per part and a cluster with a CTA per part give the same.  Short chains also keep fp32 results closer (200 rows of K 2 048, error against
+// 64 bits: one part 2.1e-6, four 4.7e-7).  The rule is the split of a cycle model of 128-row products (a k-block costs (rows + bn) 128 / 90 + 90 cycles, a cluster's exchange 2 300 and
+// 17 bytes per cycle).  At a few sizes it goes by the rows, and a row's rounding with it by the rows beside it (1 024 x 1 024: one part up to 24 rows, then four; 6 144 x 2 560: four up to 48, then two).
+int sums_of(const nvc_ctx* ctx, int M, int N, int K) {
+  const int rows = ((M + 7) / 8) * 8, kb = K / BK;
+  int sums = 1;
+  double best = 1e30;
+  const double hbm_floor = (double)N * K * 2 / 3400.0 + 3000.0;     // 6.5 TB/s at 1.9 GHz
+  for (int bn : {32, 64, 128, 256})
+    for (int S : {1, 2, 4}) {
+      if (S > 1 && (!g_nvc_gemm_ks || kb / S < 4)) continue;
+      if (bn / 2 >= N) continue;
+      const int cap = S == 1 ? ctx->num_sms : S * (ctx->pair_clusters[S / 2] > 0 ? ctx->pair_clusters[S / 2] : ctx->num_sms / (S == 2 ? 2 : 5));
+      const double waves = ceil((double)((N + bn - 1) / bn) * S / cap);
+      const double per_kb = (double)(rows + bn) * 128.0 / 90.0 + 90.0;
+      const double tail = S == 1 ? 300.0 + 6.0 * bn : 2300.0 + (double)(S - 1) * rows * (bn / S) * 4.0 / 17.0;
+      const double t = waves * (2200.0 + per_kb * ((kb + S - 1) / S) + tail);
+      // below the HBM floor every candidate takes the floor: rank those by the modeled CTA time (most slack)
+      const double key = t > hbm_floor ? t : hbm_floor * (1.0 + 1e-3 * t / hbm_floor);
+      if (key < best * 0.98 || (key < best && t < hbm_floor)) { best = key; sums = S; }
+    }
+  return sums;
+}
+
+// Tile choice: one wave where it can, several k-blocks per pipeline stage; split K through the workspace (a ticket and two round trips, 6 us and more) only when forced.
+void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, int* bn_out, int* kps_out, int* splits_out, int* ks_out, int* sums_out) {
   *splits_out = 1;
   *ks_out = 0;
-  if (M <= BM && !f32) {
-    // Decode with bf16 results, in us: fitted to measured products of K 512 - 12 288 and N 256 - 24 576, by size of the tensor products they run on.
-    // 64 rows: 1 675 configurations of 28 products, those within 15 % of a product's best (residual 4.3 %); what it picks is 0.6 % slower than the best in the mean, 7 % at most,
-    // beside what was picked and run with 128 rows 9.8 % faster, nowhere slower.  128 rows: 28 products of 72 - 128 rows; 0.1 % and 6 % slower than the best; beside the cycle model in
-    // its place, on 16 more products too, 1.1 % faster in the mean (2 048 x 1 024 5.47 -> 4.8, 6 144 x 2 560 13.2 -> 11.7, 6 144 x 4 096 18.8 -> 17.4), at most 1.5 % slower.
-    // A cluster's start waits for all of its SMs, the longer the fuller the chip: the cube.
+  *sums_out = 1;
+  if (M <= BM) {
+    // Decode, in us: fitted to measured products of K 512 - 12 288 and N 256 - 24 576, by size of the tensor products they run on.
+    // 64 rows: 1 675 configurations of 28 products, those within 15 % of a product's best (residual 4.3 %).  128 rows: 28 products of 72 - 128 rows.
+    // A cluster's start waits for all of its SMs, the longer the fuller the chip: the cube.  Several sums in one CTA cost their accumulators' starts and reads (0.21, 0.31, 0.53 us for four of
+    // 32, 64, 128 columns), at 128 rows within the residual.  Of the measured tiles with the right sums what it picks is 0.8 % slower than the best in the mean (16 products, 1 - 128 rows).
+    // Beside one sum wherever no cluster pays, several cost 1.3 % in the mean up to 64 rows, 0.7 % up to 128 (6 144 x 4 096, 100 rows 16.7 / 17.9), and beside clusters wherever there are
+    // several sums, on products of 128 rows, they save 8.7 % and 1.9 % (us, that / this: 2 048 x 1 024 4.3 / 3.45, 6 144 x 2 560 11.1 / 8.9, 6 144 x 4 096 16.2 / 13.6, 128 rows 18.4 / 18.5)
     const bool few = M <= 64;
-    const int rows = ((M + 7) / 8) * 8, kb = K / BK;
+    const int rows = ((M + 7) / 8) * 8, kb = K / BK, sums = allow_split ? sums_of(ctx, M, N, K) : 1;
     double best = 1e30;
     for (int bn : {32, 64, 128, 256})
       for (int S : {1, 2, 4}) {
-        if (S > 1 && (!allow_split || !g_nvc_gemm_ks || kb / S < 4)) continue;
+        if (S > 1 ? S != sums : bn * sums > 512) continue;
         if (bn / 2 >= N) continue;
         const int ctas = (N + bn - 1) / bn * S, cap = S == 1 ? ctx->num_sms : S * (ctx->pair_clusters[S / 2] > 0 ? ctx->pair_clusters[S / 2] : ctx->num_sms / (S == 2 ? 2 : 5));
         const double fill = ctas < cap ? (double)ctas / cap : 1.0;
         double t = ceil((double)ctas / cap) * (few ? 2.17 + (kb + S - 1) / S * (0.0331 + 0.00077 * bn + 0.00018 * rows)
                                                    : 1.65 + (kb + S - 1) / S * (0.096 + 0.00168 * bn + 0.000277 * rows));
+        if (S == 1 && few && sums > 1) t += 0.1 + 0.0011 * bn * (sums - 1);
         if (S > 1) t += few ? 0.69 + 0.73 * fill * fill * fill + 0.00021 * rows * bn * (S - 1) / S : 1.22 + 1.02 * fill * fill * fill + 0.000164 * rows * bn * (S - 1) / S;
         if (t < best) { best = t; *bn_out = bn; *splits_out = S; }
       }
     if (best > 1e29) *bn_out = 32;
     *kps_out = *bn_out == 256 ? 1 : (*bn_out == 128 ? 2 : 4);
     *ks_out = *splits_out > 1 ? 1 : 0;
-    return;
-  }
-  if (M <= BM) {
-    // fp32 results keep the splits of this model: the accumulators' error grows with the length of their chains, and the model above takes longer ones where a cluster does not pay.
-    // (100 rows, error against 64 bits: 2 048 x 1 024 in fp32 2.3e-7 with these splits, 1.0e-6 without, in bf16 1.660e-3 both; 200 rows of K 2 048 4.7e-7 with, 2.1e-6 without.)
-    // Cycle model fitted to CTA phase traces (tools/gemm_microbench.py --trace-decode):
-    // the TMA unit of an SM moves ~90 B/clk plus ~30 cycles per box (two loads + one L2 prefetch per k-block),
-    // whatever the source (the L2 prefetch before the PDL wait hides HBM), and the activation rows are re-read
-    // by every n-tile, so a k-block costs (rows + BN) * 128 / 90 + 90 cycles; ~2200 cycles of prologue +
-    // first-load latency; epilogue 300 + 6 * BN, or, with split-K inside a cluster (1,1,S), ~2300 + the DSMEM
-    // exchange at ~17 B/clk.  The winners are always ONE wave of ~96-132 CTAs with the widest tile that allows it
-    // (co-resident: 148 CTAs, 74 clusters of 2, 33 clusters of 4).
-    const int rows = ((M + 7) / 8) * 8;
-    const int kb = K / BK;
-    const int bns[4] = {32, 64, 128, 256};
-    const int ss[3] = {1, 2, 4};
-    double best = 1e30;
-    int best_bn = 32, best_s = 1;
-    const double hbm_floor = (double)N * K * 2 / 3400.0 + 3000.0;     // 6.5 TB/s at 1.9 GHz
-    for (int i = 0; i < 4; ++i) {
-      for (int j = 0; j < 3; ++j) {
-        const int bn = bns[i], S = ss[j];
-        if (S > 1 && (!allow_split || !g_nvc_gemm_ks || kb / S < 4)) continue;
-        if (bn / 2 >= N) continue;
-        const int tiles = (N + bn - 1) / bn;
-        const int cap = S == 1 ? ctx->num_sms : (S == 2 ? 2 * (ctx->pair_clusters[1] > 0 ? ctx->pair_clusters[1] : ctx->num_sms / 2)
-                                                       : 4 * (ctx->pair_clusters[2] > 0 ? ctx->pair_clusters[2] : ctx->num_sms / 5));
-        const double waves = ceil((double)tiles * S / cap);
-        const double per_kb = (double)(rows + bn) * 128.0 / 90.0 + 90.0;
-        const double tail = S == 1 ? 300.0 + 6.0 * bn : 2300.0 + (double)(S - 1) * rows * (bn / S) * 4.0 / 17.0;
-        const double t = waves * (2200.0 + per_kb * ((kb + S - 1) / S) + tail);
-        // below the HBM floor every candidate takes the floor: rank those by the modeled CTA time (most slack)
-        const double key = t > hbm_floor ? t : hbm_floor * (1.0 + 1e-3 * t / hbm_floor);
-        if (key < best * 0.98 || (key < best && t < hbm_floor)) { best = key; best_bn = bn; best_s = S; }
-      }
-    }
-    *bn_out = best_bn;
-    *kps_out = best_bn == 256 ? 1 : (best_bn == 128 ? 2 : 4);
-    *splits_out = best_s;
-    *ks_out = best_s > 1 ? 1 : 0;
+    if (*splits_out == 1) *sums_out = sums;
     return;
   }
   const int kb = K / BK;
@@ -605,32 +619,35 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   }
   // Decode batches of 129 to 256 rows with short k-loops: two row tiles of the narrowest 1-CTA tiles that stay in one wave.  Few 256-row tiles leave pairs idle or pay an exchange of
   // partial sums, 6 us before the first k-block (200 rows, us, pair / this: 2 048 x 512 gated 5.7 / 3.65, 1 024 x 1 024 7.2 / 4.6, 4 096 x 1 024 8.0 / 6.0, 8 192 x 1 024 9.2 / 7.7,
-  // 3 584 x 1 792 11.6 / 8.3, 2 048 x 2 048 9.5 / 7.5, 4 096 x 2 048 10.8 / 8.9, 1 024 x 2 048 7.4 / 7.2; longer k-loops read the rows too often: 768 x 2 304 7.2 / 7.35,
-  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4).  bf16 results only: pairs that split K sum fp32 results in shorter chains
+  // 3 584 x 1 792 11.6 / 8.5, 2 048 x 2 048 9.5 / 7.5, 4 096 x 2 048 10.8 / 9.0, 1 024 x 2 048 7.4 / 7.3; longer k-loops read the rows too often: 768 x 2 304 7.2 / 7.35,
+  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4).  Each sums K in the parts of the pairs' schedule.  fp32 results are left on pairs
   if (force_bn == 0 && force_splits == 0 && M > BM && M <= 2 * BM && K <= 2048 && out_dtype == NVC_DT_BF16 && g_nvc_gemm_pair) {
     for (int bn : {32, 64, 128})
       if (2 * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
         force_bn = bn + (bn == 128 ? 2000 : 4000);
+        force_splits = 200 + nvc_gemm_pair_sums(ctx, M, Nout, K);
         break;
       }
   }
   if (force_bn == 512 || vocab_pair || (force_bn == 0 && M > BM && g_nvc_gemm_pair))
     return nvc_gemm_pair(ctx, A, lda, W, C, ldc, out_dtype == NVC_DT_F32, M, Nout, K, force_splits, epi, stream, trace);
-  int bn, kps, splits, ks = 0;
-  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, out_dtype == NVC_DT_F32, &bn, &kps, &splits, &ks);
+  int bn, kps, splits, ks = 0, sums = 1;
+  choose_config(ctx, M, Nout, K, epi == NVC_EPI_NONE, &bn, &kps, &splits, &ks, &sums);
   if (force_bn) {          // force_bn = BN + 1000 * KPS (KPS 0: the first instantiation of that BN); a digit in front of KPS has no meaning
     bn = force_bn % 1000;
     kps = (force_bn / 1000) % 10;
     if (kps == 0) kps = bn >= 128 ? 1 : (bn == 64 ? 2 : 4);
     ks = 0;
     splits = 1;
+    sums = 1;
   }
-  // force_splits: 1..99 = split-K through the global workspace; 100 + S = split-K inside a cluster (1,1,S), S <= 8
-  if (force_splits >= 100) { splits = force_splits - 100; ks = 1; }
-  else if (force_splits) { splits = force_splits; ks = 0; }
+  // force_splits: 1..99 = split-K through the global workspace; 100 + S = split-K inside a cluster (1,1,S), S <= 8; 200 + S = S sums in one CTA, S <= 4
+  if (force_splits > 200) { splits = 1; ks = 0; sums = force_splits - 200; }
+  else if (force_splits >= 100) { splits = force_splits - 100; ks = 1; sums = 1; }
+  else if (force_splits) { splits = force_splits; ks = 0; sums = 1; }
   NVC_REQUIRE(ctx, !ks || splits <= 8, NVC_EINVAL, "cluster split-K supports at most 8 splits");
   if (epi != NVC_EPI_NONE) {       // the fused epilogue lives in the direct-store path: no split-K, tiles of >= 32 columns
-    NVC_REQUIRE(ctx, force_splits == 0 || force_splits == 1, NVC_EINVAL, "fused epilogue cannot be combined with split-K");
+    NVC_REQUIRE(ctx, force_splits == 0 || force_splits == 1 || force_splits > 200, NVC_EINVAL, "fused epilogue cannot be combined with split-K");
     splits = 1;
     ks = 0;
     if (bn < 32) { bn = 32; kps = 4; }
@@ -644,12 +661,12 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
   cudaStream_t st = nvc_stream(stream);
   const int f32 = out_dtype == NVC_DT_F32;
   if (M <= 64 && (splits == 1 || ks)) {
-#define X(BN, KPS) if (bn == BN && kps == KPS) return launch<BN, KPS, 64>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
+#define X(BN, KPS) if (bn == BN && kps == KPS) return launch<BN, KPS, 64>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, sums, epi, st, trace);
     NVC_GEMM_FEW_ROWS(X)
 #undef X
   }
 #define X(BN, KPS) \
-  if (bn == BN && kps == KPS) return launch<BN, KPS>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, epi, st, trace);
+  if (bn == BN && kps == KPS) return launch<BN, KPS>(ctx, A, lda, W, C, ldc, f32, M, Nout, K, splits, ks, sums, epi, st, trace);
   NVC_GEMM_CONFIGS(X)
 #undef X
   NVC_REQUIRE(ctx, false, NVC_EINVAL, "unsupported tile configuration");

@@ -25,6 +25,7 @@ int nvc_gemm_grouped_init(nvc_ctx* ctx);
 // CTA-pair (cta_group::2) GEMM for M > 128; force_splits 0 = choose the in-cluster split-K factor
 int nvc_gemm_pair(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
                   int N, int K, int force_splits, int epi, void* stream, long long* trace);
+int nvc_gemm_pair_sums(const nvc_ctx* ctx, int M, int N, int K);
 // fp32 C [M <= 128 tokens, N] = X . W^T with the operands swapped in the pair kernel (lm_head at decode batch sizes)
 int nvc_gemm_pair_swapped(nvc_ctx* ctx, const nvc_bf16* X, int ldx, const nvc_bf16* W, float* C, int ldc, int M, int N, int K,
                           void* stream, long long* trace);

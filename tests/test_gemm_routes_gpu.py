@@ -86,3 +86,51 @@ def test_two_row_tiles(ctx, M, N, K):
     """129 to 256 rows over K up to 2 048 run on two row tiles of 32, 64 or 128 columns as long as these are one wave; a column tile more, a row more or a longer K does not.
     The same bounds as for few rows."""
     test_few_rows(ctx, M, N, K)
+
+
+@pytest.mark.parametrize("bn,kps", [(32, 4), (64, 4), (128, 2), (256, 1)])
+@pytest.mark.parametrize("M", [1, 17, 63, 64, 65, 100, 128])
+@pytest.mark.parametrize("S", [2, 3, 4])
+def test_sums_in_one_block_are_those_of_a_cluster(ctx, M, bn, kps, S):
+    """Parts of K that one CTA sums in accumulators of its own and those of a cluster of one CTA per part: the same bits, inside bands that keep their marks.  22 k-blocks: a short last part; 1 040
+    columns: a ragged last tile.  Sums of exact products in fp32: 1e-4 of the largest."""
+    N, K = 1040, 1408
+    g = torch.Generator(device="cuda").manual_seed(M + bn + S)
+    a, w = torch.randn(M, K, generator=g, device="cuda").to(BF16), (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    want = a.double() @ w.double().T
+    for dt in (BF16, torch.float32):
+        apart = ctx.gemm(a, w, out_dtype=dt, force_bn=bn + 1000 * kps, force_splits=100 + S)
+        assert float(((apart.double() - want).abs() - (2.0 ** -8 if dt == BF16 else 0) * want.abs()).max()) <= 1e-4 * float(want.abs().max())
+        buf = torch.full((M + 1, N + 16), 7.0, device="cuda", dtype=dt)
+        if bn * S > 512:
+            with pytest.raises(RuntimeError):
+                ctx.gemm(a, w, out_dtype=dt, out=buf[:M, :N], force_bn=bn + 1000 * kps, force_splits=200 + S)
+            continue
+        ctx.gemm(a, w, out_dtype=dt, out=buf[:M, :N], force_bn=bn + 1000 * kps, force_splits=200 + S)
+        assert torch.equal(buf[:M, :N], apart) and bool((buf[M] == 7.0).all()) and bool((buf[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("N,K,S", [(1024, 2048, 4), (2048, 2048, 4), (4096, 2048, 4), (2560, 4096, 4), (4096, 4096, 4), (6144, 4096, 4), (5120, 8192, 4), (1024, 3072, 4), (4096, 1024, 1)])
+@pytest.mark.parametrize("dt", [BF16, torch.float32])
+def test_a_row_alone_and_beside_others(ctx, N, K, S, dt):
+    """Products of up to 128 rows sum K in as many parts as before, whichever tile runs them: those of the forced cluster, bit by bit, and the same for a row alone and beside any number of others."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a, w = torch.randn(128, K, generator=g, device="cuda").to(BF16), (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    forced = ctx.gemm(a, w, out_dtype=dt, force_bn=4064, force_splits=100 + S if S > 1 else 1)
+    for M in (1, 16, 17, 40, 41, 49, 64, 65, 100, 128):
+        assert torch.equal(ctx.gemm(a[:M], w, out_dtype=dt), forced[:M])
+
+
+@pytest.mark.parametrize("M", [129, 200, 256])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (1024, 2048), (4096, 2048), (2048, 2048), (3584, 1792), (64, 2048), (9472, 576), (4096, 3072)])
+def test_two_row_tiles_sum_like_pairs(ctx, M, N, K):
+    """129 to 256 rows: the same bits as on CTA pairs with the splits of their schedule, plain and gated, inside bands that keep their marks"""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g, device="cuda").to(BF16), (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    buf = torch.full((M + 1, N + 16), 7.0, device="cuda", dtype=BF16)
+    ctx.gemm(a, w, out=buf[:M, :N])
+    assert torch.equal(buf[:M, :N], ctx.gemm(a, w, force_bn=512)) and bool((buf[M] == 7.0).all()) and bool((buf[:, N:] == 7.0).all())
+    if N % 32 == 0:
+        buf = torch.full((M + 1, N // 2 + 16), 7.0, device="cuda", dtype=BF16)
+        ctx.gemm_silu_mul(a, w, out=buf[:M, :N // 2])
+        assert torch.equal(buf[:M, :N // 2], ctx.gemm_silu_mul(a, w, force_bn=512)) and bool((buf[M] == 7.0).all()) and bool((buf[:, N // 2:] == 7.0).all())
