@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
         } else {
           for (int i = 0; i < taps; ++i) apply(i, input(i));
         }
-        y[k] = make_float4(acc.x * sigmoid_f32(acc.x), acc.y * sigmoid_f32(acc.y), acc.z * sigmoid_f32(acc.z), acc.w * sigmoid_f32(acc.w));
+        y[k] = silu4(acc);
         ss4 += y[k].x * y[k].x + y[k].y * y[k].y + y[k].z * y[k].z + y[k].w * y[k].w;
       }
     }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128, 8) delta_prep_kernel(const DeltaArgs a) {
       else x = fresh ? 0.f : cs[(int64_t)(p.taps - 1 + src) * C + ch + j];
       acc = fmaf(__ldg(p.conv_w + (int64_t)i * C + ch + j), x, acc);
     }
-    const float y = acc * sigmoid_f32(acc);
+    const float y = silu_f32(acc);
     out[j] = y;
     ss += y * y;
   }

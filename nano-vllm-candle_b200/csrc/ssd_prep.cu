@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kPrepThreads) ssd_prep_kernel(const SsdArgs a)
     }
   }
 #pragma unroll
-  for (int u = 0; u < CW; ++u) y[u] = acc[u] * sigmoid_f32(acc[u]);
+  for (int u = 0; u < CW; ++u) y[u] = silu_f32(acc[u]);
   float* out;
   if (c < inner) {
     const float dt = s_dt[c / p.vdim - h_first];
