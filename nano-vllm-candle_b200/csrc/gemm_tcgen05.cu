@@ -607,25 +607,20 @@ static int gemm_impl(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W
                              swap_n && g_nvc_gemm_pair;
   if (vocab_swapped || (force_bn == 513 && out_dtype == NVC_DT_F32 && epi == NVC_EPI_NONE && M <= BM))
     return nvc_gemm_pair_swapped(ctx, A, lda, W, reinterpret_cast<float*>(C), ldc, M, Nout, K, stream, trace);
-  // Narrow products over many rows (a router: 64 columns) fill few CTA pairs and are one k-loop long: the narrowest 1-CTA tiles that stay in one wave
-  // (us, pair / this: 1 000 x 64 x 1 024 8.1 / 4.7, 4 000 x 64 x 2 048 10.8 / 7.0, 4 000 x 256 x 1 024 10.6 / 6.1, 16 000 x 128 x 1 024 11.6 / 8.4; two waves lose:
-  // 16 000 x 256 x 2 048 17.5 / 23.5, and so does a long k-loop over few rows: 200 x 64 x 4 096 8.2 / 10.8, 160 x 16 x 2 048 6.4 / 6.7, 384 x 16 x 2 048 9.0 / 6.7)
-  if (force_bn == 0 && force_splits == 0 && epi == NVC_EPI_NONE && M > BM && Nout <= 256 && K <= (M <= 2 * BM ? 1536 : 2048)) {
+  // Two kinds of products above 128 rows fill few CTA pairs and are one short k-loop: they run on the narrowest 1-CTA tiles that stay in one wave.
+  // Narrow ones over many rows (a router: 64 columns; us, pair / this: 1 000 x 64 x 1 024 8.1 / 4.7, 4 000 x 64 x 2 048 10.8 / 7.0, 4 000 x 256 x 1 024 10.6 / 6.1, 16 000 x 128 x 1 024
+  // 11.6 / 8.4, 384 x 16 x 2 048 9.0 / 6.7; 160 x 16 6.3 / 4.0 at K 1 024 and 5.5 / 5.0 at 1 536; two waves lose: 16 000 x 256 x 2 048 17.5 / 23.5), K in one sum.
+  // bf16 results of 129 to 256 rows, K summed in the parts of the pairs' schedule: few 256-row tiles leave pairs idle or pay an exchange of partial sums, 6 us before the first k-block
+  // (200 rows: 2 048 x 512 gated 5.7 / 3.65, 1 024 x 1 024 7.2 / 4.6, 4 096 x 1 024 8.0 / 6.0, 8 192 x 1 024 9.2 / 7.7, 3 584 x 1 792 11.6 / 8.5, 2 048 x 2 048 9.5 / 7.5,
+  // 4 096 x 2 048 10.8 / 9.0, 1 024 x 2 048 7.4 / 7.3); longer k-loops read the rows too often (768 x 2 304 7.2 / 7.35, 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4), those of few
+  // columns, whose pairs split K in four, sooner (64 columns of K 1 600 5.95 / 5.6, 1 792 5.97 / 5.96, 2 048 6.15 / 6.45; 512 of 1 600 6.1 / 5.9, 1 792 6.15 / 6.24, 2 048 6.35 / 6.7).
+  const bool narrow = epi == NVC_EPI_NONE && M > BM && Nout <= 256 && K <= (M <= 2 * BM ? 1536 : 2048);
+  const bool two_rows = M > BM && M <= 2 * BM && K <= (Nout < 1024 ? 1664 : 2048) && out_dtype == NVC_DT_BF16 && g_nvc_gemm_pair;
+  if (force_bn == 0 && force_splits == 0 && (narrow || two_rows)) {
     for (int bn : {32, 64, 128})
       if ((int64_t)((M + BM - 1) / BM) * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
         force_bn = bn + (bn == 128 ? 2000 : 4000);
-        break;
-      }
-  }
-  // Decode batches of 129 to 256 rows with short k-loops: two row tiles of the narrowest 1-CTA tiles that stay in one wave.  Few 256-row tiles leave pairs idle or pay an exchange of
-  // partial sums, 6 us before the first k-block (200 rows, us, pair / this: 2 048 x 512 gated 5.7 / 3.65, 1 024 x 1 024 7.2 / 4.6, 4 096 x 1 024 8.0 / 6.0, 8 192 x 1 024 9.2 / 7.7,
-  // 3 584 x 1 792 11.6 / 8.5, 2 048 x 2 048 9.5 / 7.5, 4 096 x 2 048 10.8 / 9.0, 1 024 x 2 048 7.4 / 7.3; longer k-loops read the rows too often: 768 x 2 304 7.2 / 7.35,
-  // 6 144 x 2 560 13.0 / 14.0, 1 024 x 3 072 8.4 / 10.4).  Each sums K in the parts of the pairs' schedule.  fp32 results are left on pairs
-  if (force_bn == 0 && force_splits == 0 && M > BM && M <= 2 * BM && K <= 2048 && out_dtype == NVC_DT_BF16 && g_nvc_gemm_pair) {
-    for (int bn : {32, 64, 128})
-      if (2 * ((Nout + bn - 1) / bn) <= ctx->num_sms) {
-        force_bn = bn + (bn == 128 ? 2000 : 4000);
-        force_splits = 200 + nvc_gemm_pair_sums(ctx, M, Nout, K);
+        if (!narrow) force_splits = 200 + nvc_gemm_pair_sums(ctx, M, Nout, K);
         break;
       }
   }
