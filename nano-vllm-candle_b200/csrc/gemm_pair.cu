@@ -760,11 +760,13 @@ extern "C" int nvc_gemm_pair_qk(nvc_ctx* ctx, const nvc_bf16* A, int lda, const 
   auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   if (N != (nh + 2 * kv) * 128 || K % BK != 0 || lda < K || (lda | ldc) % 8 || !al16(A) || !al16(W) || !al16(C)) return NVC_ENOTIMPL;
   // The fusion saves a pass over the rows and lengthens the epilogue, of which all but the last wave's runs under the next tile's main loop; but it is bound to 256-wide
-  // tiles without splits.  It wins wherever these fill the chip: from two waves on, and at one or two waves that are 85 % full (one call against two kernels, us:
+  // tiles without splits.  It wins wherever these fill the chip: above two waves, and at one or two waves that are 85 % full (one call against two kernels, us:
   // 3 000 x 4 096 x 1 024, 2.6 waves: 30.5 / 36.6; 6 555 rows, 5.6: 50 / 72; 2 600 x 4 096 x 2 048, 2.4: 42.8 / 46.3; 2 000 x 4 096 x 1 024, 1.73: 23.3 / 27.8; 1 000, 0.86:
-  // 16.1 / 18.2; 700 x 6 144 x 2 560, 0.97: 30.7 / 33.6; it loses at 1 300 x 4 096 x 2 048, 1.3: 31.2 / 29.7, and 500 x 6 144 x 4 096, 0.65: 34.7 / 28.9)
+  // 16.1 / 18.2; 700 x 6 144 x 2 560, 0.97: 30.7 / 33.6; it loses at 1 300 x 4 096 x 2 048, 1.3: 31.2 / 29.7, and 500 x 6 144 x 4 096, 0.65: 34.7 / 28.9).  From K 2 048 on a third wave has to be a
+  // quarter full too (6 144 columns, 2.05 waves: K 2 048 43.7 / 42.9, K 4 096 83 / 73; 2.16: 45.0 / 42.8, 87 / 75; 2.27: 43.6 / 48.9, 71 - 86 / 75 - 82; 2.38: 44.4 / 48.5, 84.5 / 87.4; but
+  // 2.05 of K 1 024 26.6 / 28.2 and of 512 21.6 / 23.6; 3.03 of K 4 096 109 / 110)
   const int pairs = ctx->num_sms / 2, tiles = ((M + 255) / 256) * ((N + 255) / 256), waves = (tiles + pairs - 1) / pairs;
-  if (M <= kTileM || (waves <= 2 && 20 * tiles < 17 * waves * pairs)) return NVC_ENOTIMPL;
+  if (M <= kTileM || (waves <= 2 && 20 * tiles < 17 * waves * pairs) || (K >= 2048 && 4 * tiles < 3 * waves * pairs)) return NVC_ENOTIMPL;
   int nt = 256, S = 1;
   choose_schedule(ctx, M, N, K / BK, false, true, &nt, &S);
   if (nt != 256 || S != 1) return NVC_ENOTIMPL;
