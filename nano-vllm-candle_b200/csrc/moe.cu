@@ -466,10 +466,11 @@ static int sort_padded(nvc_ctx* ctx, const int32_t* topk_idx, int N, int top, in
   NVC_REQUIRE(ctx, !tile_group || (align > 1 && (int64_t)tiles_cap * align >= (int64_t)N * top + (int64_t)E * (align - 1)), NVC_EINVAL,
               "tile_group needs align > 1 and room for every group's padding");
   const int P = N * top;
-  // Eight CTAs cost 0.8 - 1.1 us of cluster launch and barriers.  They divide the pairs, and a warp's walks over padded groups where there are more than 32 of them (us, one / eight CTAs, pairs to
-  // experts, groups of 128 rows: to 8 experts 3 200 4.2 / 4.4, 4 800 4.8 / 4.4; to 16 2 000 4.0 / 4.5, 3 200 4.8 / 4.5, 8 000 7.6 / 4.6; to 64 1 000 5.3 / 6.05, 2 000 6.4 / 6.2; to 95 32 4.7 / 5.1,
-  // 1 000 6.45 / 6.5, 2 000 7.6 / 6.6; to 128 8 5.3 / 5.5, 128 6.5 / 5.9, 32 000 43.8 / 11.0; to 256 8 8.2 / 7.15; unpadded to 128 2 000 6.2 / 6.3, 4 800 9.0 / 6.6)
-  const int C = P + (int64_t)((E + 31) / 32 - 1) * (align - 1) * 9 > 3500 ? 8 : 1;
+  // Eight CTAs cost 0.8 - 1.1 us of cluster launch and barriers.  They divide the pairs, which take longer the more experts there are, and the walks over padded groups, 32 of them at a time (us, one /
+  // eight CTAs, pairs to experts, groups of 128 rows: to 8 experts 3 200 4.2 / 4.4, 4 800 4.8 / 4.4; to 16 2 000 4.0 / 4.5, 3 200 4.8 / 4.5, 8 000 7.6 / 4.6; to 32 2 000 5.0 / 5.5, 3 200 5.95 /
+  // 5.55; to 64 1 000 5.3 / 6.05, 2 000 6.4 / 6.2; to 95 32 4.7 / 5.1, 1 000 6.45 / 6.5, 2 000 7.6 / 6.6; to 128 8 5.35 / 5.5, with the rows behind the groups filled 6.15 / 5.6, 128 6.5 / 5.9,
+  // 32 000 43.8 / 11.0; to 256 8 8.2 / 7.15; unpadded to 128 2 000 6.2 / 6.3, 3 200 7.25 / 6.5)
+  const int C = P + (int64_t)E * E * (align - 1) / 690 > (E > 16 ? 3000 : 3500) ? 8 : 1;
   auto kernel = C == 8 ? moe_sort_kernel<8> : moe_sort_kernel<1>;
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster(ctx, kernel, dim3(C), dim3(1024), (size_t)(32 * (E | 1) + (C > 1 ? 4 : 2) * E + 1) * sizeof(int32_t), nvc_stream(stream), C,
                                          topk_idx, P, top, E, E_real, align, offsets, src_rows, pos, tile_group, tiles_cap, tail_cap, tail));
