@@ -138,7 +138,7 @@ def test_guard_qk_norm_rope_store_and_attention(ctx):
 
 
 def test_guard_qkv_proj_norm_rope_fused(ctx):
-    """K3 + K2 as one kernel (M >= 8192 takes the fused epilogue at any K): qkv rows and both caches inside sentinel bands, M ragged"""
+    """K3 + K2 as one kernel (132 tiles: two waves that are 89 % full take the fused epilogue): qkv rows and both caches inside sentinel bands, M ragged"""
     g = torch.Generator().manual_seed(9)
     nh, kv, hd, bs, K = 4, 2, 128, 16, 256
     M = 8192 + 77
