@@ -64,8 +64,9 @@ __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
 // however few columns there are, so a decode product of K 1 024 spent 1.2 us on rows that do not exist; and with half the bytes per k-block of activations the ring holds
 // half as many weights again in front of the dependency (64 rows, us, 128 / 64: 6 144 x 1 024 gated 5.75 / 5.1, 2 048 x 1 024 4.45 / 3.8, 12 288 x 2 048 gated 13.9 / 13.2,
 // 2 048 x 6 144 9.7 / 8.9, 3 072 x 2 048 gated 6.9 / 5.6; 1 row 6 144 x 1 024 gated 5.5 / 4.8)
-// sums: the parts of K that are summed apart and added in order by the epilogue (choose_config), each in BN columns of tensor memory of its own, up to 512 together
-template <int BN, int KPS, bool kExt = false, int RM = BM>
+// kSums: K is summed in `sums` parts (sums_of), each in BN columns of tensor memory of its own, up to 512 together, added in order by the epilogue.  A variant, because its
+// registers (106 -> 110 to 154) keep the next kernel's CTAs off the SM: 6 144 x 1 024 gated in a chain of layers 5.1 -> 5.4 us when all products had them
+template <int BN, int KPS, bool kExt = false, int RM = BM, bool kSums = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                          void* __restrict__ C, int ldc, int out_f32, int M, int N, int k_blocks_total,
@@ -96,7 +97,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   const int kb_end = min(k_blocks_total, kb_begin + k_blocks_per_split);
   const int num_kb = kb_end - kb_begin;
   const int num_it = (num_kb + KPS - 1) / KPS;       // pipeline iterations (stages consumed)
-  const uint32_t tmem_cols = cfg::kTmemCols * (sums <= 2 ? sums : 4);
+  const uint32_t tmem_cols = cfg::kTmemCols * (!kSums ? 1 : (sums == 2 ? 2 : 4));
 
   if (warp == 0 && lane == 0) {
     ptx::tma_prefetch_desc(&tma_a);
@@ -201,9 +202,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
               // 16 bf16 = 32 bytes along K inside the 128-byte swizzle span: +2 in the address field
               ptx::umma_bf16_ss(acc, ptx::umma_desc(a_lo + j * (cfg::kBytesA >> 4) + 2 * k, desc_hi),
                                 ptx::umma_desc(b_lo + j * (cfg::kBytesB >> 4) + 2 * k, desc_hi), idesc,
-                                (in_sum | k) != 0 ? 1u : 0u);
+                                ((kSums ? in_sum : it | j) | k) != 0 ? 1u : 0u);
             }
-            if (++in_sum == k_blocks_per_sum) {
+            if (kSums && ++in_sum == k_blocks_per_sum) {
               in_sum = 0;
               acc += BN;
             }
@@ -235,30 +236,28 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       if constexpr (BN >= 32) {
 #pragma unroll 1
         for (int c = 0; c < BN / 16; c += 2) {          // two 16-column chunks per tensor-memory round trip
-          uint32_t v[32];
           float f[32];
-          ptx::tmem_ld_32x32b_x16(taddr + c * 16, v);
-          ptx::tmem_ld_32x32b_x16(taddr + c * 16 + 16, v + 16);
-          if (sums > 1) {                               // every sum in one round trip, added in order and from zero as a cluster does (-0 becomes 0)
-            uint32_t v1[32], v2[32], v3[32];
-            ptx::tmem_ld_32x32b_x16(taddr + BN + c * 16, v1);
-            ptx::tmem_ld_32x32b_x16(taddr + BN + c * 16 + 16, v1 + 16);
-            if (sums > 2) {
-              ptx::tmem_ld_32x32b_x16(taddr + 2 * BN + c * 16, v2);
-              ptx::tmem_ld_32x32b_x16(taddr + 2 * BN + c * 16 + 16, v2 + 16);
-            }
-            if (sums > 3) {
-              ptx::tmem_ld_32x32b_x16(taddr + 3 * BN + c * 16, v3);
-              ptx::tmem_ld_32x32b_x16(taddr + 3 * BN + c * 16 + 16, v3 + 16);
-            }
-            ptx::tmem_ld_wait();
+          if constexpr (kSums) {                        // 16 columns of every sum in one round trip, added in order and from zero as a cluster does (-0 becomes 0)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              f[j] = 0.f + __uint_as_float(v[j]) + __uint_as_float(v1[j]);
-              if (sums > 2) f[j] += __uint_as_float(v2[j]);
-              if (sums > 3) f[j] += __uint_as_float(v3[j]);
+            for (int i = 0; i < 2; ++i) {
+              uint32_t v[4][16];
+#pragma unroll
+              for (int z = 0; z < 4; ++z)
+                if (z < sums) ptx::tmem_ld_32x32b_x16(taddr + z * BN + (c + i) * 16, v[z]);
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) f[16 * i + j] = 0.f + __uint_as_float(v[0][j]);
+#pragma unroll
+              for (int z = 1; z < 4; ++z)
+                if (z < sums) {
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) f[16 * i + j] += __uint_as_float(v[z][j]);
+                }
             }
           } else {
+            uint32_t v[32];
+            ptx::tmem_ld_32x32b_x16(taddr + c * 16, v);
+            ptx::tmem_ld_32x32b_x16(taddr + c * 16 + 16, v + 16);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
@@ -429,6 +428,9 @@ int make_tma_2d(nvc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t inner
   return NVC_OK;
 }
 
+// the tiles and epilogues that may sum K in parts: products of up to 64 rows split where there is no epilogue only, and 16 and 96 columns, and rings of other depths, are reached by force alone
+constexpr bool has_sums(int bn, int kps, int rm, bool ext) { return bn == 256 ? !ext : (bn == 128 ? kps == 2 : (bn == 64 || bn == 32) && kps == 4) && (rm == BM || !ext); }
+
 template <int BN, int KPS, int RM = BM>
 int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C, int ldc, int out_f32, int M,
            int N, int K, int splits, int ks_cluster, int sums, int epi, cudaStream_t stream, long long* trace) {
@@ -445,7 +447,7 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   const int eff_splits = (kb_total + kb_per - 1) / kb_per;   // no empty splits
   const int kb_sum = (kb_total + sums - 1) / sums;
   sums = (kb_total + kb_sum - 1) / kb_sum;
-  NVC_REQUIRE(ctx, sums == 1 || (eff_splits == 1 && BN >= 32 && sums <= 4 && sums * BN <= 512), NVC_EINVAL, "these sums do not fit the tensor memory of one CTA");
+  NVC_REQUIRE(ctx, sums == 1 || (eff_splits == 1 && sums <= 4 && sums * BN <= 512), NVC_EINVAL, "these sums do not fit the tensor memory of one CTA");
   const int n_tiles = (N + BN - 1) / BN;
   dim3 grid(n_tiles, (M + BM - 1) / BM, eff_splits);
   // ks_cluster: the eff_splits CTAs of one output tile form a cluster (1,1,S) and reduce over DSMEM
@@ -455,6 +457,12 @@ int launch(nvc_ctx* ctx, const nvc_bf16* A, int lda, const nvc_bf16* W, void* C,
   NVC_REQUIRE(ctx, !ext || has_ext(BN), NVC_EINVAL, "no element-wise epilogue on this tile");
   auto kernel = gemm_bf16_tcgen05_kernel<BN, KPS, false, RM>;
   if constexpr (has_ext(BN)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true, RM>; }
+  if (sums > 1) {
+    kernel = nullptr;
+    if constexpr (has_sums(BN, KPS, RM, false)) { if (!ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, false, RM, true>; }
+    if constexpr (has_sums(BN, KPS, RM, true)) { if (ext) kernel = gemm_bf16_tcgen05_kernel<BN, KPS, true, RM, true>; }
+    NVC_REQUIRE(ctx, kernel, NVC_EINVAL, "no sums in parts on this tile");
+  }
   NVC_CUDA_CHECK(ctx, nvc_launch_cluster3(ctx, kernel, grid, dim3(kThreads), cfg::kSmemBytes,
                                           stream, dim3(1, 1, ks ? eff_splits : 1), ta, tb, C, ldc, out_f32, M, N, kb_total,
                                           kb_per, sums, kb_sum, a_rows,
@@ -554,20 +562,21 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
 
 }  // namespace
 
+template <int BN, int KPS, int RM>
+static cudaError_t allow_smem() {
+  auto allow = [](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS, RM>::kSmemBytes); };
+  cudaError_t e = allow(gemm_bf16_tcgen05_kernel<BN, KPS, false, RM>);
+  if constexpr (has_ext(BN)) { if (e == cudaSuccess) e = allow(gemm_bf16_tcgen05_kernel<BN, KPS, true, RM>); }
+  if constexpr (has_sums(BN, KPS, RM, false)) { if (e == cudaSuccess) e = allow(gemm_bf16_tcgen05_kernel<BN, KPS, false, RM, true>); }
+  if constexpr (has_sums(BN, KPS, RM, true)) { if (e == cudaSuccess) e = allow(gemm_bf16_tcgen05_kernel<BN, KPS, true, RM, true>); }
+  return e;
+}
+
 extern "C" int nvc_gemm_init(nvc_ctx* ctx) {
-#define X(BN, KPS)                                                                                                       \
-  NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, false>,                                     \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS>::kSmemBytes));      \
-  if constexpr (has_ext(BN))                                                                                             \
-    NVC_CUDA_CHECK(ctx, cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, true>,                                    \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS>::kSmemBytes));
+#define X(BN, KPS) NVC_CUDA_CHECK(ctx, (allow_smem<BN, KPS, BM>()));
   NVC_GEMM_CONFIGS(X)
 #undef X
-#define X(BN, KPS)                                                                                                       \
-  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, false, 64>,                                \
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS, 64>::kSmemBytes))); \
-  NVC_CUDA_CHECK(ctx, (cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, KPS, true, 64>,                                 \
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, KPS, 64>::kSmemBytes)));
+#define X(BN, KPS) NVC_CUDA_CHECK(ctx, (allow_smem<BN, KPS, 64>()));
   NVC_GEMM_FEW_ROWS(X)
 #undef X
   return NVC_OK;
