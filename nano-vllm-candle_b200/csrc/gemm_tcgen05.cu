@@ -519,8 +519,9 @@ void choose_config(const nvc_ctx* ctx, int M, int N, int K, bool allow_split, in
     // 64 rows: 1 675 configurations of 28 products, those within 15 % of a product's best (residual 4.3 %).  128 rows: 28 products of 72 - 128 rows.
     // A cluster's start waits for all of its SMs, the longer the fuller the chip: the cube.  Several sums in one CTA cost their accumulators' starts and reads (0.21, 0.31, 0.53 us for four of
     // 32, 64, 128 columns), at 128 rows within the residual.  Of the measured tiles with the right sums what it picks is 0.8 % slower than the best in the mean (16 products, 1 - 128 rows).
-    // Beside one sum wherever no cluster pays, several cost 1.3 % in the mean up to 64 rows, 0.7 % up to 128 (6 144 x 4 096, 100 rows 16.7 / 17.9), and beside clusters wherever there are
-    // several sums, on products of 128 rows, they save 8.7 % and 1.9 % (us, that / this: 2 048 x 1 024 4.3 / 3.45, 6 144 x 2 560 11.1 / 8.9, 6 144 x 4 096 16.2 / 13.6, 128 rows 18.4 / 18.5)
+    // Beside one sum wherever no cluster pays, several cost 1 % in the mean (6 144 x 2 560, 8 rows 8.45 / 9.35; 6 144 x 4 096, 100 rows 16.4 / 17.65); beside products of 128 rows
+    // with the cycle model's width, which gave several sums a cluster, this choice saves 8.7 % up to 64 rows and 1.4 % up to 128 (us, that / this: 2 048 x 1 024 4.3 / 3.45, 6 144 x 2 560 10.95 / 9.0,
+    // 6 144 x 4 096 16.2 / 13.6, 128 rows 18.4 / 18.45)
     const bool few = M <= 64;
     const int rows = ((M + 7) / 8) * 8, kb = K / BK, sums = allow_split ? sums_of(ctx, M, N, K) : 1;
     double best = 1e30;
