@@ -192,9 +192,13 @@ __device__ __forceinline__ void pair_reduce(const float4* __restrict__ ws_cluste
   }
 }
 
-// Tile number -> row tile, column tile: bands of `band` row tiles, the row tiles of a band fastest (band 1: column tiles fastest).
+// Tile number -> row tile, column tile: bands of `band` row tiles, the row tiles of a band fastest (band 1: column tiles fastest).  Only large weights have bands: the other divisions
+// were 0.2 - 0.4 us of a product of few tiles, one is 0.1 - 0.2 of a decode product (us, three divisions / now: 200 x 1 024 x 3 072 8.41 / 8.27, 2 533 x 16 x 4 864 10.28 / 9.9)
 __device__ __forceinline__ int2 tile_at(int tile, int num_tiles, int n_tiles, int band) {
-  if (num_tiles == n_tiles) return make_int2(0, tile);     // one row tile: four divisions were 0.2 us of a decode product (200 rows, 1 024 x 3 072 8.41 / 8.27)
+  if (band == 1) {
+    const int m = num_tiles == n_tiles ? 0 : tile / n_tiles;
+    return make_int2(m, tile - m * n_tiles);
+  }
   const int b = tile / (band * n_tiles), rest = tile - b * band * n_tiles, rows = min(band, num_tiles / n_tiles - b * band), n = rest / rows;
   return make_int2(b * band + rest - n * rows, n);
 }
