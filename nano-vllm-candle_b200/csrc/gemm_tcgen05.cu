@@ -65,7 +65,8 @@ __device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
 // half as many weights again in front of the dependency (64 rows, us, 128 / 64: 6 144 x 1 024 gated 5.75 / 5.1, 2 048 x 1 024 4.45 / 3.8, 12 288 x 2 048 gated 13.9 / 13.2,
 // 2 048 x 6 144 9.7 / 8.9, 3 072 x 2 048 gated 6.9 / 5.6; 1 row 6 144 x 1 024 gated 5.5 / 4.8)
 // kSums: K is summed in `sums` parts (sums_of), each in BN columns of tensor memory of its own, up to 512 together, added in order by the epilogue.  A variant, because its
-// registers (106 -> 110 to 154) keep the next kernel's CTAs off the SM: 6 144 x 1 024 gated in a chain of layers 5.1 -> 5.4 us when all products had them
+// registers (106 -> 110 to 154) keep the next kernel's CTAs off the SM: 6 144 x 1 024 gated in a chain of layers 5.1 -> 5.4 us when all products had them.  All 512 columns may be taken: no other
+// kernel with tensor memory fits on the SM beside a ring of 160 KB and more (97 KB the smallest)
 template <int BN, int KPS, bool kExt = false, int RM = BM, bool kSums = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
